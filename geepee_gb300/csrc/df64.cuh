@@ -14,7 +14,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-struct df64 {
+struct __align__(8) df64 {   // 8-byte alignment: an element in memory is one access
   float hi, lo;
 };
 
@@ -244,6 +244,69 @@ __device__ __forceinline__ df64 exp_tab(df64 x, const Tab& tab) {
   return scale2(res, m);
 }
 
+// ---- exp2 of a fixed-point argument (the psi2 pair sweeps) ----
+// x is a base-2 exponent in units of 2^-52, plus the half step 2^-12 that centres the table
+// reduction (the caller folds kFxHalf into one of x's terms).  The table T[j] = 2^(j/2048) takes
+// x's top 11 fraction bits, so that the remainder r, |r| <= 2^-12, needs only the first-order term
+// in two floats: 2^r - 1 = p + p^2/2 + p^3/6, p = r ln 2 < 1.7e-4, whose p^2/2 < 2^-26 is exact to
+// 2^-50 in one float.  ~30 instructions where the double-float argument reduction and polynomial
+// of exp_tab take ~80, and the argument's sums are integer additions (2 instructions instead
+// of 11).  Results below 2^-126 are flushed to zero; x must be below 127 * 2^52.
+constexpr int kFxTab = 2048;
+constexpr long long kFxHalf = 1LL << 40;
+// T[j], j < 2048, from the 256-entry table: T[8 j + i] = 2^(j/256) 2^(i/2048); 2^(i/2048) - 1 as
+// double-float constants (60-digit decimal arithmetic, rounded as in exp2_table.cuh)
+__device__ __forceinline__ void load_exp2_table(float2* s_tab) {
+  const float c_hi[8] = {0.000000000e+00f, 3.385080490e-04f, 6.771307089e-04f, 1.015867922e-03f, 1.354719861e-03f, 1.693686470e-03f, 2.032767981e-03f, 2.371964045e-03f};
+  const float c_lo[8] = {0.000000000e+00f, 3.656181261e-12f, -1.587024435e-11f, 3.841724161e-11f, 3.069764928e-11f, 5.799375910e-11f, -7.369679866e-11f, 2.371333858e-11f};
+  for (int k = threadIdx.x; k < kFxTab; k += blockDim.x) {
+    const int i = k & 7;
+    const float2 t = kExp2Tab[k >> 3];
+    float ch = 0.f, cl = 0.f;
+#pragma unroll
+    for (int u = 1; u < 8; ++u) {
+      ch = i == u ? c_hi[u] : ch;
+      cl = i == u ? c_lo[u] : cl;
+    }
+    // t (1 + c): the product's exact high part and its cross terms added to t
+    const df64 w = two_prod(t.x, ch);
+    const float e = __fadd_rn(__fmaf_rn(t.x, cl, w.lo), __fmaf_rn(t.y, ch, t.y));
+    df64 r = quick_two_sum(t.x, w.hi);
+    r = quick_two_sum(r.hi, __fadd_rn(r.lo, e));
+    s_tab[k] = make_float2(r.hi, r.lo);
+  }
+}
+__device__ __forceinline__ df64 exp2_fx(long long x, const float2* tab) {
+  const unsigned xl = (unsigned)x;
+  const int xh = (int)(x >> 32);
+  const float2 T = tab[(xh >> 9) & (kFxTab - 1)];
+  // the 41 remainder bits as two floats, by exponent splicing: 23 bits of [1, 2), then 18
+  const float f = __uint_as_float(0x3f800000u | (__funnelshift_l(xl, (unsigned)xh, 14) & 0x7fffffu));
+  const float g = __uint_as_float(0x4b000000u | (xl & 0x3ffffu));   // 2^23 + the low 18 bits
+  const float a = __fsub_rn(f, 1.5f);                               // r = a 2^-11 + (low bits) 2^-52
+  const float c1 = 3.384507727e-04f, c1l = -9.300069395e-13f, c2 = 1.539095923e-16f;                // ln2 2^-11 (hi, lo), ln2 2^-52
+  const float p = __fmul_rn(a, c1);
+  float t = __fmaf_rn(g, c2, -8388608.f * c2);
+  t = __fmaf_rn(a, c1l, t);
+  float e = __fadd_rn(t, __fmaf_rn(a, c1, -p));
+  e = __fmaf_rn(p, e, e);
+  e = __fmaf_rn(__fmul_rn(p, p), __fmaf_rn(p, 0.16666667f, 0.5f), e);   // 2^r = 1 + p + e
+  // T 2^r, then 2^m by one multiply a word
+  const float w = __fmul_rn(T.x, p);
+  float l = __fmaf_rn(T.x, e, __fmaf_rn(T.x, p, -w));
+  l = __fadd_rn(l, __fmaf_rn(T.y, p, T.y));
+  const float h = __fadd_rn(T.x, w);
+  l = __fadd_rn(l, __fsub_rn(w, __fsub_rn(h, T.x)));
+  const float s = xh >= -(126 << 20) ? __int_as_float(((xh << 3) & 0xff800000) + 0x3f800000) : 0.f;
+  return make_df(__fmul_rn(h, s), __fmul_rn(l, s));
+}
+// round(v 2^e) of a double-float (|v 2^e| < 2^62)
+__device__ __forceinline__ long long fx_of(df64 v, float two_e) {
+  return __float2ll_rn(__fmul_rn(v.hi, two_e)) + __float2ll_rn(__fmul_rn(v.lo, two_e));
+}
+// log2(e) in the precision of the argument
+__device__ __forceinline__ df64 log2e_of(df64) { return make_df(1.442695022e+00f, 1.925963034e-08f); }
+
 // log by one Newton step on exp: y1 = y0 + x exp(-y0) - 1
 template <typename Tab>
 __device__ __forceinline__ df64 log_tab(df64 x, const Tab& tab) {
@@ -285,12 +348,13 @@ __device__ __forceinline__ float rsqrt_(float a) { return __frsqrt_rn(a); }
 __device__ __forceinline__ float scale2(float a, int e) { return scale2f(a, e); }
 template <typename Tab> __device__ __forceinline__ float exp_tab(float x, const Tab&) { return expf(x); }
 template <typename Tab> __device__ __forceinline__ float log_tab(float x, const Tab&) { return logf(x); }
-// The exp of the psi2 pair sweeps (one per pair and point, the bulk of those kernels): the
-// double-float exp_tab, or in FP32 CUDA's __expf intrinsic (documented maximum error
-// 2 + floor(|1.173 x|) ulp; the terms that dominate a sweep's sums have |x| near 0, and the
-// FP32 path's statistics are held to 1e-5 and its gradients to 1e-4 relative).
+// The exp of the psi2 pair sweeps' rare path (arguments outside the fixed-point range)
 template <typename Tab> __device__ __forceinline__ df64 exp_pair(df64 x, const Tab& tab) { return exp_tab<true>(x, tab); }
 template <typename Tab> __device__ __forceinline__ float exp_pair(float x, const Tab&) { return __expf(x); }
+
+__device__ __forceinline__ float log2e_of(float) { return 1.44269504f; }
+// max that returns NaN when either is NaN
+__device__ __forceinline__ float fmax_nan(float a, float b) { return (a != a || b != b) ? __int_as_float(0x7fffffff) : fmaxf(a, b); }
 
 // Warp sums of K values at once (K a power of two <= 32): in each of the first log2 K steps
 // of the butterfly a lane keeps half of its values and adds its partner's copies of them,
@@ -316,14 +380,6 @@ __device__ __forceinline__ void warp_sum_many(T (&v)[K]) {
 }
 
 // conversions between storage (double / float) and compute (df64 / float) types
-// A compute-type element read as one 8-byte access (df64) when its address is known to be
-// 8-byte aligned (df64 itself is only 4-byte aligned, so plain loads may split in two).
-__device__ __forceinline__ df64 ld_al8(const df64* p) {
-  const float2 v = *reinterpret_cast<const float2*>(p);
-  return make_df(v.x, v.y);
-}
-__device__ __forceinline__ float ld_al8(const float* p) { return *p; }
-
 template <typename T> struct Num;
 template <> struct Num<df64> {
   typedef double store_t;

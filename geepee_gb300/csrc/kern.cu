@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(256) det_fwd_kernel(int N, int M, int D, int D
 // (geepee/aep_models.py:142-158 once Kfu is formed).  A CTA takes CR rows; warp w works on row
 // w % CR and column half w / CR, lane l on columns b = 64 h + l + 32 j (j < 2), for all DB
 // outputs, so each thread runs 2 DB independent sums over a.  All of B (Dout M^2) and the CTA's
-// kernel rows sit in shared memory (asynchronous copies, converted in place, 8-byte aligned so
-// that each element is one shared-memory access); m and v are warp sums, then the two halves'
+// kernel rows sit in shared memory (asynchronous copies, converted in place);
+// m and v are warp sums, then the two halves'
 // sums are added in a fixed order.
 constexpr int CR = 8;              // rows per CTA
 constexpr int CT = CR * 2 * 32;    // threads: (row, column half) per warp
@@ -280,8 +280,8 @@ __global__ void __launch_bounds__(CT) det_contract_kernel(int N, int M, int Dout
 #pragma unroll
     for (int d = 0; d < DB; ++d) {
       // det_fwd's operand order, so that the sums match its arithmetic
-      acc[d][0] = fma_(ld_al8(B0[d] + ra), ka, acc[d][0]);
-      acc[d][1] = fma_(ld_al8(B1[d] + ra), ka, acc[d][1]);
+      acc[d][0] = fma_(B0[d][ra], ka, acc[d][0]);
+      acc[d][1] = fma_(B1[d][ra], ka, acc[d][1]);
     }
   }
   T pm[DB], pv[DB];
@@ -722,10 +722,10 @@ __global__ void __launch_bounds__(GP_T) gram_pairs_kernel(int N, int M, int Dout
       const T* ur = us + (size_t)rl * M;
       T wd[DB];
 #pragma unroll
-      for (int d = 0; d < DB; ++d) wd[d] = ld_al8(ws + rl * DO_MAX + d);
+      for (int d = 0; d < DB; ++d) wd[d] = ws[rl * DO_MAX + d];
 #pragma unroll
       for (int k = 0; k < GP_PPT; ++k) {
-        const T kk = mul(ld_al8(ur + ia[k]), ld_al8(ur + ib[k]));
+        const T kk = mul(ur[ia[k]], ur[ib[k]]);
 #pragma unroll
         for (int d = 0; d < DB; ++d) acc[k][d] = fma_(wd[d], kk, acc[k][d]);
       }

@@ -95,7 +95,7 @@ extern "C" int gpk_psi_bwd_ex(int prec, int N, int M, int Q, int Dout, const voi
 
 long psi_bwd_work_elems(int M, int Q, int Dout) {
   const long P = (long)M * (M + 1) / 2;
-  return (long)gpk::sm_count() * (Dout * P + (long)Dout * M + (long)M * Q + 1 + Q);
+  return 2L * gpk::sm_count() * (Dout * P + (long)Dout * M + (long)M * Q + 1 + Q);
 }
 
 extern "C" int gpk_psi_bwd_ws(int prec, int N, int M, int Q, int Dout, const void* mu, const void* var,

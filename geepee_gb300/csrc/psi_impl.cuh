@@ -9,13 +9,19 @@
 // per-pair quantities (sum_n psi2, dB = sum_n dv psi2) stay in registers until one atomic
 // flush per CTA.  psi2 per point is never materialised in HBM (unless requested).
 //
-// log psi2[n,a,b] = u_a + u_b + G_ab - sum_q h_aq z_bq   with
-//   G_ab = -sum_q (z_aq - z_bq)^2 / (4 l_q)                      (per call, shared memory)
-//   u_a  = k_n/2 + sum_q c_q z_aq (mu_q - z_aq/4),  h_aq = c_q z_aq / 2   (per point)
-//   k_n  = 2 log sf2 + 1/2 sum_q log(l_q / (l_q + 2 S_q)) - sum_q c_q mu_q^2,
-//   c_q  = 1 / (l_q + 2 S_q)
-// which is the reference's exponent (geepee/kernels.py:219-225) regrouped so that the
-// inner loop costs Q multiply-adds plus one exp.
+// log2 psi2[n,a,b] = u_a + u_b + G_ab - sum_q t_aq t_bq   with
+//   t_aq = (mu_q - z_aq) sqrt(c_q log2(e) / 2),  c_q = 1 / (l_q + 2 S_q)     (per point)
+//   u_a  = k_n/2 - 1/2 sum_q t_aq^2                                         (per point)
+//   k_n  = log2(e) (2 log sf2 + 1/2 sum_q log(l_q / (l_q + 2 S_q)))
+//   G_ab = -log2(e) sum_q (z_aq - z_bq)^2 / (4 l_q)                          (per call)
+// which is the reference's exponent (geepee/kernels.py:219-225) regrouped about the point, so
+// that no term is larger than the exponent itself needs: where psi2 is not negligible,
+// sum_q t_aq^2 < k_n + 127 (l + 2S >= l gives log2 psi2 <= k_n - sum_q (t_aq^2 + t_bq^2)).  In
+// double-float precision u, t and G are therefore kept as fixed-point integers: the sums are
+// integer additions, the cross terms 32 x 32 -> 64-bit multiply-adds, and the exponential reads
+// its table index and remainder from the bits (exp2_fx).  Against double-float sums and exp_tab
+// that is ~55 instead of ~140 instructions per pair and point for two dimensions; forward moments
+// at N = 10000, Q = 5, M = 100: 498 -> 366 us.
 //
 // Template parameters: T compute type (df64 or float); PPT pairs per thread held in
 // registers (0: plain strided sweep); QC a compile-time cap on Q and DB on Dout, so
@@ -28,14 +34,15 @@ namespace psi_impl {
 constexpr int QMAX = 8;
 constexpr int DMAX = 4;
 constexpr int NT = 512;        // threads per CTA (forward)
-// threads per CTA of the backward (one CTA per SM): 32 warps when Q <= 2 (64 registers a
-// thread, no spills), 16 when the per-dimension sums of Q <= 8 need more registers
-__host__ __device__ constexpr int nt_bwd(int QC) { return QC <= 2 ? 1024 : 512; }
 // Q is QC itself in an exact instantiation (every width other than the two catch-all ones, 2
 // for Q <= 2 and QMAX above): the per-dimension loops then carry no runtime test
 __host__ __device__ constexpr bool exact_q(int QC) { return QC != 2 && QC != QMAX; }
+// a pseudo-input's record in a point's table: u, t_1 .. t_QC (zeros past Q), padded to an odd
+// count so that the lanes of a warp (consecutive pseudo-inputs) read different banks
+__host__ __device__ constexpr int rec_len(int QC) { return (1 + QC) | 1; }
+constexpr size_t SMEM_CAP = 227 * 1024 - 64;   // dynamic shared memory of a CTA, beside the kernels' static words
 constexpr int PPT_MAX = 16;    // pairs per thread for register-resident per-pair sums
-constexpr int RED = 48;        // reduction slots per warp
+constexpr int FRED = 16;        // reduction slots per warp: forward
 
 template <typename S>
 struct PsiArgs {
@@ -58,8 +65,7 @@ struct PsiArgs {
   const S* dpsi1;    // optional [N,M]: replaces dm_all A
   int chain;         // forward rollout: point n > 0 takes point n-1's (m, v) as its (mu, var)
   int bs_smem;       // symmetrised B staged in shared memory (set by the launcher)
-  int accb_smem;     // backward: dBhat accumulates in shared memory (else atomically in dB)
-  int pab_smem;      // backward: the pair table fits in shared memory (set by the launcher)
+  int g_smem;        // G_ab in shared memory (set by the launcher)
   long b_stride;     // != 0: B is per point (B + n*b_stride), dv treated as 1
   double* dsf2;
   double* dl;
@@ -75,11 +81,103 @@ struct PsiArgs {
 
 __device__ __forceinline__ void pair_of(int p, int& a, int& b) { tri_pair(p, a, b); }
 
+// How a precision keeps the pair exponent's terms (log2 units): R a table element, arg() the
+// exponent of a pair from the two records and G, ev() its exponential.
+template <typename T>
+struct PairExp;
+
+// FP32: floats, and the hardware's base-2 exponential
+template <>
+struct PairExp<float> {
+  typedef float R;
+  static constexpr int TAB = 0;    // exp table entries in shared memory
+  static __device__ __forceinline__ R u_of(float x) { return x; }
+  static __device__ __forceinline__ R t_of(float x) { return x; }
+  static __device__ __forceinline__ R g_of(float x) { return x; }
+  template <int QC>
+  static __device__ __forceinline__ R arg(const R* a, const R* b, R g) {
+    R x = (a[0] + b[0]) + g;
+#pragma unroll
+    for (int q = 1; q <= QC; ++q) x = __fmaf_rn(-a[q], b[q], x);
+    return x;
+  }
+  static __device__ __forceinline__ float ev(R x, const float2*) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+  }
+};
+
+// double-float: u and G in units of 2^-52, t in units of 2^-58 as a balanced pair (high word the
+// nearest multiple of 2^32, low word signed), so that t_a t_b in units of 2^-52 is the product of
+// the high words plus the upper half of the two mixed products.  |t| < 16 (see above) bounds the
+// high words by 2^30 and a mixed sum over three dimensions by 2^63.
+template <>
+struct PairExp<df64> {
+  typedef long long R;
+  static constexpr int TAB = kFxTab;
+  static __device__ __forceinline__ R u_of(df64 x) { return fx_of(x, 4503599627370496.f); }
+  static __device__ __forceinline__ R t_of(df64 x) {
+    const long long t = fx_of(x, 288230376151711744.f);
+    return ((t + 0x80000000LL) & ~0xffffffffLL) | (t & 0xffffffffLL);
+  }
+  // below -1024 every pair's psi2 is zero already (the other terms sum to less than 127); the
+  // half step of exp2_fx enters here
+  static __device__ __forceinline__ R g_of(df64 x) {
+    return (x.hi > -1024.f ? fx_of(x, 4503599627370496.f) : -(1024LL << 52)) + kFxHalf;
+  }
+  // a record whose pairs are all zero: u + u_b + G < -126 for every live b (u_b <= 63.5), and no
+  // sum leaves the range of +-2048
+  // a t as its two words (low, high), one 8-byte access
+  static __device__ __forceinline__ int2 ld2(const R* p) { return *reinterpret_cast<const int2*>(p); }
+  // a b + c of 32-bit factors in one instruction (from C, the compiler widened the factors to 64
+  // bits first: three multiply-adds and two shifts a product)
+  static __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+  }
+  static __device__ __forceinline__ R dead_u() { return -(400LL << 52); }
+  template <int QC>
+  static __device__ __forceinline__ R arg(const R* a, const R* b, R g) {
+    long long x = a[0] + b[0] + g;
+#pragma unroll
+    for (int q0 = 1; q0 <= QC; q0 += 3) {
+      long long mid = 0;
+      int2 ta[3], tb[3];
+#pragma unroll
+      for (int u = 0; u < 3 && q0 + u <= QC; ++u) {
+        ta[u] = ld2(a + q0 + u);
+        tb[u] = ld2(b + q0 + u);
+        mid = mad_wide(ta[u].y, tb[u].x, mid);
+        mid = mad_wide(ta[u].x, tb[u].y, mid);
+      }
+      long long hi = (int)(mid >> 32);
+#pragma unroll
+      for (int u = 0; u < 3 && q0 + u <= QC; ++u) hi = mad_wide(ta[u].y, tb[u].y, hi);
+      x -= hi;
+    }
+    return x;
+  }
+  static __device__ __forceinline__ df64 ev(R x, const float2* tab) { return exp2_fx(x, tab); }
+};
+
+// the 256-entry exp table of exp_tab inside the kernels' shared table (every 8th entry)
+struct ExpTab {
+  const float2* p;
+  __device__ __forceinline__ float2 operator[](int j) const { return p[8 * j]; }
+};
+template <typename T>
+__device__ __forceinline__ void load_pair_table(float2* tab) {
+  if (PairExp<T>::TAB) load_exp2_table(tab);
+}
+__host__ __device__ inline size_t pair_table_bytes(size_t tsz) { return tsz == 8 ? kFxTab * sizeof(float2) : 0; }
+
 // The symmetrised weights of the packed pairs, Bs[d P + p] = B_d[a,b] + B_d[b,a] (a != b) or
-// B_d[a,a]: each thread keeps eight pairs' global loads in flight before converting them, so
+// B_d[a,a] (half: (B_d[a,b] + B_d[b,a]) / 2 off the diagonal): each thread keeps eight pairs' global loads in flight before converting them, so
 // the table costs a few memory latencies per CTA instead of one per pair.
 template <typename T, int NTH>
-__device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int D, int P) {
+__device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int D, int P, bool half = false) {
   typedef typename Num<T>::store_t S;
   constexpr int K = 8;
   for (int d = 0; d < D; ++d) {
@@ -101,7 +199,10 @@ __device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int
         const int p = p0 + k * NTH;
         if (p < P) {
           T w = Num<T>::ld(x1[k]);
-          if (off[k]) w = add(w, Num<T>::ld(x2[k]));
+          if (off[k]) {
+            w = add(w, Num<T>::ld(x2[k]));
+            if (half) w = scale2(w, -1);
+          }
           Bs[d * P + p] = w;
         }
       }
@@ -109,33 +210,10 @@ __device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int
   }
 }
 
-// CTA-wide sum of K (<= RED) values per thread; the result is valid in warp 0.  Only the
-// first `nact` warps hold non-zero values (the others skip the shuffles; default: all).
-template <typename T, int K>
-__device__ __forceinline__ void block_sum(T* vals, T* red, int nact = 0) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = nact > 0 ? nact : (int)(blockDim.x >> 5);
-  if (warp < nw) {
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      T s = warp_sum(vals[i]);
-      if (lane == 0) red[warp * RED + i] = s;
-    }
-  }
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-      T s = lane < nw ? red[lane * RED + i] : Num<T>::zero();
-      vals[i] = warp_sum(s);
-    }
-  }
-}
-
-// block_sum for a point's handful of values: each warp reduces them in multi-value butterflies
+// CTA-wide sum of K values per thread (valid in warp 0) from the first nact warps: each warp reduces them in multi-value butterflies
 // of eight (warp_sum_many; lane 4v then holds value c0 + v), lane i of warp 0 adds value i (and
 // i + 32) over the warps in order and shuffles it to the warp.  Fixed order; K <= RED.
-template <typename T, int K>
+template <typename T, int K, int RED>
 __device__ __forceinline__ void block_sum_many(T (&vals)[K], T* red, int nact) {
   static_assert(K <= RED, "K values per warp slot");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -165,22 +243,27 @@ __device__ __forceinline__ void block_sum_many(T (&vals)[K], T* red, int nact) {
 }
 
 // Per-point tables of one data point n: per-dimension constants (pmu, pis1 = 1/(l+S),
-// pc = 1/(l+2S), pld1/pld2 = 1/2 log(l/(l+S)), 1/2 log(l/(l+2S))) and per-pseudo-input terms
-// (u_a, h_aq).  The backward keeps one point's tables, the forward NPB points' side by side.
+// pc = 1/(l+2S), psq = sqrt(pc log2(e)/2), pld1/pld2 = 1/2 log(l/(l+S)), 1/2 log(l/(l+2S))) and
+// the pseudo-inputs' records (u_a, t_aq).  The backward keeps one point's tables, the forward NPB
+// points' side by side.
+constexpr int PD = 6;   // arrays of QMAX per-dimension constants
 template <typename T>
 struct PointSlot {
   T* pmu;
   T* pis1;
   T* pc;
+  T* psq;
   T* pld1;
   T* pld2;
-  T* u;   // [M]
-  T* h;   // [M*Q]
+  typename PairExp<T>::R* rec;   // [M][rec_len]
+  __device__ __forceinline__ PointSlot(T* pd, typename PairExp<T>::R* r)
+      : pmu(pd), pis1(pd + QMAX), pc(pd + 2 * QMAX), psq(pd + 3 * QMAX), pld1(pd + 4 * QMAX), pld2(pd + 5 * QMAX),
+        rec(r) {}
 };
 
 // per-point constants for dimension q of point n
-template <typename T, typename S>
-__device__ __forceinline__ void dims_of(const PsiArgs<S>& a, const T* ell2, const T* lnl, const float2* tab,
+template <typename T, typename S, typename Tab>
+__device__ __forceinline__ void dims_of(const PsiArgs<S>& a, const T* ell2, const T* lnl, const Tab& tab,
                                         const PointSlot<T>& ps, int n, int q, int part) {
   // a rollout reads the previous point's outputs (written before the pass's last barrier)
   const S* pmu = a.chain ? (n > 0 ? a.m_out + (size_t)(n - 1) * a.Q : a.mu) : a.mu + (size_t)n * a.Q;
@@ -192,7 +275,9 @@ __device__ __forceinline__ void dims_of(const PsiArgs<S>& a, const T* ell2, cons
     ps.pmu[q] = Num<T>::ld(pmu[q]);
     ps.pis1[q] = recip(s);
   } else if (part == 1) {
-    ps.pc[q] = recip(s);
+    const T c = recip(s);
+    ps.pc[q] = c;
+    ps.psq[q] = sqrt_(mul(c, scale2(log2e_of(c), -1)));
   } else if (part == 2) {
     ps.pld1[q] = scale2(sub(lnl[q], log_tab(s, tab)), -1);
   } else {
@@ -200,31 +285,61 @@ __device__ __forceinline__ void dims_of(const PsiArgs<S>& a, const T* ell2, cons
   }
 }
 
-// per-pseudo-input terms of one point: psi1_a (returned), u_a and h_aq (written to the slot)
-template <typename T, int QC>
-__device__ __forceinline__ T rows_of(const T* z, T lsf, const float2* tab, const PointSlot<T>& ps, int Q, int ia) {
-  T e1 = lsf;
-  T kap = add(lsf, lsf);
+// The record of one pseudo-input at one point in fixed point: a dead record (zero for every
+// pair) where k_n - sum_q t_q^2 < -127.5.  *flag is set where the fixed-point range does not hold
+// and the whole pass takes psi2_general: non-finite terms, k_n above 126, or l + 2S < l (a
+// negative variance; the rounding of a zero one is tolerated), for which the bound on t fails.
+template <int QC>
+__device__ __forceinline__ void put_rec(long long* r, df64 k2, df64 s2, const df64* t, float ld2, int* flag) {
+  const bool in = s2.hi < 1e38f && k2.hi < 63.f && k2.hi > -1e38f && ld2 < 1e-6f;   // false for NaN
+  if (!in) *flag = 1;
+  const bool live = in && 2.f * k2.hi - s2.hi >= -127.5f;
+  r[0] = live ? PairExp<df64>::u_of(sub(k2, scale2(s2, -1))) : PairExp<df64>::dead_u();
+#pragma unroll
+  for (int q = 0; q < QC; ++q) r[1 + q] = live ? PairExp<df64>::t_of(t[q]) : 0;
+}
+template <int QC>
+__device__ __forceinline__ void put_rec(float* r, float k2, float s2, const float* t, float, int*) {
+  r[0] = k2 - 0.5f * s2;
+#pragma unroll
+  for (int q = 0; q < QC; ++q) r[1 + q] = t[q];
+}
+
+// per-pseudo-input terms of one point: psi1_a (returned) and the record (u_a, t_aq)
+template <typename T, int QC, typename Tab>
+__device__ __forceinline__ T rows_of(const T* z, T lsf, const Tab& tab, const PointSlot<T>& ps, int Q, int ia,
+                                     int* flag) {
+  T e1 = lsf, kap = lsf, s2 = Num<T>::zero();
+  T t[QC];
+  float ld2 = -1e30f;
 #pragma unroll
   for (int q = 0; q < QC; ++q) {
+    t[q] = Num<T>::zero();
     if (q < Q) {
-      T d = sub(ps.pmu[q], z[ia * Q + q]);
+      const T d = sub(ps.pmu[q], z[ia * Q + q]);
       e1 = add(e1, sub(ps.pld1[q], scale2(mul(mul(d, d), ps.pis1[q]), -1)));
-      kap = add(kap, sub(ps.pld2[q], mul(mul(ps.pmu[q], ps.pmu[q]), ps.pc[q])));
+      kap = add(kap, scale2(ps.pld2[q], -1));
+      ld2 = fmax_nan(ld2, Num<T>::approx(ps.pld2[q]));
+      t[q] = mul(d, ps.psq[q]);
+      s2 = fma_(t[q], t[q], s2);
     }
   }
-  T u = scale2(kap, -1);
-#pragma unroll
-  for (int q = 0; q < QC; ++q) {
-    if (q < Q) {
-      T zq = z[ia * Q + q];
-      T czq = mul(ps.pc[q], zq);
-      u = add(u, mul(czq, sub(ps.pmu[q], scale2(zq, -2))));
-      ps.h[ia * Q + q] = scale2(czq, -1);
-    }
-  }
-  ps.u[ia] = u;
+  put_rec<QC>(ps.rec + ia * rec_len(QC), mul(kap, log2e_of(kap)), s2, t, ld2, flag);
   return exp_tab(e1, tab);
+}
+
+// psi2 of one pair outside the fixed-point range, from the point's constants and the two
+// pseudo-inputs (df64 only; rare, so out of line)
+template <typename T>
+__device__ __noinline__ T psi2_general(const T* za, const T* zb, const T* pd, const T* inv4l, T lsf, int Q,
+                                       const float2* tab) {
+  const T *pmu = pd, *pc = pd + 2 * QMAX, *pld2 = pd + 5 * QMAX;
+  T x = add(lsf, lsf);
+  for (int q = 0; q < Q; ++q) {
+    const T v = sub(pmu[q], scale2(add(za[q], zb[q]), -1)), d = sub(za[q], zb[q]);
+    x = add(x, sub(pld2[q], add(mul(mul(v, v), pc[q]), mul(mul(d, d), inv4l[q]))));
+  }
+  return exp_pair(x, ExpTab{tab});
 }
 
 // ---------------------------------------------------------------------------------
@@ -243,59 +358,72 @@ struct FSmem {
   T* lnl;    // [QMAX]
   T* inv4l;  // [QMAX]
   T* misc;   // [4] log sf2, sf2
-  T* pd;     // [NPB][5][QMAX] per-point constants
-  T* u;      // [NPB][M]
-  T* h;      // [NPB][M*Q]
+  T* pd;     // [NPB][PD][QMAX] per-point constants
+  typename PairExp<T>::R* rec;   // [NPB][M][rec_len]
   T* p1;     // [NPB][M]
   T* As;     // [Dout][M]
-  T* G;      // [P]
+  typename PairExp<T>::R* G;      // [P] or nullptr (then formed for each pair)
   T* Bs;     // [Dout*P] or nullptr
-  T* red;    // [32*RED]
+  T* red;    // [NT/32][FRED]
 };
 
-__host__ __device__ inline size_t fwd_smem_bytes(int M, int Q, int P, int D, int npb, size_t tsz, int nbs) {
-  size_t n = (size_t)M * Q + 3 * QMAX + 4 + (size_t)npb * 5 * QMAX + (size_t)npb * M * (2 + Q) + (size_t)D * M + P +
-             nbs + 32 * RED;
-  return 256 * 8 + n * tsz;
+__host__ __device__ inline size_t fwd_smem_bytes(int M, int Q, int QC, int D, int npb, size_t tsz, int ng, int nbs) {
+  size_t n = (size_t)M * Q + 3 * QMAX + 4 + (size_t)npb * PD * QMAX + (size_t)npb * M * (1 + rec_len(QC)) +
+             (size_t)D * M + ng + nbs + (size_t)(NT / 32) * FRED;
+  return pair_table_bytes(tsz) + n * tsz;
 }
 
-template <typename T>
-__device__ FSmem<T> fcarve(char* base, int M, int Q, int P, int D, int npb, int nbs) {
+template <typename T, int QC>
+__device__ FSmem<T> fcarve(char* base, int M, int Q, int D, int npb, int ng, int nbs) {
+  typedef typename PairExp<T>::R R;
+  static_assert(sizeof(R) == sizeof(T), "table elements as large as T");
   FSmem<T> s;
   s.tab = reinterpret_cast<float2*>(base);
-  T* t = reinterpret_cast<T*>(base + 256 * sizeof(float2));
+  T* t = reinterpret_cast<T*>(base + pair_table_bytes(sizeof(T)));
   s.z = t; t += M * Q;
   s.ell2 = t; t += QMAX;
   s.lnl = t; t += QMAX;
   s.inv4l = t; t += QMAX;
   s.misc = t; t += 4;
-  s.pd = t; t += npb * 5 * QMAX;
-  s.u = t; t += npb * M;
-  s.h = t; t += npb * M * Q;
+  s.pd = t; t += npb * PD * QMAX;
+  s.rec = reinterpret_cast<R*>(t); t += npb * M * rec_len(QC);
   s.p1 = t; t += npb * M;
   s.As = t; t += D * M;
-  s.G = t; t += P;
+  s.G = ng ? reinterpret_cast<R*>(t) : nullptr; t += ng;
   s.Bs = nbs ? t : nullptr; t += nbs;
   s.red = t;
   return s;
 }
 
-template <typename T>
-__device__ __forceinline__ PointSlot<T> fslot(const FSmem<T>& s, int pt, int M, int Q) {
-  T* pd = s.pd + pt * 5 * QMAX;
-  return PointSlot<T>{pd, pd + QMAX, pd + 2 * QMAX, pd + 3 * QMAX, pd + 4 * QMAX, s.u + pt * M, s.h + pt * M * Q};
+// G_ab (log2 units) of a pair from the pseudo-inputs
+template <typename T, int QC>
+__device__ __forceinline__ typename PairExp<T>::R pair_G(const T* za, const T* zb, const T* inv4l, int Q) {
+  T g = Num<T>::zero();
+#pragma unroll
+  for (int q = 0; q < QC; ++q) {
+    if (q < Q) {
+      const T d = sub(za[q], zb[q]);
+      g = fma_(mul(d, d), inv4l[q], g);
+    }
+  }
+  return PairExp<T>::g_of(neg(mul(g, log2e_of(g))));
 }
 
 template <typename T, int NPB, int PPT, int QC, int DB>
 __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::store_t> a) {
   typedef typename Num<T>::store_t S;
+  typedef PairExp<T> X;
+  typedef typename X::R R;
+  constexpr int RL = rec_len(QC);
   extern __shared__ __align__(16) char smem_raw[];
   const int M = a.M, Q = exact_q(QC) ? QC : a.Q, D = a.Dout;
   const int P = M * (M + 1) / 2;
   const bool contract = (a.A != nullptr) && (a.B != nullptr) && (a.m_out != nullptr || a.v_out != nullptr);
-  FSmem<T> s = fcarve<T>(smem_raw, M, Q, P, contract ? D : 0, NPB, a.bs_smem ? D * P : 0);
+  FSmem<T> s = fcarve<T, QC>(smem_raw, M, Q, contract ? D : 0, NPB, a.g_smem ? P : 0, a.bs_smem ? D * P : 0);
+  __shared__ int s_flag;   // the pass holds a point outside the fixed-point range
+  const ExpTab etab{s.tab};
   // ---- per-CTA tables: exp table, Z, lengthscales, sf2, A, G_ab and the symmetrised B
-  load_exp_table(s.tab);
+  load_pair_table<T>(s.tab);
   for (int i = threadIdx.x; i < M * Q; i += NT) s.z[i] = Num<T>::ld(a.Z[i]);
   if (contract)
     for (int i = threadIdx.x; i < D * M; i += NT) s.As[i] = Num<T>::ld(a.A[i]);
@@ -303,7 +431,7 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
   if (threadIdx.x < Q) {
     const int q = threadIdx.x;
     T lnl = Num<T>::ld(static_cast<S>(a.lls2[q]));
-    T l2 = exp_tab(lnl, s.tab);
+    T l2 = exp_tab(lnl, etab);
     s.lnl[q] = lnl;
     s.ell2[q] = l2;
     s.inv4l[q] = recip(mul(l2, Num<T>::c(4.f)));
@@ -311,21 +439,15 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
   if (threadIdx.x == 32) {
     T lsf = Num<T>::ld(static_cast<S>(a.lsf2[0]));
     s.misc[0] = lsf;
-    s.misc[1] = exp_tab(lsf, s.tab);
+    s.misc[1] = exp_tab(lsf, etab);
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < P; p += NT) {
-    int ia, ib;
-    pair_of(p, ia, ib);
-    T g = Num<T>::zero();
-#pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      if (q < Q) {
-        T d = sub(s.z[ia * Q + q], s.z[ib * Q + q]);
-        g = fma_(mul(d, d), s.inv4l[q], g);
-      }
+  if (s.G) {
+    for (int p = threadIdx.x; p < P; p += NT) {
+      int ia, ib;
+      pair_of(p, ia, ib);
+      s.G[p] = pair_G<T, QC>(s.z + ia * Q, s.z + ib * Q, s.inv4l, Q);
     }
-    s.G[p] = neg(g);
   }
   if (s.Bs) stage_sym_B<T, NT>(s.Bs, a.B, M, D, P);
   constexpr int KP = PPT > 0 ? PPT : 1;
@@ -346,20 +468,23 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
   const int nend = (int)((long)a.N * (blockIdx.x + 1) / gridDim.x);
   for (int n0 = nbeg; n0 < nend; n0 += NPB) {
     const int npts = min(NPB, nend - n0);
+    auto slot = [&](int pt) { return PointSlot<T>(s.pd + pt * PD * QMAX, s.rec + pt * M * RL); };
     // ---- per-dimension constants of the NPB points
+    if (threadIdx.x == 0) s_flag = 0;
     for (int t = threadIdx.x; t < 4 * npts * Q; t += NT) {
       const int part = t & 3, pq = t >> 2, pt = pq / Q, q = pq - pt * Q;
-      dims_of<T, S>(a, s.ell2, s.lnl, s.tab, fslot(s, pt, M, Q), n0 + pt, q, part);
+      dims_of<T, S>(a, s.ell2, s.lnl, etab, slot(pt), n0 + pt, q, part);
     }
     __syncthreads();
     // ---- per-pseudo-input terms (and psi1)
     for (int t = threadIdx.x; t < npts * M; t += NT) {
       const int pt = t / M, ia = t - pt * M;
-      const T v1 = rows_of<T, QC>(s.z, lsf, s.tab, fslot(s, pt, M, Q), Q, ia);
+      const T v1 = rows_of<T, QC>(s.z, lsf, etab, slot(pt), Q, ia, &s_flag);
       s.p1[pt * M + ia] = v1;
       if (a.psi1) a.psi1[(size_t)(n0 + pt) * M + ia] = Num<T>::st(v1);
     }
     __syncthreads();
+    const bool general = X::TAB && s_flag;
     // ---- pairs
     T vacc[NPB][DB];
 #pragma unroll
@@ -367,10 +492,7 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
 #pragma unroll
       for (int d = 0; d < DB; ++d) vacc[pt][d] = Num<T>::zero();
     auto do_pair = [&](int p, int ia, int ib, T& sum) {
-      const T gab = s.G[p];
-      T zb[QC];
-#pragma unroll
-      for (int q = 0; q < QC; ++q) zb[q] = q < Q ? s.z[ib * Q + q] : Num<T>::zero();
+      const R gab = s.G ? s.G[p] : pair_G<T, QC>(s.z + ia * Q, s.z + ib * Q, s.inv4l, Q);
       T w[DB];
       if (contract) {
 #pragma unroll
@@ -390,14 +512,9 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
 #pragma unroll
       for (int pt = 0; pt < NPB; ++pt) {
         if (pt < npts) {
-          const T* hu = s.u + pt * M;
-          const T* hh = s.h + pt * M * Q + ia * Q;
-          T x = add(add(hu[ia], hu[ib]), gab);
-          T cr = Num<T>::zero();
-#pragma unroll
-          for (int q = 0; q < QC; ++q)
-            if (q < Q) cr = fma_(hh[q], zb[q], cr);
-          const T ps = exp_pair(sub(x, cr), s.tab);
+          const R* rec = s.rec + pt * M * RL;
+          const T ps = general ? psi2_general(s.z + ia * Q, s.z + ib * Q, s.pd + pt * PD * QMAX, s.inv4l, lsf, Q, s.tab)
+                               : X::ev(X::template arg<QC>(rec + ia * RL, rec + ib * RL, gab), s.tab);
           if (a.psi2) {
             const S v = Num<T>::st(ps);
             const size_t o = (size_t)(n0 + pt) * M;
@@ -413,33 +530,27 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
         }
       }
     };
-    // the common configuration (m and v only, Q == QC, Dout == DB, B in shared memory): the same
+    // the common configuration (m and v only, Dout == DB, B and G in shared memory): the same
     // sums without branches, so the NPB points' exps interleave.  In a pass with fewer than NPB
     // points the extra slots run on stale tables; their sums are never read.
     auto do_pair_fast = [&](int p, int ia, int ib) {
       p = GPK_IDX(p, P, 3);
-      const T gab = s.G[p];
+      const R gab = s.G[p];
       T w[DB];
 #pragma unroll
       for (int d = 0; d < DB; ++d) w[d] = s.Bs[d * P + p];
-      T arg[NPB];
+      const R *ra = s.rec + ia * RL, *rb = s.rec + ib * RL;
+      R arg[NPB];
+#pragma unroll
+      for (int pt = 0; pt < NPB; ++pt) arg[pt] = X::template arg<QC>(ra + pt * M * RL, rb + pt * M * RL, gab);
 #pragma unroll
       for (int pt = 0; pt < NPB; ++pt) {
-        const T* hu = s.u + pt * M;
-        const T* hh = s.h + pt * M * QC + ia * QC;
-        T cr = mul(hh[0], s.z[ib * QC]);   // = fma_ from zero, bit for bit
-#pragma unroll
-        for (int q = 1; q < QC; ++q) cr = fma_(hh[q], s.z[ib * QC + q], cr);
-        arg[pt] = sub(add(add(hu[ia], hu[ib]), gab), cr);
-      }
-#pragma unroll
-      for (int pt = 0; pt < NPB; ++pt) {
-        const T ps = exp_pair(arg[pt], s.tab);
+        const T ps = X::ev(arg[pt], s.tab);
 #pragma unroll
         for (int d = 0; d < DB; ++d) vacc[pt][d] = fma_(w[d], ps, vacc[pt][d]);
       }
     };
-    const bool fast = PPT == 0 && contract && !a.psi2 && Q == QC && D == DB && s.Bs;
+    const bool fast = PPT == 0 && contract && !a.psi2 && D == DB && s.Bs && s.G && !general;
     if (fast) {
       for (int p = threadIdx.x; p < P; p += NT) {
         int ia, ib;
@@ -473,7 +584,7 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
           vals[(pt * DB + d) * 2] = mm;
           vals[(pt * DB + d) * 2 + 1] = vacc[pt][d];
         }
-      block_sum_many<T, 2 * NPB * DB>(vals, s.red, NT / 32);
+      block_sum_many<T, 2 * NPB * DB, FRED>(vals, s.red, NT / 32);
       if (threadIdx.x == 0) {
 #pragma unroll
         for (int pt = 0; pt < NPB; ++pt)
@@ -506,465 +617,514 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
 }
 
 // ---------------------------------------------------------------------------------
-// Backward, NPB points per pass.  Per point: psi1 terms per pseudo-input; per pair
-// L = W psi2 with W = sum_d dv_d (B_d[a,b] + B_d[b,a]) (the symmetrised upstream gradient, as
-// psi2compDer does, geepee/kernels.py:415-418) staged in shared memory; then per row a the
-// full-square sums R_a = sum_b L~_ab, S_aq = sum_b L~_ab z_bq (L~ the symmetric half-weight
-// matrix).  Every psi2 gradient is an affine function of R and S:
-//   dZ_aq += R_a(-z_aq/l + 2 c mu - c z_aq) + S_aq (1/l - c)
-//   dmu_q  = -2c (mu Rt - St)                    (Rt = sum_a R_a, St = sum_a S_a)
-//   dS_q   = -c Rt + 2c^2 (mu^2 Rt - 2 mu St + Z2R/2 + ZS/2)
-//   dl_q  += 2 ell (Rt (1/(2l) - c/2) + (Z2R - ZS)/(2 l^2) + c^2 (mu^2 Rt - 2 mu St + Z2R/2 + ZS/2))
-// with Z2R = sum_a z_a^2 R_a, ZS = sum_a z_a S_a; these restate psi2compDer
-// (geepee/kernels.py:402-444) without its N x M x M temporaries.  A pass evaluates each of a
-// thread's pairs for all NPB points (the pair's G_ab, z_b and B weights loaded once), and the
-// per-point phases and barriers are shared by the NPB points.
+// Backward.  Per point: psi1 terms per pseudo-input; per pair L = W psi2 with
+// W = sum_d dv_d (B_d[a,b] + B_d[b,a]) / 2 (the symmetrised upstream gradient, as psi2compDer does,
+// geepee/kernels.py:415-418) staged in shared memory; then per row a the full-square sums
+// R_a = sum_b L_ab, S_aq = sum_b L_ab z_bq.  With d_a = mu - z_a, A_a = S_a - z_a R_a,
+// H_a = R_a d_a - A_a / 2 (sum_a A_a = 0, L being symmetric), every psi2 gradient follows:
+//   dZ_aq += (1/l - c) A_a + 2 c R_a d_a
+//   dmu_q  = -2 c sum_a R_a d_a,   dS_q = c sum_a (2 c d_a H_a - R_a)
+//   dl_q  += ell (sum_a R_a / l + dS_q - sum_a z_a A_a / l^2)
+// and with L1_a = dpsi1_a psi1_a, y = L1 d / (l + S) the psi1 ones:
+//   dZ_aq += y,  dmu_q = -sum y,  2 dS_q = sum (y d - L1) / (l + S),  dl_q += ell (sum L1 / l + 2 dS_q)
+// which restate psi2compDer and psi1compDer (geepee/kernels.py:355-378, 402-444) without their
+// N x M x M temporaries.  Only dmu and the two parts of dS are reduced per point (3 Q values); every
+// other sum stays with the thread of its row until the end.
+//
+// The CTA is split by warps into NS sweep, NB back and NF front warps, which work side by side:
+//   stage A: sweep warps: pair sweep of point i -> L, dB-hat  | back warps: gradients of point i-1
+//   stage B: sweep and back warps: row sums of point i (SEG threads a row)
+//   through both: front warps: constants, psi1 terms and records of point i+1
+// with one CTA barrier after each stage.  In one-role form (every warp doing each phase in
+// turn, six barriers a point) the per-row phases kept 4 of 16 warps busy and the barriers were
+// the largest stall.  Measured (df64, with the reduction of the partial blocks): N = 10000, Q = 5,
+// M = 100: 1591 -> 766 us, 660 -> ~400 instructions a pair and point, 65% of issue slots; N = 1000,
+// Q = 2, M = 100: 128 -> 84 us, of which ~35 us are per-CTA tables and the flush; N = 4999, Q = 2,
+// M = 50, two outputs: 295 -> 128 us; FP32 at N = 10000: 416 -> 236 us.  Bound by instruction
+// issue, half of it FP32 additions of the double-float sums.  Records alternate between two
+// slots, the small per-point arrays between three.
+// dZ's row sums in the back threads' registers: one row a thread, and room for them
+__host__ __device__ constexpr bool bwd_dz_reg(int QC, int M, int nb) { return QC < QMAX && M <= nb * 32; }
+__host__ __device__ constexpr int zlen(int QC) { return (QC + 1) & ~1; }   // a z row, padded to pairs
 template <typename T>
 struct BSmem {
+  typedef typename PairExp<T>::R R;
   float2* tab;
-  T* z;      // [M*Q]
+  T* z;      // [M][zlen]
   T* ell2;   // [QMAX]
   T* lnl;    // [QMAX]
   T* inv4l;  // [QMAX]
   T* il;     // [QMAX]
   T* misc;   // [4] log sf2, sf2
-  T* pd;     // [NPB][5][QMAX] per-point constants
-  T* pg;     // [NPB][2*DMAX] dm_all, dv per point
-  T* u;      // [NPB][M]
-  T* h;      // [NPB][M*Q]
-  T* G;      // [P]
+  T* pd;     // [3][PDN] per-point constants
+  T* pg;     // [3][2*DMAX] dm_all, dv
+  T* As;     // [Dout][M]
+  R* rec;    // [2][M][rec_len]
+  T* L1;     // [3][M]
+  T* dz;     // [QC][M] where a back thread has several rows (else in its registers)
+  T* gA;     // [Dout][M]
+  T* rows;   // [SEG][1+QC][M]
+  T* red;    // [back warps][3 QC + 2]
+  T* L;      // [P]
+  R* G;      // [P] or nullptr (then formed for each pair)
   T* Bs;     // [Dout*P] or nullptr
-  T* L;      // [NPB][P]
-  T* rows;   // [NPB][M][1+QMAX]
-  T* dz;     // [M*Q]
-  T* accB;   // [Dout*P] sum over the CTA's points of dv psi2 (dBhat)
-  T* red;    // [32*RED]
-  int* pab;  // [P] the pairs (a << 16 | b), the same for every point
+  T* accB;   // [Dout*P] or nullptr: sum over the CTA's points of dv psi2 (dBhat)
+  unsigned short* pab;  // [P] or nullptr: the pairs (a << 8 | b)
 };
+// the per-point constants: PD arrays of QMAX, then log sf2 + sum pld1, k_n / 2, max pld2
+constexpr int PDN = PD * QMAX + 4;
 
-__host__ __device__ inline size_t bwd_smem_bytes(int M, int Q, int P, int nacc, int npb, size_t tsz, int nbs) {
-  size_t n = (size_t)M * Q + 4 * QMAX + 4 + (size_t)npb * (5 * QMAX + 2 * DMAX) + (size_t)npb * M * (1 + Q) + P +
-             nbs + (size_t)npb * P + (size_t)npb * M * (1 + QMAX) + (size_t)M * Q + nacc + 32 * RED;
-  return 256 * 8 + n * tsz;
-}
-
+struct BLayout {
+  int seg, ng, nbs, nacc, pab;   // row segments, elements of G, B, dB-hat; pair table or not
+};
 template <typename T>
-__device__ BSmem<T> bcarve(char* base, int M, int Q, int P, int nacc, int npb, int nbs) {
+__host__ __device__ inline size_t bcarve(BSmem<T>* out, char* base, int M, int QC, int P, int D, int nb,
+                                         const BLayout& lo) {
+  typedef typename PairExp<T>::R R;
+  static_assert(sizeof(R) == sizeof(T), "table elements as large as T");
   BSmem<T> s;
-  s.tab = reinterpret_cast<float2*>(base);
-  T* t = reinterpret_cast<T*>(base + 256 * sizeof(float2));
-  s.z = t; t += M * Q;
-  s.ell2 = t; t += QMAX;
-  s.lnl = t; t += QMAX;
-  s.inv4l = t; t += QMAX;
-  s.il = t; t += QMAX;
-  s.misc = t; t += 4;
-  s.pd = t; t += npb * 5 * QMAX;
-  s.pg = t; t += npb * 2 * DMAX;
-  s.u = t; t += npb * M;
-  s.h = t; t += npb * M * Q;
-  s.G = t; t += P;
-  s.Bs = nbs ? t : nullptr; t += nbs;
-  s.L = t; t += npb * P;
-  s.rows = t; t += npb * M * (1 + QMAX);
-  s.dz = t; t += M * Q;
-  s.accB = nacc ? t : nullptr; t += nacc;
-  s.red = t; t += 32 * RED;
-  s.pab = reinterpret_cast<int*>(t);
-  return s;
+  size_t o = 0;
+  auto take = [&](size_t n) {
+    char* p = base + o;
+    o += n;
+    return p;
+  };
+  const size_t e = sizeof(T);
+  s.tab = (float2*)take(PairExp<T>::TAB * sizeof(float2));
+  s.z = (T*)take((size_t)zlen(QC) * M * e);   // (16-byte aligned: read in pairs)
+  s.ell2 = (T*)take(QMAX * e);
+  s.lnl = (T*)take(QMAX * e);
+  s.inv4l = (T*)take(QMAX * e);
+  s.il = (T*)take(QMAX * e);
+  s.misc = (T*)take(4 * e);
+  s.pd = (T*)take(3 * PDN * e);
+  s.pg = (T*)take(3 * 2 * DMAX * e);
+  s.As = (T*)take((size_t)D * M * e);
+  s.rec = (R*)take(2 * (size_t)M * rec_len(QC) * e);
+  s.L1 = (T*)take(3 * (size_t)M * e);
+  s.dz = (T*)take(bwd_dz_reg(QC, M, nb) ? 0 : (size_t)QC * M * e);
+  s.gA = (T*)take((size_t)D * M * e);
+  s.rows = (T*)take((size_t)lo.seg * (1 + QC) * M * e);
+  s.red = (T*)take((size_t)nb * (3 * QC + 2) * e);
+  s.L = (T*)take((size_t)P * e);
+  s.G = lo.ng ? (R*)take((size_t)lo.ng * e) : nullptr;
+  s.Bs = lo.nbs ? (T*)take((size_t)lo.nbs * e) : nullptr;
+  s.accB = lo.nacc ? (T*)take((size_t)lo.nacc * e) : nullptr;
+  s.pab = lo.pab ? (unsigned short*)take((size_t)P * sizeof(unsigned short)) : nullptr;
+  if (out) *out = s;
+  return o;
 }
 
-template <typename T>
-__device__ __forceinline__ PointSlot<T> bslot(const BSmem<T>& s, int pt, int M, int Q) {
-  T* pd = s.pd + pt * 5 * QMAX;
-  return PointSlot<T>{pd, pd + QMAX, pd + 2 * QMAX, pd + 3 * QMAX, pd + 4 * QMAX, s.u + pt * M, s.h + pt * M * Q};
+// a running sum kept as (hi, lo) without renormalising: for sums of a few dozen terms (the low
+// word's own rounding stays below the normalised sum's)
+__device__ __forceinline__ void acc_add(df64& a, df64 x) {
+  const df64 s = two_sum(a.hi, x.hi);
+  a.hi = s.hi;
+  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, x.lo));
+}
+__device__ __forceinline__ void acc_fma(df64& a, df64 x, df64 y) {
+  const float p = __fmul_rn(x.hi, y.hi);
+  float e = __fmaf_rn(x.hi, y.hi, -p);
+  e = __fmaf_rn(x.hi, y.lo, e);
+  e = __fmaf_rn(x.lo, y.hi, e);
+  const df64 s = two_sum(a.hi, p);
+  a.hi = s.hi;
+  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, e));
+}
+__device__ __forceinline__ df64 acc_done(df64 a) { return quick_two_sum(a.hi, a.lo); }
+__device__ __forceinline__ void acc_add(float& a, float x) { a += x; }
+__device__ __forceinline__ void acc_fma(float& a, float x, float y) { a = __fmaf_rn(x, y, a); }
+__device__ __forceinline__ float acc_done(float a) { return a; }
+
+// barrier ID over NW warps of the CTA
+template <int ID, int NW>
+__device__ __forceinline__ void warps_sync() {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(NW * 32) : "memory");
+}
+// two consecutive elements in one access
+__device__ __forceinline__ void ld_two(const df64* p, df64& a, df64& b) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  a = make_df(v.x, v.y);
+  b = make_df(v.z, v.w);
+}
+__device__ __forceinline__ void ld_two(const float* p, float& a, float& b) {
+  const float2 v = *reinterpret_cast<const float2*>(p);
+  a = v.x;
+  b = v.y;
 }
 
-template <typename T, int NPB, int DB, int QC>
-__global__ void __launch_bounds__(nt_bwd(QC)) psi_bwd_kernel(PsiArgs<typename Num<T>::store_t> a) {
-  constexpr int NTB = nt_bwd(QC);
+template <typename T, int DB, int QC, int NS, int NB, int NF>
+__global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
+    psi_bwd_kernel(PsiArgs<typename Num<T>::store_t> a, BLayout lo) {
   typedef typename Num<T>::store_t S;
+  typedef PairExp<T> X;
+  typedef typename X::R R;
+  constexpr int RL = rec_len(QC), ZL = zlen(QC), NTH = (NS + NB + NF) * 32, NTS = NS * 32;
   extern __shared__ __align__(16) char smem_raw[];
   const int M = a.M, Q = exact_q(QC) ? QC : a.Q, D = a.Dout;
   const int P = M * (M + 1) / 2;
-  BSmem<T> s = bcarve<T>(smem_raw, M, Q, P, a.accb_smem ? D * P : 0, NPB, a.bs_smem ? D * P : 0);
-  // ---- per-CTA tables: exp table, Z, lengthscales, sf2, G_ab and the symmetrised B
-  load_exp_table(s.tab);
-  for (int i = threadIdx.x; i < M * Q; i += NTB) {
-    s.z[i] = Num<T>::ld(a.Z[i]);
-    s.dz[i] = Num<T>::zero();
+  BSmem<T> s;
+  bcarve<T>(&s, smem_raw, M, QC, P, D, NB, lo);
+  __shared__ int s_flag[3];   // the slot's point lies outside the fixed-point range
+  const ExpTab etab{s.tab};
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool back_warp = tid >= NTS && tid < NTS + NB * 32, front_warp = tid >= NTS + NB * 32;
+  // ---- per-CTA tables: exp table, Z, A, lengthscales, sf2
+  load_pair_table<T>(s.tab);
+  for (int i = tid; i < M * ZL; i += NTH) {
+    const int ia = i / ZL, q = i - ia * ZL;
+    s.z[i] = q < Q ? Num<T>::ld(a.Z[ia * Q + q]) : Num<T>::zero();
   }
-  if (s.accB)
-    for (int i = threadIdx.x; i < D * P; i += NTB) s.accB[i] = Num<T>::zero();
+  const bool dz_reg = bwd_dz_reg(QC, M, NB);
+  if (!dz_reg)
+    for (int i = tid; i < M * QC; i += NTH) s.dz[i] = Num<T>::zero();
+  for (int i = tid; i < D * M; i += NTH) {
+    s.As[i] = a.dpsi1 ? Num<T>::zero() : Num<T>::ld(a.A[i]);
+    s.gA[i] = Num<T>::zero();
+  }
   double* const part = a.part ? a.part + (size_t)blockIdx.x * a.part_stride : nullptr;
-  if (part && !s.accB)   // dBhat accumulates in this CTA's partial block (each pair has one owner)
-    for (int i = threadIdx.x; i < D * P; i += NTB) part[i] = 0.0;
   __syncthreads();
-  if (threadIdx.x < Q) {
-    const int q = threadIdx.x;
-    T lnl = Num<T>::ld(static_cast<S>(a.lls2[q]));
-    T l2 = exp_tab(lnl, s.tab);
-    s.lnl[q] = lnl;
-    s.ell2[q] = l2;
-    s.il[q] = recip(l2);
-    s.inv4l[q] = recip(mul(l2, Num<T>::c(4.f)));
+  if (tid < Q) {
+    const T lnl = Num<T>::ld(static_cast<S>(a.lls2[tid]));
+    const T l2 = exp_tab(lnl, etab);
+    s.lnl[tid] = lnl;
+    s.ell2[tid] = l2;
+    s.il[tid] = recip(l2);
+    s.inv4l[tid] = recip(mul(l2, Num<T>::c(4.f)));
   }
-  if (threadIdx.x == 32) {
-    T lsf = Num<T>::ld(static_cast<S>(a.lsf2[0]));
+  if (tid == 32) {
+    const T lsf = Num<T>::ld(static_cast<S>(a.lsf2[0]));
     s.misc[0] = lsf;
-    s.misc[1] = exp_tab(lsf, s.tab);
+    s.misc[1] = exp_tab(lsf, etab);
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < P; p += NTB) {
-    int ia, ib;
-    pair_of(p, ia, ib);
-    if (a.pab_smem) s.pab[p] = (ia << 16) | ib;
-    T g = Num<T>::zero();
-#pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      if (q < Q) {
-        T d = sub(s.z[ia * Q + q], s.z[ib * Q + q]);
-        g = fma_(mul(d, d), s.inv4l[q], g);
-      }
-    }
-    s.G[p] = neg(g);
-  }
-  if (s.Bs) stage_sym_B<T, NTB>(s.Bs, a.B, M, D, P);
-  // per-thread accumulators over points
-  T g_sf = Num<T>::zero();                 // sum L1 + 2 sum L (for dsf2 * sf2)
-  T g_l[QC];                               // dl (before the ell factor)
-  T g_A[DB];
-#pragma unroll
-  for (int q = 0; q < QC; ++q) g_l[q] = Num<T>::zero();
-#pragma unroll
-  for (int d = 0; d < DB; ++d) g_A[d] = Num<T>::zero();
   const T lsf = s.misc[0];
-  __syncthreads();
-
-  // each CTA takes a contiguous range of points, NPB at a time
+  // each CTA takes a contiguous range of points
   const int nbeg = (int)((long)a.N * blockIdx.x / gridDim.x);
   const int nend = (int)((long)a.N * (blockIdx.x + 1) / gridDim.x);
-  const int ia0 = threadIdx.x;   // the pseudo-input of this thread in the per-row phases (M <= NTB)
-  for (int n0 = nbeg; n0 < nend; n0 += NPB) {
-    const int npts = min(NPB, nend - n0);
-    // ---- per-point constants and upstream gradients
-    for (int t = threadIdx.x; t < 4 * npts * Q; t += NTB) {
-      const int part = t & 3, pq = t >> 2, pt = pq / Q, q = pq - pt * Q;
-      dims_of<T, S>(a, s.ell2, s.lnl, s.tab, bslot(s, pt, M, Q), n0 + pt, q, part);
-    }
-    if (threadIdx.x >= 256 && threadIdx.x < 256 + npts * D) {
-      const int t = threadIdx.x - 256, pt = t / D, d = t - pt * D, n = n0 + pt;
-      T dvv = a.b_stride ? Num<T>::c(1.f) : Num<T>::ld(a.dv[(size_t)n * D + d]);
+  const int cnt = nend - nbeg;
+
+  // ---- front warps: constants, psi1 terms and records of point i
+  auto front = [&](int i) {
+    const int rt = tid - (NTS + NB * 32), rw = rt >> 5;
+    const int n = nbeg + i, sl = i % 3;
+    T* pd = s.pd + sl * PDN;
+    const PointSlot<T> ps(pd, s.rec + (size_t)(i & 1) * M * RL);
+    T* pg = s.pg + sl * 2 * DMAX;
+    if (rw == 0) {
+      if (lane < 4 * Q) dims_of<T, S>(a, s.ell2, s.lnl, etab, ps, n, lane >> 2, lane & 3);
+      __syncwarp();
+      if (lane == 0) {
+        T c1 = lsf;
+        for (int q = 0; q < Q; ++q) c1 = add(c1, ps.pld1[q]);
+        pd[PD * QMAX] = c1;
+      } else if (lane == 1) {
+        T k = lsf;
+        float ld2 = -1e30f;
+        for (int q = 0; q < Q; ++q) {
+          k = add(k, scale2(ps.pld2[q], -1));
+          ld2 = fmax_nan(ld2, Num<T>::approx(ps.pld2[q]));
+        }
+        pd[PD * QMAX + 1] = mul(k, log2e_of(k));
+        pd[PD * QMAX + 2] = Num<T>::c(ld2);
+      } else if (lane == 2) {
+        s_flag[sl] = 0;
+      }
+    } else if (rw == 1 && lane < D) {
+      const T dvv = a.b_stride ? Num<T>::c(1.f) : Num<T>::ld(a.dv[(size_t)n * D + lane]);
       if (!a.dpsi1) {
-        T mm = Num<T>::ld(a.m[(size_t)n * D + d]);
-        T dmv = Num<T>::ld(a.dm[(size_t)n * D + d]);
-        s.pg[pt * 2 * DMAX + d] = sub(dmv, mul(scale2(dvv, 1), mm));     // dm_all
+        const T mm = Num<T>::ld(a.m[(size_t)n * D + lane]);
+        const T dmv = Num<T>::ld(a.dm[(size_t)n * D + lane]);
+        pg[lane] = sub(dmv, mul(scale2(dvv, 1), mm));     // dm_all
       }
-      s.pg[pt * 2 * DMAX + DMAX + d] = dvv;
+      pg[DMAX + lane] = dvv;
     }
-    __syncthreads();
-    // ---- psi1 terms, one pseudo-input per thread for all the pass's points
-    // vals[pt]: dmu, dS (psi1 part, 2Q) then Rt, St (Q), Z2R (Q), ZS (Q) - reduced together
-    constexpr int KV = 5 * QC + 1;
-    T vals[NPB * KV];
+    warps_sync<2, NF>();
+    const T k2 = pd[PD * QMAX + 1];
+    const float ld2 = Num<T>::approx(pd[PD * QMAX + 2]);
+    for (int ia = rt; ia < M; ia += NF * 32) {
+      T e1 = pd[PD * QMAX], s2 = Num<T>::zero(), t[QC];
 #pragma unroll
-    for (int i = 0; i < NPB * KV; ++i) vals[i] = Num<T>::zero();
-    if (ia0 < M) {
+      for (int q = 0; q < QC; ++q) {
+        t[q] = Num<T>::zero();
+        if (q < Q) {
+          const T d = sub(ps.pmu[q], s.z[ia * ZL + q]);
+          e1 = fma_(mul(d, d), scale2(neg(ps.pis1[q]), -1), e1);
+          t[q] = mul(d, ps.psq[q]);
+          s2 = fma_(t[q], t[q], s2);
+        }
+      }
+      put_rec<QC>(ps.rec + ia * RL, k2, s2, t, ld2, &s_flag[sl]);
+      const T p1 = exp_tab(e1, etab);
+      T dp1 = Num<T>::zero();
+      if (a.dpsi1) {
+        dp1 = Num<T>::ld(a.dpsi1[(size_t)n * M + ia]);
+      } else {
 #pragma unroll
-      for (int pt = 0; pt < NPB; ++pt) {
-        if (pt < npts) {
-          const int n = n0 + pt;
-          const PointSlot<T> ps = bslot(s, pt, M, Q);
-          const T* pg = s.pg + pt * 2 * DMAX;
-          T p1 = rows_of<T, QC>(s.z, lsf, s.tab, ps, Q, ia0);
-          T dp1 = Num<T>::zero();
-          if (a.dpsi1) {
-            dp1 = Num<T>::ld(a.dpsi1[(size_t)n * M + ia0]);
-          } else {
-#pragma unroll
-            for (int d = 0; d < DB; ++d) {
-              if (d < D) {
-                dp1 = fma_(pg[d], Num<T>::ld(a.A[d * M + ia0]), dp1);
-                g_A[d] = fma_(pg[d], p1, g_A[d]);
-              }
-            }
+        for (int d = 0; d < DB; ++d) {
+          if (d < D) {
+            dp1 = fma_(pg[d], s.As[d * M + ia], dp1);
+            s.gA[d * M + ia] = fma_(pg[d], p1, s.gA[d * M + ia]);
           }
-          T L1 = mul(dp1, p1);
-          g_sf = add(g_sf, L1);
+        }
+      }
+      s.L1[sl * M + ia] = mul(dp1, p1);
+    }
+    warps_sync<2, NF>();   // (the constants' slot is written again three points later)
+  };
+
+  // ---- back warps: gradients of point i from its row sums
+  T g1 = Num<T>::zero(), g2 = Num<T>::zero();   // sum L1, sum R
+  T dzr[QC];                                    // this thread's row of dZ (dz_reg)
+  T g_z[QC], g_l = Num<T>::zero();              // sum z A; lane QC + q of the first back warp: sum (2 dS1 + dS2)
 #pragma unroll
-          for (int q = 0; q < QC; ++q) {
-            if (q < Q) {
-              T dd = sub(ps.pmu[q], s.z[ia0 * Q + q]);
-              T ds = mul(dd, ps.pis1[q]);                       // (mu - z)/s1
-              T ds2 = mul(ds, ds);
-              T L1ds = mul(L1, ds);
-              vals[pt * KV + q] = neg(L1ds);                    // dmu
-              vals[pt * KV + QC + q] = scale2(mul(L1, sub(ds2, ps.pis1[q])), -1);   // dS
-              s.dz[ia0 * Q + q] = add(s.dz[ia0 * Q + q], L1ds);  // dZ (psi1)
-              g_l[q] = add(g_l[q], mul(L1, add(sub(s.il[q], ps.pis1[q]), ds2)));   // 1/l - 1/s1 + d^2/s1^2
-            }
+  for (int q = 0; q < QC; ++q) g_z[q] = dzr[q] = Num<T>::zero();
+  constexpr int RW = 3 * QC + 2;
+  auto back = [&](int i) {
+    const int rt = tid - NTS, rw = rt >> 5;
+    const int n = nbeg + i, sl = i % 3;
+    const PointSlot<T> ps(s.pd + sl * PDN, s.rec);
+    T tot = Num<T>::zero();
+    for (int r0 = 0; r0 < M; r0 += NB * 32) {
+      const int ia = r0 + rt;
+      T vals[3 * QC];   // per dimension: -dmu, 2 dS of psi1, dS of psi2
+#pragma unroll
+      for (int k = 0; k < 3 * QC; ++k) vals[k] = Num<T>::zero();
+      if (ia < M) {
+        const T L1 = s.L1[sl * M + ia];
+        const T* row = s.rows + ia;
+        T Ra = row[0], Sa[QC];
+#pragma unroll
+        for (int q = 0; q < QC; ++q) Sa[q] = row[(1 + q) * M];
+        for (int g = 1; g < lo.seg; ++g) {
+          row += (1 + QC) * M;
+          acc_add(Ra, row[0]);
+#pragma unroll
+          for (int q = 0; q < QC; ++q) acc_add(Sa[q], row[(1 + q) * M]);
+        }
+        Ra = acc_done(Ra);
+        g1 = add(g1, L1);
+        g2 = add(g2, Ra);
+#pragma unroll
+        for (int q = 0; q < QC; ++q) {
+          if (q < Q) {
+            const T z = s.z[ia * ZL + q], d = sub(ps.pmu[q], z), is1 = ps.pis1[q], c = ps.pc[q];
+            const T y = mul(is1, mul(L1, d));
+            const T A = sub(acc_done(Sa[q]), mul(Ra, z)), Rd = mul(Ra, d);
+            const T yg = add(y, mul(scale2(c, 1), Rd));
+            const T dz = fma_(sub(s.il[q], c), A, add(dz_reg ? dzr[q] : s.dz[q * M + ia], yg));
+            if (dz_reg) dzr[q] = dz;
+            else s.dz[q * M + ia] = dz;
+            g_z[q] = fma_(z, A, g_z[q]);
+            const T H = sub(Rd, scale2(A, -1));
+            vals[q] = yg;
+            vals[QC + q] = mul(is1, sub(mul(y, d), L1));
+            vals[2 * QC + q] = mul(c, sub(scale2(mul(c, mul(d, H)), 1), Ra));
           }
+        }
+      }
+      // 3 Q values over the back warps: multi-value butterflies, then lane k adds value k over warps
+#pragma unroll
+      for (int c0 = 0; c0 < 3 * QC; c0 += 8) {
+        T t[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t[u] = c0 + u < 3 * QC ? vals[c0 + u] : Num<T>::zero();
+        warp_sum_many<8>(t);
+        if ((lane & 3) == 0 && c0 + (lane >> 2) < 3 * QC) s.red[rw * RW + c0 + (lane >> 2)] = t[0];
+      }
+      warps_sync<1, NB>();
+      if (rw == 0 && lane < 3 * QC)
+        for (int w = 0; w < NB; ++w) tot = add(tot, s.red[w * RW + lane]);
+      warps_sync<1, NB>();   // red and the constants' slot are free again
+    }
+    if (rw == 0) {
+      const T e2 = shfl_idx(tot, lane + QC);
+      const int q = lane < QC ? lane : lane - QC;
+      if (lane < 2 * QC && q < Q) {
+        if (lane < QC) {
+          a.dmu[(size_t)n * Q + q] = Num<T>::st(neg(tot));
+        } else {
+          a.dvar[(size_t)n * Q + q] = Num<T>::st(add(scale2(tot, -1), e2));
+          g_l = add(g_l, add(tot, e2));
         }
       }
     }
-    __syncthreads();
-    // ---- pairs: L = W psi2 -> shared memory; dBhat accumulates in shared memory (each
-    // pair has one owner thread)
-    T dvr[NPB][DB];
-#pragma unroll
-    for (int pt = 0; pt < NPB; ++pt)
-#pragma unroll
-      for (int d = 0; d < DB; ++d)
-        dvr[pt][d] = (pt < npts && d < D) ? s.pg[pt * 2 * DMAX + DMAX + d] : Num<T>::zero();
-    if (NPB == 1 && Q == QC && D == DB && s.Bs && s.accB && !a.b_stride) {
-      // the common configuration, branch-free: two pairs (p, p + NTB) per iteration, each step
-      // written for both, so that their dependent double-float chains interleave
-      const T* hu = s.u;
-      for (int p0 = threadIdx.x; p0 < P; p0 += 2 * NTB) {
-        int pp[2], ia[2], ib[2];
-        bool ok[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          ok[u] = p0 + u * NTB < P;
-          pp[u] = GPK_IDX(ok[u] ? p0 + u * NTB : p0, P, 2);
-          if (a.pab_smem) {   // the pair's (a, b) from the per-CTA table (CTA-uniform test)
-            const int ab = s.pab[pp[u]];
-            ia[u] = ab >> 16;
-            ib[u] = ab & 0xffff;
-          } else {
-            pair_of(pp[u], ia[u], ib[u]);
-          }
-        }
-        T arg[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const T* hh = s.h + ia[u] * QC;
-          T cr = mul(hh[0], s.z[ib[u] * QC]);   // = fma_ from zero, bit for bit
-#pragma unroll
-          for (int q = 1; q < QC; ++q) cr = fma_(hh[q], s.z[ib[u] * QC + q], cr);
-          arg[u] = sub(add(add(hu[ia[u]], hu[ib[u]]), s.G[pp[u]]), cr);
-        }
-        T ps[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) ps[u] = exp_pair(arg[u], s.tab);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          T ab[DB];
-#pragma unroll
-          for (int d = 0; d < DB; ++d) ab[d] = mul(dvr[0][d], ps[u]);
-          // L~ (half weight off the diagonal: the symmetric matrix entry) = psi2 sum_d dv_d Bs_d:
-          // for one output (dv psi2) Bs, reusing the dB-hat term
-          T l;
-          if (DB == 1) {
-            l = mul(ab[0], s.Bs[pp[u]]);
-          } else {
-            T w = mul(dvr[0][0], s.Bs[pp[u]]);
-#pragma unroll
-            for (int d = 1; d < DB; ++d) w = fma_(dvr[0][d], s.Bs[d * P + pp[u]], w);
-            l = mul(w, ps[u]);
-          }
-          if (ok[u]) {
-            s.L[pp[u]] = ia[u] == ib[u] ? l : scale2(l, -1);
-#pragma unroll
-            for (int d = 0; d < DB; ++d) s.accB[d * P + pp[u]] = add(s.accB[d * P + pp[u]], ab[d]);
-          }
-        }
-      }
-    } else
-    for (int p = threadIdx.x; p < P; p += NTB) {
+  };
+
+  if (front_warp) {
+    if (cnt > 0) front(0);
+  } else {
+    constexpr int NTA = NTS + NB * 32;
+    for (int p = tid; p < P; p += NTA) {
       int ia, ib;
       pair_of(p, ia, ib);
-      const T gab = s.G[p];
-      T zb[QC];
+      if (s.pab) s.pab[p] = (unsigned short)((ia << 8) | ib);
+      if (s.G) s.G[p] = pair_G<T, QC>(s.z + ia * ZL, s.z + ib * ZL, s.inv4l, Q);
+    }
+    if (s.Bs) stage_sym_B<T, NTA>(s.Bs, a.B, M, D, P, true);
+    if (s.accB)
+      for (int i = tid; i < D * P; i += NTA) s.accB[i] = Num<T>::zero();
+    else if (part && a.dB)   // dBhat accumulates in this CTA's partial block (each pair has one owner)
+      for (int i = tid; i < D * P; i += NTA) part[i] = 0.0;
+  }
+  __syncthreads();
+  for (int i = 0; i < cnt; ++i) {
+    const int n = nbeg + i, sl = i % 3;
+    // ---- stage A
+    if (front_warp) {
+      if (i + 1 < cnt) front(i + 1);
+    } else if (back_warp) {
+      if (i > 0) back(i - 1);
+    } else {
+      const R* rec = s.rec + (size_t)(i & 1) * M * RL;
+      const bool general = X::TAB && s_flag[sl];
+      T dvr[DB];
 #pragma unroll
-      for (int q = 0; q < QC; ++q) zb[q] = q < Q ? s.z[ib * Q + q] : Num<T>::zero();
-      T bb[DB], ab[DB];
+      for (int d = 0; d < DB; ++d) dvr[d] = d < D ? s.pg[sl * 2 * DMAX + DMAX + d] : Num<T>::zero();
+      if (D == DB && s.Bs && s.accB && s.G && s.pab && !general) {
+        // the common configuration, branch-free: two pairs (p, p + NTS) per iteration, each step
+        // written for both, so that their dependent chains interleave
+        for (int p0 = tid; p0 < P; p0 += 2 * NTS) {
+          int pp[2], ia[2], ib[2];
+          bool ok[2];
 #pragma unroll
-      for (int d = 0; d < DB; ++d) {
-        bb[d] = ab[d] = Num<T>::zero();
-        if (d < D) {
-          if (s.Bs) {
-            bb[d] = s.Bs[d * P + p];
-          } else {
-            const S* Bd = a.B + (size_t)d * M * M + (size_t)n0 * a.b_stride;
-            bb[d] = Num<T>::ld(Bd[ia * M + ib]);
-            if (ia != ib) bb[d] = add(bb[d], Num<T>::ld(Bd[ib * M + ia]));
+          for (int u = 0; u < 2; ++u) {
+            ok[u] = p0 + u * NTS < P;
+            pp[u] = GPK_IDX(ok[u] ? p0 + u * NTS : p0, P, 2);
+            const int ab = s.pab[pp[u]];
+            ia[u] = ab >> 8;
+            ib[u] = ab & 0xff;
+          }
+          R arg[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) arg[u] = X::template arg<QC>(rec + ia[u] * RL, rec + ib[u] * RL, s.G[pp[u]]);
+          T ps2[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) ps2[u] = X::ev(arg[u], s.tab);
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            T ab[DB];
+#pragma unroll
+            for (int d = 0; d < DB; ++d) ab[d] = mul(dvr[d], ps2[u]);
+            T l;
+            if (DB == 1) {   // (dv psi2) B, reusing the dB-hat term
+              l = mul(ab[0], s.Bs[pp[u]]);
+            } else {
+              T w = mul(dvr[0], s.Bs[pp[u]]);
+#pragma unroll
+              for (int d = 1; d < DB; ++d) w = fma_(dvr[d], s.Bs[d * P + pp[u]], w);
+              l = mul(w, ps2[u]);
+            }
+            if (ok[u]) {
+              s.L[pp[u]] = l;
+#pragma unroll
+              for (int d = 0; d < DB; ++d) s.accB[d * P + pp[u]] = add(s.accB[d * P + pp[u]], ab[d]);
+            }
           }
         }
-      }
-#pragma unroll
-      for (int pt = 0; pt < NPB; ++pt) {
-        if (pt < npts) {
-          if (a.b_stride && pt > 0) {   // per-point B (Dout == 1): reload for this point
-            const S* Bd = a.B + (size_t)(n0 + pt) * a.b_stride;
-            bb[0] = Num<T>::ld(Bd[ia * M + ib]);
-            if (ia != ib) bb[0] = add(bb[0], Num<T>::ld(Bd[ib * M + ia]));
+      } else {
+        for (int p = tid; p < P; p += NTS) {
+          int ia, ib;
+          pair_of(p, ia, ib);
+          T ps2;
+          if (general) {
+            ps2 = psi2_general(s.z + ia * ZL, s.z + ib * ZL, s.pd + sl * PDN, s.inv4l, lsf, Q, s.tab);
+          } else {
+            const R gab = s.G ? s.G[p] : pair_G<T, QC>(s.z + ia * ZL, s.z + ib * ZL, s.inv4l, Q);
+            ps2 = X::ev(X::template arg<QC>(rec + ia * RL, rec + ib * RL, gab), s.tab);
           }
-          const T* hu = s.u + pt * M;
-          const T* hh = s.h + pt * M * Q + ia * Q;
-          T x = add(add(hu[ia], hu[ib]), gab);
-          T cr = Num<T>::zero();
-#pragma unroll
-          for (int q = 0; q < QC; ++q)
-            if (q < Q) cr = fma_(hh[q], zb[q], cr);
-          const T ps = exp_pair(sub(x, cr), s.tab);
           T w = Num<T>::zero();
 #pragma unroll
           for (int d = 0; d < DB; ++d) {
             if (d < D) {
-              w = fma_(dvr[pt][d], bb[d], w);
-              ab[d] = fma_(dvr[pt][d], ps, ab[d]);
+              T bb;
+              if (s.Bs) {
+                bb = s.Bs[d * P + p];
+              } else {
+                const S* Bd = a.B + (size_t)d * M * M + (size_t)n * a.b_stride;
+                bb = Num<T>::ld(Bd[ia * M + ib]);
+                if (ia != ib) bb = scale2(add(bb, Num<T>::ld(Bd[ib * M + ia])), -1);
+              }
+              w = fma_(dvr[d], bb, w);
             }
           }
-          // L~ (half weight off the diagonal: the symmetric matrix entry)
-          const T l = mul(w, ps);
-          s.L[pt * P + p] = ia == ib ? l : scale2(l, -1);
-        }
-      }
+          s.L[p] = mul(w, ps2);
 #pragma unroll
-      for (int d = 0; d < DB; ++d) {
-        if (d < D) {
-          if (s.accB) {
-            s.accB[d * P + p] = add(s.accB[d * P + p], ab[d]);
-          } else if (part) {   // no room for the accumulators: this thread's pair of the partial block
-            part[d * P + p] += (double)Num<T>::st(ab[d]);
-          } else if (a.dB) {   // no room for the accumulators: straight into dB
-            const double v = (double)Num<T>::st(ab[d]);
-            atomicAdd(&a.dB[((size_t)d * M + ia) * M + ib], v);
-            if (ia != ib) atomicAdd(&a.dB[((size_t)d * M + ib) * M + ia], v);
-          }
-        }
-      }
-    }
-    __syncthreads();
-    // ---- row sums, 8 threads per (point, row)
-    for (int rid0 = 0; rid0 < npts * M; rid0 += NTB / 8) {
-      const int rid = rid0 + (threadIdx.x >> 3), sl = threadIdx.x & 7;
-      const int pt = rid / M, ia = rid - pt * M;
-      T R = Num<T>::zero();
-      T Sq[QC];
-#pragma unroll
-      for (int q = 0; q < QC; ++q) Sq[q] = Num<T>::zero();
-      if (rid < npts * M) {
-        const T* Lp = s.L + pt * P;
-        const int rowbase = ia * (ia + 1) / 2;
-        // two interleaved partial sums (b = sl + 16 j and sl + 8 + 16 j) halve the chains
-        T R1 = Num<T>::zero(), S1[QC];
-#pragma unroll
-        for (int q = 0; q < QC; ++q) S1[q] = Num<T>::zero();
-        // branch-free: a second column past M contributes zero, and dimensions q >= Q reuse
-        // dimension 0's coordinate in sums that are never stored
-        for (int ib = sl; ib < M; ib += 16) {
-          const int jb = ib + 8, jc = jb < M ? jb : ib;
-          const int p = ia >= ib ? rowbase + ib : ib * (ib + 1) / 2 + ia;
-          const int p1 = ia >= jc ? rowbase + jc : jc * (jc + 1) / 2 + ia;
-          const T l = Lp[p];
-          const T l1 = jb < M ? Lp[p1] : Num<T>::zero();
-          R = add(R, l);
-          R1 = add(R1, l1);
-#pragma unroll
-          for (int q = 0; q < QC; ++q) {
-            const int qq = q < Q ? q : 0;
-            Sq[q] = fma_(l, s.z[ib * Q + qq], Sq[q]);
-            S1[q] = fma_(l1, s.z[jc * Q + qq], S1[q]);
-          }
-        }
-        R = add(R, R1);
-#pragma unroll
-        for (int q = 0; q < QC; ++q) Sq[q] = add(Sq[q], S1[q]);
-      }
-#pragma unroll
-      for (int m = 1; m < 8; m <<= 1) {
-        R = add(R, shfl_xor(R, m));
-#pragma unroll
-        for (int q = 0; q < QC; ++q) Sq[q] = add(Sq[q], shfl_xor(Sq[q], m));
-      }
-      if (rid < npts * M && sl == 0) {
-        T* row = s.rows + (pt * M + ia) * (1 + QMAX);
-        row[0] = R;
-#pragma unroll
-        for (int q = 0; q < QC; ++q)
-          if (q < Q) row[1 + q] = Sq[q];
-      }
-    }
-    __syncthreads();
-    // ---- dZ from the row sums, and this row's share of the per-point totals
-    if (ia0 < M) {
-#pragma unroll
-      for (int pt = 0; pt < NPB; ++pt) {
-        if (pt < npts) {
-          const PointSlot<T> ps = bslot(s, pt, M, Q);
-          const T* row = s.rows + (pt * M + ia0) * (1 + QMAX);
-          const T R = row[0];
-          vals[pt * KV + 2 * QC] = R;
-#pragma unroll
-          for (int q = 0; q < QC; ++q) {
-            if (q < Q) {
-              T zq = s.z[ia0 * Q + q];
-              T il = s.il[q];
-              T cq = ps.pc[q];
-              const T Sa = row[1 + q];
-              // R(-z/l + 2 c mu - c z) + S (1/l - c)
-              T t = sub(add(neg(mul(zq, il)), scale2(mul(cq, ps.pmu[q]), 1)), mul(cq, zq));
-              s.dz[ia0 * Q + q] = add(s.dz[ia0 * Q + q], add(mul(R, t), mul(Sa, sub(il, cq))));
-              vals[pt * KV + 2 * QC + 1 + q] = Sa;                          // St
-              vals[pt * KV + 3 * QC + 1 + q] = mul(mul(zq, zq), R);         // Z2R
-              vals[pt * KV + 4 * QC + 1 + q] = mul(zq, Sa);                 // ZS
+          for (int d = 0; d < DB; ++d) {
+            if (d < D) {
+              const T ab = mul(dvr[d], ps2);
+              if (s.accB) {
+                s.accB[d * P + p] = add(s.accB[d * P + p], ab);
+              } else if (part && a.dB) {   // no room for the accumulators: this thread's pair of the partial block
+                part[d * P + p] += (double)Num<T>::st(ab);
+              } else if (a.dB) {   // no room for the accumulators: straight into dB
+                const double v = (double)Num<T>::st(ab);
+                atomicAdd(&a.dB[((size_t)d * M + ia) * M + ib], v);
+                if (ia != ib) atomicAdd(&a.dB[((size_t)d * M + ib) * M + ia], v);
+              }
             }
           }
         }
       }
     }
-    // ---- per-point totals: one CTA reduction, then lane q of warp 0 finalises dimension q
-    block_sum_many<T, NPB * KV>(vals, s.red, (M + 31) >> 5);   // vals live in the row threads ia0 < M
-    if (threadIdx.x < 32) {
+    if (!front_warp) {
+      warps_sync<3, NS + NB>();
+      // ---- stage B: thread (segment, row) sums the row's columns [b0, b1) of the symmetric L;
+      // lanes take consecutive rows, so z_b is one broadcast
+      const int W = (M + lo.seg - 1) / lo.seg;
+      for (int t = tid; t < lo.seg * M; t += NTS + NB * 32) {
+        const int g = t / M, ia = t - g * M;
+        const int b0 = g * W, b1 = min(M, b0 + W);
+        const T* l = s.L + (ia >= b0 ? ia * (ia + 1) / 2 + b0 : b0 * (b0 + 1) / 2 + ia);
+        const T* zb = s.z + b0 * ZL;
+        T Rs = Num<T>::zero(), Sq[ZL];
 #pragma unroll
-      for (int pt = 0; pt < NPB; ++pt) {
-        if (pt < npts) {
-          const int n = n0 + pt;
-          const PointSlot<T> ps = bslot(s, pt, M, Q);
-          const T Rt = vals[pt * KV + 2 * QC];
+        for (int q = 0; q < ZL; ++q) Sq[q] = Num<T>::zero();
+#pragma unroll 4
+        for (int b = b0; b < b1; ++b) {
+          const T lv = *l;
+          l += b < ia ? 1 : b + 1;   // the next column of this row in the packed triangle
+          acc_add(Rs, lv);
 #pragma unroll
-          for (int q = 0; q < QC; ++q) {
-            if (q < Q && q == (int)threadIdx.x) {
-              const T St = vals[pt * KV + 2 * QC + 1 + q], Z2R = vals[pt * KV + 3 * QC + 1 + q];
-              const T ZS = vals[pt * KV + 4 * QC + 1 + q];
-              T mu = ps.pmu[q], cq = ps.pc[q], il = s.il[q];
-              T e2 = add(sub(mul(mul(mu, mu), Rt), scale2(mul(mu, St), 1)), scale2(add(Z2R, ZS), -1));
-              T dmu = add(vals[pt * KV + q], mul(scale2(cq, 1), sub(St, mul(mu, Rt))));
-              T dS = add(vals[pt * KV + QC + q], add(neg(mul(cq, Rt)), scale2(mul(mul(cq, cq), e2), 1)));
-              // (dl / 2 ell) accumulates: Rt (1/(2l) - c/2) + (Z2R - ZS)/(2 l^2) + c^2 e2
-              T t = add(add(scale2(mul(Rt, sub(il, cq)), -1), scale2(mul(sub(Z2R, ZS), mul(il, il)), -1)),
-                        mul(mul(cq, cq), e2));
-              g_l[q] = add(g_l[q], scale2(t, 1));
-              a.dmu[(size_t)n * Q + q] = Num<T>::st(dmu);
-              a.dvar[(size_t)n * Q + q] = Num<T>::st(dS);
-            }
+          for (int q = 0; q < ZL; q += 2) {
+            T z0, z1;
+            ld_two(zb + q, z0, z1);
+            acc_fma(Sq[q], lv, z0);
+            if (q + 1 < QC) acc_fma(Sq[q + 1], lv, z1);
           }
-          if (threadIdx.x == 0) g_sf = add(g_sf, scale2(Rt, 1));
+          zb += ZL;
         }
+        T* o = s.rows + (size_t)g * (1 + QC) * M + ia;
+        o[0] = acc_done(Rs);
+#pragma unroll
+        for (int q = 0; q < QC; ++q) o[(1 + q) * M] = acc_done(Sq[q]);
       }
     }
     __syncthreads();
   }
-  // ---- flush CTA accumulators: into the partial block (fixed-order path) or atomically
-  T fin[1 + QC];
-  fin[0] = g_sf;
+  if (back_warp && cnt > 0) back(cnt - 1);
+  T* const dzo = dz_reg ? s.rows : s.dz;   // (a back thread has read its own column of rows)
+  if (back_warp && dz_reg && tid - NTS < M) {
 #pragma unroll
-  for (int q = 0; q < QC; ++q) fin[1 + q] = g_l[q];
+    for (int q = 0; q < QC; ++q)
+      if (q < Q) dzo[q * M + tid - NTS] = dzr[q];
+  }
+  __syncthreads();
+  // ---- flush CTA accumulators: into the partial block ([dB pairs D*P | dA D*M | dZ M*Q | dsf2 |
+  // dl Q], fixed-order path) or atomically
   if (part) {
     const bool wantA = a.dA && !a.dpsi1;
     if (s.accB)
-      for (int i = threadIdx.x; i < D * P; i += NTB) part[i] = (double)Num<T>::st(s.accB[i]);
-    if (threadIdx.x < M) {
-#pragma unroll
-      for (int d = 0; d < DB; ++d)
-        if (d < D) part[D * P + d * M + threadIdx.x] = wantA ? (double)Num<T>::st(g_A[d]) : 0.0;
+      for (int i = tid; i < D * P; i += NTH) part[i] = (double)Num<T>::st(s.accB[i]);
+    for (int i = tid; i < D * M; i += NTH) part[D * P + i] = wantA ? (double)Num<T>::st(s.gA[i]) : 0.0;
+    for (int i = tid; i < M * Q; i += NTH) {
+      const int ia = i / Q, q = i - ia * Q;
+      part[D * P + D * M + i] = (double)Num<T>::st(dzo[q * M + ia]);
     }
-    for (int i = threadIdx.x; i < M * Q; i += blockDim.x) part[D * P + D * M + i] = (double)Num<T>::st(s.dz[i]);
   } else {
     if (a.dB && s.accB) {
-      for (int p = threadIdx.x; p < P; p += NTB) {
+      for (int p = tid; p < P; p += NTH) {
         int ia, ib;
         pair_of(p, ia, ib);
         for (int d = 0; d < D; ++d) {
@@ -974,28 +1134,44 @@ __global__ void __launch_bounds__(nt_bwd(QC)) psi_bwd_kernel(PsiArgs<typename Nu
         }
       }
     }
-    if (threadIdx.x < M) {
-#pragma unroll
-      for (int d = 0; d < DB; ++d)
-        if (d < D && a.dA && !a.dpsi1) atomicAdd(&a.dA[d * M + threadIdx.x], (double)Num<T>::st(g_A[d]));
+    if (a.dA && !a.dpsi1)
+      for (int i = tid; i < D * M; i += NTH) atomicAdd(&a.dA[i], (double)Num<T>::st(s.gA[i]));
+    for (int i = tid; i < M * Q; i += NTH) {
+      const int ia = i / Q, q = i - ia * Q;
+      atomicAdd(&a.dZ[i], (double)Num<T>::st(dzo[q * M + ia]));
     }
-    for (int i = threadIdx.x; i < M * Q; i += blockDim.x) atomicAdd(&a.dZ[i], (double)Num<T>::st(s.dz[i]));
   }
-  // dsf2 and dl need the ell / sf2 factors: (sum L1 + 2 sum L) / sf2 and ell * g_l
-  __syncthreads();
-  block_sum<T, 1 + QC>(fin, s.red);
-  if (threadIdx.x == 0) {
-    const double vsf = (double)Num<T>::st(div(fin[0], s.misc[1]));
-    if (part) part[D * P + D * M + M * Q] = vsf;
-    else atomicAdd(a.dsf2, vsf);
+  // dsf2 and dl: (sum L1 + 2 sum R) / sf2 and ell ((sum L1 + sum R) / l + g_l - g_z / l^2)
+  if (back_warp) {
+    const int rt = tid - NTS, rw = rt >> 5;
+    auto put = [&](int k, T v) {
+      v = warp_sum(v);
+      if (lane == 0) s.red[rw * RW + k] = v;
+    };
+    put(0, g1);
+    put(1, g2);
 #pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      if (q < Q) {
-        T ell = sqrt_(s.ell2[q]);
-        const double vl = (double)Num<T>::st(mul(fin[1 + q], ell));
-        if (part) part[D * P + D * M + M * Q + 1 + q] = vl;
-        else atomicAdd(&a.dl[q], vl);
+    for (int q = 0; q < QC; ++q) put(2 + q, g_z[q]);
+    if (rw == 0 && lane >= QC && lane < 2 * QC) s.red[2 + lane] = g_l;   // value 2 + QC + q
+    warps_sync<1, NB>();
+    if (rt < 1 + Q) {
+      auto tot = [&](int k) {
+        T v = s.red[k];
+        for (int w = 1; w < NB; ++w) v = add(v, s.red[w * RW + k]);
+        return v;
+      };
+      const T t1 = tot(0), t2 = tot(1);
+      double out;
+      if (rt == 0) {
+        out = (double)Num<T>::st(div(add(t1, scale2(t2, 1)), s.misc[1]));
+      } else {
+        const int q = rt - 1;
+        const T il = s.il[q];
+        const T g = add(mul(add(t1, t2), il), sub(s.red[2 + QC + q], mul(tot(2 + q), mul(il, il))));
+        out = (double)Num<T>::st(mul(g, sqrt_(s.ell2[q])));
       }
+      if (part) part[D * P + D * M + M * Q + rt] = out;
+      else atomicAdd(rt == 0 ? a.dsf2 : a.dl + (rt - 1), out);
     }
   }
 }
@@ -1041,353 +1217,30 @@ int launch_fwd(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) {
   const bool sum = a.psi2_sum != nullptr;
   const int npb = a.chain ? 1 : ((sum || (contract && a.Dout > 2)) ? 2 : 4);
   const int D = contract ? a.Dout : 0;
-  a.bs_smem = contract && fwd_smem_bytes(a.M, a.Q, P, D, npb, sizeof(T), a.Dout * P) <= 200 * 1024;
-  size_t sm = fwd_smem_bytes(a.M, a.Q, P, D, npb, sizeof(T), a.bs_smem ? a.Dout * P : 0);
-  if (sm > 227 * 1024) return gpk::fail(GPK_EUNSUPPORTED, "psi_fwd: M=%d needs %zu B of shared memory", a.M, sm);
+  // accepted sizes: a pair table and the points' tables within shared memory
+  const size_t need = 2048 + ((size_t)a.M * a.Q + 28 + (size_t)npb * 40 + (size_t)npb * a.M * (2 + a.Q) +
+                              (size_t)D * a.M + P + 1536) * sizeof(T);
+  if (need > 227 * 1024) return gpk::fail(GPK_EUNSUPPORTED, "psi_fwd: M=%d needs %zu B of shared memory", a.M, need);
   if (sum && P > PPT_MAX * NT)
     return gpk::fail(GPK_EUNSUPPORTED, "psi_fwd: psi2_sum needs M(M+1)/2 <= %d (M=%d)", PPT_MAX * NT, a.M);
+  // five input dimensions, one output, moments only (the psi-statistics workload's shape): an
+  // exact instantiation
+  const bool five = a.Q == 5 && !sum && !a.chain && contract && a.Dout == 1 && !a.psi2;
+  const int QC = a.Q <= 2 ? 2 : (five ? 5 : QMAX);
+  // G and the symmetrised B in shared memory as far as they fit; B first (from global memory it
+  // costs two loads and conversions per pair, G a few operations per dimension)
+  const size_t cap = SMEM_CAP;
+  auto bytes = [&](int ng, int nbs) { return fwd_smem_bytes(a.M, a.Q, QC, D, npb, sizeof(T), ng, nbs); };
+  const int nbs = contract ? a.Dout * P : 0;
+  a.bs_smem = contract && bytes(0, nbs) <= cap;
+  a.g_smem = bytes(P, a.bs_smem ? nbs : 0) <= cap;
+  const size_t sm = bytes(a.g_smem ? P : 0, a.bs_smem ? nbs : 0);
   int per_sm = (int)((227 * 1024) / (sm + 1024));
   if (per_sm < 1) per_sm = 1;
   if (per_sm > 2) per_sm = 2;
-  if (a.Q <= 2) return fwd_variant<T, 2>(a, sum, contract, P, per_sm, sm, st);
-  // five input dimensions, one output, moments only (the psi-statistics workload's shape): an
-  // exact instantiation, so that the pair loop is the branch-free one (Q == QC)
-  if (a.Q == 5 && !sum && !a.chain && contract && a.Dout == 1 && !a.psi2 && a.bs_smem)
-    return run_fwd<T, 4, 0, 5, 1>(a, per_sm, sm, st);
+  if (QC == 2) return fwd_variant<T, 2>(a, sum, contract, P, per_sm, sm, st);
+  if (QC == 5) return run_fwd<T, 4, 0, 5, 1>(a, per_sm, sm, st);
   return fwd_variant<T, QMAX>(a, sum, contract, P, per_sm, sm, st);
-}
-
-// ---------------------------------------------------------------------------------
-// Backward, software-pipelined over points (the common configuration: Q == QC, Dout == DB,
-// B and the dB-hat accumulators in shared memory, the fixed-order partial block).  Iteration
-// i overlaps point i's front half with point i-1's back half, so a point costs three CTA
-// barriers instead of six and the short phases share them:
-//   phase 1: row sums of point i-1 (8 threads a row)    | per-point constants of point i
-//   phase 2: dZ and totals of point i-1 (warps 4..7)     | psi1 terms of point i (warps 0..3)
-//            one CTA reduction of both; warp 0 then finalises point i-1 (dmu, dS)
-//   phase 3: the pair sweep of point i (L, dB-hat)
-// L, the row sums and the per-pseudo-input tables are read in the phase after the one that
-// writes them, so one copy of each suffices; the per-dimension constants, which point i-1's
-// finalisation still reads while point i's are formed, alternate between two slots.  The
-// psi1 part of a point's dmu, dS waits in shared memory (`carry`) for its finalisation.  The
-// arithmetic of every term is psi_bwd_kernel's.
-template <typename T>
-struct PSmem {
-  float2* tab;
-  T *z, *ell2, *lnl, *inv4l, *il, *misc;
-  T* pd;      // [2][5][QMAX]
-  T* pg;      // [2*DMAX] dm_all, dv of the current point
-  T* u;       // [M]
-  T* h;       // [M*Q]
-  T* G;       // [P]
-  T* Bs;      // [Dout*P]
-  T* L;       // [P]
-  T* rows;    // [M][1+QC]
-  T* dz;      // [M*Q] psi1 part of dZ
-  T* dzr;     // [M*Q] row-sum part of dZ
-  T* accB;    // [Dout*P]
-  T* carry;   // [2*QC] psi1 part of the previous point's dmu, dS
-  T* red;     // [32*RED]
-  int* pab;   // [P] the pairs (a << 16 | b), the same for every point
-};
-
-__host__ __device__ inline size_t pipe_smem_bytes(int M, int Q, int QC, int P, int D, size_t tsz) {
-  const size_t n = (size_t)M * Q + 4 * QMAX + 4 + 2 * 5 * QMAX + 2 * DMAX + M + (size_t)M * Q + P + (size_t)D * P + P +
-                   (size_t)M * (1 + QC) + 2 * (size_t)M * Q + (size_t)D * P + 2 * QC + 32 * RED;
-  return 256 * 8 + n * tsz + (size_t)P * sizeof(int);
-}
-
-template <typename T, int QC>
-__device__ PSmem<T> pcarve(char* base, int M, int Q, int P, int D) {
-  PSmem<T> s;
-  s.tab = reinterpret_cast<float2*>(base);
-  T* t = reinterpret_cast<T*>(base + 256 * sizeof(float2));
-  s.z = t; t += M * Q;
-  s.ell2 = t; t += QMAX;
-  s.lnl = t; t += QMAX;
-  s.inv4l = t; t += QMAX;
-  s.il = t; t += QMAX;
-  s.misc = t; t += 4;
-  s.pd = t; t += 2 * 5 * QMAX;
-  s.pg = t; t += 2 * DMAX;
-  s.u = t; t += M;
-  s.h = t; t += M * Q;
-  s.G = t; t += P;
-  s.Bs = t; t += D * P;
-  s.L = t; t += P;
-  s.rows = t; t += M * (1 + QC);
-  s.dz = t; t += M * Q;
-  s.dzr = t; t += M * Q;
-  s.accB = t; t += D * P;
-  s.carry = t; t += 2 * QC;
-  s.red = t; t += 32 * RED;
-  s.pab = reinterpret_cast<int*>(t);
-  return s;
-}
-
-template <typename T, int DB, int QC>
-__global__ void __launch_bounds__(nt_bwd(QC)) psi_bwd_pipe_kernel(PsiArgs<typename Num<T>::store_t> a) {
-  constexpr int NTB = nt_bwd(QC);
-  constexpr int Q = QC, D = DB;
-  constexpr int KV = 5 * QC + 1;   // [dmu, dS psi1 parts (2QC) | Rt, St (QC), Z2R (QC), ZS (QC)]
-  typedef typename Num<T>::store_t S;
-  static_assert(NTB >= 8 * 128, "the row phase takes 8 threads for each of up to 128 rows");
-  extern __shared__ __align__(16) char smem_raw[];
-  const int M = a.M;
-  const int P = M * (M + 1) / 2;
-  PSmem<T> s = pcarve<T, QC>(smem_raw, M, Q, P, D);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // ---- per-CTA tables (as psi_bwd_kernel)
-  load_exp_table(s.tab);
-  for (int i = tid; i < M * Q; i += NTB) {
-    s.z[i] = Num<T>::ld(a.Z[i]);
-    s.dz[i] = Num<T>::zero();
-    s.dzr[i] = Num<T>::zero();
-  }
-  for (int i = tid; i < D * P; i += NTB) s.accB[i] = Num<T>::zero();
-  __syncthreads();
-  if (tid < Q) {
-    const int q = tid;
-    T lnl = Num<T>::ld(static_cast<S>(a.lls2[q]));
-    T l2 = exp_tab(lnl, s.tab);
-    s.lnl[q] = lnl;
-    s.ell2[q] = l2;
-    s.il[q] = recip(l2);
-    s.inv4l[q] = recip(mul(l2, Num<T>::c(4.f)));
-  }
-  if (tid == 32) {
-    T lsf = Num<T>::ld(static_cast<S>(a.lsf2[0]));
-    s.misc[0] = lsf;
-    s.misc[1] = exp_tab(lsf, s.tab);
-  }
-  __syncthreads();
-  for (int p = tid; p < P; p += NTB) {
-    int ia, ib;
-    pair_of(p, ia, ib);
-    s.pab[p] = (ia << 16) | ib;
-    T g = Num<T>::zero();
-#pragma unroll
-    for (int q = 0; q < QC; ++q) {
-      T dd = sub(s.z[ia * Q + q], s.z[ib * Q + q]);
-      g = fma_(mul(dd, dd), s.inv4l[q], g);
-    }
-    s.G[p] = neg(g);
-  }
-  stage_sym_B<T, NTB>(s.Bs, a.B, M, D, P);
-  T g_sf = Num<T>::zero();
-  T g_l[QC], g_A[DB];
-#pragma unroll
-  for (int q = 0; q < QC; ++q) g_l[q] = Num<T>::zero();
-#pragma unroll
-  for (int d = 0; d < DB; ++d) g_A[d] = Num<T>::zero();
-  const T lsf = s.misc[0];
-  __syncthreads();
-
-  const int nbeg = (int)((long)a.N * blockIdx.x / gridDim.x);
-  const int nend = (int)((long)a.N * (blockIdx.x + 1) / gridDim.x);
-  const int cnt = nend - nbeg;
-  auto slot = [&](int i) {
-    T* pd = s.pd + (i & 1) * 5 * QMAX;
-    return PointSlot<T>{pd, pd + QMAX, pd + 2 * QMAX, pd + 3 * QMAX, pd + 4 * QMAX, s.u, s.h};
-  };
-  for (int i = 0; i <= cnt; ++i) {
-    const bool cur = i < cnt, prev = i > 0;
-    const int n = nbeg + i;
-    // ---- phase 1: row sums of the previous point | constants of this point.  Whole warps
-    // enter (the 8-lane sums below shuffle with a full mask); lanes of rows past M add nothing.
-    if (prev && warp < (8 * M + 31) / 32) {
-      const int ia = tid >> 3, sl = tid & 7;
-      const bool live = ia < M;
-      T R = Num<T>::zero(), R1 = Num<T>::zero(), Sq[QC], S1[QC];
-#pragma unroll
-      for (int q = 0; q < QC; ++q) Sq[q] = S1[q] = Num<T>::zero();
-      const int rowbase = ia * (ia + 1) / 2;
-      for (int ib = sl; live && ib < M; ib += 16) {
-        const int jb = ib + 8, jc = jb < M ? jb : ib;
-        const int p = ia >= ib ? rowbase + ib : ib * (ib + 1) / 2 + ia;
-        const int p1 = ia >= jc ? rowbase + jc : jc * (jc + 1) / 2 + ia;
-        const T l = s.L[GPK_IDX(p, P, 6)];
-        const T l1 = jb < M ? s.L[GPK_IDX(p1, P, 6)] : Num<T>::zero();
-        R = add(R, l);
-        R1 = add(R1, l1);
-#pragma unroll
-        for (int q = 0; q < QC; ++q) {
-          Sq[q] = fma_(l, s.z[ib * Q + q], Sq[q]);
-          S1[q] = fma_(l1, s.z[jc * Q + q], S1[q]);
-        }
-      }
-      R = add(R, R1);
-#pragma unroll
-      for (int q = 0; q < QC; ++q) Sq[q] = add(Sq[q], S1[q]);
-#pragma unroll
-      for (int m = 1; m < 8; m <<= 1) {
-        R = add(R, shfl_xor(R, m));
-#pragma unroll
-        for (int q = 0; q < QC; ++q) Sq[q] = add(Sq[q], shfl_xor(Sq[q], m));
-      }
-      if (live && sl == 0) {
-        T* row = s.rows + ia * (1 + QC);
-        row[0] = R;
-#pragma unroll
-        for (int q = 0; q < QC; ++q) row[1 + q] = Sq[q];
-      }
-    }
-    if (cur) {
-      const int t = tid - (NTB - 64);   // the last two warps (beside the row threads while 8 M <= NTB - 64)
-      if (t >= 0 && t < 4 * Q) dims_of<T, S>(a, s.ell2, s.lnl, s.tab, slot(i), n, t >> 2, t & 3);
-      const int g = tid - (NTB - 32);
-      if (g >= 0 && g < D) {
-        const T dvv = Num<T>::ld(a.dv[(size_t)n * D + g]);
-        const T mm = Num<T>::ld(a.m[(size_t)n * D + g]);
-        const T dmv = Num<T>::ld(a.dm[(size_t)n * D + g]);
-        s.pg[g] = sub(dmv, mul(scale2(dvv, 1), mm));   // dm_all
-        s.pg[DMAX + g] = dvv;
-      }
-    }
-    __syncthreads();
-    // ---- phase 2: psi1 terms of this point (warps 0..3) | dZ and totals of the previous (4..7)
-    T vals[KV];
-#pragma unroll
-    for (int k = 0; k < KV; ++k) vals[k] = Num<T>::zero();
-    if (cur && tid < M) {
-      const int ia0 = tid;
-      const PointSlot<T> ps = slot(i);
-      const T p1 = rows_of<T, QC>(s.z, lsf, s.tab, ps, Q, ia0);
-      T dp1 = Num<T>::zero();
-#pragma unroll
-      for (int d = 0; d < DB; ++d) {
-        dp1 = fma_(s.pg[d], Num<T>::ld(a.A[d * M + ia0]), dp1);
-        g_A[d] = fma_(s.pg[d], p1, g_A[d]);
-      }
-      const T L1 = mul(dp1, p1);
-      g_sf = add(g_sf, L1);
-#pragma unroll
-      for (int q = 0; q < QC; ++q) {
-        const T dd = sub(ps.pmu[q], s.z[ia0 * Q + q]);
-        const T ds = mul(dd, ps.pis1[q]);
-        const T ds2 = mul(ds, ds);
-        const T L1ds = mul(L1, ds);
-        vals[q] = neg(L1ds);                                            // dmu
-        vals[QC + q] = scale2(mul(L1, sub(ds2, ps.pis1[q])), -1);       // dS
-        s.dz[ia0 * Q + q] = add(s.dz[ia0 * Q + q], L1ds);               // dZ (psi1)
-        g_l[q] = add(g_l[q], mul(L1, add(sub(s.il[q], ps.pis1[q]), ds2)));
-      }
-    }
-    if (prev && tid >= 128 && tid < 128 + M) {
-      const int ia0 = tid - 128;
-      const PointSlot<T> ps = slot(i - 1);
-      const T* row = s.rows + ia0 * (1 + QC);
-      const T R = row[0];
-      vals[2 * QC] = R;
-#pragma unroll
-      for (int q = 0; q < QC; ++q) {
-        const T zq = s.z[ia0 * Q + q], il = s.il[q], cq = ps.pc[q], Sa = row[1 + q];
-        const T t = sub(add(neg(mul(zq, il)), scale2(mul(cq, ps.pmu[q]), 1)), mul(cq, zq));
-        s.dzr[ia0 * Q + q] = add(s.dzr[ia0 * Q + q], add(mul(R, t), mul(Sa, sub(il, cq))));
-        vals[2 * QC + 1 + q] = Sa;                       // St
-        vals[3 * QC + 1 + q] = mul(mul(zq, zq), R);      // Z2R
-        vals[4 * QC + 1 + q] = mul(zq, Sa);              // ZS
-      }
-    }
-    block_sum_many<T, KV>(vals, s.red, (128 + M + 31) >> 5);   // warps past the dZ threads hold zeros
-    if (warp == 0) {
-      if (prev) {   // finalise the previous point with its carried psi1 part
-        const int np = n - 1;
-        const PointSlot<T> ps = slot(i - 1);
-        const T Rt = vals[2 * QC];
-#pragma unroll
-        for (int q = 0; q < QC; ++q) {
-          if (q == lane) {
-            const T St = vals[2 * QC + 1 + q], Z2R = vals[3 * QC + 1 + q], ZS = vals[4 * QC + 1 + q];
-            const T mu = ps.pmu[q], cq = ps.pc[q], il = s.il[q];
-            const T e2 = add(sub(mul(mul(mu, mu), Rt), scale2(mul(mu, St), 1)), scale2(add(Z2R, ZS), -1));
-            const T dmu = add(s.carry[q], mul(scale2(cq, 1), sub(St, mul(mu, Rt))));
-            const T dS = add(s.carry[QC + q], add(neg(mul(cq, Rt)), scale2(mul(mul(cq, cq), e2), 1)));
-            const T t = add(add(scale2(mul(Rt, sub(il, cq)), -1), scale2(mul(sub(Z2R, ZS), mul(il, il)), -1)),
-                            mul(mul(cq, cq), e2));
-            g_l[q] = add(g_l[q], scale2(t, 1));
-            a.dmu[(size_t)np * Q + q] = Num<T>::st(dmu);
-            a.dvar[(size_t)np * Q + q] = Num<T>::st(dS);
-          }
-        }
-        if (lane == 0) g_sf = add(g_sf, scale2(Rt, 1));
-      }
-      __syncwarp();
-      if (cur && lane < 2 * QC) s.carry[lane] = vals[lane];   // this point's psi1 part, for its finalisation
-    }
-    // ---- phase 3: the pair sweep of this point (as psi_bwd_kernel's branch-free loop)
-    if (cur) {
-      T dvr[DB];
-#pragma unroll
-      for (int d = 0; d < DB; ++d) dvr[d] = s.pg[DMAX + d];
-      for (int p0 = tid; p0 < P; p0 += 2 * NTB) {
-        int pp[2], ia[2], ib[2];
-        bool ok[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          ok[u] = p0 + u * NTB < P;
-          pp[u] = ok[u] ? p0 + u * NTB : p0;
-          pp[u] = GPK_IDX(pp[u], P, 2);
-          const int ab = s.pab[pp[u]];
-          ia[u] = ab >> 16;
-          ib[u] = ab & 0xffff;
-        }
-        T arg[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const T* hh = s.h + ia[u] * QC;
-          T cr = mul(hh[0], s.z[ib[u] * QC]);   // = fma_ from zero, bit for bit
-#pragma unroll
-          for (int q = 1; q < QC; ++q) cr = fma_(hh[q], s.z[ib[u] * QC + q], cr);
-          arg[u] = sub(add(add(s.u[ia[u]], s.u[ib[u]]), s.G[pp[u]]), cr);
-        }
-        T ps2[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) ps2[u] = exp_pair(arg[u], s.tab);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          T ab[DB];
-#pragma unroll
-          for (int d = 0; d < DB; ++d) ab[d] = mul(dvr[d], ps2[u]);
-          // L = psi2 sum_d dv_d Bs_d: for one output (dv psi2) Bs, reusing the dB-hat term
-          T l;
-          if (DB == 1) {
-            l = mul(ab[0], s.Bs[pp[u]]);
-          } else {
-            T w = mul(dvr[0], s.Bs[pp[u]]);
-#pragma unroll
-            for (int d = 1; d < DB; ++d) w = fma_(dvr[d], s.Bs[d * P + pp[u]], w);
-            l = mul(w, ps2[u]);
-          }
-          if (ok[u]) {
-            s.L[pp[u]] = ia[u] == ib[u] ? l : scale2(l, -1);
-#pragma unroll
-            for (int d = 0; d < DB; ++d) s.accB[d * P + pp[u]] = add(s.accB[d * P + pp[u]], ab[d]);
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  // ---- flush into the partial block: [dB pairs D*P | dA D*M | dZ M*Q | dsf2 | dl Q]
-  double* const part = a.part + (size_t)blockIdx.x * a.part_stride;
-  for (int i = tid; i < D * P; i += NTB) part[i] = (double)Num<T>::st(s.accB[i]);
-  if (tid < M) {
-#pragma unroll
-    for (int d = 0; d < DB; ++d) part[D * P + d * M + tid] = a.dA ? (double)Num<T>::st(g_A[d]) : 0.0;
-  }
-  for (int i = tid; i < M * Q; i += NTB) part[D * P + D * M + i] = (double)Num<T>::st(add(s.dz[i], s.dzr[i]));
-  T fin[1 + QC];
-  fin[0] = g_sf;
-#pragma unroll
-  for (int q = 0; q < QC; ++q) fin[1 + q] = g_l[q];
-  __syncthreads();
-  block_sum<T, 1 + QC>(fin, s.red);
-  if (tid == 0) {
-    part[D * P + D * M + M * Q] = (double)Num<T>::st(div(fin[0], s.misc[1]));
-#pragma unroll
-    for (int q = 0; q < QC; ++q) part[D * P + D * M + M * Q + 1 + q] = (double)Num<T>::st(mul(fin[1 + q], sqrt_(s.ell2[q])));
-  }
 }
 
 // the destinations of the backward's partial block (layout in PsiArgs::part)
@@ -1403,78 +1256,76 @@ gpk::RedPlan bwd_plan(const PsiArgs<S>& a) {
   return r;
 }
 
-template <typename T, int NPB, int DB, int QC>
-int run_bwd(const PsiArgs<typename Num<T>::store_t>& a, size_t sm, cudaStream_t st) {
-  auto k = psi_bwd_kernel<T, NPB, DB, QC>;
+template <typename T, int DB, int QC, int NS, int NB, int NF>
+int run_bwd(const PsiArgs<typename Num<T>::store_t>& a, const BLayout& lo, size_t sm, cudaStream_t st) {
+  auto k = psi_bwd_kernel<T, DB, QC, NS, NB, NF>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  int grid = gpk::sm_count();
+  int grid = gpk::sm_count() * (NS < 12 ? 2 : 1);
   if (grid > a.N) grid = a.N;
   if (grid < 1) return GPK_OK;
-  k<<<grid, nt_bwd(QC), sm, st>>>(a);
+  k<<<grid, (NS + NB + NF) * 32, sm, st>>>(a, lo);
   int rc = gpk::check_launch("psi_bwd");
   if (rc != GPK_OK || !a.part) return rc;
   return gpk::reduce_partials(a.part, grid, bwd_plan(a), st);
 }
 
-template <typename T, int DB>
-int run_bwd_pipe(const PsiArgs<typename Num<T>::store_t>& a, size_t sm, cudaStream_t st) {
-  auto k = psi_bwd_pipe_kernel<T, DB, 2>;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  int grid = gpk::sm_count();
-  if (grid > a.N) grid = a.N;
-  if (grid < 1) return GPK_OK;
-  k<<<grid, nt_bwd(2), sm, st>>>(a);
-  int rc = gpk::check_launch("psi_bwd_pipe");
-  if (rc != GPK_OK) return rc;
-  return gpk::reduce_partials(a.part, grid, bwd_plan(a), st);
+template <typename T, int QC, int NS, int NB, int NF>
+int bwd_db(const PsiArgs<typename Num<T>::store_t>& a, const BLayout& lo, size_t sm, cudaStream_t st) {
+  if (a.Dout == 1) return run_bwd<T, 1, QC, NS, NB, NF>(a, lo, sm, st);
+  if (a.Dout == 2) return run_bwd<T, 2, QC, NS, NB, NF>(a, lo, sm, st);
+  return run_bwd<T, 4, QC, NS, NB, NF>(a, lo, sm, st);
 }
 
-template <typename T, int NPB, int QC>
-int bwd_db(const PsiArgs<typename Num<T>::store_t>& a, size_t sm, cudaStream_t st) {
-  if (a.Dout == 1) return run_bwd<T, NPB, 1, QC>(a, sm, st);
-  if (a.Dout == 2) return run_bwd<T, NPB, 2, QC>(a, sm, st);
-  return run_bwd<T, NPB, 4, QC>(a, sm, st);
+// the warp split: 12 + 4 + 4 with one CTA an SM (128 rows at a time), 6 + 2 + 2 with two
+template <typename T, bool TWO>
+int bwd_qc(const PsiArgs<typename Num<T>::store_t>& a, int QC, const BLayout& lo, size_t sm, cudaStream_t st) {
+  constexpr int NS = TWO ? 6 : 12, NR = TWO ? 2 : 4;
+  if (QC == 2) return bwd_db<T, 2, NS, NR, NR>(a, lo, sm, st);
+  if (QC == 5) return bwd_db<T, 5, NS, NR, NR>(a, lo, sm, st);
+  return bwd_db<T, QMAX, NS, NR, NR>(a, lo, sm, st);
 }
 
-// points per pass: BWD_NPB when their tables fit in shared memory and the per-point sums
-// (NPB (5 Q + 1) values) fit one reduction; else one
-#ifndef GPK_BWD_NPB
-#define GPK_BWD_NPB 1
-#endif
-constexpr int BWD_NPB = GPK_BWD_NPB;
 template <typename T>
-int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) {
-  PsiArgs<typename Num<T>::store_t> a = a_in;
-  const int P = a.M * (a.M + 1) / 2;
-  if (a.M > nt_bwd(QMAX)) return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d > %d", a.M, nt_bwd(QMAX));
-  if (5 * (a.Q <= 2 ? 2 : QMAX) + 1 > RED) return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: Q=%d too large", a.Q);
-  const size_t cap = 227 * 1024;
-  // the pipelined kernel: Q == 2, Dout <= 2, the fixed-order path, B in shared memory
-  if (a.Q == 2 && a.Dout <= 2 && a.part && !a.b_stride && !a.dpsi1 && a.A && a.m && a.dm && a.M <= 128) {
-    const size_t sm = pipe_smem_bytes(a.M, 2, 2, P, a.Dout, sizeof(T));
-    if (sm <= cap) return a.Dout == 1 ? run_bwd_pipe<T, 1>(a, sm, st) : run_bwd_pipe<T, 2>(a, sm, st);
+int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
+  const int M = a.M, P = M * (M + 1) / 2;
+  if (M > 512) return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d > %d", M, 512);
+  const size_t cap = SMEM_CAP;
+  // accepted sizes: two pair tables and the point's tables within shared memory
+  const size_t need = 2048 + ((size_t)M * a.Q + 84 + (size_t)M * (1 + a.Q) + 2 * (size_t)P + (size_t)M * 9 +
+                              (size_t)M * a.Q + 1536) * sizeof(T);
+  if (need > 227 * 1024) return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d needs too much shared memory", M);
+  const int QC = a.Q <= 2 ? 2 : (a.Q == 5 ? 5 : QMAX);   // 5: the psi-statistics workload's width, exact
+  const int nbs = a.b_stride == 0 ? a.Dout * P : 0, nacc = a.dB ? a.Dout * P : 0;
+  auto bytes = [&](const BLayout& lo, int nb) { return bcarve<T>(nullptr, nullptr, M, QC, P, a.Dout, nb, lo); };
+  auto segs = [&](int threads) { return threads / M > 8 ? 8 : (threads / M < 1 ? 1 : threads / M); };
+  // two CTAs of ten warps an SM where everything fits twice (M <= ~60 in double-float precision):
+  // the phases of one then overlap the other's
+  {
+    const BLayout lo{segs(256), P, nbs, nacc, M <= 255};
+    const size_t sm = bytes(lo, 2);
+    if (lo.pab && sm <= (cap - 2048) / 2) return bwd_qc<T, true>(a, QC, lo, sm, st);
   }
-  const int nbs = a.b_stride == 0 ? a.Dout * P : 0, nacc = a.Dout * P;
-  for (int npb = (a.Q <= 2 ? BWD_NPB : 1); npb >= 1; --npb) {
-    // preference: B and the dBhat accumulators both in shared memory, then without B, then
-    // without either (dBhat then accumulates with atomics in global memory)
-    const int opts[3][2] = {{nbs, nacc}, {0, nacc}, {0, 0}};
-    for (int o = 0; o < 3; ++o) {
-      size_t sm = bwd_smem_bytes(a.M, a.Q, P, opts[o][1], npb, sizeof(T), opts[o][0]);
-      if (sm > cap) continue;
-      a.bs_smem = opts[o][0] > 0;
-      a.accb_smem = opts[o][1] > 0;
-      // the pair table only where it fits on top of this option (it never displaces B or the
-      // dB-hat accumulators)
-      a.pab_smem = sm + (size_t)P * sizeof(int) <= cap;
-      if (a.pab_smem) sm += (size_t)P * sizeof(int);
-      if (npb == 2) return bwd_db<T, 2, 2>(a, sm, st);
-      if (a.Q <= 2) return bwd_db<T, 1, 2>(a, sm, st);
-      if (a.Q == 5) return bwd_db<T, 1, 5>(a, sm, st);   // the psi-statistics workload's width, exact
-      return bwd_db<T, 1, QMAX>(a, sm, st);
+  // preference: G, B, the dBhat accumulators and the pair table in shared memory; without the pair
+  // table; then without G (a few operations per dimension and pair), without B (two loads and
+  // conversions), without both, and without the accumulators (dBhat then accumulates in the
+  // partial block, or with atomics).  Four row segments instead of five where that makes room.
+  const int opts[6][3] = {{P, nbs, nacc}, {0, nbs, nacc}, {P, 0, nacc}, {0, 0, nacc}, {P, 0, 0}, {0, 0, 0}};
+  const int smax = segs(512);
+  for (int o = 0; o < 6; ++o) {
+    for (int pab = M <= 255; pab >= 0; --pab) {
+      for (int seg = smax; seg >= (smax > 4 ? 4 : smax); --seg) {
+        const BLayout lo{seg, opts[o][0], opts[o][1], opts[o][2], pab};
+        const size_t sm = bytes(lo, 4);
+        if (sm <= cap) return bwd_qc<T, false>(a, QC, lo, sm, st);
+      }
     }
   }
-  return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d needs too much shared memory", a.M);
+  for (int seg = smax; seg >= 1; --seg) {   // the largest M accepted
+    const BLayout lo{seg, 0, 0, 0, 0};
+    const size_t sm = bytes(lo, 4);
+    if (sm <= cap) return bwd_qc<T, false>(a, QC, lo, sm, st);
+  }
+  return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d needs too much shared memory", M);
 }
 
 }  // namespace psi_impl

@@ -1,0 +1,128 @@
+"""The psi statistics at the edges of their kernels' ranges: ragged sizes around the row, pair and
+shared-memory limits of the backward's layouts, every input width, and points whose exponents lie
+outside the fixed-point range of the double-float pair sweep (they take its general form)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import geepee_np as O
+from tests._helpers import assert_close
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-9   # double-float sums (~48 bits) of a few thousand terms against float64
+
+
+def dev(a, dtype=torch.float64):
+    return torch.as_tensor(np.asarray(a, dtype=np.float64), device='cuda').to(dtype).contiguous()
+
+
+def z(*s):
+    return torch.zeros(s, dtype=torch.float64, device='cuda')
+
+
+@pytest.mark.parametrize('M,Q,Dout,N,fixed', [
+    (2, 1, 1, 5, True), (13, 2, 3, 9, True), (59, 2, 1, 400, True), (64, 3, 2, 33, True), (65, 4, 1, 35, True),
+    (70, 5, 2, 21, False), (104, 2, 1, 170, True), (110, 2, 1, 20, True), (100, 5, 1, 20, True), (96, 6, 1, 11, True),
+    (129, 2, 1, 9, True), (129, 7, 1, 5, False), (150, 1, 2, 7, True), (155, 2, 1, 6, False), (31, 8, 4, 40, True)])
+def test_psi_layer_edge_sizes(M, Q, Dout, N, fixed):
+    """Forward moments and every backward output against the oracle, with the fixed-order sums
+    (twice, bit for bit) or the atomic ones."""
+    from geepee_gb300 import gpk, workloads as W
+    wl = W.psi_workload(seed=3 * M + Q, N=N, Q=Q, M=M, Dout=Dout)
+    lls2, lsf2 = 2 * wl['ls'], 2 * wl['sf'] + 0.1
+    p1, p2 = O.psi_stats(lls2, lsf2, wl['mu'], wl['S'], wl['Z'])
+    A, B, sf2 = wl['Ahat'], wl['Bhat'], float(np.exp(lsf2[0]))
+    m_ref = p1 @ A.T
+    v_ref = sf2 + np.einsum('dab,nab->nd', B, p2) - m_ref ** 2
+    dm, dv = wl['dm'], wl['dv']
+    dm_all = dm - 2 * dv * m_ref
+    r = O.psi_derivatives(dm_all @ A, p1, np.einsum('nd,dab->nab', dv, B), p2, np.exp(wl['ls']), sf2,
+                          wl['mu'], wl['S'], wl['Z'])
+    t = {k: dev(wl[k]) for k in ('mu', 'S', 'Z')}
+    l2, s2, At, Bt = dev(lls2), dev(lsf2), dev(A), dev(B)
+    m, v = z(N, Dout), z(N, Dout)
+    gpk.psi_fwd(t['mu'], t['S'], t['Z'], l2, s2, At, Bt, m_out=m, v_out=v)
+    assert_close(m.cpu().numpy(), m_ref, TOL, 'm')
+    assert_close(v.cpu().numpy(), v_ref, TOL, 'v')
+    work = z(gpk.work_elems(gpk.OP_PSI_BWD, N, M, Q, Dout)) if fixed else None
+    outs = []
+    for _ in range(2):
+        out = dict(dsf2=z(1), dl=z(Q), dZ=z(M, Q), dA=z(Dout, M), dB=z(Dout, M, M), dmu=z(N, Q), dS=z(N, Q))
+        gpk.psi_bwd(t['mu'], t['S'], t['Z'], l2, s2, At, Bt, dev(m_ref), dev(dm), dev(dv), out['dsf2'], out['dl'],
+                    out['dZ'], out['dA'], out['dB'], out['dmu'], out['dS'], work=work)
+        outs.append(out)
+    for name, val in zip(('dsf2', 'dl', 'dZ', 'dmu', 'dS'), r):
+        assert_close(outs[0][name].cpu().numpy(), val, TOL, name)
+    assert_close(outs[0]['dA'].cpu().numpy(), dm_all.T @ p1, TOL, 'dA')
+    assert_close(outs[0]['dB'].cpu().numpy(), np.einsum('nd,nab->dab', dv, p2), TOL, 'dB')
+    if fixed:
+        for name in outs[0]:
+            assert torch.equal(outs[0][name], outs[1][name]), name + ' differs between calls'
+
+
+@pytest.mark.parametrize('kind', ['far', 'negative_variance', 'large_sf', 'mixed'])
+@pytest.mark.parametrize('Q', [2, 5])
+def test_psi_outside_fixed_point_range(kind, Q):
+    """Far points (every psi2 zero), slightly negative variances and a kernel variance near the
+    float range, alone and beside ordinary points, forward and backward."""
+    from geepee_gb300 import gpk, workloads as W
+    N, M, Dout = 23, 37, 1
+    wl = W.psi_workload(seed=11 + Q, N=N, Q=Q, M=M, Dout=Dout)
+    lls2, lsf2 = 2 * wl['ls'], np.array([0.3])
+    mu, S = wl['mu'].copy(), wl['S'].copy()
+    if kind in ('far', 'mixed'):
+        mu[5] = 40.0
+        mu[6, 0] = -1e4
+        S[6] = 1e-6
+        mu[9] *= 8.0
+    if kind in ('negative_variance', 'mixed'):
+        S[::4] = -0.05 * np.exp(lls2)
+        S[7] = 0.0
+    if kind == 'large_sf':
+        lsf2 = np.array([43.85])   # psi2 up to e^87.7, within the float range; k_n above 126
+    p1, p2 = O.psi_stats(lls2, lsf2, mu, S, wl['Z'])
+    psi1, psi2 = z(N, M), z(N, M, M)
+    t = dict(mu=dev(mu), S=dev(S), Z=dev(wl['Z']))
+    l2, s2 = dev(lls2), dev(lsf2)
+    gpk.psi_fwd(t['mu'], t['S'], t['Z'], l2, s2, psi1=psi1, psi2=psi2)
+    # results below e^-87 may be flushed to zero
+    floor = 2e-38
+    np.testing.assert_allclose(psi2.cpu().numpy(), p2, rtol=1e-10, atol=floor)
+    np.testing.assert_allclose(psi1.cpu().numpy(), p1, rtol=1e-10, atol=floor)
+    if kind == 'large_sf':
+        return   # sums of such terms leave the float range
+    A, B, sf2 = wl['Ahat'], wl['Bhat'], float(np.exp(lsf2[0]))
+    m_ref = p1 @ A.T
+    m, v = z(N, Dout), z(N, Dout)
+    gpk.psi_fwd(t['mu'], t['S'], t['Z'], l2, s2, dev(A), dev(B), m_out=m, v_out=v)
+    assert_close(m.cpu().numpy(), m_ref, TOL, 'm')
+    assert_close(v.cpu().numpy(), sf2 + np.einsum('dab,nab->nd', B, p2) - m_ref ** 2, TOL, 'v')
+    dm, dv = wl['dm'], wl['dv']
+    dm_all = dm - 2 * dv * m_ref
+    r = O.psi_derivatives(dm_all @ A, p1, np.einsum('nd,dab->nab', dv, B), p2, np.exp(wl['ls']), sf2, mu, S, wl['Z'])
+    out = dict(dsf2=z(1), dl=z(Q), dZ=z(M, Q), dA=z(Dout, M), dB=z(Dout, M, M), dmu=z(N, Q), dS=z(N, Q))
+    gpk.psi_bwd(t['mu'], t['S'], t['Z'], l2, s2, dev(A), dev(B), dev(m_ref), dev(dm), dev(dv), out['dsf2'],
+                out['dl'], out['dZ'], out['dA'], out['dB'], out['dmu'], out['dS'],
+                work=z(gpk.work_elems(gpk.OP_PSI_BWD, N, M, Q, Dout)))
+    for name, val in zip(('dsf2', 'dl', 'dZ', 'dmu', 'dS'), r):
+        assert_close(out[name].cpu().numpy(), val, TOL, name)
+
+
+def test_psi_nan_stays_with_its_point():
+    """A point with a NaN moment gives NaN there and leaves the others of its pass unchanged."""
+    from geepee_gb300 import gpk, workloads as W
+    N, M, Q = 9, 20, 2
+    wl = W.psi_workload(seed=4, N=N, Q=Q, M=M, Dout=1)
+    mu = wl['mu'].copy()
+    mu[2, 1] = np.nan
+    res = []
+    for x in (wl['mu'], mu):
+        m, v = z(N, 1), z(N, 1)
+        gpk.psi_fwd(dev(x), dev(wl['S']), dev(wl['Z']), dev(2 * wl['ls']), dev(2 * wl['sf']), dev(wl['Ahat']),
+                    dev(wl['Bhat']), m_out=m, v_out=v)
+        res.append((m.cpu().numpy(), v.cpu().numpy()))
+    ok = np.arange(N) != 2
+    assert np.isnan(res[1][0][2]) and np.isnan(res[1][1][2])
+    for a, b in zip(*res):
+        assert_close(b[ok], a[ok], 1e-12)
