@@ -110,11 +110,28 @@ long trace_kzz_work_elems(int M, int Q);
 
 // Pair p of the row-major lower triangle, p = a (a + 1) / 2 + b with 0 <= b <= a.
 __host__ __device__ __forceinline__ void tri_pair(int p, int& a, int& b) {
+#ifdef __CUDA_ARCH__
+  float q;   // (the hardware root: within a few ulp, which the two corrections below absorb)
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(q) : "f"(8.f * (float)p + 1.f));
+  int r = (int)((q - 1.f) * 0.5f);
+#else
   int r = (int)((sqrtf(8.f * (float)p + 1.f) - 1.f) * 0.5f);
+#endif
   if ((r + 1) * (r + 2) / 2 <= p) ++r;
   if (r * (r + 1) / 2 > p) --r;
   a = r;
   b = p - r * (r + 1) / 2;
+}
+
+// One 8- or 4-byte element from global to shared memory, asynchronously (cp.async.wait_all follows)
+template <typename S>
+__device__ __forceinline__ void async_copy(S* dst, const S* src) {
+  static_assert(sizeof(S) == 8 || sizeof(S) == 4, "8- or 4-byte elements");
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if (sizeof(S) == 8)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 
 // Copies n storage-type elements (8 or 4 bytes) from global memory into shared memory with

@@ -259,6 +259,7 @@ constexpr long long kFxHalf = 1LL << 40;
 __device__ __forceinline__ void load_exp2_table(float2* s_tab) {
   const float c_hi[8] = {0.000000000e+00f, 3.385080490e-04f, 6.771307089e-04f, 1.015867922e-03f, 1.354719861e-03f, 1.693686470e-03f, 2.032767981e-03f, 2.371964045e-03f};
   const float c_lo[8] = {0.000000000e+00f, 3.656181261e-12f, -1.587024435e-11f, 3.841724161e-11f, 3.069764928e-11f, 5.799375910e-11f, -7.369679866e-11f, 2.371333858e-11f};
+#pragma unroll 1
   for (int k = threadIdx.x; k < kFxTab; k += blockDim.x) {
     const int i = k & 7;
     const float2 t = kExp2Tab[k >> 3];
@@ -276,10 +277,12 @@ __device__ __forceinline__ void load_exp2_table(float2* s_tab) {
     s_tab[k] = make_float2(r.hi, r.lo);
   }
 }
-__device__ __forceinline__ df64 exp2_fx(long long x, const float2* tab) {
+// 2^(x's fraction) as h + l, h in (0.999, 2); tab: the table's shared-memory address
+__device__ __forceinline__ df64 exp2_fx_frac(long long x, unsigned tab) {
   const unsigned xl = (unsigned)x;
   const int xh = (int)(x >> 32);
-  const float2 T = tab[(xh >> 9) & (kFxTab - 1)];
+  float2 T;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(T.x), "=f"(T.y) : "r"(tab + ((xh >> 6) & ((kFxTab - 1) << 3))));
   // the 41 remainder bits as two floats, by exponent splicing: 23 bits of [1, 2), then 18
   const float f = __uint_as_float(0x3f800000u | (__funnelshift_l(xl, (unsigned)xh, 14) & 0x7fffffu));
   const float g = __uint_as_float(0x4b000000u | (xl & 0x3ffffu));   // 2^23 + the low 18 bits
@@ -297,15 +300,62 @@ __device__ __forceinline__ df64 exp2_fx(long long x, const float2* tab) {
   l = __fadd_rn(l, __fmaf_rn(T.y, p, T.y));
   const float h = __fadd_rn(T.x, w);
   l = __fadd_rn(l, __fsub_rn(w, __fsub_rn(h, T.x)));
+  return make_df(h, l);
+}
+__device__ __forceinline__ df64 exp2_fx(long long x, unsigned tab) {
+  const df64 r = exp2_fx_frac(x, tab);
+  const int xh = (int)(x >> 32);
   const float s = xh >= -(126 << 20) ? __int_as_float(((xh << 3) & 0xff800000) + 0x3f800000) : 0.f;
-  return make_df(__fmul_rn(h, s), __fmul_rn(l, s));
+  return make_df(__fmul_rn(r.hi, s), __fmul_rn(r.lo, s));
 }
-// round(v 2^e) of a double-float (|v 2^e| < 2^62)
-__device__ __forceinline__ long long fx_of(df64 v, float two_e) {
-  return __float2ll_rn(__fmul_rn(v.hi, two_e)) + __float2ll_rn(__fmul_rn(v.lo, two_e));
+// the same as a float64, by integer operations: h's bits widened, l added in units of h's last
+// float64 place (below 1 the unit halves; h = 1 with a negative l counts as below)
+__device__ __forceinline__ double exp2_fx_double(long long x, unsigned tab) {
+  const df64 r = exp2_fx_frac(x, tab);
+  const int xh = (int)(x >> 32);
+  const bool below = r.hi < 1.f || (r.hi == 1.f && r.lo < 0.f);
+  const int li = __float2int_rn(__fmul_rn(r.lo, below ? 9007199254740992.f : 4503599627370496.f));
+  const unsigned hb = __float_as_uint(r.hi);
+  long long d = ((long long)hb << 29) + ((896LL + (xh >> 20)) << 52) + li;
+  return __longlong_as_double(xh >= -(126 << 20) ? d : 0LL);
 }
+// x 2^F truncated to an integer (|x 2^F| < 2^63, the exponent field at most 189 - F), by shifting
+// the significand: the float-to-64-bit-integer conversion issues on the FP64 pipe, 16 cycles a warp
+template <int F>
+__device__ __forceinline__ long long fx_bits(float x) {
+  const unsigned b = __float_as_uint(x);
+  const int s = min(189 - F - (int)((b >> 23) & 0xffu), 63);
+  const long long v = (long long)(((unsigned long long)(((b & 0x7fffffu) | 0x800000u) << 7) << 32) >> s);
+  return (int)b < 0 ? -v : v;
+}
+// a double-float in units of 2^-52 (|v| < 1024)
+__device__ __forceinline__ long long fx52_of(df64 v) { return fx_bits<52>(v.hi) + fx_bits<52>(v.lo); }
+// a double-float (|v| < 16) as two words, high 2^-26 + low 2^-57 with |low| <= 2^30
+__device__ __forceinline__ long long fx57_words_of(df64 v) {
+  const long long t = fx_bits<57>(v.hi) + fx_bits<57>(v.lo) + (1LL << 30);
+  const int high = (int)(t >> 31), low = (int)((unsigned)t & 0x7fffffffu) - (1 << 30);
+  return ((long long)high << 32) | (unsigned)low;
+}
+// hi + lo as a float64 by integer operations (df_to_double's three FP64-pipe instructions take 48
+// cycles a warp): hi's bits widened, lo added in units of hi's last float64 place (half of it
+// below a power of two).  Values whose words leave the normal range take the FP64 path.
+__device__ __forceinline__ double df_to_double_int(df64 a) {
+  const unsigned hb = __float_as_uint(a.hi), lb = __float_as_uint(a.lo);
+  const int he = (int)((hb >> 23) & 0xffu), le = (int)((lb >> 23) & 0xffu);
+  const bool against = (int)(hb ^ lb) < 0;                          // lo takes away from |hi|
+  const int k = 127 + 52 + (((hb & 0x7fffffu) == 0u && against) ? 1 : 0) - he;   // lo 2^k: exponent field le + k
+  if (he == 0 || he == 255 || (le == 0 && (lb << 1) != 0u) || le + k > 158) return df_to_double(a);
+  const int li = le == 0 || le + k < 1 ? 0 : __float2int_rn(__uint_as_float((lb & 0x7fffffu) | ((unsigned)(le + k) << 23)));
+  const long long mag = ((long long)(hb & 0x7fffffffu) << 29) + (896LL << 52) + (against ? -li : li);
+  return __longlong_as_double(mag | ((long long)(hb & 0x80000000u) << 32));
+}
+
 // log2(e) in the precision of the argument
 __device__ __forceinline__ df64 log2e_of(df64) { return make_df(1.442695022e+00f, 1.925963034e-08f); }
+
+// the storage value of a compute value by integer operations (see df_to_double_int)
+__device__ __forceinline__ double st_int(df64 a) { return df_to_double_int(a); }
+__device__ __forceinline__ double st_int(float a) { return (double)a; }
 
 // log by one Newton step on exp: y1 = y0 + x exp(-y0) - 1
 template <typename Tab>

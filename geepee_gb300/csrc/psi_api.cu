@@ -1,12 +1,39 @@
 // C ABI of the psi-statistics kernels (see psi_impl.cuh for the algorithm).
 #include "psi_impl.cuh"
 
-int psi_fwd_df64(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
+int psi_fwd_df64_q2(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
+int psi_fwd_df64_q5(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
+int psi_fwd_df64_q8(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
 int psi_bwd_df64(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
-int psi_fwd_f32(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
+int psi_fwd_f32_q2(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
+int psi_fwd_f32_q5(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
+int psi_fwd_f32_q8(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
 int psi_bwd_f32(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
 using psi_impl::QMAX;
 using psi_impl::DMAX;
+
+// five input dimensions (the psi-statistics workload's width) have kernels of their own for the
+// plain forms; other forms and widths take the catch-all ones
+static int psi_fwd_df64(const psi_impl::PsiArgs<double>& a, cudaStream_t st) {
+  const int rc = psi_impl::check_fwd(a);
+  if (rc != GPK_OK) return rc;
+  if (a.Q <= 2) return psi_fwd_df64_q2(a, st);
+  if (a.Q == 5) {
+    const int r5 = psi_fwd_df64_q5(a, st);
+    if (r5 != GPK_EUNSUPPORTED) return r5;
+  }
+  return psi_fwd_df64_q8(a, st);
+}
+static int psi_fwd_f32(const psi_impl::PsiArgs<float>& a, cudaStream_t st) {
+  const int rc = psi_impl::check_fwd(a);
+  if (rc != GPK_OK) return rc;
+  if (a.Q <= 2) return psi_fwd_f32_q2(a, st);
+  if (a.Q == 5) {
+    const int r5 = psi_fwd_f32_q5(a, st);
+    if (r5 != GPK_EUNSUPPORTED) return r5;
+  }
+  return psi_fwd_f32_q8(a, st);
+}
 
 template <typename S>
 static psi_impl::PsiArgs<S> make_args(int N, int M, int Q, int Dout, const void* mu, const void* var, const void* Z,

@@ -81,6 +81,39 @@ struct PsiArgs {
 
 __device__ __forceinline__ void pair_of(int p, int& a, int& b) { tri_pair(p, a, b); }
 
+// The pair loops address shared memory by 32-bit addresses: through the table pointers every access
+// cost a 64-bit address computation (two integer instructions each).
+typedef unsigned saddr;
+__device__ __forceinline__ saddr sm_addr(const void* p) { return (saddr)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ int2 lds_i2(saddr a) {
+  int2 v;
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void lds(saddr a, long long& v) { asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(saddr a, df64& v) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.hi), "=f"(v.lo) : "r"(a));
+}
+__device__ __forceinline__ void lds(saddr a, float& v) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
+__device__ __forceinline__ void lds_st(saddr a, double& v) { asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
+__device__ __forceinline__ void lds_st(saddr a, float& v) { lds(a, v); }
+__device__ __forceinline__ int lds_u16(saddr a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts(saddr a, df64 v) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.hi), "f"(v.lo) : "memory");
+}
+__device__ __forceinline__ void sts(saddr a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts(saddr a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
+template <typename V>
+__device__ __forceinline__ V ldsv(saddr a) {
+  V v;
+  lds(a, v);
+  return v;
+}
+
 // How a precision keeps the pair exponent's terms (log2 units): R a table element, arg() the
 // exponent of a pair from the two records and G, ev() its exponential.
 template <typename T>
@@ -95,41 +128,37 @@ struct PairExp<float> {
   static __device__ __forceinline__ R t_of(float x) { return x; }
   static __device__ __forceinline__ R g_of(float x) { return x; }
   template <int QC>
-  static __device__ __forceinline__ R arg(const R* a, const R* b, R g) {
-    R x = (a[0] + b[0]) + g;
+  static __device__ __forceinline__ R arg(saddr a, saddr b, R g) {
+    R x = (ldsv<R>(a) + ldsv<R>(b)) + g;
 #pragma unroll
-    for (int q = 1; q <= QC; ++q) x = __fmaf_rn(-a[q], b[q], x);
+    for (int q = 1; q <= QC; ++q) x = __fmaf_rn(-ldsv<R>(a + 4 * q), ldsv<R>(b + 4 * q), x);
     return x;
   }
-  static __device__ __forceinline__ float ev(R x, const float2*) {
+  static __device__ __forceinline__ float ev(R x, saddr) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
   }
+  static __device__ __forceinline__ float ev_st(R x, saddr tab) { return ev(x, tab); }
 };
 
-// double-float: u and G in units of 2^-52, t in units of 2^-58 as a balanced pair (high word the
-// nearest multiple of 2^32, low word signed), so that t_a t_b in units of 2^-52 is the product of
-// the high words plus the upper half of the two mixed products.  |t| < 16 (see above) bounds the
-// high words by 2^30 and a mixed sum over three dimensions by 2^63.
+// double-float: u and G in units of 2^-52; t as two words, t = high 2^-26 + low 2^-57 (|low| <= 2^30),
+// so that t_a t_b in units of 2^-52 is the product of the high words plus the mixed products
+// shifted by 31.  sum_q t_q^2 < 254 (see above) bounds the high words by 2^30 and a mixed sum over
+// eight dimensions by 2^62.5.
 template <>
 struct PairExp<df64> {
   typedef long long R;
   static constexpr int TAB = kFxTab;
-  static __device__ __forceinline__ R u_of(df64 x) { return fx_of(x, 4503599627370496.f); }
-  static __device__ __forceinline__ R t_of(df64 x) {
-    const long long t = fx_of(x, 288230376151711744.f);
-    return ((t + 0x80000000LL) & ~0xffffffffLL) | (t & 0xffffffffLL);
-  }
+  static __device__ __forceinline__ R u_of(df64 x) { return fx52_of(x); }
+  static __device__ __forceinline__ R t_of(df64 x) { return fx57_words_of(x); }
   // below -1024 every pair's psi2 is zero already (the other terms sum to less than 127); the
   // half step of exp2_fx enters here
   static __device__ __forceinline__ R g_of(df64 x) {
-    return (x.hi > -1024.f ? fx_of(x, 4503599627370496.f) : -(1024LL << 52)) + kFxHalf;
+    return (x.hi > -1024.f ? fx52_of(x) : -(1024LL << 52)) + kFxHalf;
   }
   // a record whose pairs are all zero: u + u_b + G < -126 for every live b (u_b <= 63.5), and no
   // sum leaves the range of +-2048
-  // a t as its two words (low, high), one 8-byte access
-  static __device__ __forceinline__ int2 ld2(const R* p) { return *reinterpret_cast<const int2*>(p); }
   // a b + c of 32-bit factors in one instruction (from C, the compiler widened the factors to 64
   // bits first: three multiply-adds and two shifts a product)
   static __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
@@ -139,27 +168,26 @@ struct PairExp<df64> {
   }
   static __device__ __forceinline__ R dead_u() { return -(400LL << 52); }
   template <int QC>
-  static __device__ __forceinline__ R arg(const R* a, const R* b, R g) {
-    long long x = a[0] + b[0] + g;
+  static __device__ __forceinline__ R arg(saddr a, saddr b, R g) {
+    long long x = ldsv<R>(a) + ldsv<R>(b) + g;
+    long long mid = 0;
+    int2 ta[QC], tb[QC];
 #pragma unroll
-    for (int q0 = 1; q0 <= QC; q0 += 3) {
-      long long mid = 0;
-      int2 ta[3], tb[3];
-#pragma unroll
-      for (int u = 0; u < 3 && q0 + u <= QC; ++u) {
-        ta[u] = ld2(a + q0 + u);
-        tb[u] = ld2(b + q0 + u);
-        mid = mad_wide(ta[u].y, tb[u].x, mid);
-        mid = mad_wide(ta[u].x, tb[u].y, mid);
-      }
-      long long hi = (int)(mid >> 32);
-#pragma unroll
-      for (int u = 0; u < 3 && q0 + u <= QC; ++u) hi = mad_wide(ta[u].y, tb[u].y, hi);
-      x -= hi;
+    for (int q = 0; q < QC; ++q) {
+      ta[q] = lds_i2(a + 8 * (1 + q));   // (low, high) words of t
+      tb[q] = lds_i2(b + 8 * (1 + q));
+      mid = mad_wide(ta[q].y, tb[q].x, mid);
+      mid = mad_wide(ta[q].x, tb[q].y, mid);
     }
+    long long hi = mid >> 31;
+#pragma unroll
+    for (int q = 0; q < QC; ++q) hi = mad_wide(ta[q].y, tb[q].y, hi);
+    x -= hi;
     return x;
   }
-  static __device__ __forceinline__ df64 ev(R x, const float2* tab) { return exp2_fx(x, tab); }
+  static __device__ __forceinline__ df64 ev(R x, saddr tab) { return exp2_fx(x, tab); }
+  // the same as a float64
+  static __device__ __forceinline__ double ev_st(R x, saddr tab) { return exp2_fx_double(x, tab); }
 };
 
 // the 256-entry exp table of exp_tab inside the kernels' shared table (every 8th entry)
@@ -174,10 +202,10 @@ __device__ __forceinline__ void load_pair_table(float2* tab) {
 __host__ __device__ inline size_t pair_table_bytes(size_t tsz) { return tsz == 8 ? kFxTab * sizeof(float2) : 0; }
 
 // The symmetrised weights of the packed pairs, Bs[d P + p] = B_d[a,b] + B_d[b,a] (a != b) or
-// B_d[a,a] (half: (B_d[a,b] + B_d[b,a]) / 2 off the diagonal): each thread keeps eight pairs' global loads in flight before converting them, so
+// B_d[a,a]: each thread keeps eight pairs' global loads in flight before converting them, so
 // the table costs a few memory latencies per CTA instead of one per pair.
 template <typename T, int NTH>
-__device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int D, int P, bool half = false) {
+__device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int D, int P) {
   typedef typename Num<T>::store_t S;
   constexpr int K = 8;
   for (int d = 0; d < D; ++d) {
@@ -199,10 +227,7 @@ __device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int
         const int p = p0 + k * NTH;
         if (p < P) {
           T w = Num<T>::ld(x1[k]);
-          if (off[k]) {
-            w = add(w, Num<T>::ld(x2[k]));
-            if (half) w = scale2(w, -1);
-          }
+          if (off[k]) w = add(w, Num<T>::ld(x2[k]));
           Bs[d * P + p] = w;
         }
       }
@@ -287,7 +312,7 @@ __device__ __forceinline__ void dims_of(const PsiArgs<S>& a, const T* ell2, cons
 
 // The record of one pseudo-input at one point in fixed point: a dead record (zero for every
 // pair) where k_n - sum_q t_q^2 < -127.5.  *flag is set where the fixed-point range does not hold
-// and the whole pass takes psi2_general: non-finite terms, k_n above 126, or l + 2S < l (a
+// and the point takes psi2_general: non-finite terms, k_n above 126, or l + 2S < l (a
 // negative variance; the rounding of a zero one is tolerated), for which the bound on t fails.
 template <int QC>
 __device__ __forceinline__ void put_rec(long long* r, df64 k2, df64 s2, const df64* t, float ld2, int* flag) {
@@ -328,6 +353,51 @@ __device__ __forceinline__ T rows_of(const T* z, T lsf, const Tab& tab, const Po
   return exp_tab(e1, tab);
 }
 
+// the per-point constants beside the arrays: log sf2 + sum pld1, k_n / 2 (log2 units), max pld2
+constexpr int PDN = PD * QMAX + 4;
+// point n's constants by one warp (4 Q <= 32 lanes), *flag cleared
+template <typename T, typename S, typename Tab>
+__device__ __forceinline__ void consts_of(const PsiArgs<S>& a, const T* ell2, const T* lnl, const Tab& tab, T lsf,
+                                          const PointSlot<T>& ps, int n, int Q, int lane, int* flag) {
+  T* pd = ps.pmu;
+  if (lane < 4 * Q) dims_of<T, S>(a, ell2, lnl, tab, ps, n, lane >> 2, lane & 3);
+  __syncwarp();
+  if (lane == 0) {
+    T c1 = lsf;
+    for (int q = 0; q < Q; ++q) c1 = add(c1, ps.pld1[q]);
+    pd[PD * QMAX] = c1;
+  } else if (lane == 1) {
+    T k = lsf;
+    float ld2 = -1e30f;
+    for (int q = 0; q < Q; ++q) {
+      k = add(k, scale2(ps.pld2[q], -1));
+      ld2 = fmax_nan(ld2, Num<T>::approx(ps.pld2[q]));
+    }
+    pd[PD * QMAX + 1] = mul(k, log2e_of(k));
+    pd[PD * QMAX + 2] = Num<T>::c(ld2);
+  } else if (lane == 2) {
+    *flag = 0;
+  }
+}
+// pseudo-input ia's record at the point, and its psi1 (z: its coordinates)
+template <typename T, int QC, typename Tab>
+__device__ __forceinline__ T row_of(const T* z, const Tab& tab, const PointSlot<T>& ps, int Q, int ia, int* flag) {
+  const T* pd = ps.pmu;
+  T e1 = pd[PD * QMAX], s2 = Num<T>::zero(), t[QC];
+#pragma unroll
+  for (int q = 0; q < QC; ++q) {
+    t[q] = Num<T>::zero();
+    if (q < Q) {
+      const T d = sub(ps.pmu[q], z[q]);
+      e1 = fma_(mul(d, d), scale2(neg(ps.pis1[q]), -1), e1);
+      t[q] = mul(d, ps.psq[q]);
+      s2 = fma_(t[q], t[q], s2);
+    }
+  }
+  put_rec<QC>(ps.rec + ia * rec_len(QC), pd[PD * QMAX + 1], s2, t, Num<T>::approx(pd[PD * QMAX + 2]), flag);
+  return exp_tab(e1, tab);
+}
+
 // psi2 of one pair outside the fixed-point range, from the point's constants and the two
 // pseudo-inputs (df64 only; rare, so out of line)
 template <typename T>
@@ -342,14 +412,125 @@ __device__ __noinline__ T psi2_general(const T* za, const T* zb, const T* pd, co
   return exp_pair(x, ExpTab{tab});
 }
 
+// a running sum kept as (hi, lo) without renormalising: for sums of a few dozen terms (the low
+// word's own rounding stays below the normalised sum's)
+__device__ __forceinline__ void acc_add(df64& a, df64 x) {
+  const df64 s = two_sum(a.hi, x.hi);
+  a.hi = s.hi;
+  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, x.lo));
+}
+__device__ __forceinline__ void acc_fma(df64& a, df64 x, df64 y) {
+  const float p = __fmul_rn(x.hi, y.hi);
+  float e = __fmaf_rn(x.hi, y.hi, -p);
+  e = __fmaf_rn(x.hi, y.lo, e);
+  e = __fmaf_rn(x.lo, y.hi, e);
+  const df64 s = two_sum(a.hi, p);
+  a.hi = s.hi;
+  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, e));
+}
+__device__ __forceinline__ df64 acc_done(df64 a) { return quick_two_sum(a.hi, a.lo); }
+__device__ __forceinline__ void acc_add(float& a, float x) { a += x; }
+__device__ __forceinline__ void acc_fma(float& a, float x, float y) { a = __fmaf_rn(x, y, a); }
+__device__ __forceinline__ float acc_done(float a) { return a; }
+
+// barrier ID over NW warps of the CTA
+template <int ID, int NW>
+__device__ __forceinline__ void warps_sync() {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(NW * 32) : "memory");
+}
+__host__ __device__ constexpr int zlen(int QC) { return (QC + 1) & ~1; }   // a z row, padded to pairs
+// G_ab (log2 units) of a pair from the pseudo-inputs
+template <typename T, int QC>
+__device__ __forceinline__ typename PairExp<T>::R pair_G(const T* za, const T* zb, const T* inv4l, int Q) {
+  T g = Num<T>::zero();
+#pragma unroll
+  for (int q = 0; q < QC; ++q) {
+    if (q < Q) {
+      const T d = sub(za[q], zb[q]);
+      g = fma_(mul(d, d), inv4l[q], g);
+    }
+  }
+  return PairExp<T>::g_of(neg(mul(g, log2e_of(g))));
+}
+
+// The per-CTA pair tables by NW warps (the CTA's first): the pair table, G (where wanted) and the
+// symmetrised weights Bs[d P + p] = B_d[a,b] + B_d[b,a] (half of that with `half`), B_d[a,a] on the
+// diagonal.  B is read along its rows by asynchronous copies, the triangle at and below the
+// diagonal into Bs, the one above into `tmp` ([P], e.g. G before it is formed), and converted
+// from there; reading each pair's two entries together took a 32-byte sector per transposed entry
+// (36 MB of L2 reads over 152 CTAs at M = 100).  The loops are kept rolled: this code runs
+// once per CTA, and unrolled its instruction fetches took longer than its work.
+template <typename T, int QC, int NW, int BAR>
+__device__ __forceinline__ void stage_pairs(const T* z, const T* inv4l, int Q, int M, int P, int D,
+                                         const typename Num<T>::store_t* B, bool half, unsigned short* pab,
+                                         typename PairExp<T>::R* G, T* Bs, T* tmp) {
+  typedef typename Num<T>::store_t S;
+  constexpr int ZL = zlen(QC), NTH = NW * 32;
+  const int tid = threadIdx.x;
+  for (int d = 0; Bs && d < D; ++d, B += (size_t)M * M, Bs += P) {
+#pragma unroll 1
+    for (int p = tid; p < P; p += NTH) {
+      int ia, ib;
+      pair_of(p, ia, ib);
+      if (pab && d == 0) pab[p] = (unsigned short)((ia << 8) | ib);
+      const int ja = M - 1 - ib, jb = M - 1 - ia;   // row jb, column ja >= jb: consecutive threads descend
+      async_copy(reinterpret_cast<S*>(Bs) + p, B + ia * M + ib);
+      async_copy(reinterpret_cast<S*>(tmp) + ja * (ja + 1) / 2 + jb, B + jb * M + ja);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    warps_sync<BAR, NW>();
+#pragma unroll 1
+    for (int p = tid; p < P; p += NTH) {
+      bool off;
+      if (pab) {
+        off = (pab[p] >> 8) != (pab[p] & 0xff);
+      } else {
+        int ia, ib;
+        pair_of(p, ia, ib);
+        off = ia != ib;
+      }
+      T w = Num<T>::ld(reinterpret_cast<const S*>(Bs)[p]);
+      if (off) {
+        w = add(w, Num<T>::ld(reinterpret_cast<const S*>(tmp)[p]));
+        if (half) w = scale2(w, -1);
+      }
+      Bs[p] = w;
+    }
+    warps_sync<BAR, NW>();
+  }
+  const bool have = Bs && pab;
+#pragma unroll 1
+  for (int p = tid; p < P && (G || !have); p += NTH) {
+    int ia, ib;
+    if (have) {
+      const int ab = pab[p];
+      ia = ab >> 8;
+      ib = ab & 0xff;
+    } else {
+      pair_of(p, ia, ib);
+      if (pab) pab[p] = (unsigned short)((ia << 8) | ib);
+    }
+    if (G) G[p] = pair_G<T, QC>(z + ia * ZL, z + ib * ZL, inv4l, Q);
+  }
+}
+
+// two consecutive elements in one access
+__device__ __forceinline__ void lds_two(saddr p, df64& a, df64& b) {
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.hi), "=f"(a.lo), "=f"(b.hi), "=f"(b.lo) : "r"(p));
+}
+__device__ __forceinline__ void lds_two(saddr p, float& a, float& b) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(p));
+}
+
 // ---------------------------------------------------------------------------------
-// Forward, NPB points per pass.  Per pass: the NPB points' per-dimension constants (threads
-// over (point, q)), then their per-pseudo-input terms (threads over (point, a)), then the pair
-// sweep, in which each thread loads a pair's point-independent data once (G_ab, z_b, the
-// symmetrised B weights) and evaluates psi2 for all NPB points - NPB independent exp chains
-// per pair - and finally one CTA reduction for the NPB points' m and v.  PPT > 0 keeps
-// sum_n psi2 of each thread's pairs in registers (pairs tid + k*NT); PPT == 0 sweeps any number
-// of pairs.  The pass count, barriers and reductions per point are 1/NPB of a per-point sweep.
+// Forward, general form (sum_n psi2, rollouts, psi2 together with moments, sizes whose tables do not
+// fit): NPB points per pass.  Per pass: the NPB points' per-dimension constants (threads over
+// (point, q)), then their per-pseudo-input terms (threads over (point, a)), then the pair
+// sweep, in which each thread loads a pair's point-independent data once (G_ab, the symmetrised B
+// weights) and evaluates psi2 for all NPB points, and finally one CTA reduction for the NPB
+// points' m and v.  PPT > 0 keeps sum_n psi2 of each thread's pairs in registers (pairs
+// tid + k*NT); PPT == 0 sweeps any number of pairs.
 template <typename T>
 struct FSmem {
   float2* tab;
@@ -395,22 +576,8 @@ __device__ FSmem<T> fcarve(char* base, int M, int Q, int D, int npb, int ng, int
   return s;
 }
 
-// G_ab (log2 units) of a pair from the pseudo-inputs
-template <typename T, int QC>
-__device__ __forceinline__ typename PairExp<T>::R pair_G(const T* za, const T* zb, const T* inv4l, int Q) {
-  T g = Num<T>::zero();
-#pragma unroll
-  for (int q = 0; q < QC; ++q) {
-    if (q < Q) {
-      const T d = sub(za[q], zb[q]);
-      g = fma_(mul(d, d), inv4l[q], g);
-    }
-  }
-  return PairExp<T>::g_of(neg(mul(g, log2e_of(g))));
-}
-
 template <typename T, int NPB, int PPT, int QC, int DB>
-__global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::store_t> a) {
+__global__ void __launch_bounds__(NT) psi_fwd_gen_kernel(PsiArgs<typename Num<T>::store_t> a) {
   typedef typename Num<T>::store_t S;
   typedef PairExp<T> X;
   typedef typename X::R R;
@@ -420,7 +587,7 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
   const int P = M * (M + 1) / 2;
   const bool contract = (a.A != nullptr) && (a.B != nullptr) && (a.m_out != nullptr || a.v_out != nullptr);
   FSmem<T> s = fcarve<T, QC>(smem_raw, M, Q, contract ? D : 0, NPB, a.g_smem ? P : 0, a.bs_smem ? D * P : 0);
-  __shared__ int s_flag;   // the pass holds a point outside the fixed-point range
+  __shared__ int s_flag[NPB];   // a point of the pass lies outside the fixed-point range
   const ExpTab etab{s.tab};
   // ---- per-CTA tables: exp table, Z, lengthscales, sf2, A, G_ab and the symmetrised B
   load_pair_table<T>(s.tab);
@@ -470,7 +637,7 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
     const int npts = min(NPB, nend - n0);
     auto slot = [&](int pt) { return PointSlot<T>(s.pd + pt * PD * QMAX, s.rec + pt * M * RL); };
     // ---- per-dimension constants of the NPB points
-    if (threadIdx.x == 0) s_flag = 0;
+    if (threadIdx.x < NPB) s_flag[threadIdx.x] = 0;
     for (int t = threadIdx.x; t < 4 * npts * Q; t += NT) {
       const int part = t & 3, pq = t >> 2, pt = pq / Q, q = pq - pt * Q;
       dims_of<T, S>(a, s.ell2, s.lnl, etab, slot(pt), n0 + pt, q, part);
@@ -479,12 +646,11 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
     // ---- per-pseudo-input terms (and psi1)
     for (int t = threadIdx.x; t < npts * M; t += NT) {
       const int pt = t / M, ia = t - pt * M;
-      const T v1 = rows_of<T, QC>(s.z, lsf, etab, slot(pt), Q, ia, &s_flag);
+      const T v1 = rows_of<T, QC>(s.z, lsf, etab, slot(pt), Q, ia, &s_flag[pt]);
       s.p1[pt * M + ia] = v1;
       if (a.psi1) a.psi1[(size_t)(n0 + pt) * M + ia] = Num<T>::st(v1);
     }
     __syncthreads();
-    const bool general = X::TAB && s_flag;
     // ---- pairs
     T vacc[NPB][DB];
 #pragma unroll
@@ -513,8 +679,8 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
       for (int pt = 0; pt < NPB; ++pt) {
         if (pt < npts) {
           const R* rec = s.rec + pt * M * RL;
-          const T ps = general ? psi2_general(s.z + ia * Q, s.z + ib * Q, s.pd + pt * PD * QMAX, s.inv4l, lsf, Q, s.tab)
-                               : X::ev(X::template arg<QC>(rec + ia * RL, rec + ib * RL, gab), s.tab);
+          const T ps = X::TAB && s_flag[pt] ? psi2_general(s.z + ia * Q, s.z + ib * Q, s.pd + pt * PD * QMAX, s.inv4l, lsf, Q, s.tab)
+                               : X::ev(X::template arg<QC>(sm_addr(rec + ia * RL), sm_addr(rec + ib * RL), gab), sm_addr(s.tab));
           if (a.psi2) {
             const S v = Num<T>::st(ps);
             const size_t o = (size_t)(n0 + pt) * M;
@@ -530,34 +696,7 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
         }
       }
     };
-    // the common configuration (m and v only, Dout == DB, B and G in shared memory): the same
-    // sums without branches, so the NPB points' exps interleave.  In a pass with fewer than NPB
-    // points the extra slots run on stale tables; their sums are never read.
-    auto do_pair_fast = [&](int p, int ia, int ib) {
-      p = GPK_IDX(p, P, 3);
-      const R gab = s.G[p];
-      T w[DB];
-#pragma unroll
-      for (int d = 0; d < DB; ++d) w[d] = s.Bs[d * P + p];
-      const R *ra = s.rec + ia * RL, *rb = s.rec + ib * RL;
-      R arg[NPB];
-#pragma unroll
-      for (int pt = 0; pt < NPB; ++pt) arg[pt] = X::template arg<QC>(ra + pt * M * RL, rb + pt * M * RL, gab);
-#pragma unroll
-      for (int pt = 0; pt < NPB; ++pt) {
-        const T ps = X::ev(arg[pt], s.tab);
-#pragma unroll
-        for (int d = 0; d < DB; ++d) vacc[pt][d] = fma_(w[d], ps, vacc[pt][d]);
-      }
-    };
-    const bool fast = PPT == 0 && contract && !a.psi2 && D == DB && s.Bs && s.G && !general;
-    if (fast) {
-      for (int p = threadIdx.x; p < P; p += NT) {
-        int ia, ib;
-        pair_of(p, ia, ib);
-        do_pair_fast(p, ia, ib);
-      }
-    } else if (PPT > 0) {
+    if (PPT > 0) {
 #pragma unroll
       for (int k = 0; k < KP; ++k) {
         const int p = threadIdx.x + k * NT;
@@ -645,7 +784,6 @@ __global__ void __launch_bounds__(NT) psi_fwd_kernel(PsiArgs<typename Num<T>::st
 // slots, the small per-point arrays between three.
 // dZ's row sums in the back threads' registers: one row a thread, and room for them
 __host__ __device__ constexpr bool bwd_dz_reg(int QC, int M, int nb) { return QC < QMAX && M <= nb * 32; }
-__host__ __device__ constexpr int zlen(int QC) { return (QC + 1) & ~1; }   // a z row, padded to pairs
 template <typename T>
 struct BSmem {
   typedef typename PairExp<T>::R R;
@@ -671,9 +809,6 @@ struct BSmem {
   T* accB;   // [Dout*P] or nullptr: sum over the CTA's points of dv psi2 (dBhat)
   unsigned short* pab;  // [P] or nullptr: the pairs (a << 8 | b)
 };
-// the per-point constants: PD arrays of QMAX, then log sf2 + sum pld1, k_n / 2, max pld2
-constexpr int PDN = PD * QMAX + 4;
-
 struct BLayout {
   int seg, ng, nbs, nacc, pab;   // row segments, elements of G, B, dB-hat; pair table or not
 };
@@ -715,45 +850,6 @@ __host__ __device__ inline size_t bcarve(BSmem<T>* out, char* base, int M, int Q
   return o;
 }
 
-// a running sum kept as (hi, lo) without renormalising: for sums of a few dozen terms (the low
-// word's own rounding stays below the normalised sum's)
-__device__ __forceinline__ void acc_add(df64& a, df64 x) {
-  const df64 s = two_sum(a.hi, x.hi);
-  a.hi = s.hi;
-  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, x.lo));
-}
-__device__ __forceinline__ void acc_fma(df64& a, df64 x, df64 y) {
-  const float p = __fmul_rn(x.hi, y.hi);
-  float e = __fmaf_rn(x.hi, y.hi, -p);
-  e = __fmaf_rn(x.hi, y.lo, e);
-  e = __fmaf_rn(x.lo, y.hi, e);
-  const df64 s = two_sum(a.hi, p);
-  a.hi = s.hi;
-  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, e));
-}
-__device__ __forceinline__ df64 acc_done(df64 a) { return quick_two_sum(a.hi, a.lo); }
-__device__ __forceinline__ void acc_add(float& a, float x) { a += x; }
-__device__ __forceinline__ void acc_fma(float& a, float x, float y) { a = __fmaf_rn(x, y, a); }
-__device__ __forceinline__ float acc_done(float a) { return a; }
-
-// barrier ID over NW warps of the CTA
-template <int ID, int NW>
-__device__ __forceinline__ void warps_sync() {
-  __syncwarp();
-  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(NW * 32) : "memory");
-}
-// two consecutive elements in one access
-__device__ __forceinline__ void ld_two(const df64* p, df64& a, df64& b) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  a = make_df(v.x, v.y);
-  b = make_df(v.z, v.w);
-}
-__device__ __forceinline__ void ld_two(const float* p, float& a, float& b) {
-  const float2 v = *reinterpret_cast<const float2*>(p);
-  a = v.x;
-  b = v.y;
-}
-
 template <typename T, int DB, int QC, int NS, int NB, int NF>
 __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
     psi_bwd_kernel(PsiArgs<typename Num<T>::store_t> a, BLayout lo) {
@@ -772,6 +868,7 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
   const bool back_warp = tid >= NTS && tid < NTS + NB * 32, front_warp = tid >= NTS + NB * 32;
   // ---- per-CTA tables: exp table, Z, A, lengthscales, sf2
   load_pair_table<T>(s.tab);
+#pragma unroll 1
   for (int i = tid; i < M * ZL; i += NTH) {
     const int ia = i / ZL, q = i - ia * ZL;
     s.z[i] = q < Q ? Num<T>::ld(a.Z[ia * Q + q]) : Num<T>::zero();
@@ -779,6 +876,7 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
   const bool dz_reg = bwd_dz_reg(QC, M, NB);
   if (!dz_reg)
     for (int i = tid; i < M * QC; i += NTH) s.dz[i] = Num<T>::zero();
+#pragma unroll 1
   for (int i = tid; i < D * M; i += NTH) {
     s.As[i] = a.dpsi1 ? Num<T>::zero() : Num<T>::ld(a.A[i]);
     s.gA[i] = Num<T>::zero();
@@ -809,28 +907,10 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
   auto front = [&](int i) {
     const int rt = tid - (NTS + NB * 32), rw = rt >> 5;
     const int n = nbeg + i, sl = i % 3;
-    T* pd = s.pd + sl * PDN;
-    const PointSlot<T> ps(pd, s.rec + (size_t)(i & 1) * M * RL);
+    const PointSlot<T> ps(s.pd + sl * PDN, s.rec + (size_t)(i & 1) * M * RL);
     T* pg = s.pg + sl * 2 * DMAX;
     if (rw == 0) {
-      if (lane < 4 * Q) dims_of<T, S>(a, s.ell2, s.lnl, etab, ps, n, lane >> 2, lane & 3);
-      __syncwarp();
-      if (lane == 0) {
-        T c1 = lsf;
-        for (int q = 0; q < Q; ++q) c1 = add(c1, ps.pld1[q]);
-        pd[PD * QMAX] = c1;
-      } else if (lane == 1) {
-        T k = lsf;
-        float ld2 = -1e30f;
-        for (int q = 0; q < Q; ++q) {
-          k = add(k, scale2(ps.pld2[q], -1));
-          ld2 = fmax_nan(ld2, Num<T>::approx(ps.pld2[q]));
-        }
-        pd[PD * QMAX + 1] = mul(k, log2e_of(k));
-        pd[PD * QMAX + 2] = Num<T>::c(ld2);
-      } else if (lane == 2) {
-        s_flag[sl] = 0;
-      }
+      consts_of<T, S>(a, s.ell2, s.lnl, etab, lsf, ps, n, Q, lane, &s_flag[sl]);
     } else if (rw == 1 && lane < D) {
       const T dvv = a.b_stride ? Num<T>::c(1.f) : Num<T>::ld(a.dv[(size_t)n * D + lane]);
       if (!a.dpsi1) {
@@ -841,22 +921,8 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
       pg[DMAX + lane] = dvv;
     }
     warps_sync<2, NF>();
-    const T k2 = pd[PD * QMAX + 1];
-    const float ld2 = Num<T>::approx(pd[PD * QMAX + 2]);
     for (int ia = rt; ia < M; ia += NF * 32) {
-      T e1 = pd[PD * QMAX], s2 = Num<T>::zero(), t[QC];
-#pragma unroll
-      for (int q = 0; q < QC; ++q) {
-        t[q] = Num<T>::zero();
-        if (q < Q) {
-          const T d = sub(ps.pmu[q], s.z[ia * ZL + q]);
-          e1 = fma_(mul(d, d), scale2(neg(ps.pis1[q]), -1), e1);
-          t[q] = mul(d, ps.psq[q]);
-          s2 = fma_(t[q], t[q], s2);
-        }
-      }
-      put_rec<QC>(ps.rec + ia * RL, k2, s2, t, ld2, &s_flag[sl]);
-      const T p1 = exp_tab(e1, etab);
+      const T p1 = row_of<T, QC>(s.z + ia * ZL, etab, ps, Q, ia, &s_flag[sl]);
       T dp1 = Num<T>::zero();
       if (a.dpsi1) {
         dp1 = Num<T>::ld(a.dpsi1[(size_t)n * M + ia]);
@@ -956,14 +1022,9 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
     if (cnt > 0) front(0);
   } else {
     constexpr int NTA = NTS + NB * 32;
-    for (int p = tid; p < P; p += NTA) {
-      int ia, ib;
-      pair_of(p, ia, ib);
-      if (s.pab) s.pab[p] = (unsigned short)((ia << 8) | ib);
-      if (s.G) s.G[p] = pair_G<T, QC>(s.z + ia * ZL, s.z + ib * ZL, s.inv4l, Q);
-    }
-    if (s.Bs) stage_sym_B<T, NTA>(s.Bs, a.B, M, D, P, true);
+    stage_pairs<T, QC, NS + NB, 3>(s.z, s.inv4l, Q, M, P, D, a.B, true, s.pab, s.G, s.Bs, s.L);
     if (s.accB)
+#pragma unroll 1
       for (int i = tid; i < D * P; i += NTA) s.accB[i] = Num<T>::zero();
     else if (part && a.dB)   // dBhat accumulates in this CTA's partial block (each pair has one owner)
       for (int i = tid; i < D * P; i += NTA) part[i] = 0.0;
@@ -985,23 +1046,22 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
       if (D == DB && s.Bs && s.accB && s.G && s.pab && !general) {
         // the common configuration, branch-free: two pairs (p, p + NTS) per iteration, each step
         // written for both, so that their dependent chains interleave
+        constexpr int E = sizeof(T);
+        const saddr ar = sm_addr(rec), aG = sm_addr(s.G), aB = sm_addr(s.Bs), aL = sm_addr(s.L), aC = sm_addr(s.accB),
+                    ap = sm_addr(s.pab), at = sm_addr(s.tab);
         for (int p0 = tid; p0 < P; p0 += 2 * NTS) {
-          int pp[2], ia[2], ib[2];
-          bool ok[2];
+          saddr o[2];   // the pairs' byte offsets
+          R arg[2];
+          const bool two = p0 + NTS < P;
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            ok[u] = p0 + u * NTS < P;
-            pp[u] = GPK_IDX(ok[u] ? p0 + u * NTS : p0, P, 2);
-            const int ab = s.pab[pp[u]];
-            ia[u] = ab >> 8;
-            ib[u] = ab & 0xff;
+            const int p = GPK_IDX(u && two ? p0 + NTS : p0, P, 2), ab = lds_u16(ap + 2 * p);
+            o[u] = p * E;
+            arg[u] = X::template arg<QC>(ar + (ab >> 8) * (RL * E), ar + (ab & 0xff) * (RL * E), ldsv<R>(aG + o[u]));
           }
-          R arg[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) arg[u] = X::template arg<QC>(rec + ia[u] * RL, rec + ib[u] * RL, s.G[pp[u]]);
           T ps2[2];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) ps2[u] = X::ev(arg[u], s.tab);
+          for (int u = 0; u < 2; ++u) ps2[u] = X::ev(arg[u], at);
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             T ab[DB];
@@ -1009,17 +1069,18 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
             for (int d = 0; d < DB; ++d) ab[d] = mul(dvr[d], ps2[u]);
             T l;
             if (DB == 1) {   // (dv psi2) B, reusing the dB-hat term
-              l = mul(ab[0], s.Bs[pp[u]]);
+              l = mul(ab[0], ldsv<T>(aB + o[u]));
             } else {
-              T w = mul(dvr[0], s.Bs[pp[u]]);
+              T w = mul(dvr[0], ldsv<T>(aB + o[u]));
 #pragma unroll
-              for (int d = 1; d < DB; ++d) w = fma_(dvr[d], s.Bs[d * P + pp[u]], w);
+              for (int d = 1; d < DB; ++d) w = fma_(dvr[d], ldsv<T>(aB + d * P * E + o[u]), w);
               l = mul(w, ps2[u]);
             }
-            if (ok[u]) {
-              s.L[pp[u]] = l;
+            if (u == 0 || two) {
+              sts(aL + o[u], l);
 #pragma unroll
-              for (int d = 0; d < DB; ++d) s.accB[d * P + pp[u]] = add(s.accB[d * P + pp[u]], ab[d]);
+              for (int d = 0; d < DB; ++d)
+                sts(aC + d * P * E + o[u], add(ldsv<T>(aC + d * P * E + o[u]), ab[d]));
             }
           }
         }
@@ -1032,7 +1093,7 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
             ps2 = psi2_general(s.z + ia * ZL, s.z + ib * ZL, s.pd + sl * PDN, s.inv4l, lsf, Q, s.tab);
           } else {
             const R gab = s.G ? s.G[p] : pair_G<T, QC>(s.z + ia * ZL, s.z + ib * ZL, s.inv4l, Q);
-            ps2 = X::ev(X::template arg<QC>(rec + ia * RL, rec + ib * RL, gab), s.tab);
+            ps2 = X::ev(X::template arg<QC>(sm_addr(rec + ia * RL), sm_addr(rec + ib * RL), gab), sm_addr(s.tab));
           }
           T w = Num<T>::zero();
 #pragma unroll
@@ -1076,24 +1137,25 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
       for (int t = tid; t < lo.seg * M; t += NTS + NB * 32) {
         const int g = t / M, ia = t - g * M;
         const int b0 = g * W, b1 = min(M, b0 + W);
-        const T* l = s.L + (ia >= b0 ? ia * (ia + 1) / 2 + b0 : b0 * (b0 + 1) / 2 + ia);
-        const T* zb = s.z + b0 * ZL;
+        constexpr int E = sizeof(T);
+        saddr l = sm_addr(s.L) + (ia >= b0 ? ia * (ia + 1) / 2 + b0 : b0 * (b0 + 1) / 2 + ia) * E;
+        saddr zb = sm_addr(s.z) + b0 * (ZL * E);
         T Rs = Num<T>::zero(), Sq[ZL];
 #pragma unroll
         for (int q = 0; q < ZL; ++q) Sq[q] = Num<T>::zero();
 #pragma unroll 4
         for (int b = b0; b < b1; ++b) {
-          const T lv = *l;
-          l += b < ia ? 1 : b + 1;   // the next column of this row in the packed triangle
+          const T lv = ldsv<T>(l);
+          l += b < ia ? E : (b + 1) * E;   // the next column of this row in the packed triangle
           acc_add(Rs, lv);
 #pragma unroll
           for (int q = 0; q < ZL; q += 2) {
             T z0, z1;
-            ld_two(zb + q, z0, z1);
+            lds_two(zb + q * E, z0, z1);
             acc_fma(Sq[q], lv, z0);
             if (q + 1 < QC) acc_fma(Sq[q + 1], lv, z1);
           }
-          zb += ZL;
+          zb += ZL * E;
         }
         T* o = s.rows + (size_t)g * (1 + QC) * M + ia;
         o[0] = acc_done(Rs);
@@ -1116,11 +1178,14 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
   if (part) {
     const bool wantA = a.dA && !a.dpsi1;
     if (s.accB)
-      for (int i = tid; i < D * P; i += NTH) part[i] = (double)Num<T>::st(s.accB[i]);
-    for (int i = tid; i < D * M; i += NTH) part[D * P + i] = wantA ? (double)Num<T>::st(s.gA[i]) : 0.0;
+#pragma unroll 1
+      for (int i = tid; i < D * P; i += NTH) part[i] = st_int(s.accB[i]);
+#pragma unroll 1
+    for (int i = tid; i < D * M; i += NTH) part[D * P + i] = wantA ? st_int(s.gA[i]) : 0.0;
+#pragma unroll 1
     for (int i = tid; i < M * Q; i += NTH) {
       const int ia = i / Q, q = i - ia * Q;
-      part[D * P + D * M + i] = (double)Num<T>::st(dzo[q * M + ia]);
+      part[D * P + D * M + i] = st_int(dzo[q * M + ia]);
     }
   } else {
     if (a.dB && s.accB) {
@@ -1176,14 +1241,428 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
   }
 }
 
+// ---------------------------------------------------------------------------------
+// Forward moments (m, v and optionally psi1), NPB points per pass, split by warps like the backward:
+// NS sweep warps take the pairs of pass i (each thread a pair for all NPB points, G and B loaded
+// once) while NF front warps form the constants, psi1, m and the records of pass i + 1 and finish
+// pass i - 1's v from the sweep warps' sums: one CTA barrier a pass.  Measured (df64), general form
+// of the same sweep -> this: N = 10000, Q = 5, M = 100: 366 -> 285 us (64% of issue slots; 143
+// instructions a pair and point); N = 1000, Q = 2: 50 -> 41 us, of which ~18 us are the per-CTA
+// tables; N = 4999, Q = 2, M = 50, two outputs: 85 -> 62 us.
+template <typename T>
+struct MSmem {
+  typedef typename PairExp<T>::R R;
+  float2* tab;
+  T* z;      // [M][zlen]
+  T* ell2;   // [QMAX]
+  T* lnl;    // [QMAX]
+  T* inv4l;  // [QMAX]
+  T* misc;   // [4] log sf2, sf2
+  T* pd;     // [2][NPB][PDN] per-point constants
+  T* As;     // [Dout][M]
+  T* p1;     // [NPB][M]
+  T* ms;     // [3][NPB][DMAX] m of three passes
+  T* red;    // [2][NS][NPB*DB]
+  R* rec;    // [2][NPB][M][rec_len]
+  R* G;      // [P]
+  T* Bs;     // [Dout*P]
+  unsigned short* pab;   // [P] or nullptr
+};
+template <typename T>
+__host__ __device__ inline size_t mcarve(MSmem<T>* out, char* base, int M, int QC, int P, int D, int npb, int ns,
+                                         int db, int pab) {
+  typedef typename PairExp<T>::R R;
+  MSmem<T> s;
+  size_t o = 0;
+  auto take = [&](size_t n) {
+    char* p = base + o;
+    o += n;
+    return p;
+  };
+  const size_t e = sizeof(T);
+  s.tab = (float2*)take(PairExp<T>::TAB * sizeof(float2));
+  s.z = (T*)take((size_t)zlen(QC) * M * e);
+  s.ell2 = (T*)take(QMAX * e);
+  s.lnl = (T*)take(QMAX * e);
+  s.inv4l = (T*)take(QMAX * e);
+  s.misc = (T*)take(4 * e);
+  s.pd = (T*)take((size_t)2 * npb * PDN * e);
+  s.As = (T*)take((size_t)D * M * e);
+  s.p1 = (T*)take((size_t)npb * M * e);
+  s.ms = (T*)take((size_t)3 * npb * DMAX * e);
+  s.red = (T*)take((size_t)2 * ns * npb * db * e);
+  s.rec = (R*)take((size_t)2 * npb * M * rec_len(QC) * e);
+  s.G = (R*)take((size_t)P * e);
+  s.Bs = (T*)take((size_t)D * P * e);
+  s.pab = pab ? (unsigned short*)take((size_t)P * sizeof(unsigned short)) : nullptr;
+  if (out) *out = s;
+  return o;
+}
+
+template <typename T, int NPB, int QC, int DB, int NS, int NF>
+__global__ void __launch_bounds__((NS + NF) * 32, NS < 16 ? 2 : 1)
+    psi_fwd_kernel(PsiArgs<typename Num<T>::store_t> a, int use_pab) {
+  typedef typename Num<T>::store_t S;
+  typedef PairExp<T> X;
+  typedef typename X::R R;
+  constexpr int RL = rec_len(QC), ZL = zlen(QC), NTH = (NS + NF) * 32, NTS = NS * 32, K = NPB * DB;
+  static_assert(K <= 8, "one butterfly of eight values");
+  extern __shared__ __align__(16) char smem_raw[];
+  const int M = a.M, Q = exact_q(QC) ? QC : a.Q, D = a.Dout;
+  const int P = M * (M + 1) / 2;
+  MSmem<T> s;
+  mcarve<T>(&s, smem_raw, M, QC, P, D, NPB, NS, DB, use_pab);
+  __shared__ int s_flag[2][NPB];   // a point of the pass lies outside the fixed-point range
+  const ExpTab etab{s.tab};
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool front_warp = tid >= NTS;
+  // ---- per-CTA tables
+  load_pair_table<T>(s.tab);
+#pragma unroll 1
+  for (int i = tid; i < M * ZL; i += NTH) {
+    const int ia = i / ZL, q = i - ia * ZL;
+    s.z[i] = q < Q ? Num<T>::ld(a.Z[ia * Q + q]) : Num<T>::zero();
+  }
+#pragma unroll 1
+  for (int i = tid; i < D * M; i += NTH) s.As[i] = Num<T>::ld(a.A[i]);
+  __syncthreads();
+  if (tid < Q) {
+    const T lnl = Num<T>::ld(static_cast<S>(a.lls2[tid]));
+    const T l2 = exp_tab(lnl, etab);
+    s.lnl[tid] = lnl;
+    s.ell2[tid] = l2;
+    s.inv4l[tid] = recip(mul(l2, Num<T>::c(4.f)));
+  }
+  if (tid == 32) {
+    const T lsf = Num<T>::ld(static_cast<S>(a.lsf2[0]));
+    s.misc[0] = lsf;
+    s.misc[1] = exp_tab(lsf, etab);
+  }
+  __syncthreads();
+  const T lsf = s.misc[0];
+  const int nbeg = (int)((long)a.N * blockIdx.x / gridDim.x);
+  const int nend = (int)((long)a.N * (blockIdx.x + 1) / gridDim.x);
+  const int passes = (nend - nbeg + NPB - 1) / NPB;
+  auto npts_of = [&](int i) { return min(NPB, nend - nbeg - i * NPB); };
+
+  // ---- front warps: constants, records, psi1 and m of pass i
+  auto front = [&](int i) {
+    const int rt = tid - NTS, rw = rt >> 5, n0 = nbeg + i * NPB, npts = npts_of(i);
+    auto slot = [&](int pt) { return PointSlot<T>(s.pd + ((i & 1) * NPB + pt) * PDN, s.rec + (size_t)((i & 1) * NPB + pt) * M * RL); };
+    for (int pt = rw; pt < npts; pt += NF)
+      consts_of<T, S>(a, s.ell2, s.lnl, etab, lsf, slot(pt), n0 + pt, Q, lane, &s_flag[i & 1][pt]);
+    if (rw == 0 && lane >= npts && lane < NPB) s_flag[i & 1][lane] = 0;
+    warps_sync<1, NF>();
+    for (int t = rt; t < npts * M; t += NF * 32) {
+      const int pt = t / M, ia = t - pt * M;
+      const T v1 = row_of<T, QC>(s.z + ia * ZL, etab, slot(pt), Q, ia, &s_flag[i & 1][pt]);
+      s.p1[pt * M + ia] = v1;
+      if (a.psi1) a.psi1[(size_t)(n0 + pt) * M + ia] = Num<T>::st(v1);
+    }
+    warps_sync<1, NF>();
+    for (int pt = rw; pt < npts; pt += NF) {   // m = psi1 . A_d, a warp a point
+#pragma unroll
+      for (int d = 0; d < DB; ++d) {
+        if (d < D) {
+          T mm = Num<T>::zero();
+          for (int ia = lane; ia < M; ia += 32) mm = fma_(s.p1[pt * M + ia], s.As[d * M + ia], mm);
+          mm = warp_sum(mm);
+          if (lane == 0) {
+            s.ms[((i % 3) * NPB + pt) * DMAX + d] = mm;
+            if (a.m_out) a.m_out[(size_t)(n0 + pt) * D + d] = Num<T>::st(mm);
+          }
+        }
+      }
+    }
+    warps_sync<1, NF>();
+  };
+  // ---- front warps: v of pass i from the sweep warps' sums, a thread an output
+  auto finish = [&](int i) {
+    const int rt = tid - NTS, pt = rt / DB, d = rt - pt * DB;
+    if (rt < K && pt < npts_of(i) && d < D && a.v_out) {
+      const T* r = s.red + (size_t)(i & 1) * NS * K + rt;
+      T v = r[0];
+      for (int w = 1; w < NS; ++w) v = add(v, r[w * K]);
+      const T mm = s.ms[((i % 3) * NPB + pt) * DMAX + d];
+      a.v_out[(size_t)(nbeg + i * NPB + pt) * D + d] = Num<T>::st(sub(add(s.misc[1], v), mul(mm, mm)));
+    }
+  };
+
+  if (front_warp) {
+    if (passes > 0) front(0);
+  } else {
+    stage_pairs<T, QC, NS, 2>(s.z, s.inv4l, Q, M, P, D, a.B, false, s.pab, s.G, s.Bs,
+                              reinterpret_cast<T*>(s.G));
+  }
+  __syncthreads();
+  for (int i = 0; i < passes; ++i) {
+    if (front_warp) {
+      if (i > 0) finish(i - 1);
+      if (i + 1 < passes) front(i + 1);
+    } else {
+      const R* rec = s.rec + (size_t)(i & 1) * NPB * M * RL;
+      int general = 0;
+      if (X::TAB) {
+#pragma unroll
+        for (int pt = 0; pt < NPB; ++pt) general |= s_flag[i & 1][pt];
+      }
+      T vacc[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) vacc[k] = Num<T>::zero();
+      constexpr int E = sizeof(T);
+      const saddr ar = sm_addr(rec), aG = sm_addr(s.G), aB = sm_addr(s.Bs), ap = use_pab ? sm_addr(s.pab) : 0u,
+                  at = sm_addr(s.tab);
+      const saddr ps_ = M * (RL * E);   // from one point's records to the next
+      for (int p = tid; p < P; p += NTS) {
+        p = GPK_IDX(p, P, 3);
+        int ia, ib;
+        if (use_pab) {
+          const int ab = lds_u16(ap + 2 * p);
+          ia = ab >> 8;
+          ib = ab & 0xff;
+        } else {
+          pair_of(p, ia, ib);
+        }
+        T w[DB];
+#pragma unroll
+        for (int d = 0; d < DB; ++d) w[d] = d < D ? ldsv<T>(aB + (d * P + p) * E) : Num<T>::zero();
+        const R gab = ldsv<R>(aG + p * E);
+        saddr ra = ar + ia * (RL * E), rb = ar + ib * (RL * E);
+        if (!general) {
+          // branch-free, so that the NPB points' exps interleave; in a pass with fewer points the
+          // extra slots run on stale tables and their sums are never read
+          R arg[NPB];
+#pragma unroll
+          for (int pt = 0; pt < NPB; ++pt) {
+            arg[pt] = X::template arg<QC>(ra, rb, gab);
+            ra += ps_;
+            rb += ps_;
+          }
+#pragma unroll
+          for (int pt = 0; pt < NPB; ++pt) {
+            const T ps = X::ev(arg[pt], at);
+#pragma unroll
+            for (int d = 0; d < DB; ++d) acc_fma(vacc[pt * DB + d], w[d], ps);
+          }
+        } else {
+          const int npts = npts_of(i);
+#pragma unroll
+          for (int pt = 0; pt < NPB; ++pt) {
+            if (pt < npts) {
+              const T ps = s_flag[i & 1][pt]
+                               ? psi2_general(s.z + ia * ZL, s.z + ib * ZL, s.pd + ((i & 1) * NPB + pt) * PDN, s.inv4l,
+                                              lsf, Q, s.tab)
+                               : X::ev(X::template arg<QC>(ra, rb, gab), at);
+#pragma unroll
+              for (int d = 0; d < DB; ++d) acc_fma(vacc[pt * DB + d], w[d], ps);
+            }
+            ra += ps_;
+            rb += ps_;
+          }
+        }
+      }
+      T t[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t[k] = k < K ? acc_done(vacc[k]) : Num<T>::zero();
+      warp_sum_many<8>(t);
+      if ((lane & 3) == 0 && (lane >> 2) < K) s.red[((size_t)(i & 1) * NS + (tid >> 5)) * K + (lane >> 2)] = t[0];
+    }
+    __syncthreads();
+  }
+  if (front_warp && passes > 0) finish(passes - 1);
+}
+
+// ---------------------------------------------------------------------------------
+// Forward with psi2 per point written out [N, M, M] (psi1 optionally): the sweep warps leave point
+// i's packed pairs in shared memory as storage values while they write point i - 1's full square
+// from the other buffer, each row as consecutive columns (straight from the sweep, the entries
+// above the diagonal are one 8-byte store per 32-byte sector); the front warps form point i + 1.
+// N = 1000, Q = 2, M = 100 (81 MB): 67 -> 45 us; FP32 24 us.  The double-float pairs become float64 by
+// integer operations (exp2_fx_double): two conversions
+// and an addition on the FP64 pipe took longer than the sweep itself.
+template <typename T>
+struct OSmem {
+  typedef typename PairExp<T>::R R;
+  typedef typename Num<T>::store_t S;
+  float2* tab;
+  T* z;      // [M][zlen]
+  T* ell2;   // [QMAX]
+  T* lnl;    // [QMAX]
+  T* inv4l;  // [QMAX]
+  T* misc;   // [4]
+  T* pd;     // [2][PDN]
+  R* rec;    // [2][M][rec_len]
+  S* L;      // [2][P]
+  R* G;      // [P] or nullptr
+  unsigned short* pab;   // [P] or nullptr
+};
+template <typename T>
+__host__ __device__ inline size_t ocarve(OSmem<T>* out, char* base, int M, int QC, int P, int ng, int pab) {
+  typedef typename PairExp<T>::R R;
+  typedef typename Num<T>::store_t S;
+  OSmem<T> s;
+  size_t o = 0;
+  auto take = [&](size_t n) {
+    char* p = base + o;
+    o += n;
+    return p;
+  };
+  const size_t e = sizeof(T);
+  s.tab = (float2*)take(PairExp<T>::TAB * sizeof(float2));
+  s.z = (T*)take((size_t)zlen(QC) * M * e);
+  s.ell2 = (T*)take(QMAX * e);
+  s.lnl = (T*)take(QMAX * e);
+  s.inv4l = (T*)take(QMAX * e);
+  s.misc = (T*)take(4 * e);
+  s.pd = (T*)take(2 * PDN * e);
+  s.rec = (R*)take(2 * (size_t)M * rec_len(QC) * e);
+  s.L = (S*)take(2 * (size_t)P * e);
+  s.G = ng ? (R*)take((size_t)ng * e) : nullptr;
+  s.pab = pab ? (unsigned short*)take((size_t)P * sizeof(unsigned short)) : nullptr;
+  if (out) *out = s;
+  return o;
+}
+
+template <typename T, int QC, int NS, int NF>
+__global__ void __launch_bounds__((NS + NF) * 32, NS < 12 ? 2 : 1)
+    psi_out_kernel(PsiArgs<typename Num<T>::store_t> a, int use_pab) {
+  typedef typename Num<T>::store_t S;
+  typedef PairExp<T> X;
+  typedef typename X::R R;
+  constexpr int RL = rec_len(QC), ZL = zlen(QC), NTH = (NS + NF) * 32, NTS = NS * 32;
+  extern __shared__ __align__(16) char smem_raw[];
+  const int M = a.M, Q = exact_q(QC) ? QC : a.Q;
+  const int P = M * (M + 1) / 2;
+  OSmem<T> s;
+  ocarve<T>(&s, smem_raw, M, QC, P, a.g_smem ? P : 0, use_pab);
+  __shared__ int s_flag[2];
+  const ExpTab etab{s.tab};
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool front_warp = tid >= NTS;
+  load_pair_table<T>(s.tab);
+#pragma unroll 1
+  for (int i = tid; i < M * ZL; i += NTH) {
+    const int ia = i / ZL, q = i - ia * ZL;
+    s.z[i] = q < Q ? Num<T>::ld(a.Z[ia * Q + q]) : Num<T>::zero();
+  }
+  __syncthreads();
+  if (tid < Q) {
+    const T lnl = Num<T>::ld(static_cast<S>(a.lls2[tid]));
+    const T l2 = exp_tab(lnl, etab);
+    s.lnl[tid] = lnl;
+    s.ell2[tid] = l2;
+    s.inv4l[tid] = recip(mul(l2, Num<T>::c(4.f)));
+  }
+  const T lsf = Num<T>::ld(static_cast<S>(a.lsf2[0]));
+  __syncthreads();
+  const int nbeg = (int)((long)a.N * blockIdx.x / gridDim.x);
+  const int nend = (int)((long)a.N * (blockIdx.x + 1) / gridDim.x);
+  const int cnt = nend - nbeg;
+  auto front = [&](int i) {
+    const int rt = tid - NTS, n = nbeg + i;
+    const PointSlot<T> ps(s.pd + (i & 1) * PDN, s.rec + (size_t)(i & 1) * M * RL);
+    if (rt < 32) consts_of<T, S>(a, s.ell2, s.lnl, etab, lsf, ps, n, Q, lane, &s_flag[i & 1]);
+    warps_sync<1, NF>();
+    for (int ia = rt; ia < M; ia += NF * 32) {
+      const T v1 = row_of<T, QC>(s.z + ia * ZL, etab, ps, Q, ia, &s_flag[i & 1]);
+      if (a.psi1) a.psi1[(size_t)n * M + ia] = Num<T>::st(v1);
+    }
+  };
+  if (front_warp) {
+    if (cnt > 0) front(0);
+  } else {
+    stage_pairs<T, QC, NS, 2>(s.z, s.inv4l, Q, M, P, 0, (const S*)nullptr, false, s.pab, s.G, (T*)nullptr,
+                              (T*)nullptr);
+  }
+  __syncthreads();
+  for (int i = 0; i <= cnt; ++i) {
+    if (front_warp) {
+      if (i + 1 < cnt) front(i + 1);
+    } else {
+      if (i < cnt) {
+        S* L = s.L + (size_t)(i & 1) * P;
+        const R* rec = s.rec + (size_t)(i & 1) * M * RL;
+        const bool general = X::TAB && s_flag[i & 1];
+        constexpr int E = sizeof(T);
+        const saddr ar = sm_addr(rec), aG = a.g_smem ? sm_addr(s.G) : 0u, aL = sm_addr(L),
+                    ap = use_pab ? sm_addr(s.pab) : 0u, at = sm_addr(s.tab);
+        // two pairs (p, p + NTS) per iteration, so that their chains interleave
+        for (int p0 = tid; p0 < P; p0 += 2 * NTS) {
+          R arg[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int p = u && p0 + NTS < P ? p0 + NTS : p0;
+            int ia, ib;
+            if (use_pab) {
+              const int ab = lds_u16(ap + 2 * p);
+              ia = ab >> 8;
+              ib = ab & 0xff;
+            } else {
+              pair_of(p, ia, ib);
+            }
+            if (general) {
+              sts(aL + p * E, Num<T>::st(psi2_general(s.z + ia * ZL, s.z + ib * ZL, s.pd + (i & 1) * PDN, s.inv4l, lsf, Q,
+                                                      s.tab)));
+            } else {
+              arg[u] = X::template arg<QC>(ar + ia * (RL * E), ar + ib * (RL * E),
+                                           a.g_smem ? ldsv<R>(aG + p * E)
+                                                    : pair_G<T, QC>(s.z + ia * ZL, s.z + ib * ZL, s.inv4l, Q));
+            }
+          }
+          if (!general) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) sts(aL + (u && p0 + NTS < P ? p0 + NTS : p0) * E, X::ev_st(arg[u], at));
+          }
+        }
+      }
+      if (i > 0) {   // the previous point's square, a warp a row, 128 columns at a time
+        constexpr int E = sizeof(T);
+        const saddr aL = sm_addr(s.L + (size_t)((i - 1) & 1) * P);
+        S* const out = a.psi2 + (size_t)(nbeg + i - 1) * M * M;
+        for (int c0 = 0; c0 < M; c0 += 128) {
+          saddr up[4];   // the lane's columns: where their entries below the diagonal begin
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int b = c0 + lane + 32 * k;
+            up[k] = aL + b * (b + 1) / 2 * E;
+          }
+          for (int ia = tid >> 5; ia < M; ia += NS) {
+            const saddr row = aL + (ia * (ia + 1) / 2 + c0 + lane) * E;
+            S* const o = out + (size_t)ia * M + c0 + lane;
+            const int left = M - c0 - lane, below = ia - c0 - lane;   // columns left, columns up to the diagonal
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              if (32 * k < left) {
+                S v;
+                lds_st(32 * k <= below ? row + 32 * k * E : up[k] + ia * E, v);
+                o[32 * k] = v;
+              }
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
 template <typename T, int NPB, int PPT, int QC, int DB>
-int run_fwd(const PsiArgs<typename Num<T>::store_t>& a, int per_sm, size_t sm, cudaStream_t st) {
-  auto k = psi_fwd_kernel<T, NPB, PPT, QC, DB>;
+int run_fwd_gen(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) {
+  PsiArgs<typename Num<T>::store_t> a = a_in;
+  const int P = a.M * (a.M + 1) / 2;
+  const bool contract = a.A && a.B && (a.m_out || a.v_out);
+  const int D = contract ? a.Dout : 0, nbs = D * P;
+  // G and the symmetrised B in shared memory as far as they fit; B first (from global memory it
+  // costs two loads and conversions per pair, G a few operations per dimension)
+  auto bytes = [&](int ng, int nb) { return fwd_smem_bytes(a.M, a.Q, QC, D, NPB, sizeof(T), ng, nb); };
+  a.bs_smem = contract && bytes(0, nbs) <= SMEM_CAP;
+  a.g_smem = bytes(P, a.bs_smem ? nbs : 0) <= SMEM_CAP;
+  const size_t sm = bytes(a.g_smem ? P : 0, a.bs_smem ? nbs : 0);
+  auto k = psi_fwd_gen_kernel<T, NPB, PPT, QC, DB>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   int resident = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k, NT, sm);
-  if (resident < 1) resident = 1;
-  if (resident > per_sm) resident = per_sm;
+  resident = resident < 1 ? 1 : (resident > 2 ? 2 : resident);
   int grid = a.chain ? 1 : gpk::sm_count() * resident;   // a rollout is one CTA's sequence
   if (grid > a.N) grid = a.N;
   if (grid < 1) return GPK_OK;
@@ -1193,25 +1672,99 @@ int run_fwd(const PsiArgs<typename Num<T>::store_t>& a, int per_sm, size_t sm, c
 
 // points per pass: 4 for Dout <= 2, 2 for Dout <= 4 (so 2*NPB*Dout sums fit one reduction)
 template <typename T, int QC>
-int fwd_variant(const PsiArgs<typename Num<T>::store_t>& a, bool sum, bool contract, int P, int per_sm, size_t sm,
-                cudaStream_t st) {
+int fwd_gen(const PsiArgs<typename Num<T>::store_t>& a, bool sum, bool contract, int P, cudaStream_t st) {
   if (sum) {
-    if (P <= 4 * NT) return run_fwd<T, 2, 4, QC, 4>(a, per_sm, sm, st);
-    return run_fwd<T, 2, 16, QC, 4>(a, per_sm, sm, st);
+    if (P <= 4 * NT) return run_fwd_gen<T, 2, 4, QC, 4>(a, st);
+    return run_fwd_gen<T, 2, 16, QC, 4>(a, st);
   }
   if (a.chain) {   // one point per pass: each point needs the previous one's moments
-    if (a.Dout == 1) return run_fwd<T, 1, 0, QC, 1>(a, per_sm, sm, st);
-    if (a.Dout == 2) return run_fwd<T, 1, 0, QC, 2>(a, per_sm, sm, st);
-    return run_fwd<T, 1, 0, QC, 4>(a, per_sm, sm, st);
+    if (a.Dout == 1) return run_fwd_gen<T, 1, 0, QC, 1>(a, st);
+    if (a.Dout == 2) return run_fwd_gen<T, 1, 0, QC, 2>(a, st);
+    return run_fwd_gen<T, 1, 0, QC, 4>(a, st);
   }
-  if (!contract || a.Dout == 1) return run_fwd<T, 4, 0, QC, 1>(a, per_sm, sm, st);
-  if (a.Dout == 2) return run_fwd<T, 4, 0, QC, 2>(a, per_sm, sm, st);
-  return run_fwd<T, 2, 0, QC, 4>(a, per_sm, sm, st);
+  if (!contract || a.Dout == 1) return run_fwd_gen<T, 4, 0, QC, 1>(a, st);
+  if (a.Dout == 2) return run_fwd_gen<T, 4, 0, QC, 2>(a, st);
+  return run_fwd_gen<T, 2, 0, QC, 4>(a, st);
 }
 
-template <typename T>
-int launch_fwd(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) {
+// the moments kernel, or -1 where its tables do not fit
+template <typename T, int NPB, int QC, int DB, int NS, int NF>
+int run_fwd(const PsiArgs<typename Num<T>::store_t>& a, size_t cap, cudaStream_t st) {
+  const int P = a.M * (a.M + 1) / 2;
+  int pab = a.M <= 255;
+  // whether this split is taken depends on the sizes of the full pass only, not on N
+  constexpr int NPBF = DB <= 2 ? 4 : 2;
+  if (mcarve<T>(nullptr, nullptr, a.M, QC, P, a.Dout, NPBF, NS, DB, pab) > cap && NS >= 16) pab = 0;
+  if (mcarve<T>(nullptr, nullptr, a.M, QC, P, a.Dout, NPBF, NS, DB, pab) > cap) return -1;
+  const size_t sm = mcarve<T>(nullptr, nullptr, a.M, QC, P, a.Dout, NPB, NS, DB, pab);
+  auto k = psi_fwd_kernel<T, NPB, QC, DB, NS, NF>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  int grid = gpk::sm_count() * (NS < 16 ? 2 : 1);
+  if (grid > a.N) grid = a.N;
+  if (grid < 1) return GPK_OK;
+  k<<<grid, (NS + NF) * 32, sm, st>>>(a, pab);
+  return gpk::check_launch("psi_fwd");
+}
+
+template <typename T, int QC, int NS, int NF>
+int fwd_npb(const PsiArgs<typename Num<T>::store_t>& a, size_t cap, cudaStream_t st) {
+  // points per pass: one where every CTA has a single point (a pass evaluates all its slots), else
+  // four (two for Dout > 2: eight sums a thread)
+  const bool one = a.N <= gpk::sm_count() * (NS < 16 ? 2 : 1);
+  if (a.Dout == 1) return one ? run_fwd<T, 1, QC, 1, NS, NF>(a, cap, st) : run_fwd<T, 4, QC, 1, NS, NF>(a, cap, st);
+  if (a.Dout == 2) return one ? run_fwd<T, 1, QC, 2, NS, NF>(a, cap, st) : run_fwd<T, 4, QC, 2, NS, NF>(a, cap, st);
+  return run_fwd<T, 2, QC, 4, NS, NF>(a, cap, st);
+}
+
+template <typename T, int QC, int NS, int NF>
+int run_out(const PsiArgs<typename Num<T>::store_t>& a_in, size_t cap, cudaStream_t st) {
   PsiArgs<typename Num<T>::store_t> a = a_in;
+  const int P = a.M * (a.M + 1) / 2;
+  // G and the pair table as far as they fit (two CTAs an SM only with both)
+  for (int o = 0; o < (NS < 12 ? 1 : 3); ++o) {
+    const int pab = o == 0 && a.M <= 255;
+    a.g_smem = o < 2;
+    const size_t sm = ocarve<T>(nullptr, nullptr, a.M, QC, P, a.g_smem ? P : 0, pab);
+    if (sm > cap) continue;
+    auto k = psi_out_kernel<T, QC, NS, NF>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    int grid = gpk::sm_count() * (NS < 12 ? 2 : 1);
+    if (grid > a.N) grid = a.N;
+    if (grid < 1) return GPK_OK;
+    k<<<grid, (NS + NF) * 32, sm, st>>>(a, pab);
+    return gpk::check_launch("psi_out");
+  }
+  return -1;
+}
+
+// one input width's kernels (each width is a translation unit of its own)
+template <typename T, int QC>
+int launch_fwd_q(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
+  const int P = a.M * (a.M + 1) / 2;
+  const bool contract = a.A && a.B && (a.m_out || a.v_out);
+  const bool sum = a.psi2_sum != nullptr;
+  const size_t half = (SMEM_CAP - 2048) / 2;   // two CTAs an SM
+  int rc = -1;
+  if (!sum && !a.chain && !a.psi2 && contract) {
+    // the split of the sums may not depend on N: a point's moments are the same, bit for bit, in any
+    // batch (the points per pass do not enter a point's sums)
+    rc = fwd_npb<T, QC, 8, 4>(a, half, st);
+    if (rc == -1) rc = fwd_npb<T, QC, 16, 4>(a, SMEM_CAP, st);
+  } else if (!sum && !a.chain && a.psi2 && !contract) {
+    if (a.N > gpk::sm_count()) rc = run_out<T, QC, 8, 4>(a, half, st);
+    if (rc == -1) rc = run_out<T, QC, 16, 4>(a, SMEM_CAP, st);
+  }
+  if (rc != -1) return rc;
+  if constexpr (exact_q(QC)) {
+    return GPK_EUNSUPPORTED;   // the caller falls back to the catch-all width
+  } else {
+    return fwd_gen<T, QC>(a, sum, contract, P, st);
+  }
+}
+
+// the size limits, the same for every form
+template <typename S>
+int check_fwd(const PsiArgs<S>& a) {
   const int P = a.M * (a.M + 1) / 2;
   const bool contract = a.A && a.B && (a.m_out || a.v_out);
   const bool sum = a.psi2_sum != nullptr;
@@ -1219,28 +1772,11 @@ int launch_fwd(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) {
   const int D = contract ? a.Dout : 0;
   // accepted sizes: a pair table and the points' tables within shared memory
   const size_t need = 2048 + ((size_t)a.M * a.Q + 28 + (size_t)npb * 40 + (size_t)npb * a.M * (2 + a.Q) +
-                              (size_t)D * a.M + P + 1536) * sizeof(T);
+                              (size_t)D * a.M + P + 1536) * sizeof(S);
   if (need > 227 * 1024) return gpk::fail(GPK_EUNSUPPORTED, "psi_fwd: M=%d needs %zu B of shared memory", a.M, need);
   if (sum && P > PPT_MAX * NT)
     return gpk::fail(GPK_EUNSUPPORTED, "psi_fwd: psi2_sum needs M(M+1)/2 <= %d (M=%d)", PPT_MAX * NT, a.M);
-  // five input dimensions, one output, moments only (the psi-statistics workload's shape): an
-  // exact instantiation
-  const bool five = a.Q == 5 && !sum && !a.chain && contract && a.Dout == 1 && !a.psi2;
-  const int QC = a.Q <= 2 ? 2 : (five ? 5 : QMAX);
-  // G and the symmetrised B in shared memory as far as they fit; B first (from global memory it
-  // costs two loads and conversions per pair, G a few operations per dimension)
-  const size_t cap = SMEM_CAP;
-  auto bytes = [&](int ng, int nbs) { return fwd_smem_bytes(a.M, a.Q, QC, D, npb, sizeof(T), ng, nbs); };
-  const int nbs = contract ? a.Dout * P : 0;
-  a.bs_smem = contract && bytes(0, nbs) <= cap;
-  a.g_smem = bytes(P, a.bs_smem ? nbs : 0) <= cap;
-  const size_t sm = bytes(a.g_smem ? P : 0, a.bs_smem ? nbs : 0);
-  int per_sm = (int)((227 * 1024) / (sm + 1024));
-  if (per_sm < 1) per_sm = 1;
-  if (per_sm > 2) per_sm = 2;
-  if (QC == 2) return fwd_variant<T, 2>(a, sum, contract, P, per_sm, sm, st);
-  if (QC == 5) return run_fwd<T, 4, 0, 5, 1>(a, per_sm, sm, st);
-  return fwd_variant<T, QMAX>(a, sum, contract, P, per_sm, sm, st);
+  return GPK_OK;
 }
 
 // the destinations of the backward's partial block (layout in PsiArgs::part)
