@@ -29,27 +29,58 @@ def _c(t):
     return t.detach().contiguous()
 
 
-def _hyp_grads(dsf2, dl, dv, lls2, lsf2):
-    """(d/d lls2, d/d lsf2) from the kernels' d/d sf2 (psi or kfu part) and d/d ell, plus the
-    direct sf2 of v = sf2 + ...: d ell / d lls2 = ell / 2, d sf2 / d lsf2 = sf2."""
-    ell = torch.exp(0.5 * lls2.detach().double())
-    sf2 = torch.exp(lsf2.detach().double())
-    g_l = (dl * ell * 0.5).to(lls2.dtype)
-    g_s = (sf2 * (dsf2 + dv.double().sum())).reshape(lsf2.shape).to(lsf2.dtype)
-    return g_l, g_s
+def _hyp(lls2, lsf2):
+    """The hyperparameters as the kernels take them: contiguous float64."""
+    return _c(lls2).double(), _c(lsf2).double().reshape(1)
+
+
+def _up(g, like):
+    """An upstream gradient (None: zero) as a contiguous tensor of the outputs' type."""
+    return torch.zeros_like(like) if g is None else g.contiguous().to(like.dtype)
+
+
+class _Acc:
+    """The float64 sums of one backward call in one zeroed buffer: dsf2, dl, dZ, dA, dB."""
+
+    def __init__(self, Q, M, D, device):
+        o = [0, 1, 1 + Q, 1 + Q + M * Q, 1 + Q + M * Q + D * M, 1 + Q + M * Q + D * M + D * M * M]
+        self.Q, self.shapes, self.o = Q, ((M, Q), (D, M), (D, M, M)), o
+        self.buf = torch.zeros(o[5], dtype=torch.float64, device=device)
+        self.dsf2, self.dl = self.buf[0:1], self.buf[1:1 + Q]
+        self.dZ, self.dA, self.dB = self._rest(self.buf, 0)
+
+    def _rest(self, buf, shift):
+        o = self.o
+        return [buf[o[2 + i] - shift:o[3 + i] - shift].view(s) for i, s in enumerate(self.shapes)]
+
+    def grads(self, l2, s2, dv, hyp):
+        """(dZ, g_lls2, g_lsf2, dA, dB) in the inputs' types, one launch: d ell / d lls2 = ell / 2,
+        d sf2 / d lsf2 = sf2, and v's direct sf2."""
+        (lt, _), (st, sshape) = hyp
+        g = torch.empty(self.Q + 1, dtype=torch.float64, device=self.buf.device)
+        if dv.dtype == torch.float64:
+            rest, cast = (self.dZ, self.dA, self.dB), None
+        else:
+            cast = torch.empty(self.buf.numel() - 1 - self.Q, dtype=dv.dtype, device=dv.device)
+            rest = self._rest(cast, 1 + self.Q)
+        gpk.moment_grads(self.Q, l2, s2, self.buf, dv, g[:self.Q], g[self.Q:], cast)
+        return rest[0], g[:self.Q].to(lt), g[self.Q:].reshape(sshape).to(st), rest[1], rest[2]
+
+
+def _hyp_kind(lls2, lsf2):
+    return ((lls2.dtype, lls2.shape), (lsf2.dtype, lsf2.shape))
 
 
 class PsiMoments(torch.autograd.Function):
     @staticmethod
     def forward(ctx, mu, S, Z, lls2, lsf2, A, B):
         mu, S, Z, A, B = _c(mu), _c(S), _c(Z), _c(A), _c(B)
-        l2, s2 = _c(lls2).double(), _c(lsf2).double().reshape(1)
-        N, D = mu.shape[0], A.shape[0]
-        m = torch.empty((N, D), dtype=mu.dtype, device=mu.device)
+        l2, s2 = _hyp(lls2, lsf2)
+        m = torch.empty((mu.shape[0], A.shape[0]), dtype=mu.dtype, device=mu.device)
         v = torch.empty_like(m)
         gpk.psi_fwd(mu, S, Z, l2, s2, A, B, m_out=m, v_out=v)
         ctx.save_for_backward(mu, S, Z, l2, s2, A, B, m)
-        ctx.hyp = (lls2, lsf2)
+        ctx.hyp = _hyp_kind(lls2, lsf2)
         return m, v
 
     @staticmethod
@@ -57,22 +88,20 @@ class PsiMoments(torch.autograd.Function):
         mu, S, Z, l2, s2, A, B, m = ctx.saved_tensors
         N, Q = mu.shape
         M, D = Z.shape[0], A.shape[0]
-        dm = torch.zeros_like(m) if dm is None else dm.contiguous().to(m.dtype)
-        dv = torch.zeros_like(m) if dv is None else dv.contiguous().to(m.dtype)
-        z = lambda *s: torch.zeros(s, dtype=torch.float64, device=mu.device)
-        dsf2, dl, dZ, dA, dB = z(1), z(Q), z(M, Q), z(D, M), z(D, M, M)
+        dm, dv = _up(dm, m), _up(dv, m)
+        acc = _Acc(Q, M, D, mu.device)
         dmu, dS = torch.empty_like(mu), torch.empty_like(S)
-        work = z(gpk.work_elems(gpk.OP_PSI_BWD, N, M, Q, D))
-        gpk.psi_bwd(mu, S, Z, l2, s2, A, B, m, dm, dv, dsf2, dl, dZ, dA, dB, dmu, dS, work=work)
-        g_l, g_s = _hyp_grads(dsf2, dl, dv, *ctx.hyp)
-        return dmu, dS, dZ.to(Z.dtype), g_l, g_s, dA.to(A.dtype), dB.to(B.dtype)
+        work = torch.empty(gpk.work_elems(gpk.OP_PSI_BWD, N, M, Q, D), dtype=torch.float64, device=mu.device)
+        gpk.psi_bwd(mu, S, Z, l2, s2, A, B, m, dm, dv, acc.dsf2, acc.dl, acc.dZ, acc.dA, acc.dB, dmu, dS, work=work)
+        dZ, g_l, g_s, dA, dB = acc.grads(l2, s2, dv, ctx.hyp)
+        return dmu, dS, dZ, g_l, g_s, dA, dB
 
 
 class DetMoments(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, Z, lls2, lsf2, A, B):
         x, Z, A, B = _c(x), _c(Z), _c(A), _c(B)
-        l2, s2 = _c(lls2).double(), _c(lsf2).double().reshape(1)
+        l2, s2 = _hyp(lls2, lsf2)
         N, M, D = x.shape[0], Z.shape[0], A.shape[0]
         kfu = torch.empty((N, M), dtype=x.dtype, device=x.device)
         Bk = torch.empty((N, D, M), dtype=x.dtype, device=x.device)
@@ -80,7 +109,7 @@ class DetMoments(torch.autograd.Function):
         v = torch.empty_like(m)
         gpk.det_fwd(x, Z, l2, s2, A, B, kfu, Bk, m, v)
         ctx.save_for_backward(x, Z, l2, s2, A, kfu, Bk)
-        ctx.hyp = (lls2, lsf2)
+        ctx.hyp = _hyp_kind(lls2, lsf2)
         return m, v
 
     @staticmethod
@@ -88,16 +117,16 @@ class DetMoments(torch.autograd.Function):
         x, Z, l2, s2, A, kfu, Bk = ctx.saved_tensors
         N, Q = x.shape
         M, D = Z.shape[0], A.shape[0]
-        dm = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dm is None else dm.contiguous().to(x.dtype)
-        dv = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dv is None else dv.contiguous().to(x.dtype)
-        z = lambda *s: torch.zeros(s, dtype=torch.float64, device=x.device)
-        dsf2, dl, dZ, dA, dB = z(1), z(Q), z(M, Q), z(D, M), z(D, M, M)
+        dm = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dm is None else _up(dm, x)
+        dv = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dv is None else _up(dv, x)
+        acc = _Acc(Q, M, D, x.device)
         dx = torch.empty_like(x)
-        gpk.det_bwd(x, Z, l2, s2, A, kfu, Bk, dm, dv, dsf2, dl, dZ, dA, dx=dx,
-                    work=z(gpk.work_elems(gpk.OP_DET_BWD, N, M, Q, D)))
-        gpk.gram(kfu, kfu, dv, dB, work=z(gpk.work_elems(gpk.OP_GRAM, N, M, Q, D)))
-        g_l, g_s = _hyp_grads(dsf2, dl, dv, *ctx.hyp)
-        return dx, dZ.to(Z.dtype), g_l, g_s, dA.to(A.dtype), dB.to(A.dtype)
+        n1, n2 = gpk.work_elems(gpk.OP_DET_BWD, N, M, Q, D), gpk.work_elems(gpk.OP_GRAM, N, M, Q, D)
+        work = torch.empty(max(n1, n2), dtype=torch.float64, device=x.device)   # one after the other
+        gpk.det_bwd(x, Z, l2, s2, A, kfu, Bk, dm, dv, acc.dsf2, acc.dl, acc.dZ, acc.dA, dx=dx, work=work)
+        gpk.gram(kfu, kfu, dv, acc.dB, work=work)
+        dZ, g_l, g_s, dA, dB = acc.grads(l2, s2, dv, ctx.hyp)
+        return dx, dZ, g_l, g_s, dA, dB
 
 
 def psi_moments(mu, S, Z, lls2, lsf2, A, B):

@@ -404,6 +404,13 @@ def hyp_grads(ls, sf, dl, dsf2, dv, g_ls, g_sf):
          ptr(g_sf), stream())
 
 
+def moment_grads(Q, lls2, lsf2, acc, dv, g_l, g_s, cast=None):
+    """gpk_moment_grads: the chain rule to (lls2, lsf2) from acc = [dsf2 | dl Q | rest] and dv, and
+    acc's rest as float32 into `cast` when given."""
+    call('gpk_moment_grads', prec_of(dv.dtype), Q, acc.numel() - 1 - Q, ptr(lls2), ptr(lsf2), ptr(acc), ptr(dv),
+         dv.numel(), ptr(g_l), ptr(g_s), ptr(cast), stream())
+
+
 def aep_phi(D, M, N, alpha, logdetK, ldSuinv, ldShinv, mu, mh, th2, w, out):
     call('gpk_aep_phi', D, M, float(N), float(alpha), ptr(logdetK), ptr(ldSuinv), ptr(ldShinv), ptr(mu), ptr(mh),
          ptr(th2), float(w), ptr(out), stream())

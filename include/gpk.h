@@ -331,6 +331,15 @@ int gpk_triu_pack(int D, int M, const double* dR, const double* R, double* out, 
 int gpk_hyp_grads(int Q, const double* ls, const double* sf, const double* dl, const double* dsf2,
                   const double* dv, int ndv, double* g_ls, double* g_sf, void* stream);
 
+/* The end of a layer's backward in the log parameterisation of its inputs: acc holds
+ * [dsf2 | dl Q | ncast further sums] (the float64 outputs of gpk_psi_bwd or gpk_det_bwd laid out in
+ * that order), dv [ndv] the upstream gradient of v in the storage type:
+ *   g_l[q] = acc[1+q] exp(lls2[q]/2) / 2,  g_s[0] = exp(lsf2) (acc[0] + sum(dv))   (float64),
+ *   cast[i] = acc[1+Q+i] rounded to float, i < ncast (GPK_FP32 only; NULL to skip).
+ * The chain rule of geepee/aep_models.py:226-231 for lls2 = log ell^2, lsf2 = log sf^2. */
+int gpk_moment_grads(int prec, int Q, long ncast, const double* lls2, const double* lsf2, const double* acc,
+                     const void* dv, long ndv, double* g_l, double* g_s, void* cast, void* stream);
+
 /* *out += w * phi, the natural-parameter layer's weighted log-partition
  * phi = D/2 logdet Kuu + (N/a - 1)(-1/2 sum_d logdet Su^-1 + 1/2 mu.th2)
  *       - (N/a)(-1/2 sum_d logdet Suhat^-1 + 1/2 beta muhat.th2),  beta = (N - a)/N

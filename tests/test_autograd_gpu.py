@@ -94,3 +94,22 @@ def test_gradcheck_small():
             dev([0.1], True), dev(rng.randn(D, M) / M, True))
     f = lambda x, Z, l, s, A: det_moments(x, Z, l, s, A, Bf)
     assert torch.autograd.gradcheck(f, args, eps=1e-6, atol=1e-6, rtol=1e-5)
+
+
+@pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
+@pytest.mark.parametrize('n,Q,rest', [(0, 1, 0), (1, 2, 3), (4095, 8, 1000), (4097, 5, 1), (40000, 3, 20000)])
+def test_moment_grads(n, Q, rest, dtype):
+    """The chain-rule launch against the same expressions in float64 (a float64 sum of n values of
+    magnitude 1 in another order: n 2^-53 relative to the sum of magnitudes; the cast is exact)."""
+    from geepee_gb300 import gpk
+    g = torch.Generator(device='cuda').manual_seed(n + Q)
+    r = lambda *s: torch.randn(*s, generator=g, dtype=torch.float64, device='cuda')
+    l2, s2, acc, dv = r(Q), r(1), r(1 + Q + rest), r(n).to(dtype)
+    gl, gs = torch.empty_like(l2), torch.empty_like(s2)
+    cast = None if dtype == torch.float64 else torch.empty(rest, dtype=dtype, device='cuda')
+    gpk.moment_grads(Q, l2, s2, acc, dv, gl, gs, cast)
+    assert torch.allclose(gl, 0.5 * acc[1:1 + Q] * torch.exp(0.5 * l2), rtol=1e-14, atol=0)
+    want = torch.exp(s2) * (acc[0] + dv.double().sum())
+    assert abs(float(gs - want)) <= (2 * n + 8) * 2.0 ** -53 * float(torch.exp(s2)) * (float(dv.double().abs().sum()) + 8)
+    if cast is not None:
+        assert torch.equal(cast, acc[1 + Q:].float())
