@@ -67,6 +67,8 @@ _SIGS = {
     'gpk_triu_pack': [_c_int, _c_int, _vp, _vp, _vp, _c_int, _vp],
     'gpk_hyp_grads': [_c_int, _vp, _vp, _vp, _vp, _vp, _c_int, _vp, _vp, _vp],
     'gpk_moment_grads': [_c_int, _c_int, ctypes.c_long, _vp, _vp, _vp, _vp, ctypes.c_long, _vp, _vp, _vp, _vp],
+    'gpk_psi_layer_bwd': [_c_int] * 5 + [_vp] * 16 + [_vp, ctypes.c_long, _vp],
+    'gpk_det_layer_bwd': [_c_int] * 5 + [_vp, _c_int] + [_vp] * 13 + [_vp, ctypes.c_long, _vp],
     'gpk_aep_phi': [_c_int, _c_int, _c_dbl, _c_dbl, _vp, _vp, _vp, _vp, _vp, _vp, _c_dbl, _vp, _vp],
     'gpk_work_elems': [_c_int, _c_int, _c_int, _c_int, _c_int, _vp],
     'gpk_cavity_forms': [_c_int, _vp, _vp],
@@ -125,7 +127,9 @@ def ptr(t):
 
 
 def stream():
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream as its handle.  (torch.cuda.current_stream() builds a
+    Stream object on each call, ~10 us of host time, where this takes one.)"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def prec_of(dtype):

@@ -39,32 +39,24 @@ def _up(g, like):
     return torch.zeros_like(like) if g is None else g.contiguous().to(like.dtype)
 
 
-class _Acc:
-    """The float64 sums of one backward call in one zeroed buffer: dsf2, dl, dZ, dA, dB."""
+class _Sums:
+    """One backward call's float64 sums, [dsf2 | dl | dZ | dA | dB], with the two chained
+    hyperparameter gradients behind them, and for float32 layers the casts of dZ, dA, dB."""
 
-    def __init__(self, Q, M, D, device):
-        o = [0, 1, 1 + Q, 1 + Q + M * Q, 1 + Q + M * Q + D * M, 1 + Q + M * Q + D * M + D * M * M]
-        self.Q, self.shapes, self.o = Q, ((M, Q), (D, M), (D, M, M)), o
-        self.buf = torch.zeros(o[5], dtype=torch.float64, device=device)
-        self.dsf2, self.dl = self.buf[0:1], self.buf[1:1 + Q]
-        self.dZ, self.dA, self.dB = self._rest(self.buf, 0)
+    def __init__(self, Q, M, D, dtype, device):
+        self.sizes = [1 + Q, M * Q, D * M, D * M * M]
+        n = sum(self.sizes)
+        self.shapes = ((M, Q), (D, M), (D, M, M))
+        buf = torch.empty(n + Q + 1, dtype=torch.float64, device=device)
+        self.acc, self.g_l, self.g_s = buf.split([n, Q, 1])
+        self.cast = None if dtype == torch.float64 else torch.empty(n - 1 - Q, dtype=dtype, device=device)
 
-    def _rest(self, buf, shift):
-        o = self.o
-        return [buf[o[2 + i] - shift:o[3 + i] - shift].view(s) for i, s in enumerate(self.shapes)]
-
-    def grads(self, l2, s2, dv, hyp):
-        """(dZ, g_lls2, g_lsf2, dA, dB) in the inputs' types, one launch: d ell / d lls2 = ell / 2,
-        d sf2 / d lsf2 = sf2, and v's direct sf2."""
+    def grads(self, hyp):
+        """(dZ, g_lls2, g_lsf2, dA, dB) in the inputs' types."""
         (lt, _), (st, sshape) = hyp
-        g = torch.empty(self.Q + 1, dtype=torch.float64, device=self.buf.device)
-        if dv.dtype == torch.float64:
-            rest, cast = (self.dZ, self.dA, self.dB), None
-        else:
-            cast = torch.empty(self.buf.numel() - 1 - self.Q, dtype=dv.dtype, device=dv.device)
-            rest = self._rest(cast, 1 + self.Q)
-        gpk.moment_grads(self.Q, l2, s2, self.buf, dv, g[:self.Q], g[self.Q:], cast)
-        return rest[0], g[:self.Q].to(lt), g[self.Q:].reshape(sshape).to(st), rest[1], rest[2]
+        rest = self.acc.split(self.sizes)[1:] if self.cast is None else self.cast.split(self.sizes[1:])
+        dZ, dA, dB = [t.view(s) for t, s in zip(rest, self.shapes)]
+        return dZ, self.g_l.to(lt), self.g_s.reshape(sshape).to(st), dA, dB
 
 
 def _hyp_kind(lls2, lsf2):
@@ -89,11 +81,11 @@ class PsiMoments(torch.autograd.Function):
         N, Q = mu.shape
         M, D = Z.shape[0], A.shape[0]
         dm, dv = _up(dm, m), _up(dv, m)
-        acc = _Acc(Q, M, D, mu.device)
+        sums = _Sums(Q, M, D, mu.dtype, mu.device)
         dmu, dS = torch.empty_like(mu), torch.empty_like(S)
         work = torch.empty(gpk.work_elems(gpk.OP_PSI_BWD, N, M, Q, D), dtype=torch.float64, device=mu.device)
-        gpk.psi_bwd(mu, S, Z, l2, s2, A, B, m, dm, dv, acc.dsf2, acc.dl, acc.dZ, acc.dA, acc.dB, dmu, dS, work=work)
-        dZ, g_l, g_s, dA, dB = acc.grads(l2, s2, dv, ctx.hyp)
+        gpk.psi_layer_bwd(mu, S, Z, l2, s2, A, B, m, dm, dv, sums.acc, dmu, dS, sums.g_l, sums.g_s, sums.cast, work)
+        dZ, g_l, g_s, dA, dB = sums.grads(ctx.hyp)
         return dmu, dS, dZ, g_l, g_s, dA, dB
 
 
@@ -119,13 +111,12 @@ class DetMoments(torch.autograd.Function):
         M, D = Z.shape[0], A.shape[0]
         dm = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dm is None else _up(dm, x)
         dv = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dv is None else _up(dv, x)
-        acc = _Acc(Q, M, D, x.device)
+        sums = _Sums(Q, M, D, x.dtype, x.device)
         dx = torch.empty_like(x)
         n1, n2 = gpk.work_elems(gpk.OP_DET_BWD, N, M, Q, D), gpk.work_elems(gpk.OP_GRAM, N, M, Q, D)
         work = torch.empty(max(n1, n2), dtype=torch.float64, device=x.device)   # one after the other
-        gpk.det_bwd(x, Z, l2, s2, A, kfu, Bk, dm, dv, acc.dsf2, acc.dl, acc.dZ, acc.dA, dx=dx, work=work)
-        gpk.gram(kfu, kfu, dv, acc.dB, work=work)
-        dZ, g_l, g_s, dA, dB = acc.grads(l2, s2, dv, ctx.hyp)
+        gpk.det_layer_bwd(x, Z, l2, s2, A, kfu, Bk, dm, dv, sums.acc, dx, sums.g_l, sums.g_s, sums.cast, work)
+        dZ, g_l, g_s, dA, dB = sums.grads(ctx.hyp)
         return dx, dZ, g_l, g_s, dA, dB
 
 

@@ -109,6 +109,51 @@ int reduce_partials(const double* part, int nparts, const RedPlan& plan, cudaStr
 }
 }  // namespace gpk
 
+// acc = [dsf2 | dl Q | dZ M Q | dA Dout M | dB Dout M M], zeroed
+static int zero_acc(double* acc, int M, int Q, int Dout, long* ncast, cudaStream_t st) {
+  *ncast = (long)M * Q + (long)Dout * M + (long)Dout * M * M;
+  const cudaError_t e = cudaMemsetAsync(acc, 0, (1 + Q + *ncast) * sizeof(double), st);
+  if (e != cudaSuccess) return gpk::fail(GPK_ECUDA, "layer_bwd: %s", cudaGetErrorString(e));
+  return GPK_OK;
+}
+
+extern "C" int gpk_psi_layer_bwd(int prec, int N, int M, int Q, int Dout, const void* mu, const void* var,
+                                 const void* Z, const double* lls2, const double* lsf2, const void* A, const void* B,
+                                 const void* m, const void* dm, const void* dv, double* acc, void* dmu, void* dvar,
+                                 double* g_l, double* g_s, void* cast, double* work, long work_elems, void* stream) {
+  GPK_NVTX("gpk_psi_layer_bwd");
+  GPK_REQUIRE(N >= 0 && M >= 1 && Q >= 1 && Dout >= 1, "psi_layer_bwd: bad sizes N=%d M=%d Q=%d Dout=%d", N, M, Q, Dout);
+  GPK_REQUIRE(acc && work, "psi_layer_bwd: null accumulators or workspace");
+  long nc;
+  int rc = zero_acc(acc, M, Q, Dout, &nc, gpk::as_stream(stream));
+  double *dl = acc + 1, *dZ = dl + Q, *dA = dZ + (long)M * Q, *dB = dA + (long)Dout * M;
+  if (rc == GPK_OK)
+    rc = gpk_psi_bwd_ws(prec, N, M, Q, Dout, mu, var, Z, lls2, lsf2, A, B, m, dm, dv, nullptr, 0, acc, dl, dZ, dA, dB,
+                        dmu, dvar, work, work_elems, stream);
+  if (rc == GPK_OK)
+    rc = gpk_moment_grads(prec, Q, nc, lls2, lsf2, acc, dv, (long)N * Dout, g_l, g_s, cast, stream);
+  return rc;
+}
+
+extern "C" int gpk_det_layer_bwd(int prec, int N, int M, int D, int Dout, const void* x, int ldx, const void* Z,
+                                 const double* lls2, const double* lsf2, const void* A, const void* kfu,
+                                 const void* Bk, const void* dm, const void* dv, double* acc, void* dx, double* g_l,
+                                 double* g_s, void* cast, double* work, long work_elems, void* stream) {
+  GPK_NVTX("gpk_det_layer_bwd");
+  GPK_REQUIRE(N >= 0 && M >= 1 && D >= 1 && Dout >= 1, "det_layer_bwd: bad sizes N=%d M=%d D=%d Dout=%d", N, M, D, Dout);
+  GPK_REQUIRE(acc && work, "det_layer_bwd: null accumulators or workspace");
+  long nc;
+  int rc = zero_acc(acc, M, D, Dout, &nc, gpk::as_stream(stream));
+  double *dl = acc + 1, *dZ = dl + D, *dA = dZ + (long)M * D, *dB = dA + (long)Dout * M;
+  if (rc == GPK_OK)
+    rc = gpk_det_bwd_ws(prec, N, M, D, Dout, x, ldx, Z, lls2, lsf2, A, kfu, Bk, dm, dv, nullptr, acc, dl, dZ, dA, dx,
+                        work, work_elems, stream);
+  if (rc == GPK_OK) rc = gpk_gram_ws(prec, N, M, Dout, kfu, kfu, dv, dB, work, work_elems, stream);
+  if (rc == GPK_OK)
+    rc = gpk_moment_grads(prec, D, nc, lls2, lsf2, acc, dv, (long)N * Dout, g_l, g_s, cast, stream);
+  return rc;
+}
+
 extern "C" int gpk_work_elems(int op, int N, int M, int D, int Dout, long* elems) {
   GPK_NVTX("gpk_work_elems");
   GPK_REQUIRE(elems, "work_elems: null output");
