@@ -519,6 +519,9 @@ __device__ __forceinline__ void stage_pairs(const T* z, const T* inv4l, int Q, i
 __device__ __forceinline__ void lds_two(saddr p, df64& a, df64& b) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.hi), "=f"(a.lo), "=f"(b.hi), "=f"(b.lo) : "r"(p));
 }
+__device__ __forceinline__ void lds_two(saddr p, long long& a, long long& b) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(p));
+}
 __device__ __forceinline__ void lds_two(saddr p, float& a, float& b) {
   asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(p));
 }
@@ -1646,6 +1649,390 @@ __global__ void __launch_bounds__((NS + NF) * 32, NS < 12 ? 2 : 1)
   }
 }
 
+// ---------------------------------------------------------------------------------
+// Rollout in double-float precision: one CTA, T dependent steps, each taking the previous step's
+// moments, so a step's latency is the cost.  Against the general kernel's step (four barriers,
+// logarithms and divisions in sequence, two double-float butterflies; 5.2 us at M = 50, Q = 2):
+//  * the normalisers enter as products of reciprocal square roots (no logarithm, no division), the
+//    point-dependent scale of psi2 multiplying the finished sum;
+//  * every thread that needs the step's constants forms them itself from the summed partials (no
+//    exchange), so a step has two barriers: records ready, partial sums ready.  CH_REC warps form
+//    the records (128 rows at a time; those without rows sit out), CH_PSI1 warps psi1 and its sums
+//    beside them, CH_SWEEP warps the pairs;
+//  * the sums over threads are exact integer sums (in units of 2^-60 of sum |A| or sum |B|, which
+//    bound them): three 32-bit warp reductions a sum for what took five shuffle-and-add levels;
+//  * with up to four pairs a thread, their G and B stay in registers.
+// Measured per step: M = 50, Q = 2: 5.2 -> 2.4 us; M = 100: 9.2 -> 4.5; M = 30, Q = 3: 6.0 -> 4.9;
+// M = 10, Q = 1: 3.8 -> 2.2 (the dependent chain alone).  At M = 50 the issue rate of one SM bounds the
+// pair phase (~5000 instructions a step): twelve sweep warps of four pairs a
+// thread take fewer of them than twenty of two (each warp pays ~100 for its reduction).
+constexpr int CH_REC = 4, CH_PSI1 = 4, CH_SWEEP = 12, CH_KP = 4;
+constexpr int CH_NTH = (CH_REC + CH_PSI1 + CH_SWEEP) * 32;
+// v 2^F as an integer (|v 2^F| < 2^61)
+__device__ __forceinline__ long long fx_dyn(float x, int F) {
+  const unsigned b = __float_as_uint(x);
+  const int s = max(0, min(189 - F - (int)((b >> 23) & 0xffu), 63));
+  const long long v = (long long)(((unsigned long long)(((b & 0x7fffffu) | 0x800000u) << 7) << 32) >> s);
+  return (int)b < 0 ? -v : v;
+}
+// the warp's sum of |x| < 2^61 (so that 32 lanes stay below 2^63 - the caller's scale leaves room)
+__device__ __forceinline__ long long warp_sum_fx(long long x) {
+  const unsigned l0 = (unsigned)x & 0x3ffffffu, l1 = (unsigned)(x >> 26) & 0x3ffffffu;
+  const int l2 = (int)(x >> 52);
+  const unsigned s0 = __reduce_add_sync(0xffffffffu, l0), s1 = __reduce_add_sync(0xffffffffu, l1);
+  const int s2 = __reduce_add_sync(0xffffffffu, l2);
+  return (long long)s0 + ((long long)s1 << 26) + ((long long)s2 << 52);
+}
+// an integer times 2^-F as a double-float
+__device__ __forceinline__ df64 df_of_fx(long long x, int F) {
+  const float h = (float)(int)(x >> 38), m = (float)(int)((x >> 16) & 0x3fffff), l = (float)(int)(x & 0xffff);
+  // 26, 22 and 16 bits; h may round (its error is recovered exactly)
+  const int he = (int)(x >> 38) - __float2int_rn(h);
+  const df64 a = two_sum(__fmul_rn(h, 4194304.f), __fmaf_rn((float)he, 4194304.f, m));   // units of 2^16
+  const df64 r = add(a, __fmul_rn(l, 1.52587890625e-05f));
+  return scale2(scale2(r, 8), 8 - F);
+}
+struct ChSmem {
+  float2* tab;
+  df64 *z, *As, *ell2, *sl, *inv4l, *misc;   // misc: sf2, then a step's normalisers of psi1 and psi2
+  long long* rec;    // [M][rec_len]
+  long long* part;   // [QC][CH_PSI1] sums of m, then [QC][CH_SWEEP] of v
+  long long* G;      // [P]
+  df64* Bs;          // [QC * P]
+  unsigned short* pab;   // [P]
+};
+__host__ __device__ inline size_t chcarve(ChSmem* out, char* base, int M, int QC, int P) {
+  ChSmem s;
+  size_t o = 0;
+  auto take = [&](size_t n) {
+    char* p = base + o;
+    o += n;
+    return p;
+  };
+  s.tab = (float2*)take(kFxTab * sizeof(float2));
+  s.z = (df64*)take((size_t)zlen(QC) * M * 8);
+  s.As = (df64*)take((size_t)QC * M * 8);
+  s.ell2 = (df64*)take(QC * 8);
+  s.sl = (df64*)take(QC * 8);
+  s.inv4l = (df64*)take(QMAX * 8);
+  s.misc = (df64*)take(4 * 8);
+  s.part = (long long*)take((size_t)QC * (CH_PSI1 + CH_SWEEP) * 8);   // (16-byte aligned: read in pairs)
+  s.rec = (long long*)take((size_t)M * rec_len(QC) * 8);
+  s.G = (long long*)take((size_t)P * 8);
+  s.Bs = (df64*)take((size_t)QC * P * 8);
+  s.pab = (unsigned short*)take((size_t)P * 2);
+  if (out) *out = s;
+  return o;
+}
+
+// a sweep thread's pairs of a step outside the fixed-point range (rare, so out of line): the
+// exponents in double-float, psi2 without its point-dependent scale
+template <int QC>
+struct ChSums {
+  df64 v[QC];
+};
+template <int QC>
+__device__ __noinline__ ChSums<QC> chain_general(const double* mu, const double* var, const df64* z, const df64* ell2,
+                                                 const df64* inv4l, const float2* tab, const unsigned short* pab,
+                                                 const df64* Bs, int Q, int p0, int np, int P) {
+  df64 m[QC], c[QC];
+  ChSums<QC> r;
+#pragma unroll
+  for (int q = 0; q < QC; ++q) {
+    const df64 v = df_from_double(q < Q ? var[q] : 0.0);
+    m[q] = df_from_double(q < Q ? mu[q] : 0.0);
+    c[q] = recip(add(ell2[q], add(v, v)));
+    r.v[q] = make_df(0.f);
+  }
+  for (int p = p0; p < P; p += np) {
+    const int ia = pab[p] >> 8, ib = pab[p] & 0xff;
+    df64 x = make_df(0.f);
+#pragma unroll
+    for (int q = 0; q < QC; ++q) {
+      const df64 za = z[ia * zlen(QC) + q], zb = z[ib * zlen(QC) + q];
+      const df64 u = sub(m[q], scale2(add(za, zb), -1)), d = sub(za, zb);
+      x = sub(x, add(mul(mul(u, u), c[q]), mul(mul(d, d), inv4l[q])));
+    }
+    const df64 ps = exp_pair(x, ExpTab{tab});
+#pragma unroll
+    for (int d = 0; d < QC; ++d) acc_fma(r.v[d], Bs[d * P + p], ps);
+  }
+  return r;
+}
+
+template <int QC, bool REGS>
+__global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a) {
+  typedef PairExp<df64> X;
+  constexpr int RL = rec_len(QC), ZL = zlen(QC), NTH = CH_NTH, NTS = CH_SWEEP * 32, KP = CH_KP;
+  extern __shared__ __align__(16) char smem_raw[];
+  const int M = a.M, Q = a.Q, P = M * (M + 1) / 2, T = a.N;
+  ChSmem s;
+  chcarve(&s, smem_raw, M, QC, P);
+  __shared__ int s_flag[2], s_bad, s_amax[QC], s_bmax[QC];
+  __shared__ unsigned long long s_asum[QC], s_bsum[QC];
+  const ExpTab etab{s.tab};
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool sweep_warp = warp >= CH_REC + CH_PSI1, rec_warp = warp < CH_REC;
+  load_exp2_table(s.tab);
+#pragma unroll 1
+  for (int i = tid; i < M * ZL; i += NTH) {
+    const int ia = i / ZL, q = i - ia * ZL;
+    s.z[i] = q < Q ? df_from_double(a.Z[ia * Q + q]) : make_df(0.f);
+  }
+  if (tid < 2) s_flag[tid] = 0;
+  if (tid == 2) s_bad = 0;
+  if (tid < QC) {
+    s_amax[tid] = s_bmax[tid] = 0;
+    s_asum[tid] = s_bsum[tid] = 0;
+  }
+  for (int i = tid; i < QC * (CH_PSI1 + CH_SWEEP); i += NTH) s.part[i] = 0;
+  __syncthreads();
+  if (tid < QC) {
+    const df64 l2 = tid < Q ? exp_tab(df_from_double(a.lls2[tid]), etab) : make_df(1.f);
+    s.ell2[tid] = l2;
+    s.sl[tid] = sqrt_(l2);
+    s.inv4l[tid] = recip(mul(l2, make_df(4.f)));
+  }
+  if (tid == 32) s.misc[0] = exp_tab(df_from_double(a.lsf2[0]), etab);
+#pragma unroll 1
+  for (int i = tid; i < QC * M; i += NTH) {
+    const int d = i / M;
+    const df64 v = d < Q ? df_from_double(a.A[i]) : make_df(0.f);
+    s.As[i] = v;
+    atomicMax(&s_amax[d], __float_as_int(fabsf(v.hi)));
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int p = tid; p < P; p += NTH) {
+    int ia, ib;
+    pair_of(p, ia, ib);
+    s.pab[p] = (unsigned short)((ia << 8) | ib);
+    s.G[p] = pair_G<df64, QC>(s.z + ia * ZL, s.z + ib * ZL, s.inv4l, Q);
+    for (int d = 0; d < QC; ++d) {
+      df64 w = make_df(0.f);
+      if (d < Q) {
+        const double* B = a.B + (size_t)d * M * M;
+        w = df_from_double(B[ia * M + ib]);
+        if (ia != ib) w = add(w, df_from_double(B[ib * M + ia]));
+      }
+      s.Bs[d * P + p] = w;
+      atomicMax(&s_bmax[d], __float_as_int(fabsf(w.hi)));
+    }
+  }
+  __syncthreads();
+  // scales: |sum psi1 A| <= sum |A| and |sum psi2 B| <= sum |B| (psi1, psi2 without their
+  // normalisers are at most 1), summed as integers relative to the largest so that the result does
+  // not depend on the order; non-finite weights poison the result instead
+  int ea[QC], eb[QC];
+  bool bad_w = false;
+#pragma unroll
+  for (int d = 0; d < QC; ++d) {
+    ea[d] = max((s_amax[d] >> 23) - 126, -60);
+    eb[d] = max((s_bmax[d] >> 23) - 126, -60);
+    bad_w |= ea[d] > 128 || eb[d] > 128;
+    // |x| 2^(32 - e), rounded up (x < 2^e)
+    auto up = [](df64 x, int e) { return (unsigned long long)fx_dyn(fabsf(x.hi), 32 - e) + 2ull; };
+    unsigned long long sa = 0, sb = 0;
+    for (int i = tid; i < M; i += NTH) sa += up(s.As[d * M + i], ea[d]);
+    for (int p = tid; p < P; p += NTH) sb += up(s.Bs[d * P + p], eb[d]);
+    if (sa) atomicAdd(&s_asum[d], sa);
+    if (sb) atomicAdd(&s_bsum[d], sb);
+  }
+  __syncthreads();
+  int Fm[QC], Fv[QC];
+#pragma unroll
+  for (int d = 0; d < QC; ++d) {
+    Fm[d] = 60 - (ea[d] - 32 + 64 - __clzll(s_asum[d]));
+    Fv[d] = 60 - (eb[d] - 32 + 64 - __clzll(s_bsum[d]));
+  }
+  if (bad_w && tid == 0) s_bad = 1;
+  const df64 sf2 = s.misc[0], kq = make_df(8.493217826e-01f, 1.769906000e-08f);   // sqrt(log2(e) / 2)
+  // the pairs of a sweep thread, their G and B
+  const int st = tid - (CH_REC + CH_PSI1) * 32;
+  long long g[KP];
+  df64 w[KP][QC];
+  int off[KP];
+  if (REGS && sweep_warp) {
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+      const int p = st + k * NTS;
+      const bool in = p < P;
+      g[k] = in ? s.G[p] : 0;
+      off[k] = in ? s.pab[p] : 0;
+#pragma unroll
+      for (int d = 0; d < QC; ++d) w[k][d] = in ? s.Bs[d * P + p] : make_df(0.f);
+    }
+  }
+  __syncthreads();
+  for (int t = 0; t <= T; ++t) {
+    if (!sweep_warp) {
+      // rows of this thread: from r0 in steps of 128 (a warp without rows only keeps the barriers)
+      const int r0 = rec_warp ? tid : tid - CH_REC * 32;
+      const bool live_warp = (r0 & ~31) < M;
+      df64 m[QC], v[QC];
+#pragma unroll
+      for (int d = 0; d < QC; ++d) m[d] = v[d] = make_df(0.f);
+      if (live_warp) {
+        if (t == 0) {
+#pragma unroll
+          for (int d = 0; d < QC; ++d)
+            if (d < Q) m[d] = df_from_double(a.mu[d]), v[d] = df_from_double(a.var[d]);
+        } else {
+          // ---- the previous step's moments from the partial sums (each warp for itself)
+          const df64 K1 = s.misc[1], F2 = s.misc[2];
+          const bool bad = s_bad != 0;
+          const saddr pm = sm_addr(s.part), pv = pm + QC * CH_PSI1 * 8;
+#pragma unroll
+          for (int d = 0; d < QC; ++d) {
+            long long sm = 0, sv = 0, x0, x1;
+#pragma unroll
+            for (int k = 0; k < CH_PSI1; k += 2) {
+              lds_two(pm + (d * CH_PSI1 + k) * 8, x0, x1);
+              sm += x0 + x1;
+            }
+#pragma unroll
+            for (int k = 0; k < CH_SWEEP; k += 2) {
+              lds_two(pv + (d * CH_SWEEP + k) * 8, x0, x1);
+              sv += x0 + x1;
+            }
+            m[d] = mul(K1, df_of_fx(sm, Fm[d]));
+            v[d] = sub(fma_(F2, df_of_fx(sv, Fv[d]), sf2), mul(m[d], m[d]));
+            if (bad) m[d] = v[d] = make_df(__int_as_float(0x7fffffff));
+          }
+          if (tid == 0) {   // (before the barrier: the general form reads them)
+#pragma unroll
+            for (int d = 0; d < QC; ++d)
+              if (d < Q) {
+                a.m_out[(size_t)(t - 1) * Q + d] = df_to_double_int(m[d]);
+                a.v_out[(size_t)(t - 1) * Q + d] = df_to_double_int(v[d]);
+              }
+          }
+        }
+      }
+      if (t == T) break;
+      if (rec_warp) {
+        df64 r2[QC];
+        if (live_warp) {
+          // ---- this thread's records
+          bool minus = false;
+#pragma unroll
+          for (int q = 0; q < QC; ++q) {
+            const df64 l = s.ell2[q];
+            r2[q] = rsqrt_(add(l, add(v[q], v[q])));
+            minus |= !(v[q].hi >= -1e-6f * l.hi);   // (also NaN)
+          }
+          for (int ia = r0; ia < M; ia += CH_REC * 32) {
+            df64 s2 = make_df(0.f), tq[QC];
+#pragma unroll
+            for (int q = 0; q < QC; ++q) {
+              tq[q] = mul(sub(m[q], s.z[ia * ZL + q]), mul(r2[q], kq));
+              s2 = fma_(tq[q], tq[q], s2);
+            }
+            const bool in = s2.hi < 1e38f && !minus;
+            if (!in) s_flag[t & 1] = 1;
+            const bool live = in && s2.hi <= 127.5f;
+            long long* r = s.rec + ia * RL;
+            r[0] = live ? X::u_of(scale2(neg(s2), -1)) : X::dead_u();
+#pragma unroll
+            for (int q = 0; q < QC; ++q) r[1 + q] = live ? X::t_of(tq[q]) : X::t_of(make_df(0.f));
+          }
+        }
+        __syncthreads();   // records ready
+        if (warp == 0) {
+          df64 F2 = mul(sf2, sf2);
+#pragma unroll
+          for (int q = 0; q < QC; ++q)
+            if (q < Q) F2 = mul(F2, mul(s.sl[q], r2[q]));
+          if (lane == 0) {
+            s.misc[2] = F2;
+            s_flag[(t + 1) & 1] = 0;
+          }
+        }
+      } else {
+        // ---- psi1 and its sums
+        df64 mm[QC], r1[QC], K1 = sf2;
+        if (live_warp) {
+#pragma unroll
+          for (int q = 0; q < QC; ++q) {
+            mm[q] = make_df(0.f);
+            r1[q] = rsqrt_(add(s.ell2[q], v[q]));
+            if (q < Q) K1 = mul(K1, mul(s.sl[q], r1[q]));
+            r1[q] = mul(r1[q], kq);
+          }
+          for (int ia = r0; ia < M; ia += CH_PSI1 * 32) {
+            df64 e = make_df(0.f);
+#pragma unroll
+            for (int q = 0; q < QC; ++q) {
+              const df64 x = mul(sub(m[q], s.z[ia * ZL + q]), r1[q]);
+              e = fma_(x, x, e);
+            }
+            // psi1 / K1 = 2^-e
+            const df64 p1 = e.hi < 126.f ? exp2_fx(fx52_of(neg(e)) + kFxHalf, sm_addr(s.tab))
+                                         : (e.hi >= 126.f ? make_df(0.f) : make_df(__int_as_float(0x7fffffff)));
+#pragma unroll
+            for (int d = 0; d < QC; ++d) acc_fma(mm[d], p1, s.As[d * M + ia]);
+          }
+        }
+        __syncthreads();
+        if (live_warp) {
+#pragma unroll
+          for (int d = 0; d < QC; ++d) {
+            if (!(fabsf(mm[d].hi) < 3e38f)) s_bad = 1;
+            const long long x = warp_sum_fx(fx_dyn(mm[d].hi, Fm[d]) + fx_dyn(mm[d].lo, Fm[d]));
+            if (lane == 0) s.part[d * CH_PSI1 + warp - CH_REC] = x;
+          }
+          if (warp == CH_REC && lane == 0) s.misc[1] = K1;
+        }
+      }
+      __syncthreads();   // partial sums ready
+    } else {
+      if (t == T) break;
+      __syncthreads();
+      const bool general = s_flag[t & 1] != 0;
+      const saddr ar = sm_addr(s.rec), at = sm_addr(s.tab);
+      df64 vv[QC];
+#pragma unroll
+      for (int d = 0; d < QC; ++d) vv[d] = make_df(0.f);
+      if (!general) {
+        if (REGS) {
+          long long arg[KP];
+#pragma unroll
+          for (int k = 0; k < KP; ++k)
+            arg[k] = X::template arg<QC>(ar + (off[k] >> 8) * (RL * 8), ar + (off[k] & 0xff) * (RL * 8), g[k]);
+#pragma unroll
+          for (int k = 0; k < KP; ++k) {
+            const df64 ps = X::ev(arg[k], at);
+#pragma unroll
+            for (int d = 0; d < QC; ++d) acc_fma(vv[d], w[k][d], ps);
+          }
+        } else {
+          for (int p = st; p < P; p += NTS) {
+            const int ab = s.pab[p];
+            const df64 ps = X::ev(X::template arg<QC>(ar + (ab >> 8) * (RL * 8), ar + (ab & 0xff) * (RL * 8), s.G[p]), at);
+#pragma unroll
+            for (int d = 0; d < QC; ++d) acc_fma(vv[d], s.Bs[d * P + p], ps);
+          }
+        }
+      } else {
+        // outside the fixed-point range: from the moments as they were written out
+        const ChSums<QC> r = chain_general<QC>(t ? a.m_out + (size_t)(t - 1) * Q : a.mu,
+                                               t ? a.v_out + (size_t)(t - 1) * Q : a.var, s.z, s.ell2, s.inv4l, s.tab,
+                                               s.pab, s.Bs, Q, st, NTS, P);
+#pragma unroll
+        for (int d = 0; d < QC; ++d) vv[d] = r.v[d];
+      }
+#pragma unroll
+      for (int d = 0; d < QC; ++d) {
+        const df64 x = acc_done(vv[d]);
+        if (!(fabsf(x.hi) < 3e38f)) s_bad = 1;
+        const long long f = warp_sum_fx(fx_dyn(x.hi, Fv[d]) + fx_dyn(x.lo, Fv[d]));
+        if (lane == 0) s.part[QC * CH_PSI1 + d * CH_SWEEP + warp - CH_REC - CH_PSI1] = f;
+      }
+      __syncthreads();
+    }
+  }
+}
+
 template <typename T, int NPB, int PPT, int QC, int DB>
 int run_fwd_gen(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) {
   PsiArgs<typename Num<T>::store_t> a = a_in;
@@ -1670,6 +2057,21 @@ int run_fwd_gen(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) 
   return gpk::check_launch("psi_fwd");
 }
 
+// the double-float rollout kernel, or -1 where its tables do not fit
+template <int QC>
+int run_chain(const PsiArgs<double>& a, cudaStream_t st) {
+  const int P = a.M * (a.M + 1) / 2;
+  const size_t sm = chcarve(nullptr, nullptr, a.M, QC, P);
+  if (sm > SMEM_CAP || a.M > 255) return -1;
+  if (a.N < 1) return GPK_OK;
+  auto k = P <= CH_KP * CH_SWEEP * 32 ? psi_chain_kernel<QC, true> : psi_chain_kernel<QC, false>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  k<<<1, CH_NTH, sm, st>>>(a);
+  return gpk::check_launch("psi_rollout");
+}
+template <int QC>
+int run_chain(const PsiArgs<float>&, cudaStream_t) { return -1; }
+
 // points per pass: 4 for Dout <= 2, 2 for Dout <= 4 (so 2*NPB*Dout sums fit one reduction)
 template <typename T, int QC>
 int fwd_gen(const PsiArgs<typename Num<T>::store_t>& a, bool sum, bool contract, int P, cudaStream_t st) {
@@ -1678,6 +2080,8 @@ int fwd_gen(const PsiArgs<typename Num<T>::store_t>& a, bool sum, bool contract,
     return run_fwd_gen<T, 2, 16, QC, 4>(a, st);
   }
   if (a.chain) {   // one point per pass: each point needs the previous one's moments
+    const int rc = run_chain<QC == 2 ? 2 : 4>(a, st);
+    if (rc != -1) return rc;
     if (a.Dout == 1) return run_fwd_gen<T, 1, 0, QC, 1>(a, st);
     if (a.Dout == 2) return run_fwd_gen<T, 1, 0, QC, 2>(a, st);
     return run_fwd_gen<T, 1, 0, QC, 4>(a, st);

@@ -126,3 +126,42 @@ def test_psi_nan_stays_with_its_point():
     assert np.isnan(res[1][0][2]) and np.isnan(res[1][1][2])
     for a, b in zip(*res):
         assert_close(b[ok], a[ok], 1e-12)
+
+
+@pytest.mark.parametrize('M,Q', [(1, 1), (3, 2), (50, 2), (51, 2), (49, 3), (100, 4), (110, 1)])
+@pytest.mark.parametrize('kind', ['plain', 'far', 'negative_variance'])
+def test_psi_rollout_vs_oracle(M, Q, kind):
+    """Twelve dependent steps against the oracle's psi statistics; the first from an ordinary state,
+    one whose distances underflow every psi2, or one with a slightly negative variance."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(7 * M + Q)
+    Z = rng.uniform(-2, 2, (M, Q))
+    lls2, lsf2 = 2 * rng.uniform(-0.6, 0.2, Q), np.array([0.2])
+    A = rng.randn(Q, M) / np.sqrt(M)
+    B = rng.randn(Q, M, M) / M
+    B = 0.1 * (B + B.transpose(0, 2, 1))
+    mu, S = rng.randn(Q), np.exp(rng.uniform(-3, 0, Q))
+    if kind == 'far':
+        mu[0], S = 60.0, 1e-3 * S
+    if kind == 'negative_variance':
+        S[0] = -0.03 * np.exp(lls2[0])
+    T, sf2 = 12, float(np.exp(lsf2[0]))
+    ms, vs, m, v = [], [], mu[None], S[None]
+    for _ in range(T):
+        p1, p2 = O.psi_stats(lls2, lsf2, m, v, Z)
+        m = p1 @ A.T
+        v = sf2 + np.einsum('dab,nab->nd', B, p2) - m ** 2
+        ms.append(m[0])
+        vs.append(v[0])
+    gm, gv = gpk.psi_rollout(dev(mu), dev(S), dev(Z), dev(lls2), dev(lsf2), dev(A), dev(B), T)
+    # (a drawn layer may drive its variance below -l/2, from where on the statistics are NaN)
+    ok = int(np.isfinite(np.array(ms)).all(1).cumprod().sum())
+    assert_close(gm.cpu().numpy()[:ok], np.array(ms)[:ok], TOL, 'm')
+    assert_close(gv.cpu().numpy()[:ok], np.array(vs)[:ok], TOL, 'v')
+    assert ok >= 1 and not bool(torch.isfinite(gm[ok:]).all(1).any())
+    m1, v1 = gpk.psi_rollout(dev(mu), dev(S), dev(Z), dev(lls2), dev(lsf2), dev(A), dev(B), 1)
+    assert torch.equal(m1[0], gm[0]) and torch.equal(v1[0], gv[0])
+    bad = mu.copy()
+    bad[0] = np.nan
+    gm, gv = gpk.psi_rollout(dev(bad), dev(S), dev(Z), dev(lls2), dev(lsf2), dev(A), dev(B), 3)
+    assert bool(torch.isnan(gm).all()) and bool(torch.isnan(gv).all())
