@@ -108,6 +108,39 @@ long det_bwd_work_elems(int N, int M, int D, int Dout);
 long gram_work_elems(int N, int M, int Dout);
 long trace_kzz_work_elems(int M, int Q);
 
+// Shared memory by 32-bit addresses, for inner loops (through table pointers every access costs a
+// 64-bit address computation of two integer instructions)
+typedef unsigned saddr;
+__device__ __forceinline__ saddr sm_addr(const void* p) { return (saddr)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ int2 lds_i2(saddr a) {
+  int2 v;
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void lds(saddr a, long long& v) { asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(saddr a, df64& v) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.hi), "=f"(v.lo) : "r"(a));
+}
+__device__ __forceinline__ void lds(saddr a, float& v) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
+__device__ __forceinline__ void lds_st(saddr a, double& v) { asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
+__device__ __forceinline__ void lds_st(saddr a, float& v) { lds(a, v); }
+__device__ __forceinline__ int lds_u16(saddr a) {
+  unsigned short v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts(saddr a, df64 v) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.hi), "f"(v.lo) : "memory");
+}
+__device__ __forceinline__ void sts(saddr a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts(saddr a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
+template <typename V>
+__device__ __forceinline__ V ldsv(saddr a) {
+  V v;
+  lds(a, v);
+  return v;
+}
+
 // Pair p of the row-major lower triangle, p = a (a + 1) / 2 + b with 0 <= b <= a.
 __host__ __device__ __forceinline__ void tri_pair(int p, int& a, int& b) {
 #ifdef __CUDA_ARCH__

@@ -20,20 +20,23 @@ struct __align__(8) df64 {   // 8-byte alignment: an element in memory is one ac
 
 __host__ __device__ __forceinline__ df64 make_df(float h, float l = 0.f) { df64 r; r.hi = h; r.lo = l; return r; }
 
-// float64 -> (hi, lo): hi = x rounded to float, lo = (x - hi) rounded to float.  Done with
-// integer operations on the bit pattern (round-to-nearest-even of the 53-bit significand to
-// 24 bits, then the signed remainder normalised to 24 bits): the FP64 pipe, which the plain
-// conversion would use, issues ~64x slower than the integer pipes on this part.  Zeros are
-// taken directly (lo may come out subnormal); values whose hi would not be a normal float
-// (|x| < 2^-126 or >= 2^128, inf, nan) take the FP64 path.
-// Kept out of line: inlined, the compiler if-converts the rare branch that calls it and runs
-// its FP64 instructions for every conversion.
+// float64 -> (hi, lo): hi = x rounded to float, lo = (x - hi) rounded to float, by integer operations
+// on the bit pattern: the FP64 pipe, which the plain conversion would use, issues ~64x slower than
+// the integer pipes on this part.  hi is the pattern rounded to 24 bits (nearest even) with its
+// exponent field lowered; lo is the remainder, at most 2^28 units of x's last place, converted by the
+// 32-bit conversion (the same rounding) with its exponent field lowered: ~16 instructions where
+// normalising and rounding the remainder by hand took 45.  Zeros, and values whose lo could
+// be subnormal or hi not a normal float (|x| < 2^-74 or >= 2^128, inf, nan), are left to
+// df_from_double_rest, out of line: inlined, the compiler if-converts the rare branch and runs its
+// instructions for every conversion.
 static __device__ __noinline__ df64 df_from_double_fp64(double x) {
   float h = __double2float_rn(x);
   float l = __double2float_rn(x - (double)h);
   return make_df(h, l);
 }
-__device__ __forceinline__ df64 df_from_double(double x) {
+// the same with every rounding step in integers, for any normal hi (lo may come out subnormal); the
+// FP64 path for the rest
+static __device__ __noinline__ df64 df_from_double_rest(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int e = (int)((b >> 52) & 0x7ff);
   if ((b << 1) == 0ull) return make_df(__int_as_float((int)(b >> 32)), 0.f);   // +-0
@@ -95,6 +98,19 @@ __device__ __forceinline__ df64 df_from_double(double x) {
     }
   }
   return make_df(hi, lo);
+}
+__device__ __forceinline__ df64 df_from_double(double x) {
+  const unsigned hw = (unsigned)__double2hiint(x), lw = (unsigned)__double2loint(x);
+  const int e = (int)((hw >> 20) & 0x7ff);
+  if (e < 949 || e > 1150) {
+    if (((hw << 1) | lw) == 0u) return make_df(__int_as_float((int)hw), 0.f);   // +-0
+    return df_from_double_rest(x);
+  }
+  const unsigned long long m = ((unsigned long long)(hw & 0x7fffffffu) << 32) | lw;
+  const unsigned top = (unsigned)((m + 0x0fffffffull + ((m >> 29) & 1u)) >> 29);   // (mod 2^32: the field's excess)
+  const float g = (float)(int)(lw - (top << 29));
+  const unsigned lo = g == 0.f ? 0u : (__float_as_uint(g) + ((unsigned)(e - 1075) << 23)) ^ (hw & 0x80000000u);
+  return make_df(__uint_as_float((top - (896u << 23)) | (hw & 0x80000000u)), __uint_as_float(lo));
 }
 __device__ __forceinline__ double df_to_double(df64 a) { return (double)a.hi + (double)a.lo; }
 
@@ -277,6 +293,11 @@ __device__ __forceinline__ void load_exp2_table(float2* s_tab) {
     s_tab[k] = make_float2(r.hi, r.lo);
   }
 }
+// the 256-entry exp table of exp_tab inside that table (every 8th entry)
+struct ExpTab {
+  const float2* p;
+  __device__ __forceinline__ float2 operator[](int j) const { return p[8 * j]; }
+};
 // 2^(x's fraction) as h + l, h in (0.999, 2); tab: the table's shared-memory address
 __device__ __forceinline__ df64 exp2_fx_frac(long long x, unsigned tab) {
   const unsigned xl = (unsigned)x;
@@ -310,6 +331,8 @@ __device__ __forceinline__ df64 exp2_fx(long long x, unsigned tab) {
 }
 // the same as a float64, by integer operations: h's bits widened, l added in units of h's last
 // float64 place (below 1 the unit halves; h = 1 with a negative l counts as below)
+// results below 2^MINE are flushed to zero
+template <int MINE = -126>
 __device__ __forceinline__ double exp2_fx_double(long long x, unsigned tab) {
   const df64 r = exp2_fx_frac(x, tab);
   const int xh = (int)(x >> 32);
@@ -317,7 +340,7 @@ __device__ __forceinline__ double exp2_fx_double(long long x, unsigned tab) {
   const int li = __float2int_rn(__fmul_rn(r.lo, below ? 9007199254740992.f : 4503599627370496.f));
   const unsigned hb = __float_as_uint(r.hi);
   long long d = ((long long)hb << 29) + ((896LL + (xh >> 20)) << 52) + li;
-  return __longlong_as_double(xh >= -(126 << 20) ? d : 0LL);
+  return __longlong_as_double(xh >= MINE * (1 << 20) ? d : 0LL);
 }
 // x 2^F truncated to an integer (|x 2^F| < 2^63, the exponent field at most 189 - F), by shifting
 // the significand: the float-to-64-bit-integer conversion issues on the FP64 pipe, 16 cycles a warp
@@ -335,6 +358,14 @@ __device__ __forceinline__ long long fx57_words_of(df64 v) {
   const long long t = fx_bits<57>(v.hi) + fx_bits<57>(v.lo) + (1LL << 30);
   const int high = (int)(t >> 31), low = (int)((unsigned)t & 0x7fffffffu) - (1 << 30);
   return ((long long)high << 32) | (unsigned)low;
+}
+// a float64 in units of 2^-57, truncated (|v| < 64; the caller checks)
+__device__ __forceinline__ long long fx57_of_double(double v) {
+  const long long b = __double_as_longlong(v);
+  const int s = 1018 - (int)((b >> 52) & 0x7ff);   // v = m 2^(e - 1075): m 2^-s units
+  const long long m = (b & 0xfffffffffffffLL) | 0x10000000000000LL;
+  const long long t = s >= 0 ? m >> min(s, 63) : m << -max(s, -9);
+  return b < 0 ? -t : t;
 }
 // hi + lo as a float64 by integer operations (df_to_double's three FP64-pipe instructions take 48
 // cycles a warp): hi's bits widened, lo added in units of hi's last float64 place (half of it
@@ -403,6 +434,13 @@ template <typename Tab> __device__ __forceinline__ df64 exp_pair(df64 x, const T
 template <typename Tab> __device__ __forceinline__ float exp_pair(float x, const Tab&) { return __expf(x); }
 
 __device__ __forceinline__ float log2e_of(float) { return 1.44269504f; }
+// a b + c of 32-bit factors in one instruction (from C, the compiler widens the factors to 64 bits
+// first: three multiply-adds and two shifts a product)
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
 // max that returns NaN when either is NaN
 __device__ __forceinline__ float fmax_nan(float a, float b) { return (a != a || b != b) ? __int_as_float(0x7fffffff) : fmaxf(a, b); }
 

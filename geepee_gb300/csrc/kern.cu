@@ -25,9 +25,9 @@ __device__ void load_hyp(Hyp<T>& h, const double* lls2, const double* lsf2, int 
   }
 }
 
-// K[n,m] = exp(lsf - 1/2 sum_d (x-z)^2 / l_d) (+ jitter on the diagonal).  A CTA takes KR rows
-// and KC columns: those rows of x and columns' Z arrive in shared memory by asynchronous copies
-// and are converted once (not once per element), then 256 threads sweep the KR x KC block.
+// K[n,m] = exp(lsf - 1/2 sum_d (x-z)^2 / l_d) (+ jitter on the diagonal): FP32, and matrices with a jitter.  A CTA takes KR rows
+// and KC columns: those rows of x and columns' Z arrive in shared memory by asynchronous copies,
+// then 256 threads sweep the KR x KC block.
 constexpr int KR = 8, KC = 128;
 template <typename T>
 __global__ void __launch_bounds__(256) kern_matrix_kernel(int N, int M, int D, const typename Num<T>::store_t* x,
@@ -45,17 +45,11 @@ __global__ void __launch_bounds__(256) kern_matrix_kernel(int N, int M, int D, c
   const int nr = min(KR, N - n0), nc = min(KC, M - m0);
   for (int e = tid; e < nr * D; e += 256) {
     const int r = e / D, d = e - r * D;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(reinterpret_cast<S*>(xs) + e);
-    const S* src = x + (size_t)(n0 + r) * ldx + d;
-    if (sizeof(S) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src));
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src));
+    async_copy(reinterpret_cast<S*>(xs) + e, x + (size_t)(n0 + r) * ldx + d);
   }
   for (int e = tid; e < nc * D; e += 256) {
     const int c = e / D, d = e - c * D;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(reinterpret_cast<S*>(zs) + e);
-    const S* src = z + (size_t)(m0 + c) * ldz + d;
-    if (sizeof(S) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src));
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst), "l"(src));
+    async_copy(reinterpret_cast<S*>(zs) + e, z + (size_t)(m0 + c) * ldz + d);
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
   load_exp_table(tab);
@@ -75,6 +69,150 @@ __global__ void __launch_bounds__(256) kern_matrix_kernel(int N, int M, int D, c
     T k = exp_tab(sub(h->lsf, scale2(rr, -1)), tab);
     if (jitter != 0.0 && n == m) k = add(k, Num<T>::ld(static_cast<S>(jitter)));
     K[(size_t)n * ldk + m] = Num<T>::st(k);
+  }
+}
+
+// ---- the kernel matrix in double-float precision, exponents in fixed point ----
+// log2 K[n,m] = log2 sf^2 - sum_d (x'_nd - z'_md)^2 with the coordinates x' = x sqrt(log2(e)/2) / ell
+// as two words, high 2^-26 + low 2^-57: a difference is two integer subtractions, exact, and its
+// square two 32 x 32 -> 64-bit multiply-adds (the low word's square, at most 2^-52, is left out), where
+// the double-float difference, square and scaling take 32 instructions; the exponential then comes from
+// the exponent's bits (exp2_fx).  The sums are taken modulo 2^64 and a float sum of the squares beside them
+// says which are meant: at 256 or more the entry is zero (below 2^-128 with sf^2 < 2^126), below
+// it no sum leaves the range.  A coordinate outside +-16 (or not finite) has NaN for its float, which
+// sends the entries it meets to the double-float form (ard_general).
+struct __align__(16) ArdHyp {
+  double s[DMAXK];      // sqrt(log2(e)/2) / ell_d
+  df64 inv_l2[DMAXK];   // 1/ell_d^2 (general form)
+  df64 lsf, sf2;
+  long long c0;         // log2 sf^2 in units of 2^-52, plus exp2_fx's half step
+  int flag;             // sf^2 outside the fixed-point range: every entry takes the general form
+};
+__device__ __forceinline__ void load_ard(ArdHyp& h, const double* lls2, const double* lsf2, int D, ExpTab tab) {
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    const double l = lls2[d];
+    h.s[d] = exp(-0.5 * l) * 0.84932180028801904272;   // times sqrt(log2(e)/2); (in float64: its error counts twice the exponent)
+    h.inv_l2[d] = exp_tab(df_from_double(-l), tab);
+  }
+  if (threadIdx.x == 32) {
+    h.lsf = df_from_double(lsf2[0]);
+    h.sf2 = exp_tab(h.lsf, tab);
+    const double c = lsf2[0] * 1.4426950408889634074;
+    h.flag = !(fabs(c) < 126.0);
+    h.c0 = (h.flag ? 0LL : __double2ll_rn(c * 4503599627370496.0)) + kFxHalf;
+  }
+}
+// a coordinate in fixed point: (low, high, float, -)
+__device__ __forceinline__ int4 ard_coord(double x, double s) {
+  const double v = x * s;
+  const int e = (int)((__double_as_longlong(v) >> 52) & 0x7ff);
+  if (e >= 1027) return make_int4(0, 0, 0x7fffffff, 0);   // |v| >= 16, infinite or NaN
+  const long long t = fx57_of_double(v) + (1LL << 30);
+  const int h = (int)(t >> 31);
+  return make_int4((int)((unsigned)t & 0x7fffffffu) - (1 << 30), h, __float_as_int(__fmul_rn((float)h, 1.490116119e-08f)), 0);
+}
+__device__ __forceinline__ int4 lds_i4(saddr a) {
+  int4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+// the exponents X and float sums of squares f of R rows against one column, D coordinates each:
+// x + i * xstep (row i) and z
+template <int R>
+__device__ __forceinline__ void ard_exponents(saddr x, saddr xstep, saddr z, int D, long long c0, long long (&X)[R],
+                                              float (&f)[R]) {
+  long long mid[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) X[i] = c0, mid[i] = 0, f[i] = 0.f;
+#pragma unroll 4
+  for (int d = 0; d < D; ++d) {
+    const int4 zd = lds_i4(z);
+    z += 16;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int4 xd = lds_i4(x + i * xstep);
+      const int h = xd.y - zd.y, l = xd.x - zd.x;
+      const float t = __int_as_float(xd.z) - __int_as_float(zd.z);
+      X[i] = mad_wide(-h, h, X[i]);
+      mid[i] = mad_wide(h, l, mid[i]);
+      f[i] = __fmaf_rn(t, t, f[i]);
+    }
+    x += 16;
+  }
+#pragma unroll
+  for (int i = 0; i < R; ++i) X[i] -= mid[i] >> 30;
+}
+__device__ __noinline__ df64 ard_general(const double* x, const double* z, int D, const ArdHyp& h, const float2* tab) {
+  df64 rr = make_df(0.f);
+  for (int d = 0; d < D; ++d) {
+    const df64 df = sub(df_from_double(x[d]), df_from_double(z[d]));
+    rr = fma_(mul(df, df), h.inv_l2[d], rr);
+  }
+  return exp_tab(sub(h.lsf, scale2(rr, -1)), ExpTab{tab});
+}
+
+// K (float64): a CTA takes FC columns and row tiles of FR; a thread one column and FR / (256 / FC) rows,
+// four at a time, so that a column's coordinate is loaded once for four rows.  As many CTAs as
+// are resident at once share the tiles: the tables and the columns are staged once a CTA.
+// Bound by the integer and FP32 pipes: 20000 x 100, D = 8 in 27 us (49 before), 20000 x 200, D = 16 in
+// 66 us (256 before).
+constexpr int FR = 16, FC = 128, FCTA = 3;
+__global__ void __launch_bounds__(256, FCTA) kern_fx_kernel(int N, int M, int D, const double* x, int ldx,
+                                                            const double* z, int ldz, const double* lls2,
+                                                            const double* lsf2, double* K, int ldk) {
+  extern __shared__ __align__(16) char smem_raw[];
+  float2* tab = reinterpret_cast<float2*>(smem_raw);
+  ArdHyp* h = reinterpret_cast<ArdHyp*>(smem_raw + kFxTab * sizeof(float2));
+  int4* xs = reinterpret_cast<int4*>(h + 1);             // [2][FR][D]: this tile's and the next one's
+  const int DZ = D | 1;                                  // (odd: the columns' banks differ)
+  int4* zs = xs + 2 * FR * D;                            // [FC][DZ]
+  const int tid = threadIdx.x;
+  const int nmb = (M + FC - 1) / FC, m0 = (int)(blockIdx.x % nmb) * FC, nc = min(FC, M - m0);
+  const int ntile = (N + FR - 1) / FR, step = (int)(gridDim.x / nmb);
+  load_exp2_table(tab);
+  __syncthreads();
+  load_ard(*h, lls2, lsf2, D, ExpTab{tab});
+  __syncthreads();
+  auto rows = [&](int tile, int b) {
+    const int n0 = tile * FR, nr = min(FR, N - n0);
+    for (int e = tid; e < nr * D; e += 256) {
+      const int r = e / D, d = e - r * D;
+      xs[b * FR * D + e] = ard_coord(x[(size_t)(n0 + r) * ldx + d], h->s[d]);
+    }
+  };
+  for (int e = tid; e < nc * D; e += 256) {
+    const int c = e / D, d = e - c * D;
+    zs[c * DZ + d] = ard_coord(z[(size_t)(m0 + c) * ldz + d], h->s[d]);
+  }
+  rows((int)(blockIdx.x / nmb), 0);
+  __syncthreads();
+  const int c = tid & (FC - 1), m = m0 + c;
+  const saddr at = sm_addr(tab), az = sm_addr(zs + c * DZ);
+  const bool hf = h->flag;
+  int b = 0;
+  for (int tile = (int)(blockIdx.x / nmb); tile < ntile; tile += step, b ^= 1) {
+    const int n0 = tile * FR, nr = min(FR, N - n0);
+    if (tile + step < ntile) rows(tile + step, b ^ 1);
+    if (c < nc) {
+      for (int r0 = (tid >> 7) * 4; r0 < nr; r0 += 8) {
+        long long X[4];
+        float f[4];
+        // rows past nr read the tile's stale coordinates; their entries are not stored
+        ard_exponents<4>(sm_addr(xs + (b * FR + r0) * D), D * 16, az, D, h->c0, X, f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int n = n0 + r0 + i;
+          if (r0 + i < nr) {
+            double k = exp2_fx_double<-1022>(X[i], at);
+            if (!(f[i] < 256.f) || hf)
+              k = f[i] >= 256.f && !hf ? 0.0
+                                       : df_to_double(ard_general(x + (size_t)n * ldx, z + (size_t)m * ldz, D, *h, tab));
+            K[(size_t)n * ldk + m] = k;
+          }
+        }
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -239,7 +377,7 @@ __global__ void __launch_bounds__(CT) det_contract_kernel(int N, int M, int Dout
                                                           const typename Num<T>::store_t* B,
                                                           typename Num<T>::store_t* Bk,
                                                           typename Num<T>::store_t* m_out,
-                                                          typename Num<T>::store_t* v_out, int b_pairs) {
+                                                          typename Num<T>::store_t* v_out) {
   typedef typename Num<T>::store_t S;
   extern __shared__ __align__(16) char smem_raw[];
   float2* tab = reinterpret_cast<float2*>(smem_raw);
@@ -254,7 +392,7 @@ __global__ void __launch_bounds__(CT) det_contract_kernel(int N, int M, int Dout
   stage_async(reinterpret_cast<S*>(kr), kfu + (size_t)n0 * M, (long)nr * M, tid, CT);
   load_exp_table(tab);
   __syncthreads();
-  if (!b_pairs) convert_in_place(Bs, nB, tid, CT);   // pairs arrive in the compute type already
+  convert_in_place(Bs, nB, tid, CT);
   convert_in_place(kr, (long)nr * M, tid, CT);
   __syncthreads();
   const bool live = n < N;   // warp-uniform; a dead row still reaches the barrier below
@@ -321,6 +459,300 @@ __global__ void __launch_bounds__(CT) det_contract_kernel(int N, int M, int Dout
 
 size_t det_contract_smem(int M, int Dout, size_t tsz) {
   return 256 * sizeof(float2) + ((size_t)Dout * M * M + (size_t)CR * M + 2 * CR * DO_MAX * 2) * tsz;
+}
+
+// ---- the deterministic layer's contraction in double-float precision on the tensor cores ----
+// For rows n and one output d:  Bk_nb = sum_a B[a,b] k_na,  m_n = k_n . A,  v_n = sf2 + k_n . Bk_n, from
+// the kernel rows k.  A is column M of B.  Each row of k and each column of B is scaled by a power of two
+// to less than 1/2 and rounded to 53 bits below the point; the integer is cut into six balanced digits of
+// nine bits (each an exact f16), and a product of two such numbers is the digit products of levels
+// i + j <= 6: 26 f16 multiply-adds into f32.  Digit products are at most 2^16, so an accumulator that takes
+// at most two of them over 128 terms holds an integer of at most 2^24: the sums of levels 0 to 4 are exact
+// (nine accumulators; a longer contraction is folded into 64-bit integers every 128 terms).  Levels 5
+// and 6 have one accumulator each, whose last place is below 2^-56 of the largest product.  What is left is
+// the rounding to 53 bits, in place of a double-float multiply-add (14 instructions, every term rounded).
+// A CTA of 16 warps takes R = 16 nrt rows at a time, B's digits resident in shared memory in the order
+// of the matrix instruction's fragments (restaged by column blocks per row chunk when they do not fit);
+// a warp takes 16 x 8 results at a time.  v is summed in an order that depends on M alone, so a row's
+// results are the same in any batch.
+// One-off staging of B (~9 us at M = 100), then per 32 rows ~5500 cycles of digits, ~16000 of products (the
+// matrix pipe itself ~10000) and ~6000 of epilogue.  With the rows' kernel launch before it, N = 20000,
+// M = 100, two outputs take 168 us (752 before); N = 777, M = 200 74 us (159); the contraction
+// alone at N = 1000, M = 100 21 us (27).
+constexpr int DM_T = 512, DM_W = DM_T / 32, DM_S = 6;
+// an integer (|x| < 2^61) times 2^-F as a double-float
+__device__ __forceinline__ df64 df_of_int(long long x, int F) {
+  const float h = (float)(int)(x >> 38), m = (float)(int)((x >> 16) & 0x3fffff), l = (float)(int)(x & 0xffff);
+  const df64 a = two_sum(__fmul_rn(h, 4194304.f), m);   // all three are exact; units of 2^16
+  return scale2(scale2(add(a, __fmul_rn(l, 1.52587890625e-05f)), 8), 8 - F);
+}
+// a float in units of 2^-F, truncated (the exponent field at most 189 - F)
+__device__ __forceinline__ long long fx_bits_by(float x, int F) {
+  const unsigned b = __float_as_uint(x);
+  const int e = (int)((b >> 23) & 0xffu), s = e == 0 ? 63 : min(189 - F - e, 63);
+  const long long v = (long long)(((unsigned long long)(((b & 0x7fffffu) | 0x800000u) << 7) << 32) >> s);
+  return (int)b < 0 ? -v : v;
+}
+// v 2^(-1 - ex), less than 1/2 in magnitude, in units of 2^-53, rounded
+__device__ __forceinline__ long long digits_of(double v, int ex) {
+  const long long b = __double_as_longlong(v);
+  const int be = (int)((b >> 52) & 0x7ff), sh = 1023 + ex - be;   // at least 1
+  const long long w = (b & 0xfffffffffffffLL) | 0x10000000000000LL;
+  const long long x = sh > 60 || be == 0 ? 0 : (w + (1LL << (sh - 1))) >> sh;
+  return b < 0 ? -x : x;
+}
+// two numbers' digits (|t| <= 2^52, units of 2^-53, t0 in the low half), most significant first
+__device__ __forceinline__ void digit_pairs(long long t0, long long t1, unsigned (&w)[DM_S]) {
+  const long long bias = 256LL * (1 + (1LL << 9) + (1LL << 18) + (1LL << 27) + (1LL << 36) + (1LL << 45));
+  t0 += bias;
+  t1 += bias;
+  const unsigned l0 = (unsigned)t0 & 0x7ffffffu, l1 = (unsigned)t1 & 0x7ffffffu;
+  const unsigned h0 = (unsigned)(t0 >> 27), h1 = (unsigned)(t1 >> 27);
+#pragma unroll
+  for (int j = 0; j < DM_S; ++j) {
+    const unsigned a = j < 3 ? h0 : l0, b = j < 3 ? h1 : l1;
+    const int sh = 9 * (2 - j % 3);
+    unsigned e = ((a >> sh) & 511u) | ((b >> sh) & 511u) << 16 | 0x64006400u;   // halves 1024 + digit + 256
+    asm("sub.rn.f16x2 %0, %0, %1;" : "+r"(e) : "r"(0x65006500u));               // minus 1280
+    w[j] = e;
+  }
+}
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint4 a, const uint2 b) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y));
+}
+// the accumulator of digits i of the left and j of the right operand
+constexpr int DM_ACC = 11;
+__host__ __device__ constexpr int dm_acc(int i, int j) {
+  const int base[7] = {0, 1, 2, 4, 6, 9, 10};
+  return base[i + j] + (i + j < 5 ? i / 2 : 0);
+}
+// the accumulators' value of result j, in units of 2^-52 of the scaled operands' product in units of 2^-106
+__device__ __forceinline__ long long dm_fold(const float (&acc)[DM_ACC][4], int j) {
+  auto S = [&](int i) { return __float2int_rn(acc[i][j]); };
+  const int s6 = __float2int_rn(__fmul_rn(acc[10][j], 1.f / 512));
+  const long long X = mad_wide(S(0), 1 << 18, mad_wide(S(1), 1 << 9, (long long)(S(2) + S(3))));
+  const long long Y = mad_wide(S(4) + S(5), 1 << 18, mad_wide(S(6) + S(7) + S(8), 1 << 9, (long long)(S(9) + s6)));
+  return (X << 20) + (Y >> 7);
+}
+// one k step: all digit products of a row fragment and a column fragment (strides in fragments)
+__device__ __forceinline__ void dm_step(float (&acc)[DM_ACC][4], const uint4* fa, int sa, const uint2* fb, int sb) {
+  uint4 va[DM_S];
+#pragma unroll
+  for (int i = 0; i < DM_S; ++i) va[i] = fa[(size_t)i * sa];
+#pragma unroll
+  for (int j = 0; j < DM_S; ++j) {
+    const uint2 vb = fb[(size_t)j * sb];
+#pragma unroll
+    for (int i = 0; i < DM_S; ++i)
+      if (i + j <= 6) mma_f16(acc[dm_acc(i, j)], va[i], vb);
+  }
+}
+struct DmSmem {
+  unsigned *B, *A;      // digit pairs: [digit][column tile][k step][lane][2], [digit][row tile][k step][lane][4]
+  df64 *k, *vp, *v;     // [R][M|1] the rows, [R][NT] parts of v, [R] v
+  int *rexp, *bexp;
+};
+__host__ __device__ inline size_t dm_carve(DmSmem* out, char* base, int M, int NB, int R) {
+  DmSmem s;
+  size_t o = 0;
+  auto take = [&](size_t n) {
+    char* p = base + o;
+    o += (n + 15) & ~(size_t)15;
+    return p;
+  };
+  const int KP = (M + 15) & ~15;
+  s.B = (unsigned*)take((size_t)DM_S * NB * KP * 2);
+  s.A = (unsigned*)take((size_t)DM_S * R * KP * 2);
+  s.k = (df64*)take((size_t)R * (M | 1) * 8);
+  s.vp = (df64*)take((size_t)R * (NB / 8) * 8);
+  s.v = (df64*)take((size_t)R * 8);
+  s.rexp = (int*)take((size_t)R * 4);
+  s.bexp = (int*)take((size_t)NB * 4);
+  if (out) *out = s;
+  return o;
+}
+constexpr int DM_BAD = 1 << 20;   // exponent of a row or column with a non-finite entry
+constexpr int DM_MAX = 255;       // largest M: four pairs a lane, sums below 2^61
+
+__global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout, const double* lsf2, const double* A,
+                                                          const double* B, int b_pairs, const double* kin, double* Bk,
+                                                          double* m_out, double* v_out, int NB, int nrt) {
+  extern __shared__ __align__(16) char smem_raw[];
+  const int R = 16 * nrt, KS = (M + 15) >> 4, NT = NB >> 3, MP = M | 1;
+  DmSmem s;
+  dm_carve(&s, smem_raw, M, NB, R);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = blockIdx.y;
+  const int nblk = (M + NB) / NB;   // blocks of the M + 1 columns
+  A += (size_t)d * M;
+  B += (size_t)d * M * M;
+  const float qnan = __int_as_float(0x7fffffff);
+  __shared__ df64 s_sf2;
+  if (tid == 0) s_sf2 = df_from_double(exp(lsf2[0]));
+  // ---- columns [c0, c0 + NB) of (B, A) as digits; a lane's four entries of a column are the matrix
+  // instruction's fragment, loaded twice (for the column's exponent, then for the digits), the next
+  // item's in flight while one is worked on
+  auto stage_B = [&](int c0) {
+    double r[4], rn[4];
+    auto fetch = [&](int nt, int ks) {
+      const int c = c0 + nt * 8 + (lane >> 2), a0 = ks * 16 + 2 * (lane & 3);
+      const double* p = c == M ? A + a0 : B + (size_t)a0 * M + c;
+      const size_t st = c == M ? 1 : M;
+      const bool on = nt < NT && c <= M;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int o = (i & 1) + 8 * (i >> 1);
+        rn[i] = on && a0 + o < M ? p[o * st] : 0.0;
+      }
+    };
+    // fragment (column tile, k step) number warp, then every DM_W-th
+    auto next = [&](int& nt, int& ks) {
+      ks += DM_W;
+      while (ks >= KS) ks -= KS, ++nt;
+    };
+    int nt0 = 0, ks0 = warp - DM_W;
+    next(nt0, ks0);
+    fetch(nt0, ks0);
+    for (int i = tid; i < NB; i += DM_T) s.bexp[i] = -126;
+    __syncthreads();
+    for (int nt = nt0, ks = ks0; nt < NT;) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = rn[i];
+      const int c = nt * 8 + (lane >> 2);
+      next(nt, ks);
+      if (nt < NT) fetch(nt, ks);
+      const bool pair = b_pairs && c0 + c < M;
+      int ex = -126;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {   // |entry| < 2^ex
+        const int eh = (int)(((unsigned)__double2loint(r[i]) >> 23) & 0xffu) - 126;
+        const int ed = (int)(((__double_as_longlong(r[i]) + (1LL << 28)) >> 52) & 0x7ff) - 1022;   // (rounded as hi is)
+        ex = max(ex, pair ? eh : ed);
+      }
+      atomicMax(&s.bexp[c], ex > 128 ? DM_BAD : ex);
+    }
+    fetch(nt0, ks0);
+    __syncthreads();
+    for (int nt = nt0, ks = ks0; nt < NT;) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] = rn[i];
+      const int c = nt * 8 + (lane >> 2), F = 52 - s.bexp[c];
+      uint2* q = reinterpret_cast<uint2*>(s.B) + (nt * KS + ks) * 32 + lane;
+      next(nt, ks);
+      if (nt < NT) fetch(nt, ks);
+      const bool pair = b_pairs && c0 + c < M;
+      long long t[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {   // (an exponent of DM_BAD gives zeros)
+        df64 v = df_from_double(r[i]);   // (pairs and float64 give the same results)
+        if (pair) v = make_df(__int_as_float(__double2loint(r[i])), __int_as_float(__double2hiint(r[i])));
+        t[i] = fx_bits_by(v.hi, F) + fx_bits_by(v.lo, F);
+      }
+      unsigned w0[DM_S], w1[DM_S];
+      digit_pairs(t[0], t[1], w0);
+      digit_pairs(t[2], t[3], w1);
+#pragma unroll
+      for (int j = 0; j < DM_S; ++j) q[j * NT * KS * 32] = make_uint2(w0[j], w1[j]);
+    }
+  };
+  if (nblk == 1) stage_B(0);
+  const int ntile = (N + R - 1) / R;
+  for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+    const int n0 = tile * R, nr = min(R, N - n0);
+    // ---- a warp a row: its largest exponent (|k| < 2^ex), the integers k 2^(-1 - ex) in units of 2^-53
+    // and their digits (rows past nr keep stale digits: their results are not used)
+    for (int r = warp; r < nr; r += DM_W) {
+      const double* kr = kin + (size_t)(n0 + r) * M;
+      double kv[4][2];
+      int ex = -126;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int a = 2 * lane + 64 * i;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          kv[i][u] = a + u < M ? kr[a + u] : 0.0;
+          ex = max(ex, (int)((__double_as_longlong(kv[i][u]) >> 52) & 0x7ff) - 1022);
+        }
+      }
+      ex = __reduce_max_sync(~0u, ex);
+      if (ex > 128) ex = DM_BAD;
+      if (lane == 0) s.rexp[r] = ex;
+      unsigned* q0 = s.A + ((size_t)((r >> 4) * KS) * 32 + (r & 7) * 4) * 4 + ((r >> 3) & 1);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int p = lane + 32 * i;
+        if (p < KS * 8) {
+          long long t[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            t[u] = digits_of(kv[i][u], ex);
+            if (2 * p + u < M) s.k[r * MP + 2 * p + u] = df_from_double(kv[i][u]);
+          }
+          unsigned w[DM_S];
+          digit_pairs(t[0], t[1], w);
+          unsigned* q = q0 + ((p >> 3) * 32 + (p & 3)) * 4 + 2 * ((p >> 2) & 1);
+#pragma unroll
+          for (int j = 0; j < DM_S; ++j) q[(size_t)j * nrt * KS * 128] = w[j];
+        }
+      }
+    }
+    for (int c0 = 0; c0 <= M; c0 += NB) {
+      if (nblk > 1) stage_B(c0);
+      __syncthreads();
+      for (int it = warp; it < NT * nrt; it += DM_W) {
+        const int rt = it / NT, nt = it - rt * NT;
+        const uint4* fa = reinterpret_cast<const uint4*>(s.A) + (size_t)rt * KS * 32 + lane;
+        const uint2* fb = reinterpret_cast<const uint2*>(s.B) + (size_t)nt * KS * 32 + lane;
+        long long Z[4] = {0, 0, 0, 0};
+        for (int k0 = 0; k0 < KS; k0 += 8) {
+          float acc[DM_ACC][4];
+#pragma unroll
+          for (int i = 0; i < DM_ACC; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+          const int k1 = min(k0 + 8, KS);
+#pragma unroll 2
+          for (int ks = k0; ks < k1; ++ks) dm_step(acc, fa + ks * 32, nrt * KS * 32, fb + ks * 32, NT * KS * 32);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) Z[j] += dm_fold(acc, j);
+        }
+        df64 v[2] = {make_df(0.f), make_df(0.f)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int r = rt * 16 + (lane >> 2) + 8 * (j >> 1), cl = nt * 8 + 2 * (lane & 3) + (j & 1), c = c0 + cl;
+          if (r < nr && c <= M) {
+            const int re = s.rexp[r], be = s.bexp[cl];
+            const df64 X = re >= DM_BAD || be >= DM_BAD ? make_df(qnan) : scale2(df_of_int(Z[j], 58), re + be + 6);
+            if (c < M) {
+              if (Bk) Bk[((size_t)(n0 + r) * Dout + d) * M + c] = df_to_double_int(X);
+              v[j >> 1] = fma_(s.k[r * MP + c], X, v[j >> 1]);
+            } else if (m_out) {
+              m_out[(size_t)(n0 + r) * Dout + d] = df_to_double_int(X);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+#pragma unroll
+          for (int o = 1; o < 4; o <<= 1) v[i] = add(v[i], shfl_xor(v[i], o));
+          if ((lane & 3) == 0) s.vp[(rt * 16 + (lane >> 2) + 8 * i) * NT + nt] = v[i];
+        }
+      }
+      __syncthreads();
+      // ---- v: a warp a row, the column tiles' parts by one butterfly (NT <= 32)
+      for (int r = warp; r < nr; r += DM_W) {
+        df64 v = lane < NT ? s.vp[r * NT + lane] : make_df(0.f);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) v = add(v, shfl_xor(v, o));
+        if (lane == 0) {
+          if (c0 > 0) v = add(s.v[r], v);
+          s.v[r] = v;
+          if (c0 + NB > M && v_out) v_out[(size_t)(n0 + r) * Dout + d] = df_to_double(add(s_sf2, v));
+        }
+      }
+    }
+  }
 }
 
 // elements of one det_bwd row buffer: RG rows of kfu (or dkfu) and Bk, x, dm, dv
@@ -788,6 +1220,27 @@ __global__ void __launch_bounds__(256) wsum_kernel(int N, int M, int Dout, const
   }
 }
 
+// the tensor-core contraction, 1 <= M <= DM_MAX (8 columns and 16 rows always fit)
+int dm_launch(int N, int M, int Dout, const double* lsf2, const double* A, const double* B, int b_pairs,
+              const double* kin, double* Bk, double* m_out, double* v_out, cudaStream_t st) {
+  const size_t cap = (size_t)227 * 1024 - 64;
+  // as few column blocks as fit beside 16 rows (sizes only: the order of v's sum)
+  int nblk = 1, NB = 0;
+  for (;; ++nblk) {
+    NB = 8 * gpk::ceil_div(gpk::ceil_div(M + 1, nblk), 8);
+    if (dm_carve(nullptr, nullptr, M, NB, 16) <= cap) break;
+  }
+  // one CTA an SM over the outputs; 32 or 64 rows at a time once a CTA has that many
+  const int gx = std::max(1, gpk::sm_count() / Dout), per = gpk::ceil_div(N, gx);
+  int nrt = per <= 16 ? 1 : (per <= 32 ? 2 : 4);
+  while (nrt > 1 && dm_carve(nullptr, nullptr, M, NB, 16 * nrt) > cap) nrt >>= 1;
+  const size_t sm = dm_carve(nullptr, nullptr, M, NB, 16 * nrt);
+  cudaFuncSetAttribute(det_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  det_mma_kernel<<<dim3(std::min(gx, gpk::ceil_div(N, 16 * nrt)), Dout), DM_T, sm, st>>>(
+      N, M, Dout, lsf2, A, B, b_pairs, kin, Bk, m_out, v_out, NB, nrt);
+  return gpk::check_launch("det_mma");
+}
+
 size_t det_fwd_smem(int M, int D, bool zstage, size_t tsz) {
   return 256 * 8 + sizeof(Hyp<df64>) + ((size_t)FT * M + FKA * FCB + 8 * DO_MAX * FT + FT * D + (zstage ? (size_t)M * D : 0)) * tsz;
 }
@@ -795,6 +1248,17 @@ size_t det_bwd_smem(int bx, int rg, int dc, int M, int D, int Dk, size_t tsz) {
   const size_t red = (size_t)rg * bx * (dc + DO_MAX);   // the largest of the three uses of the area
   return 256 * 8 + sizeof(Hyp<df64>) +
          ((size_t)M * D + (size_t)Dk * M + 2 * (size_t)det_bwd_rowbuf(rg, M, D, Dk) + red) * tsz;
+}
+
+int kern_fx_launch(int N, int M, int D, const double* x, int ldx, const double* z, int ldz, const double* lls2,
+                   const double* lsf2, double* K, int ldk, cudaStream_t st) {
+  // column blocks times as many row groups as keep the chip full in one wave
+  const long nmb = gpk::ceil_div(M, FC), ntile = gpk::ceil_div(N, FR);
+  const long rg = std::min(ntile, std::max(1L, (long)gpk::sm_count() * FCTA / nmb));
+  const size_t sm = kFxTab * sizeof(float2) + sizeof(ArdHyp) + ((size_t)2 * FR * D + (size_t)FC * (D | 1)) * 16;
+  cudaFuncSetAttribute(kern_fx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  kern_fx_kernel<<<(unsigned)(nmb * rg), 256, sm, st>>>(N, M, D, x, ldx, z, ldz, lls2, lsf2, K, ldk);
+  return gpk::check_launch("kern");
 }
 
 template <typename T>
@@ -820,7 +1284,12 @@ extern "C" int gpk_kern(int prec, int N, int M, int D, const void* x, int ldx, c
   GPK_REQUIRE(ldx >= D && ldz >= D && ldk >= M, "kern: bad leading dimension");
   if (N == 0 || M == 0) return GPK_OK;
   cudaStream_t st = gpk::as_stream(stream);
-  if (prec == GPK_DF64) return kern_launch<df64>(N, M, D, x, ldx, z, ldz, lls2, lsf2, jitter, K, ldk, st);
+  // with a jitter the matrix goes into a factorisation, which amplifies its last bits by a condition
+  // number of up to 1e7: it keeps the double-float evaluation (its M x M entries cost ~10 us)
+  if (prec == GPK_DF64 && jitter != 0.0) return kern_launch<df64>(N, M, D, x, ldx, z, ldz, lls2, lsf2, jitter, K, ldk, st);
+  GPK_REQUIRE(gpk::ceil_div(N, KR) <= 65535, "kern: N=%d too large (at most %d rows)", N, 65535 * KR);
+  if (prec == GPK_DF64)
+    return kern_fx_launch(N, M, D, (const double*)x, ldx, (const double*)z, ldz, lls2, lsf2, (double*)K, ldk, st);
   if (prec == GPK_FP32) return kern_launch<float>(N, M, D, x, ldx, z, ldz, lls2, lsf2, jitter, K, ldk, st);
   return gpk::fail(GPK_EINVAL, "kern: unknown precision %d", prec);
 }
@@ -834,6 +1303,13 @@ extern "C" int gpk_det_fwd(int prec, int N, int M, int D, int Dout, const void* 
   GPK_REQUIRE(x && Z && lls2 && lsf2 && A && B, "det_fwd: null input");
   if (N == 0) return GPK_OK;
   cudaStream_t st = gpk::as_stream(stream);
+  // the kernel rows, then the contraction from them (where the caller takes the rows)
+  if (prec == GPK_DF64 && kfu && M <= DM_MAX) {
+    const int rc = kern_fx_launch(N, M, D, (const double*)x, ldx, (const double*)Z, D, lls2, lsf2, (double*)kfu, M, st);
+    if (rc != GPK_OK) return rc;
+    return dm_launch(N, M, Dout, lsf2, (const double*)A, (const double*)B, 0, (const double*)kfu, (double*)Bk,
+                     (double*)m_out, (double*)v_out, st);
+  }
   // one CTA column per output d; row tiles up to two resident CTAs per SM in all
   int gx = gpk::ceil_div(N, FT);
   const int cap = std::max(1, gpk::sm_count() * 2 / Dout);
@@ -862,20 +1338,20 @@ extern "C" int gpk_det_fwd(int prec, int N, int M, int D, int Dout, const void* 
 namespace {
 template <typename T, int DB>
 void contract_launch(int N, int M, int Dout, const void* kfu, const double* lsf2, const void* A, const void* B,
-                     int b_pairs, void* Bk, void* m_out, void* v_out, cudaStream_t st) {
+                     void* Bk, void* m_out, void* v_out, cudaStream_t st) {
   typedef typename Num<T>::store_t S;
   const size_t sm = det_contract_smem(M, Dout, sizeof(T));
   auto k = det_contract_kernel<T, DB>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k<<<gpk::ceil_div(N, CR), CT, sm, st>>>(N, M, Dout, (const S*)kfu, lsf2, (const S*)A, (const S*)B, (S*)Bk,
-                                          (S*)m_out, (S*)v_out, b_pairs);
+                                          (S*)m_out, (S*)v_out);
 }
 template <typename T>
 void contract_dispatch(int N, int M, int Dout, const void* kfu, const double* lsf2, const void* A, const void* B,
-                       int b_pairs, void* Bk, void* m_out, void* v_out, cudaStream_t st) {
-  if (Dout == 1) contract_launch<T, 1>(N, M, Dout, kfu, lsf2, A, B, b_pairs, Bk, m_out, v_out, st);
-  else if (Dout == 2) contract_launch<T, 2>(N, M, Dout, kfu, lsf2, A, B, b_pairs, Bk, m_out, v_out, st);
-  else contract_launch<T, 4>(N, M, Dout, kfu, lsf2, A, B, b_pairs, Bk, m_out, v_out, st);
+                       void* Bk, void* m_out, void* v_out, cudaStream_t st) {
+  if (Dout == 1) contract_launch<T, 1>(N, M, Dout, kfu, lsf2, A, B, Bk, m_out, v_out, st);
+  else if (Dout == 2) contract_launch<T, 2>(N, M, Dout, kfu, lsf2, A, B, Bk, m_out, v_out, st);
+  else contract_launch<T, 4>(N, M, Dout, kfu, lsf2, A, B, Bk, m_out, v_out, st);
 }
 }  // namespace
 
@@ -896,8 +1372,9 @@ extern "C" int gpk_det_contract(int prec, int N, int M, int Dout, const void* kf
   GPK_REQUIRE(kfu && lsf2 && A && B, "det_contract: null input");
   if (N == 0) return GPK_OK;
   cudaStream_t st = gpk::as_stream(stream);
-  if (prec == GPK_DF64) contract_dispatch<df64>(N, M, Dout, kfu, lsf2, A, B, b_pairs, Bk, m_out, v_out, st);
-  else contract_dispatch<float>(N, M, Dout, kfu, lsf2, A, B, 0, Bk, m_out, v_out, st);
+  if (prec == GPK_DF64)
+    return dm_launch(N, M, Dout, lsf2, (const double*)A, (const double*)B, b_pairs, (const double*)kfu, (double*)Bk, (double*)m_out, (double*)v_out, st);
+  contract_dispatch<float>(N, M, Dout, kfu, lsf2, A, B, Bk, m_out, v_out, st);
   return gpk::check_launch("det_contract");
 }
 

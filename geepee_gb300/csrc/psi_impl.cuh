@@ -81,39 +81,6 @@ struct PsiArgs {
 
 __device__ __forceinline__ void pair_of(int p, int& a, int& b) { tri_pair(p, a, b); }
 
-// The pair loops address shared memory by 32-bit addresses: through the table pointers every access
-// cost a 64-bit address computation (two integer instructions each).
-typedef unsigned saddr;
-__device__ __forceinline__ saddr sm_addr(const void* p) { return (saddr)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ int2 lds_i2(saddr a) {
-  int2 v;
-  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ void lds(saddr a, long long& v) { asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a)); }
-__device__ __forceinline__ void lds(saddr a, df64& v) {
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.hi), "=f"(v.lo) : "r"(a));
-}
-__device__ __forceinline__ void lds(saddr a, float& v) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
-__device__ __forceinline__ void lds_st(saddr a, double& v) { asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
-__device__ __forceinline__ void lds_st(saddr a, float& v) { lds(a, v); }
-__device__ __forceinline__ int lds_u16(saddr a) {
-  unsigned short v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ void sts(saddr a, df64 v) {
-  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.hi), "f"(v.lo) : "memory");
-}
-__device__ __forceinline__ void sts(saddr a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
-__device__ __forceinline__ void sts(saddr a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
-template <typename V>
-__device__ __forceinline__ V ldsv(saddr a) {
-  V v;
-  lds(a, v);
-  return v;
-}
-
 // How a precision keeps the pair exponent's terms (log2 units): R a table element, arg() the
 // exponent of a pair from the two records and G, ev() its exponential.
 template <typename T>
@@ -159,13 +126,6 @@ struct PairExp<df64> {
   }
   // a record whose pairs are all zero: u + u_b + G < -126 for every live b (u_b <= 63.5), and no
   // sum leaves the range of +-2048
-  // a b + c of 32-bit factors in one instruction (from C, the compiler widened the factors to 64
-  // bits first: three multiply-adds and two shifts a product)
-  static __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
-    long long d;
-    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
-    return d;
-  }
   static __device__ __forceinline__ R dead_u() { return -(400LL << 52); }
   template <int QC>
   static __device__ __forceinline__ R arg(saddr a, saddr b, R g) {
@@ -190,11 +150,6 @@ struct PairExp<df64> {
   static __device__ __forceinline__ double ev_st(R x, saddr tab) { return exp2_fx_double(x, tab); }
 };
 
-// the 256-entry exp table of exp_tab inside the kernels' shared table (every 8th entry)
-struct ExpTab {
-  const float2* p;
-  __device__ __forceinline__ float2 operator[](int j) const { return p[8 * j]; }
-};
 template <typename T>
 __device__ __forceinline__ void load_pair_table(float2* tab) {
   if (PairExp<T>::TAB) load_exp2_table(tab);

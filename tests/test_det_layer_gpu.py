@@ -1,0 +1,70 @@
+"""The deterministic-input layer at the edges of its fixed-point and digit forms."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    return torch.as_tensor(np.asarray(a, dtype=np.float64), device='cuda').contiguous()
+
+
+@pytest.mark.parametrize('n,m,d,dout', [(1, 1, 1, 1), (17, 15, 2, 2), (33, 16, 16, 1), (70, 129, 3, 4), (50, 200, 8, 2),
+                                        (31, 255, 5, 1), (5000, 103, 8, 2)])
+def test_det_layer_fixed_point_edges(n, m, d, dout):
+    """The fixed-point kernel rows and the digit contraction at the edges of their tiles, with rows
+    whose coordinates leave the fixed-point range, rows that are zero or NaN, columns of B from
+    1e-25 to 1e25 and a zero column.  The rows: 2^-45 (|a| + 1) of an entry with exponent a (the
+    double-float form's error, the larger one).  The contraction, from the device's own rows: each product is off by at most
+    2^-47 of the row's largest times the column's largest."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(n + m)
+    L = np.longdouble
+    x, z = rng.randn(n, d), rng.randn(m, d)
+    if n > 16:
+        x[3] = z[5 % m] + 60.0      # far from every z: coordinates out of range, rows zero
+        x[7] = np.nan
+        x[11] = 1e12
+        x[13] = z[m - 1] + 1e-9
+    if m > 16:
+        z[9] = 25.0                 # a column out of range
+        if n > 16:
+            x[14] = z[9] + 0.1
+    l2, s2 = np.log(rng.uniform(0.5, 2.0, d) * d), np.array([0.3])
+    A, B = rng.randn(dout, m), rng.randn(dout, m, m) * 10.0 ** rng.uniform(-25, 25, (dout, 1, m))
+    B[:, :, m // 2] = 0.0
+    e = lambda *s: torch.full(s, -7.0, dtype=torch.float64, device='cuda')
+    kfu, Bk, mo, vo = e(n, m), e(n, dout, m), e(n, dout), e(n, dout)
+    At, Bt, s2t = dev(A), dev(B), dev(s2)
+    gpk.det_fwd(dev(x), dev(z), dev(l2), s2t, At, Bt, kfu, Bk, mo, vo)
+    K = gpk.kern(dev(x), dev(z), dev(l2), s2t)
+    assert torch.equal(torch.nan_to_num(K, nan=-1.0), torch.nan_to_num(kfu, nan=-1.0))
+    nan = np.isnan(x).any(1)
+    a = (s2[0] - 0.5 * ((x[:, None].astype(L) - z[None]) ** 2 / np.exp(l2.astype(L))).sum(-1))[~nan]
+    k, Kg = np.exp(a), K.cpu().numpy()
+    assert np.isnan(Kg[nan]).all()
+    err = np.abs(Kg[~nan] - k)
+    assert (err <= 2.0 ** -45 * (np.abs(a) + 1) * k + 1e-37).all(), float((err / (k + 1e-300)).max())
+    kg = Kg[~nan].astype(L)
+    bk = np.einsum('na,dab->ndb', kg, B.astype(L))
+    km, bm = kg.max(1), np.abs(B).max(1)
+    g = Bk.cpu().numpy()
+    assert np.isnan(g[nan]).all() and np.isnan(mo.cpu().numpy()[nan]).all() and np.isnan(vo.cpu().numpy()[nan]).all()
+    assert (np.abs(g[~nan] - bk) <= m * 2.0 ** -47 * km[:, None, None] * bm[None] + 1e-37).all()
+    mm = np.einsum('na,da->nd', kg, A.astype(L))
+    assert (np.abs(mo.cpu().numpy()[~nan] - mm) <= m * 2.0 ** -47 * km[:, None] * np.abs(A).max(1)[None] + 1e-37).all()
+    vv = np.exp(L(s2[0])) + np.einsum('nb,ndb->nd', kg, bk)
+    vs = 2 + m * m * (km[:, None] ** 2 * bm.max(1)[None])
+    assert (np.abs(vo.cpu().numpy()[~nan] - vv) <= 2.0 ** -46 * vs).all()
+    if gpk.det_contract_supported(torch.float64, m, dout):
+        hi = B.astype(np.float32)
+        pairs = dev(np.stack([hi, (B - hi).astype(np.float32)], -1).astype(np.float32).view(np.float64)[..., 0])
+        got = []
+        for Bp, flag in ((Bt, False), (pairs, True)):
+            Bk2, m2, v2 = e(n, dout, m), e(n, dout), e(n, dout)
+            gpk.det_contract(kfu, s2t, At, Bp, Bk2, m2, v2, b_pairs=flag)
+            got.append([torch.nan_to_num(t, nan=-1.0) for t in (Bk2, m2, v2)])
+            assert (np.abs(Bk2.cpu().numpy()[~nan] - bk) <= m * 2.0 ** -47 * km[:, None, None] * bm[None] + 1e-37).all()
+        assert all(torch.equal(p, q) for p, q in zip(*got))
+        assert torch.equal(got[0][1], torch.nan_to_num(mo, nan=-1.0))
