@@ -1450,12 +1450,12 @@ struct OSmem {
   T* misc;   // [4]
   T* pd;     // [2][PDN]
   R* rec;    // [2][M][rec_len]
-  S* L;      // [2][P]
+  S* L;      // [nl][P]
   R* G;      // [P] or nullptr
   unsigned short* pab;   // [P] or nullptr
 };
 template <typename T>
-__host__ __device__ inline size_t ocarve(OSmem<T>* out, char* base, int M, int QC, int P, int ng, int pab) {
+__host__ __device__ inline size_t ocarve(OSmem<T>* out, char* base, int M, int QC, int P, int ng, int pab, int nl) {
   typedef typename PairExp<T>::R R;
   typedef typename Num<T>::store_t S;
   OSmem<T> s;
@@ -1474,7 +1474,7 @@ __host__ __device__ inline size_t ocarve(OSmem<T>* out, char* base, int M, int Q
   s.misc = (T*)take(4 * e);
   s.pd = (T*)take(2 * PDN * e);
   s.rec = (R*)take(2 * (size_t)M * rec_len(QC) * e);
-  s.L = (S*)take(2 * (size_t)P * e);
+  s.L = (S*)take((size_t)nl * P * e);
   s.G = ng ? (R*)take((size_t)ng * e) : nullptr;
   s.pab = pab ? (unsigned short*)take((size_t)P * sizeof(unsigned short)) : nullptr;
   if (out) *out = s;
@@ -1482,8 +1482,8 @@ __host__ __device__ inline size_t ocarve(OSmem<T>* out, char* base, int M, int Q
 }
 
 template <typename T, int QC, int NS, int NF>
-__global__ void __launch_bounds__((NS + NF) * 32, NS < 12 ? 2 : 1)
-    psi_out_kernel(PsiArgs<typename Num<T>::store_t> a, int use_pab) {
+__global__ void __launch_bounds__((NS + NF) * 32, NS < 8 ? 4 : NS < 12 ? 2 : 1)
+    psi_out_kernel(PsiArgs<typename Num<T>::store_t> a, int use_pab, int nl) {
   typedef typename Num<T>::store_t S;
   typedef PairExp<T> X;
   typedef typename X::R R;
@@ -1492,7 +1492,7 @@ __global__ void __launch_bounds__((NS + NF) * 32, NS < 12 ? 2 : 1)
   const int M = a.M, Q = exact_q(QC) ? QC : a.Q;
   const int P = M * (M + 1) / 2;
   OSmem<T> s;
-  ocarve<T>(&s, smem_raw, M, QC, P, a.g_smem ? P : 0, use_pab);
+  ocarve<T>(&s, smem_raw, M, QC, P, a.g_smem ? P : 0, use_pab, nl);
   __shared__ int s_flag[2];
   const ExpTab etab{s.tab};
   const int tid = threadIdx.x, lane = tid & 31;
@@ -1538,7 +1538,7 @@ __global__ void __launch_bounds__((NS + NF) * 32, NS < 12 ? 2 : 1)
       if (i + 1 < cnt) front(i + 1);
     } else {
       if (i < cnt) {
-        S* L = s.L + (size_t)(i & 1) * P;
+        S* L = s.L + (size_t)(i & (nl - 1)) * P;
         const R* rec = s.rec + (size_t)(i & 1) * M * RL;
         const bool general = X::TAB && s_flag[i & 1];
         constexpr int E = sizeof(T);
@@ -1573,10 +1573,12 @@ __global__ void __launch_bounds__((NS + NF) * 32, NS < 12 ? 2 : 1)
           }
         }
       }
-      if (i > 0) {   // the previous point's square, a warp a row, 128 columns at a time
+      if (nl == 1) warps_sync<2, NS>();
+      const int w = nl == 1 ? i : i - 1;   // the point whose square goes out, a warp a row, 128 columns at a time
+      if (w >= 0 && w < cnt) {
         constexpr int E = sizeof(T);
-        const saddr aL = sm_addr(s.L + (size_t)((i - 1) & 1) * P);
-        S* const out = a.psi2 + (size_t)(nbeg + i - 1) * M * M;
+        const saddr aL = sm_addr(s.L + (size_t)(w & (nl - 1)) * P);
+        S* const out = a.psi2 + (size_t)(nbeg + w) * M * M;
         for (int c0 = 0; c0 < M; c0 += 128) {
           saddr up[4];   // the lane's columns: where their entries below the diagonal begin
 #pragma unroll
@@ -2079,18 +2081,21 @@ template <typename T, int QC, int NS, int NF>
 int run_out(const PsiArgs<typename Num<T>::store_t>& a_in, size_t cap, cudaStream_t st) {
   PsiArgs<typename Num<T>::store_t> a = a_in;
   const int P = a.M * (a.M + 1) / 2;
-  // G and the pair table as far as they fit (two CTAs an SM only with both)
-  for (int o = 0; o < (NS < 12 ? 1 : 3); ++o) {
-    const int pab = o == 0 && a.M <= 255;
-    a.g_smem = o < 2;
-    const size_t sm = ocarve<T>(nullptr, nullptr, a.M, QC, P, a.g_smem ? P : 0, pab);
+  // G, a second buffer of pairs and the pair table as far as they fit (several CTAs an SM only with
+  // all of them); G in place of the second buffer: at M = 128, Q = 8 the pairs' G from the pseudo-inputs
+  // cost 226 us (N = 1000) against 113 us for a write that waits for its sweep
+  const int per_sm = NS >= 12 ? 1 : NS >= 8 ? 2 : 4;
+  for (int o = 0; o < (NS < 12 ? 1 : 5); ++o) {
+    const int pab = (o == 0 || o == 2) && a.M <= 255, nl = o == 2 || o == 3 ? 1 : 2;
+    a.g_smem = o < 4;
+    const size_t sm = ocarve<T>(nullptr, nullptr, a.M, QC, P, a.g_smem ? P : 0, pab, nl);
     if (sm > cap) continue;
     auto k = psi_out_kernel<T, QC, NS, NF>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    int grid = gpk::sm_count() * (NS < 12 ? 2 : 1);
+    int grid = gpk::sm_count() * per_sm;
     if (grid > a.N) grid = a.N;
     if (grid < 1) return GPK_OK;
-    k<<<grid, (NS + NF) * 32, sm, st>>>(a, pab);
+    k<<<grid, (NS + NF) * 32, sm, st>>>(a, pab, nl);
     return gpk::check_launch("psi_out");
   }
   return -1;
@@ -2110,7 +2115,10 @@ int launch_fwd_q(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
     rc = fwd_npb<T, QC, 8, 4>(a, half, st);
     if (rc == -1) rc = fwd_npb<T, QC, 16, 4>(a, SMEM_CAP, st);
   } else if (!sum && !a.chain && a.psi2 && !contract) {
-    if (a.N > gpk::sm_count()) rc = run_out<T, QC, 8, 4>(a, half, st);
+    if (a.N > gpk::sm_count()) {
+      rc = run_out<T, QC, 4, 2>(a, (SMEM_CAP - 4096) / 4, st);
+      if (rc == -1) rc = run_out<T, QC, 8, 4>(a, half, st);
+    }
     if (rc == -1) rc = run_out<T, QC, 16, 4>(a, SMEM_CAP, st);
   }
   if (rc != -1) return rc;

@@ -165,3 +165,22 @@ def test_psi_rollout_vs_oracle(M, Q, kind):
     bad[0] = np.nan
     gm, gv = gpk.psi_rollout(dev(bad), dev(S), dev(Z), dev(lls2), dev(lsf2), dev(A), dev(B), 3)
     assert bool(torch.isnan(gm).all()) and bool(torch.isnan(gv).all())
+
+
+@pytest.mark.parametrize('N,M,Q,dtype', [(160, 1, 1, 'float64'), (700, 17, 3, 'float64'), (300, 33, 8, 'float64'),
+                                         (155, 41, 2, 'float32'), (160, 101, 2, 'float64'), (153, 128, 8, 'float64'),
+                                         (153, 128, 8, 'float32'), (153, 140, 5, 'float64')])
+def test_psi_points_written_out(N, M, Q, dtype):
+    """psi2 of every point at the sizes where the split changes: several small CTAs an SM, two,
+    one, and one with a single buffer of pairs.  Same tolerances as the psi statistics'."""
+    from geepee_gb300 import gpk
+    dt = getattr(torch, dtype)
+    rng = np.random.RandomState(N + M)
+    Z, mu, S = rng.randn(M, Q), rng.randn(N, Q), rng.uniform(0.01, 1.0, (N, Q))
+    lls2, lsf2 = rng.uniform(-0.5, 0.5, Q), np.array([0.3])
+    psi1, psi2 = torch.zeros((N, M), dtype=dt, device='cuda'), torch.zeros((N, M, M), dtype=dt, device='cuda')
+    gpk.psi_fwd(dev(mu, dt), dev(S, dt), dev(Z, dt), dev(lls2), dev(lsf2), psi1=psi1, psi2=psi2)
+    p1, p2 = O.psi_stats(lls2, lsf2, mu, S, Z)
+    tol = 1e-10 if dtype == 'float64' else 1e-4
+    np.testing.assert_allclose(psi1.cpu().numpy(), p1, rtol=tol, atol=tol * np.abs(p1).max())
+    np.testing.assert_allclose(psi2.cpu().numpy(), p2, rtol=tol, atol=tol * np.abs(p2).max())
