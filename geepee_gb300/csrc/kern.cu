@@ -1175,6 +1175,157 @@ __global__ void __launch_bounds__(GP_T) gram_pairs_kernel(int N, int M, int Dout
   }
 }
 
+// ---- the symmetric weighted Gram reduction on the tensor cores (float64) ----
+// C[d]_ab = sum_n (w u_a)(u_b) over a chunk of rows for one output d, by the digit products of
+// det_mma_kernel: the contraction runs over n, so each column of w u and of u is scaled by its largest entry
+// of the rows staged (at most 128, so that the digit sums stay exact), and the staged sums, exact
+// integers, are added up in float64.  A CTA of 12 warps owns up to 60 of the 16 x 8 tiles on and below the
+// diagonal, five a warp, their float64 sums in registers; the next rows arrive by asynchronous copies while
+// these are multiplied.  The chunk's sums leave as a partial block of packed pairs for the
+// fixed-order reduction.
+// N = 20000, M = 100, two outputs: 84 us, a third of it in the matrix pipe, the rest in digits and folds
+// (356 us in double-float pairs); with the reduction 91 us (361); N = 1000, one output 21 us (26).
+constexpr int GM_T = 384, GM_W = GM_T / 32, GM_TW = 5;
+struct GmSmem {
+  unsigned *A, *B;   // digits of w u and of u, as in DmSmem (the columns in the place of the rows)
+  double *raw, *w;   // [16 KS][M], [16 KS]
+  int *aexp, *bexp;
+};
+__host__ __device__ inline size_t gm_carve(GmSmem* out, char* base, int M, int KS) {
+  GmSmem s;
+  size_t o = 0;
+  auto take = [&](size_t n) {
+    char* p = base + o;
+    o += (n + 15) & ~(size_t)15;
+    return p;
+  };
+  const int RT = (M + 15) >> 4, CT = (M + 7) >> 3;
+  s.A = (unsigned*)take((size_t)DM_S * RT * KS * 512);
+  s.B = (unsigned*)take((size_t)DM_S * CT * KS * 256);
+  s.raw = (double*)take((size_t)16 * KS * M * 8);
+  s.w = (double*)take((size_t)16 * KS * 8);
+  s.aexp = (int*)take((size_t)M * 4);
+  s.bexp = (int*)take((size_t)M * 4);
+  if (out) *out = s;
+  return o;
+}
+// tiles on and below the diagonal: row i of 16 has min(2 i + 2, CT) of 8 columns
+__host__ __device__ inline int gm_tiles(int M) {
+  const int RT = (M + 15) >> 4, CT = (M + 7) >> 3;
+  return RT * (RT - 1) + (CT < 2 * RT ? CT : 2 * RT);
+}
+__global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dout, const double* u, const double* w,
+                                                           double* part, long pstride, int rows, int KSM,
+                                                           int tw) {
+  extern __shared__ __align__(16) char smem_raw[];
+  GmSmem s;
+  gm_carve(&s, smem_raw, M, KSM);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, d = blockIdx.y;
+  const int RT = (M + 15) >> 4, CT = (M + 7) >> 3, ntile = gm_tiles(M);
+  const int nbeg = blockIdx.x * rows, nend = min(N, nbeg + rows);
+  double C[GM_TW][4];
+  int ti[GM_TW], tj[GM_TW];   // the warp's tiles (row -1: none)
+#pragma unroll
+  for (int i = 0; i < GM_TW; ++i) {
+    int t = blockIdx.z * (GM_W * tw) + warp + GM_W * i, r = 0;
+    const bool on = i < tw && t < ntile;
+    if (!on) t = 0;
+    while (t >= min(2 * r + 2, CT)) t -= min(2 * r + 2, CT), ++r;
+    ti[i] = on ? r : -1;
+    tj[i] = t;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) C[i][j] = 0.0;
+  }
+  auto fetch = [&](int n0) {
+    const int nr = min(16 * KSM, nend - n0);
+    for (int e = tid; e < nr * M; e += GM_T) async_copy(s.raw + e, u + (size_t)n0 * M + e);
+    for (int e = tid; e < nr; e += GM_T) async_copy(s.w + e, w + (size_t)(n0 + e) * Dout + d);
+  };
+  auto expo = [](double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff) - 1022; };   // |v| < 2^expo
+  fetch(nbeg);
+  for (int n0 = nbeg; n0 < nend; n0 += 16 * KSM) {
+    const int nr = min(16 * KSM, nend - n0), KS = (nr + 15) >> 4;
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    // ---- the columns' largest exponents (of w u at most: the factors' sum)
+    for (int i = tid; i < M; i += GM_T) s.aexp[i] = s.bexp[i] = -126;
+    __syncthreads();
+    for (int c = tid & 127; c < M; c += 128) {
+      int ea = -126, eb = -126;
+      for (int r = tid >> 7; r < nr; r += GM_T / 128) {
+        const int e = expo(s.raw[r * M + c]), f = expo(s.w[r]);
+        eb = max(eb, e);
+        ea = max(ea, max(e, f) == 1025 ? DM_BAD : e + f);
+      }
+      atomicMax(&s.bexp[c], eb > 300 ? DM_BAD : eb);
+      atomicMax(&s.aexp[c], ea > 300 ? DM_BAD : ea);
+    }
+    __syncthreads();
+    // ---- digits: a lane's four rows of one column
+    for (int f = warp; f < 2 * RT * KS; f += GM_W) {
+      const int ks = f / (2 * RT), c8 = f - ks * 2 * RT, c = c8 * 8 + (lane >> 2), r0 = ks * 16 + 2 * (lane & 3);
+      long long ta[4], tb[4];
+      const int ea = c < M ? s.aexp[c] : 0, eb = c < M ? s.bexp[c] : 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = r0 + (i & 1) + 8 * (i >> 1);
+        const bool on = c < M && r < nr;
+        const double v = on ? s.raw[r * M + c] : 0.0, wv = on ? s.w[r] : 0.0;
+        ta[i] = digits_of(v * wv, ea);
+        tb[i] = digits_of(v, eb);
+      }
+      unsigned w0[DM_S], w1[DM_S];
+      digit_pairs(ta[0], ta[1], w0);
+      digit_pairs(ta[2], ta[3], w1);
+      unsigned* q = s.A + ((size_t)((c8 >> 1) * KSM + ks) * 32 + lane) * 4 + (c8 & 1);
+#pragma unroll
+      for (int j = 0; j < DM_S; ++j) {
+        q[j * RT * KSM * 128] = w0[j];
+        q[j * RT * KSM * 128 + 2] = w1[j];
+      }
+      if (c8 < CT) {
+        digit_pairs(tb[0], tb[1], w0);
+        digit_pairs(tb[2], tb[3], w1);
+        uint2* p = reinterpret_cast<uint2*>(s.B) + (size_t)(c8 * KSM + ks) * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < DM_S; ++j) p[j * CT * KSM * 32] = make_uint2(w0[j], w1[j]);
+      }
+    }
+    __syncthreads();
+    if (n0 + 16 * KSM < nend) fetch(n0 + 16 * KSM);
+#pragma unroll
+    for (int i = 0; i < GM_TW; ++i) {
+      if (ti[i] < 0) continue;   // (uniform over the warp)
+      float acc[DM_ACC][4];
+#pragma unroll
+      for (int k = 0; k < DM_ACC; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[k][j] = 0.f;
+      const uint4* fa = reinterpret_cast<const uint4*>(s.A) + (size_t)ti[i] * KSM * 32 + lane;
+      const uint2* fb = reinterpret_cast<const uint2*>(s.B) + (size_t)tj[i] * KSM * 32 + lane;
+#pragma unroll 1
+      for (int ks = 0; ks < KS; ++ks) dm_step(acc, fa + ks * 32, RT * KSM * 32, fb + ks * 32, CT * KSM * 32);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int a = ti[i] * 16 + (lane >> 2) + 8 * (j >> 1), b = tj[i] * 8 + 2 * (lane & 3) + (j & 1);
+        const int e = a < M && b < M ? s.aexp[a] + s.bexp[b] : 0;
+        // 2^(e - 52), or NaN
+        const double f = __hiloint2double(e >= DM_BAD / 2 ? 0x7fffffff : (e + 971) << 20, 0);
+        C[i][j] = fma(__ll2double_rn(dm_fold(acc, j)), f, C[i][j]);
+      }
+    }
+  }
+  double* const pb = part + (size_t)blockIdx.x * pstride + (size_t)d * (M * (M + 1) / 2);
+#pragma unroll
+  for (int i = 0; i < GM_TW; ++i) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int a = ti[i] * 16 + (lane >> 2) + 8 * (j >> 1), b = tj[i] * 8 + 2 * (lane & 3) + (j & 1);
+      if (ti[i] >= 0 && a < M && b <= a) pb[a * (a + 1) / 2 + b] = C[i][j];
+    }
+  }
+}
+
 // c[d] += sum_n w[n,d] u_n  (u: [N,M]; c: [Dout,M] f64).  32 columns per CTA, rows split over
 // 8 warps and gridDim.y; each thread keeps WU rows' loads in flight at a time.
 constexpr int WU = 4;
@@ -1454,6 +1605,26 @@ int gram_pair_chunks(int N, int M) {
   if (c > cap) c = cap;
   return c < 1 ? 1 : c;
 }
+// the tensor-core form's split: rows a chunk (a multiple of 16) so that about one CTA runs per SM, tile
+// groups of up to GM_TW tiles a warp (fewer where the chunks of 16 rows leave SMs idle: a tile's
+// fold and float64 sums are then most of its time), k steps staged at a time; false where 16 rows of
+// digits do not fit
+struct GramMma {
+  int groups, rows, chunks, ks, tw;
+};
+bool gram_mma_plan(int N, int M, int Dout, GramMma* g) {
+  const size_t cap = 227 * 1024 - 64;
+  if (gm_carve(nullptr, nullptr, M, 1) > cap) return false;
+  const int tiles = gm_tiles(M), least = gpk::ceil_div(tiles, GM_W * GM_TW);
+  const int want = std::max(1, gpk::sm_count() / (Dout * least));
+  g->rows = 16 * std::max(1, gpk::ceil_div(gpk::ceil_div(N, want), 16));
+  g->chunks = std::max(1, gpk::ceil_div(N, g->rows));
+  g->tw = gpk::ceil_div(tiles, GM_W * std::max(least, std::min(tiles, gpk::sm_count() / (Dout * g->chunks))));
+  g->groups = gpk::ceil_div(tiles, GM_W * g->tw);
+  g->ks = std::min(8, g->rows / 16);
+  while (gm_carve(nullptr, nullptr, M, g->ks) > cap) --g->ks;
+  return true;
+}
 template <typename T, int DB>
 void gram_pairs_launch(dim3 grid, size_t sm, cudaStream_t st, int N, int M, int Dout, const void* u, const void* w,
                        double* work, long pstride, int GR) {
@@ -1479,7 +1650,9 @@ int gram_pair_rows(int M, size_t tsz) {
 long gram_work_elems(int N, int M, int Dout) {
   const long full = (long)gram_chunks(N, M, false) * Dout * M * M;   // u != v: full tiles
   const long pairs = (long)gram_pair_chunks(N, M) * Dout * (M * (M + 1) / 2);
-  return full > pairs ? full : pairs;
+  GramMma g;
+  const long mma = gram_mma_plan(N, M, Dout, &g) ? (long)g.chunks * Dout * (M * (M + 1) / 2) : 0;
+  return std::max(full, std::max(pairs, mma));
 }
 
 extern "C" int gpk_det_bwd_ws(int prec, int N, int M, int D, int Dout, const void* x, int ldx, const void* Z,
@@ -1533,7 +1706,9 @@ extern "C" int gpk_gram_ws(int prec, int N, int M, int Dout, const void* u, cons
   GPK_REQUIRE(u && v && w && C, "gram: null pointer");
   const int sym = u == v;   // C symmetric: the upper tiles only
   const int P = M * (M + 1) / 2;
-  const int chunks = sym ? gram_pair_chunks(N, M) : gram_chunks(N, M, false);
+  GramMma g{};
+  const bool mma = prec == GPK_DF64 && sym && work && gram_mma_plan(N, M, Dout, &g);
+  const int chunks = mma ? g.chunks : sym ? gram_pair_chunks(N, M) : gram_chunks(N, M, false);
   if (work) {
     const long need = (long)chunks * Dout * (sym ? P : M * M);
     GPK_REQUIRE(work_elems >= need, "gram: workspace of %ld doubles, %ld needed", work_elems, need);
@@ -1546,7 +1721,12 @@ extern "C" int gpk_gram_ws(int prec, int N, int M, int Dout, const void* u, cons
     const size_t sm = (size_t)GR * (M + DO_MAX) * tsz;
     const dim3 grid(gram_pair_blocks(M), chunks);
     const long pstride = (long)Dout * P;
-    if (prec == GPK_DF64) gram_pairs_dispatch<df64>(grid, sm, st, N, M, Dout, u, w, work, pstride, GR);
+    if (mma) {
+      const size_t smm = gm_carve(nullptr, nullptr, M, g.ks);
+      cudaFuncSetAttribute(gram_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smm);
+      gram_mma_kernel<<<dim3(chunks, Dout, g.groups), GM_T, smm, st>>>(N, M, Dout, (const double*)u, (const double*)w,
+                                                                       work, pstride, g.rows, g.ks, g.tw);
+    } else if (prec == GPK_DF64) gram_pairs_dispatch<df64>(grid, sm, st, N, M, Dout, u, w, work, pstride, GR);
     else if (prec == GPK_FP32) gram_pairs_dispatch<float>(grid, sm, st, N, M, Dout, u, w, work, pstride, GR);
     else return gpk::fail(GPK_EINVAL, "gram: unknown precision %d", prec);
     int rc = gpk::check_launch("gram_pairs");

@@ -68,3 +68,37 @@ def test_det_layer_fixed_point_edges(n, m, d, dout):
             assert (np.abs(Bk2.cpu().numpy()[~nan] - bk) <= m * 2.0 ** -47 * km[:, None, None] * bm[None] + 1e-37).all()
         assert all(torch.equal(p, q) for p, q in zip(*got))
         assert torch.equal(got[0][1], torch.nan_to_num(mo, nan=-1.0))
+
+
+@pytest.mark.parametrize('n,m,dout', [(1, 1, 1), (15, 7, 2), (16, 8, 1), (17, 16, 4), (129, 33, 3), (1000, 104, 1),
+                                      (3001, 100, 2), (700, 129, 2), (97, 255, 1), (40, 460, 1)])
+def test_symmetric_gram_edges(n, m, dout):
+    """The digit form of the symmetric weighted Gram reduction at the edges of its tiles and row
+    chunks (the last size takes the pair form), columns from 1e-15 to 1e15, weights over twelve
+    decades with zeros, and a column with an infinity.  Every product is off by at most 2^-47 of
+    the largest |w u_a| times the largest |u_b|."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(n + m)
+    L = np.longdouble
+    u = rng.randn(n, m) * 10.0 ** rng.uniform(-15, 15, m)
+    w = rng.randn(n, dout) * 10.0 ** rng.uniform(-6, 6, (n, dout))
+    w[n // 2] = 0.0
+    if m > 8:
+        u[:, 5] = 0.0
+    z = lambda *s: torch.zeros(s, dtype=torch.float64, device='cuda')
+    work = z(gpk.work_elems(gpk.OP_GRAM, n, m, 1, dout))
+    ref = np.einsum('nd,na,nb->dab', w.astype(L), u.astype(L), u.astype(L))
+    ua = np.abs(u).max(0)
+    wa = np.abs(w[:, :, None] * u[:, None]).max(0)
+    tol = n * 2.0 ** -47 * np.maximum(wa[:, :, None] * ua, wa[:, None] * ua[:, None]) + 1e-37
+    C = z(dout, m, m)
+    ut = dev(u)
+    gpk.gram(ut, ut, dev(w), C, work=work)
+    assert (np.abs(C.cpu().numpy() - ref) <= tol).all()
+    if m > 8:
+        u[n // 3, 6] = np.inf
+        C, ut = z(dout, m, m), dev(u)
+        gpk.gram(ut, ut, dev(w), C, work=work)
+        g, keep = C.cpu().numpy(), np.arange(m) != 6
+        assert not np.isfinite(g[:, 6]).any() and not np.isfinite(g[:, :, 6]).any()
+        assert (np.abs(g - ref) <= tol)[:, keep][:, :, keep].all()
