@@ -29,10 +29,14 @@ unsigned gpk_bounds_word_psi_api();
 unsigned gpk_bounds_word_psi_bwd_df64();
 unsigned gpk_bounds_word_psi_bwd_f32();
 unsigned gpk_bounds_word_psi_fwd_df64_q2();
+unsigned gpk_bounds_word_psi_fwd_df64_q4();
 unsigned gpk_bounds_word_psi_fwd_df64_q5();
+unsigned gpk_bounds_word_psi_bwd_df64_w();
 unsigned gpk_bounds_word_psi_fwd_df64_q8();
 unsigned gpk_bounds_word_psi_fwd_f32_q2();
+unsigned gpk_bounds_word_psi_fwd_f32_q4();
 unsigned gpk_bounds_word_psi_fwd_f32_q5();
+unsigned gpk_bounds_word_psi_bwd_f32_w();
 unsigned gpk_bounds_word_psi_fwd_f32_q8();
 
 extern "C" int gpk_debug_bounds(unsigned int* word) {
@@ -41,7 +45,8 @@ extern "C" int gpk_debug_bounds(unsigned int* word) {
   *word = gpk_bounds_word_algebra() | gpk_bounds_word_dense() | gpk_bounds_word_kern() | gpk_bounds_word_psi_api() |
           gpk_bounds_word_psi_bwd_df64() | gpk_bounds_word_psi_bwd_f32() | gpk_bounds_word_psi_fwd_df64_q2() |
           gpk_bounds_word_psi_fwd_df64_q5() | gpk_bounds_word_psi_fwd_df64_q8() | gpk_bounds_word_psi_fwd_f32_q2() |
-          gpk_bounds_word_psi_fwd_f32_q5() | gpk_bounds_word_psi_fwd_f32_q8();
+          gpk_bounds_word_psi_fwd_f32_q5() | gpk_bounds_word_psi_fwd_f32_q8() | gpk_bounds_word_psi_fwd_df64_q4() |
+          gpk_bounds_word_psi_fwd_f32_q4() | gpk_bounds_word_psi_bwd_df64_w() | gpk_bounds_word_psi_bwd_f32_w();
 #ifdef GPK_DEBUG_BOUNDS
   return 1;
 #else

@@ -2,25 +2,27 @@
 #include "psi_impl.cuh"
 
 int psi_fwd_df64_q2(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
+int psi_fwd_df64_q4(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
 int psi_fwd_df64_q5(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
 int psi_fwd_df64_q8(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
 int psi_bwd_df64(const psi_impl::PsiArgs<double>& a, cudaStream_t st);
 int psi_fwd_f32_q2(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
+int psi_fwd_f32_q4(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
 int psi_fwd_f32_q5(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
 int psi_fwd_f32_q8(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
 int psi_bwd_f32(const psi_impl::PsiArgs<float>& a, cudaStream_t st);
 using psi_impl::QMAX;
 using psi_impl::DMAX;
 
-// five input dimensions (the psi-statistics workload's width) have kernels of their own for the
-// plain forms; other forms and widths take the catch-all ones
+// three to five input dimensions have kernels of their own for the plain forms; other forms and widths
+// take the catch-all ones
 static int psi_fwd_df64(const psi_impl::PsiArgs<double>& a, cudaStream_t st) {
   const int rc = psi_impl::check_fwd(a);
   if (rc != GPK_OK) return rc;
   if (a.Q <= 2) return psi_fwd_df64_q2(a, st);
-  if (a.Q == 5) {
-    const int r5 = psi_fwd_df64_q5(a, st);
-    if (r5 != GPK_EUNSUPPORTED) return r5;
+  if (a.Q <= 5) {
+    const int rp = a.Q == 5 ? psi_fwd_df64_q5(a, st) : psi_fwd_df64_q4(a, st);
+    if (rp != GPK_EUNSUPPORTED) return rp;
   }
   return psi_fwd_df64_q8(a, st);
 }
@@ -28,9 +30,9 @@ static int psi_fwd_f32(const psi_impl::PsiArgs<float>& a, cudaStream_t st) {
   const int rc = psi_impl::check_fwd(a);
   if (rc != GPK_OK) return rc;
   if (a.Q <= 2) return psi_fwd_f32_q2(a, st);
-  if (a.Q == 5) {
-    const int r5 = psi_fwd_f32_q5(a, st);
-    if (r5 != GPK_EUNSUPPORTED) return r5;
+  if (a.Q <= 5) {
+    const int rp = a.Q == 5 ? psi_fwd_f32_q5(a, st) : psi_fwd_f32_q4(a, st);
+    if (rp != GPK_EUNSUPPORTED) return rp;
   }
   return psi_fwd_f32_q8(a, st);
 }

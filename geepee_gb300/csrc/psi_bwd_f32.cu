@@ -2,7 +2,8 @@
 // and precision, so the build compiles them in parallel).
 #include "psi_impl.cuh"
 
-int psi_bwd_f32(const psi_impl::PsiArgs<float>& a, cudaStream_t st) { return psi_impl::launch_bwd<float>(a, st); }
+int psi_bwd_f32_w(const psi_impl::PsiArgs<float>& a, int QC, const psi_impl::BLayout& lo, size_t sm, bool two, cudaStream_t st);
+int psi_bwd_f32(const psi_impl::PsiArgs<float>& a, cudaStream_t st) { return psi_impl::launch_bwd<float>(a, psi_bwd_f32_w, st); }
 
 // the translation unit's bounds word (debug build; 0 otherwise)
 GPK_BOUNDS_READER(psi_bwd_f32)

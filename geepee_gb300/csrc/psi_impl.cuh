@@ -34,9 +34,14 @@ namespace psi_impl {
 constexpr int QMAX = 8;
 constexpr int DMAX = 4;
 constexpr int NT = 512;        // threads per CTA (forward)
-// Q is QC itself in an exact instantiation (every width other than the two catch-all ones, 2
-// for Q <= 2 and QMAX above): the per-dimension loops then carry no runtime test
-__host__ __device__ constexpr bool exact_q(int QC) { return QC != 2 && QC != QMAX; }
+// The widths: 2 (Q <= 2) and QMAX are the catch-all ones; 4 (Q = 3, 4) and 5 serve the plain forms only.
+// At width QMAX, Q = 3 does nearly three times the row sums it needs: N = 2000, M = 64, Q = 3
+// At width QMAX, Q = 3 does nearly three times the row sums it needs: N = 5000, M = 90, Q = 3 took
+// 158 + 409 us forward and backward there, 119 + 293 us at width 4; Q = 4 162 + 416 against
+// 121 + 303.  Q is QC itself at width 5 (the
+// psi-statistics workload's): the per-dimension loops then carry no runtime test.
+__host__ __device__ constexpr bool exact_q(int QC) { return QC == 5; }
+__host__ __device__ constexpr bool plain_q(int QC) { return QC == 4 || QC == 5; }
 // a pseudo-input's record in a point's table: u, t_1 .. t_QC (zeros past Q), padded to an odd
 // count so that the lanes of a warp (consecutive pseudo-inputs) read different banks
 __host__ __device__ constexpr int rec_len(int QC) { return (1 + QC) | 1; }
@@ -2122,7 +2127,7 @@ int launch_fwd_q(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
     if (rc == -1) rc = run_out<T, QC, 16, 4>(a, SMEM_CAP, st);
   }
   if (rc != -1) return rc;
-  if constexpr (exact_q(QC)) {
+  if constexpr (plain_q(QC)) {
     return GPK_EUNSUPPORTED;   // the caller falls back to the catch-all width
   } else {
     return fwd_gen<T, QC>(a, sum, contract, P, st);
@@ -2180,16 +2185,21 @@ int bwd_db(const PsiArgs<typename Num<T>::store_t>& a, const BLayout& lo, size_t
 }
 
 // the warp split: 12 + 4 + 4 with one CTA an SM (128 rows at a time), 6 + 2 + 2 with two
-template <typename T, bool TWO>
-int bwd_qc(const PsiArgs<typename Num<T>::store_t>& a, int QC, const BLayout& lo, size_t sm, cudaStream_t st) {
-  constexpr int NS = TWO ? 6 : 12, NR = TWO ? 2 : 4;
-  if (QC == 2) return bwd_db<T, 2, NS, NR, NR>(a, lo, sm, st);
-  if (QC == 5) return bwd_db<T, 5, NS, NR, NR>(a, lo, sm, st);
-  return bwd_db<T, QMAX, NS, NR, NR>(a, lo, sm, st);
+template <typename T, int QC>
+int bwd_width(const PsiArgs<typename Num<T>::store_t>& a, const BLayout& lo, size_t sm, bool two, cudaStream_t st) {
+  return two ? bwd_db<T, QC, 6, 2, 2>(a, lo, sm, st) : bwd_db<T, QC, 12, 4, 4>(a, lo, sm, st);
+}
+// widths 4 and QMAX (a translation unit of their own)
+template <typename S>
+using BwdWide = int (*)(const PsiArgs<S>& a, int QC, const BLayout& lo, size_t sm, bool two, cudaStream_t st);
+template <typename T>
+int bwd_wide(const PsiArgs<typename Num<T>::store_t>& a, int QC, const BLayout& lo, size_t sm, bool two,
+             cudaStream_t st) {
+  return QC == 4 ? bwd_width<T, 4>(a, lo, sm, two, st) : bwd_width<T, QMAX>(a, lo, sm, two, st);
 }
 
 template <typename T>
-int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
+int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, BwdWide<typename Num<T>::store_t> wide, cudaStream_t st) {
   const int M = a.M, P = M * (M + 1) / 2;
   if (M > 512) return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d > %d", M, 512);
   const size_t cap = SMEM_CAP;
@@ -2197,7 +2207,12 @@ int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
   const size_t need = 2048 + ((size_t)M * a.Q + 84 + (size_t)M * (1 + a.Q) + 2 * (size_t)P + (size_t)M * 9 +
                               (size_t)M * a.Q + 1536) * sizeof(T);
   if (need > 227 * 1024) return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d needs too much shared memory", M);
-  const int QC = a.Q <= 2 ? 2 : (a.Q == 5 ? 5 : QMAX);   // 5: the psi-statistics workload's width, exact
+  const int QC = a.Q <= 2 ? 2 : a.Q <= 4 ? 4 : a.Q == 5 ? 5 : QMAX;
+  auto run = [&](const BLayout& lo, size_t sm, bool two) {
+    if (QC == 2) return bwd_width<T, 2>(a, lo, sm, two, st);
+    if (QC == 5) return bwd_width<T, 5>(a, lo, sm, two, st);
+    return wide(a, QC, lo, sm, two, st);
+  };
   const int nbs = a.b_stride == 0 ? a.Dout * P : 0, nacc = a.dB ? a.Dout * P : 0;
   auto bytes = [&](const BLayout& lo, int nb) { return bcarve<T>(nullptr, nullptr, M, QC, P, a.Dout, nb, lo); };
   auto segs = [&](int threads) { return threads / M > 8 ? 8 : (threads / M < 1 ? 1 : threads / M); };
@@ -2206,7 +2221,7 @@ int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
   {
     const BLayout lo{segs(256), P, nbs, nacc, M <= 255};
     const size_t sm = bytes(lo, 2);
-    if (lo.pab && sm <= (cap - 2048) / 2) return bwd_qc<T, true>(a, QC, lo, sm, st);
+    if (lo.pab && sm <= (cap - 2048) / 2) return run(lo, sm, true);
   }
   // preference: G, B, the dBhat accumulators and the pair table in shared memory; without the pair
   // table; then without G (a few operations per dimension and pair), without B (two loads and
@@ -2219,14 +2234,14 @@ int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, cudaStream_t st) {
       for (int seg = smax; seg >= (smax > 4 ? 4 : smax); --seg) {
         const BLayout lo{seg, opts[o][0], opts[o][1], opts[o][2], pab};
         const size_t sm = bytes(lo, 4);
-        if (sm <= cap) return bwd_qc<T, false>(a, QC, lo, sm, st);
+        if (sm <= cap) return run(lo, sm, false);
       }
     }
   }
   for (int seg = smax; seg >= 1; --seg) {   // the largest M accepted
     const BLayout lo{seg, 0, 0, 0, 0};
     const size_t sm = bytes(lo, 4);
-    if (sm <= cap) return bwd_qc<T, false>(a, QC, lo, sm, st);
+    if (sm <= cap) return run(lo, sm, false);
   }
   return gpk::fail(GPK_EUNSUPPORTED, "psi_bwd: M=%d needs too much shared memory", M);
 }

@@ -184,3 +184,10 @@ def test_psi_points_written_out(N, M, Q, dtype):
     tol = 1e-10 if dtype == 'float64' else 1e-4
     np.testing.assert_allclose(psi1.cpu().numpy(), p1, rtol=tol, atol=tol * np.abs(p1).max())
     np.testing.assert_allclose(psi2.cpu().numpy(), p2, rtol=tol, atol=tol * np.abs(p2).max())
+
+
+@pytest.mark.parametrize('M,Q,Dout,N', [(1, 3, 1, 1), (37, 3, 2, 41), (64, 4, 1, 7), (100, 4, 4, 5), (129, 3, 1, 3)])
+def test_psi_layer_three_and_four_inputs(M, Q, Dout, N):
+    """The width that serves three and four input dimensions, both warp splits, forward and backward."""
+    test_psi_layer_edge_sizes(M, Q, Dout, N, True)
+    test_psi_layer_edge_sizes(M, Q, Dout, N, False)
