@@ -35,7 +35,6 @@ constexpr int QMAX = 8;
 constexpr int DMAX = 4;
 constexpr int NT = 512;        // threads per CTA (forward)
 // The widths: 2 (Q <= 2) and QMAX are the catch-all ones; 4 (Q = 3, 4) and 5 serve the plain forms only.
-// At width QMAX, Q = 3 does nearly three times the row sums it needs: N = 2000, M = 64, Q = 3
 // At width QMAX, Q = 3 does nearly three times the row sums it needs: N = 5000, M = 90, Q = 3 took
 // 158 + 409 us forward and backward there, 119 + 293 us at width 4; Q = 4 162 + 416 against
 // 121 + 303.  Q is QC itself at width 5 (the
@@ -739,7 +738,9 @@ __global__ void __launch_bounds__(NT) psi_fwd_gen_kernel(PsiArgs<typename Num<T>
 //   through both: front warps: constants, psi1 terms and records of point i+1
 // with one CTA barrier after each stage.  In one-role form (every warp doing each phase in
 // turn, six barriers a point) the per-row phases kept 4 of 16 warps busy and the barriers were
-// the largest stall.  Measured (df64, with the reduction of the partial blocks): N = 10000, Q = 5,
+// the largest stall.  Weights of each point's own (b_stride) are staged by the sweep warps at the start
+// of stage A: fetched pair by pair inside the sweep, every pair waited for two loads (N = 301,
+// M = 67, Q = 3, with the call: 138 -> 111 us; N = 1000, M = 100, Q = 4 204 -> 139).  Measured (df64, with the reduction of the partial blocks): N = 10000, Q = 5,
 // M = 100: 1591 -> 766 us, 660 -> ~400 instructions a pair and point, 65% of issue slots; N = 1000,
 // Q = 2, M = 100: 128 -> 84 us, of which ~35 us are per-CTA tables and the flush; N = 4999, Q = 2,
 // M = 50, two outputs: 295 -> 128 us; FP32 at N = 10000: 416 -> 236 us.  Bound by instruction
@@ -985,7 +986,7 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
     if (cnt > 0) front(0);
   } else {
     constexpr int NTA = NTS + NB * 32;
-    stage_pairs<T, QC, NS + NB, 3>(s.z, s.inv4l, Q, M, P, D, a.B, true, s.pab, s.G, s.Bs, s.L);
+    stage_pairs<T, QC, NS + NB, 3>(s.z, s.inv4l, Q, M, P, D, a.B, true, s.pab, s.G, a.b_stride ? nullptr : s.Bs, s.L);
     if (s.accB)
 #pragma unroll 1
       for (int i = tid; i < D * P; i += NTA) s.accB[i] = Num<T>::zero();
@@ -1003,15 +1004,18 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
     } else {
       const R* rec = s.rec + (size_t)(i & 1) * M * RL;
       const bool general = X::TAB && s_flag[sl];
+      if (a.b_stride && s.Bs)   // this point's weights (the row sums of the last one are done with L)
+        stage_pairs<T, QC, NS, 4>(s.z, s.inv4l, Q, M, P, 1, a.B + (size_t)n * a.b_stride, true, s.pab, nullptr, s.Bs, s.L);
       T dvr[DB];
 #pragma unroll
       for (int d = 0; d < DB; ++d) dvr[d] = d < D ? s.pg[sl * 2 * DMAX + DMAX + d] : Num<T>::zero();
-      if (D == DB && s.Bs && s.accB && s.G && s.pab && !general) {
+      if (D == DB && s.Bs && (s.accB || !a.dB) && s.G && s.pab && !general) {
         // the common configuration, branch-free: two pairs (p, p + NTS) per iteration, each step
         // written for both, so that their dependent chains interleave
         constexpr int E = sizeof(T);
-        const saddr ar = sm_addr(rec), aG = sm_addr(s.G), aB = sm_addr(s.Bs), aL = sm_addr(s.L), aC = sm_addr(s.accB),
-                    ap = sm_addr(s.pab), at = sm_addr(s.tab);
+        const bool sum = s.accB;
+        const saddr ar = sm_addr(rec), aG = sm_addr(s.G), aB = sm_addr(s.Bs), aL = sm_addr(s.L),
+                    aC = sum ? sm_addr(s.accB) : 0u, ap = sm_addr(s.pab), at = sm_addr(s.tab);
         for (int p0 = tid; p0 < P; p0 += 2 * NTS) {
           saddr o[2];   // the pairs' byte offsets
           R arg[2];
@@ -1043,7 +1047,7 @@ __global__ void __launch_bounds__((NS + NB + NF) * 32, NS < 12 ? 2 : 1)
               sts(aL + o[u], l);
 #pragma unroll
               for (int d = 0; d < DB; ++d)
-                sts(aC + d * P * E + o[u], add(ldsv<T>(aC + d * P * E + o[u]), ab[d]));
+                if (sum) sts(aC + d * P * E + o[u], add(ldsv<T>(aC + d * P * E + o[u]), ab[d]));
             }
           }
         }
@@ -2213,7 +2217,7 @@ int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, BwdWide<typename Num<
     if (QC == 5) return bwd_width<T, 5>(a, lo, sm, two, st);
     return wide(a, QC, lo, sm, two, st);
   };
-  const int nbs = a.b_stride == 0 ? a.Dout * P : 0, nacc = a.dB ? a.Dout * P : 0;
+  const int nbs = a.Dout * P, nacc = a.dB ? a.Dout * P : 0;
   auto bytes = [&](const BLayout& lo, int nb) { return bcarve<T>(nullptr, nullptr, M, QC, P, a.Dout, nb, lo); };
   auto segs = [&](int threads) { return threads / M > 8 ? 8 : (threads / M < 1 ? 1 : threads / M); };
   // two CTAs of ten warps an SM where everything fits twice (M <= ~60 in double-float precision):
@@ -2227,7 +2231,9 @@ int launch_bwd(const PsiArgs<typename Num<T>::store_t>& a, BwdWide<typename Num<
   // table; then without G (a few operations per dimension and pair), without B (two loads and
   // conversions), without both, and without the accumulators (dBhat then accumulates in the
   // partial block, or with atomics).  Four row segments instead of five where that makes room.
-  const int opts[6][3] = {{P, nbs, nacc}, {0, nbs, nacc}, {P, 0, nacc}, {0, 0, nacc}, {P, 0, 0}, {0, 0, 0}};
+  // Weights of each point's own: G stays before them (they are staged again for every point).
+  const int opts[6][3] = {{P, nbs, nacc}, {a.b_stride ? P : 0, a.b_stride ? 0 : nbs, nacc},
+                          {P, 0, nacc}, {0, 0, nacc}, {P, 0, 0}, {0, 0, 0}};
   const int smax = segs(512);
   for (int o = 0; o < 6; ++o) {
     for (int pab = M <= 255; pab >= 0; --pab) {

@@ -191,3 +191,20 @@ def test_psi_layer_three_and_four_inputs(M, Q, Dout, N):
     """The width that serves three and four input dimensions, both warp splits, forward and backward."""
     test_psi_layer_edge_sizes(M, Q, Dout, N, True)
     test_psi_layer_edge_sizes(M, Q, Dout, N, False)
+
+
+@pytest.mark.parametrize('N,M,Q', [(3, 1, 1), (5, 2, 3), (9, 67, 3), (200, 100, 4), (160, 128, 8), (5, 155, 2)])
+def test_psi_derivatives_of_points_own_weights(N, M, Q):
+    """Upstream weights of each point's own, not symmetric, at the sizes where their staging and
+    the split change.  Same tolerance as the golden derivatives."""
+    from geepee_gb300 import kernels as K
+    rng = np.random.RandomState(N + M)
+    Z, mu, S = rng.randn(M, Q), rng.randn(N, Q), rng.uniform(0.01, 1.0, (N, Q))
+    lls2, lsf2 = rng.uniform(-0.5, 0.5, Q), np.array([0.3])
+    d1, d2 = rng.randn(N, M), rng.randn(N, M, M) / M
+    p1, p2 = O.psi_stats(lls2, lsf2, mu, S, Z)
+    ell, sf2 = np.exp(0.5 * lls2), float(np.exp(lsf2[0]))
+    got = K.compute_psi_derivatives(d1, p1, d2, p2, ell, sf2, mu, S, Z)
+    ref = O.psi_derivatives(d1, p1, d2, p2, ell, sf2, mu, S, Z)
+    for name, g, r in zip(('dsf2', 'dl', 'dZ', 'dmu', 'dS'), got, ref):
+        assert_close(g, r, 1e-9, name)
