@@ -161,33 +161,43 @@ __device__ __forceinline__ void load_pair_table(float2* tab) {
 __host__ __device__ inline size_t pair_table_bytes(size_t tsz) { return tsz == 8 ? kFxTab * sizeof(float2) : 0; }
 
 // The symmetrised weights of the packed pairs, Bs[d P + p] = B_d[a,b] + B_d[b,a] (a != b) or
-// B_d[a,a]: each thread keeps eight pairs' global loads in flight before converting them, so
-// the table costs a few memory latencies per CTA instead of one per pair.
+// B_d[a,a].  B is read along its rows: the triangle at and below the diagonal by asynchronous copies
+// into Bs, then the one above, four loads in flight a thread, each entry added where its mirror
+// image lies (reading a pair's two entries together took a 32-byte sector per transposed entry).
 template <typename T, int NTH>
 __device__ void stage_sym_B(T* Bs, const typename Num<T>::store_t* B, int M, int D, int P) {
   typedef typename Num<T>::store_t S;
-  constexpr int K = 8;
-  for (int d = 0; d < D; ++d) {
-    const S* Bd = B + (size_t)d * M * M;
+  constexpr int K = 4;
+  for (int d = 0; d < D; ++d, B += (size_t)M * M, Bs += P) {
+#pragma unroll 1
+    for (int p = threadIdx.x; p < P; p += NTH) {
+      int ia, ib;
+      pair_of(p, ia, ib);
+      async_copy(reinterpret_cast<S*>(Bs) + p, B + ia * M + ib);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll 1
     for (int p0 = threadIdx.x; p0 < P; p0 += K * NTH) {
-      S x1[K], x2[K];
+      S x[K];
+      int o[K];
       bool off[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const int p = p0 + k * NTH;
         int ia = 0, ib = 0;
         if (p < P) pair_of(p, ia, ib);
-        off[k] = ia != ib;
-        x1[k] = p < P ? Bd[ia * M + ib] : S(0);
-        x2[k] = off[k] ? Bd[ib * M + ia] : S(0);
+        const int ja = M - 1 - ib, jb = M - 1 - ia;   // row jb, column ja >= jb: consecutive threads descend
+        off[k] = ja != jb;
+        o[k] = p < P ? ja * (ja + 1) / 2 + jb : -1;
+        x[k] = p < P && off[k] ? B[jb * M + ja] : S(0);
       }
 #pragma unroll
       for (int k = 0; k < K; ++k) {
-        const int p = p0 + k * NTH;
-        if (p < P) {
-          T w = Num<T>::ld(x1[k]);
-          if (off[k]) w = add(w, Num<T>::ld(x2[k]));
-          Bs[d * P + p] = w;
+        if (o[k] >= 0) {
+          T w = Num<T>::ld(reinterpret_cast<const S*>(Bs)[o[k]]);
+          if (off[k]) w = add(w, Num<T>::ld(x[k]));
+          Bs[o[k]] = w;
         }
       }
     }
@@ -614,6 +624,11 @@ __global__ void __launch_bounds__(NT) psi_fwd_gen_kernel(PsiArgs<typename Num<T>
     }
     __syncthreads();
     // ---- pairs
+    bool any_flag = false;
+    if (X::TAB) {
+#pragma unroll
+      for (int pt = 0; pt < NPB; ++pt) any_flag |= s_flag[pt] != 0;
+    }
     T vacc[NPB][DB];
 #pragma unroll
     for (int pt = 0; pt < NPB; ++pt)
@@ -663,6 +678,35 @@ __global__ void __launch_bounds__(NT) psi_fwd_gen_kernel(PsiArgs<typename Num<T>
       for (int k = 0; k < KP; ++k) {
         const int p = threadIdx.x + k * NT;
         if (p < P) do_pair(p, pab[k] >> 16, pab[k] & 0xffff, acc[k]);
+      }
+    } else if (contract && !a.psi2 && s.Bs && D == DB && !any_flag) {
+      // moments only, every point in the fixed-point range: branch-free over the pass's slots, so that
+      // their exps interleave (the steps of do_pair, so the same bits; a pass with fewer points
+      // runs the extra slots on stale tables and never reads their sums).  N = 777, Q = 2, M = 200:
+      // 151 -> 138 us
+      constexpr int E = sizeof(T);
+      const saddr ar = sm_addr(s.rec), at = sm_addr(s.tab), step = M * (RL * E);
+      for (int p = threadIdx.x; p < P; p += NT) {
+        int ia, ib;
+        pair_of(p, ia, ib);
+        const R gab = s.G ? s.G[p] : pair_G<T, QC>(s.z + ia * Q, s.z + ib * Q, s.inv4l, Q);
+        T w[DB];
+#pragma unroll
+        for (int d = 0; d < DB; ++d) w[d] = s.Bs[d * P + p];
+        saddr ra = ar + ia * (RL * E), rb = ar + ib * (RL * E);
+        R arg[NPB];
+#pragma unroll
+        for (int pt = 0; pt < NPB; ++pt) {
+          arg[pt] = X::template arg<QC>(ra, rb, gab);
+          ra += step;
+          rb += step;
+        }
+#pragma unroll
+        for (int pt = 0; pt < NPB; ++pt) {
+          const T ps = X::ev(arg[pt], at);
+#pragma unroll
+          for (int d = 0; d < DB; ++d) vacc[pt][d] = fma_(w[d], ps, vacc[pt][d]);
+        }
       }
     } else {
       T dummy = Num<T>::zero();
@@ -2051,6 +2095,18 @@ int fwd_gen(const PsiArgs<typename Num<T>::store_t>& a, bool sum, bool contract,
     if (a.Dout == 1) return run_fwd_gen<T, 1, 0, QC, 1>(a, st);
     if (a.Dout == 2) return run_fwd_gen<T, 1, 0, QC, 2>(a, st);
     return run_fwd_gen<T, 1, 0, QC, 4>(a, st);
+  }
+  if (contract && a.Dout == 1 && !a.psi2) {
+    // points per pass: a pass evaluates all its slots at ~75 instructions each beside ~100 a pair for
+    // its constants, so that with few points a CTA a width that divides them leaves fewer slots idle
+    // (M = 200, Q = 2, with B read along its rows: 100 points 80 -> 55 us, 777 points 138 -> 119)
+    const int per = gpk::ceil_div(a.N, gpk::sm_count());
+    int best = 4;
+    for (int npb = 3; npb >= 1; --npb)
+      if ((long)gpk::ceil_div(per, npb) * (100 + 75 * npb) < (long)gpk::ceil_div(per, best) * (100 + 75 * best)) best = npb;
+    if (best == 1) return run_fwd_gen<T, 1, 0, QC, 1>(a, st);
+    if (best == 2) return run_fwd_gen<T, 2, 0, QC, 1>(a, st);
+    if (best == 3) return run_fwd_gen<T, 3, 0, QC, 1>(a, st);
   }
   if (!contract || a.Dout == 1) return run_fwd_gen<T, 4, 0, QC, 1>(a, st);
   if (a.Dout == 2) return run_fwd_gen<T, 4, 0, QC, 2>(a, st);

@@ -208,3 +208,28 @@ def test_psi_derivatives_of_points_own_weights(N, M, Q):
     ref = O.psi_derivatives(d1, p1, d2, p2, ell, sf2, mu, S, Z)
     for name, g, r in zip(('dsf2', 'dl', 'dZ', 'dmu', 'dS'), got, ref):
         assert_close(g, r, 1e-9, name)
+
+
+@pytest.mark.parametrize('N', [1, 153, 330, 480, 777])
+def test_psi_moments_where_the_tables_do_not_fit(N):
+    """M = 200, one to six points a CTA (every number of points a pass): against the oracle, and a
+    point's moments the same bits whatever the batch."""
+    from geepee_gb300 import gpk
+    M, Q = 200, 2
+    rng = np.random.RandomState(5)
+    Z, mu, S = rng.randn(M, Q), rng.randn(777, Q), rng.uniform(0.01, 1.0, (777, Q))
+    A, B = rng.randn(1, M) / M, rng.randn(1, M, M) / M
+    B = B + B.transpose(0, 2, 1)
+    mu[2] = 40.0   # outside the fixed-point range
+    lls2, lsf2 = np.array([0.2, -0.3]), np.array([0.3])
+    def run(n):
+        m, v = z(n, 1), z(n, 1)
+        gpk.psi_fwd(dev(mu[:n]), dev(S[:n]), dev(Z), dev(lls2), dev(lsf2), dev(A), dev(B), m_out=m, v_out=v)
+        return m, v
+    m, v = run(N)
+    p1, p2 = O.psi_stats(lls2, lsf2, mu[:N], S[:N], Z)
+    m_ref = p1 @ A.T
+    assert_close(m.cpu().numpy(), m_ref, TOL, 'm')
+    assert_close(v.cpu().numpy(), np.exp(0.3) + np.einsum('dab,nab->nd', B, p2) - m_ref ** 2, TOL, 'v')
+    m7, v7 = run(777)
+    assert torch.equal(m, m7[:N]) and torch.equal(v, v7[:N])
