@@ -184,11 +184,11 @@ def psi_bwd_bytes(N, M, Q, D):
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one psi backward launch pair (kernel and
 # reduction) of the deep GP's layer 2 in one ncu capture of the same case (1000 points, M=100,
-# Q=2): 280,064 + 41,216 bytes for the pipelined kernel (its inputs; its outputs and partial
-# blocks stay in L2) and 6,605,312 for the reduction, which ncu replays after flushing the
+# Q=2): 287,232 + 0 bytes for the kernel (its inputs; its outputs and partial blocks stay in
+# L2) and 6,605,312 for the reduction, which ncu replays after flushing the
 # caches, so that the 152 per-CTA partial blocks it reads come from DRAM (in the evaluation
 # they are still in L2)
-PSI_BWD_TRAFFIC = 280064 + 41216 + 6605312
+PSI_BWD_TRAFFIC = 287232 + 6605312
 
 
 def time_launches(fn, flush, reps=30):
@@ -434,7 +434,7 @@ def run_ours(args, world, rank, local):
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
     fp32_peak = fp32_peak_tflops(n_sm, sm_mhz)
     achieved = F / t_k / 1e12
-    roofline = {'kernel': 'psi_bwd_pipe_kernel<df64> + its fixed-order reduction (layer 2, 1000 points, M=100, Q=2)',
+    roofline = {'kernel': 'psi_bwd_kernel<df64> + its fixed-order reduction (layer 2, 1000 points, M=100, Q=2)',
                 'bound': 'fp32-pipe', 'achieved': round(achieved, 4), 'peak': round(fp32_peak, 1),
                 'unit': 'TFLOP/s', 'frac': round(achieved / fp32_peak, 5),
                 'work': 'algorithmic: (8MQ + 20PQ + 4 Dout M^2) per point, P = M(M+1)/2, x 1000 points '
@@ -444,7 +444,7 @@ def run_ours(args, world, rank, local):
                 'us_per_launch': round(t_k * 1e6, 2),
                 'df64_issue': {'fp32_ops_per_launch': ops, 'tflops': round(ops / t_k / 1e12, 3),
                                'frac': round(ops / t_k / 1e12 / fp32_peak, 4),
-                               'note': 'the FP32 instructions the double-float arithmetic issues'},
+                               'note': 'the FP32 operations of the same work in plain double-float arithmetic'},
                 'hbm_algorithmic_gbs': round(psi_bwd_bytes(MB, M_PSEUDO, HIDDEN, 1) / t_k / 1e9, 2),
                 'hbm_peak_gbs': peaks.get('hbm_gbs'),
                 # dram__bytes (read + write) of this launch pair in one ncu capture of the same case
