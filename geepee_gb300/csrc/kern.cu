@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) kern_matrix_kernel(int N, int M, int D, c
 struct __align__(16) ArdHyp {
   double s[DMAXK];      // sqrt(log2(e)/2) / ell_d
   df64 inv_l2[DMAXK];   // 1/ell_d^2 (general form)
-  df64 lsf, sf2;
+  df64 lsf;
   long long c0;         // log2 sf^2 in units of 2^-52, plus exp2_fx's half step
   int flag;             // sf^2 outside the fixed-point range: every entry takes the general form
 };
@@ -96,7 +96,6 @@ __device__ __forceinline__ void load_ard(ArdHyp& h, const double* lls2, const do
   }
   if (threadIdx.x == 32) {
     h.lsf = df_from_double(lsf2[0]);
-    h.sf2 = exp_tab(h.lsf, tab);
     const double c = lsf2[0] * 1.4426950408889634074;
     h.flag = !(fabs(c) < 126.0);
     h.c0 = (h.flag ? 0LL : __double2ll_rn(c * 4503599627370496.0)) + kFxHalf;
@@ -123,24 +122,30 @@ __device__ __forceinline__ void ard_exponents(saddr x, saddr xstep, saddr z, int
                                               float (&f)[R]) {
   long long mid[R];
 #pragma unroll
-  for (int i = 0; i < R; ++i) X[i] = c0, mid[i] = 0, f[i] = 0.f;
+  for (int i = 0; i < R; ++i) X[i] = c0, f[i] = 0.f;
+  // the cross terms of 16 dimensions stay below 2^63: sum h^2 < 2^60 where the entry is not zero, |l| < 2^31
+  for (int d0 = 0; d0 < D; d0 += 16) {
+    const int dn = min(16, D - d0);
+#pragma unroll
+    for (int i = 0; i < R; ++i) mid[i] = 0;
 #pragma unroll 4
-  for (int d = 0; d < D; ++d) {
-    const int4 zd = lds_i4(z);
-    z += 16;
+    for (int d = 0; d < dn; ++d) {
+      const int4 zd = lds_i4(z);
+      z += 16;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int4 xd = lds_i4(x + i * xstep);
-      const int h = xd.y - zd.y, l = xd.x - zd.x;
-      const float t = __int_as_float(xd.z) - __int_as_float(zd.z);
-      X[i] = mad_wide(-h, h, X[i]);
-      mid[i] = mad_wide(h, l, mid[i]);
-      f[i] = __fmaf_rn(t, t, f[i]);
+      for (int i = 0; i < R; ++i) {
+        const int4 xd = lds_i4(x + i * xstep);
+        const int h = xd.y - zd.y, l = xd.x - zd.x;
+        const float t = __int_as_float(xd.z) - __int_as_float(zd.z);
+        X[i] = mad_wide(-h, h, X[i]);
+        mid[i] = mad_wide(h, l, mid[i]);
+        f[i] = __fmaf_rn(t, t, f[i]);
+      }
+      x += 16;
     }
-    x += 16;
-  }
 #pragma unroll
-  for (int i = 0; i < R; ++i) X[i] -= mid[i] >> 30;
+    for (int i = 0; i < R; ++i) X[i] -= mid[i] >> 30;
+  }
 }
 __device__ __noinline__ df64 ard_general(const double* x, const double* z, int D, const ArdHyp& h, const float2* tab) {
   df64 rr = make_df(0.f);
@@ -1651,7 +1656,13 @@ long gram_work_elems(int N, int M, int Dout) {
   const long full = (long)gram_chunks(N, M, false) * Dout * M * M;   // u != v: full tiles
   const long pairs = (long)gram_pair_chunks(N, M) * Dout * (M * (M + 1) / 2);
   GramMma g;
-  const long mma = gram_mma_plan(N, M, Dout, &g) ? (long)g.chunks * Dout * (M * (M + 1) / 2) : 0;
+  // (a bound on chunks x Dout that grows with N and Dout: a workspace for the largest call serves smaller ones)
+  long mma = 0;
+  if (gram_mma_plan(N, M, Dout, &g)) {
+    const long least = gpk::ceil_div(gm_tiles(M), GM_W * GM_TW);
+    mma = std::min(std::max(gpk::sm_count() / least, (long)Dout), (long)Dout * std::max(1, gpk::ceil_div(N, 16))) *
+          (M * (M + 1) / 2);
+  }
   return std::max(full, std::max(pairs, mma));
 }
 

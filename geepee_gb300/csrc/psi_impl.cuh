@@ -1,7 +1,7 @@
 // Psi statistics of the ARD kernel under Gaussian inputs, fused with the
 // moment-matching contractions of a sparse-GP layer, and their backward pass.
 //
-// Work decomposition (both kernels): a CTA takes a contiguous range of data points, NPB
+// Work decomposition (the general forward; the other kernels split it by warps): a CTA takes a contiguous range of data points, NPB
 // points per pass; per pass its threads first build the points' tables in shared memory
 // (per-dimension constants, per-pseudo-input terms u_a, h_aq), then sweep the M(M+1)/2
 // unordered pairs (a <= b) of pseudo-inputs, each pair for all NPB points.  Each thread

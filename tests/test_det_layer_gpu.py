@@ -102,3 +102,20 @@ def test_symmetric_gram_edges(n, m, dout):
         g, keep = C.cpu().numpy(), np.arange(m) != 6
         assert not np.isfinite(g[:, 6]).any() and not np.isfinite(g[:, :, 6]).any()
         assert (np.abs(g - ref) <= tol)[:, keep][:, :, keep].all()
+
+
+def test_gram_workspace_of_a_larger_call():
+    """A workspace sized for the largest call serves every smaller one (fewer rows are split into more
+    chunks than twenty thousand are)."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(2)
+    m = 20
+    z = lambda *s: torch.zeros(s, dtype=torch.float64, device='cuda')
+    for dout in (1, 3):
+        work = z(gpk.work_elems(gpk.OP_GRAM, 20000, m, 1, 3))
+        for n in (1, 16, 800, 2432, 2433, 4865):
+            u, w = rng.randn(n, m), rng.randn(n, dout)
+            C, ut = z(dout, m, m), dev(u)
+            gpk.gram(ut, ut, dev(w), C, work=work)
+            ref = np.einsum('nd,na,nb->dab', w, u, u)
+            assert np.abs(C.cpu().numpy() - ref).max() <= 1e-10 * max(1.0, np.abs(ref).max())
