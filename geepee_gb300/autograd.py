@@ -53,10 +53,10 @@ class _Sums:
 
     def grads(self, hyp):
         """(dZ, g_lls2, g_lsf2, dA, dB) in the inputs' types."""
-        (lt, _), (st, sshape) = hyp
+        (lt, lshape), (st, sshape) = hyp
         rest = self.acc.split(self.sizes)[1:] if self.cast is None else self.cast.split(self.sizes[1:])
         dZ, dA, dB = [t.view(s) for t, s in zip(rest, self.shapes)]
-        return dZ, self.g_l.to(lt), self.g_s.reshape(sshape).to(st), dA, dB
+        return dZ, self.g_l.reshape(lshape).to(lt), self.g_s.reshape(sshape).to(st), dA, dB
 
 
 def _hyp_kind(lls2, lsf2):

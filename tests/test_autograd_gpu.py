@@ -113,3 +113,24 @@ def test_moment_grads(n, Q, rest, dtype):
     assert abs(float(gs - want)) <= (2 * n + 8) * 2.0 ** -53 * float(torch.exp(s2)) * (float(dv.double().abs().sum()) + 8)
     if cast is not None:
         assert torch.equal(cast, acc[1 + Q:].float())
+
+
+@pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
+@pytest.mark.parametrize('layer', ['psi', 'det'])
+def test_lengthscales_as_a_row(layer, dtype):
+    """Log-lengthscales of shape (1, Q) get the gradient of the flat ones, in their own shape."""
+    from geepee_gb300 import autograd
+    g = torch.Generator(device='cuda').manual_seed(5)
+    N, M, Q, D = 40, 12, 3, 2
+    r = lambda *s: torch.randn(*s, generator=g, dtype=torch.float64, device='cuda').to(dtype)
+    rows = [r(N, Q)] + ([torch.rand(N, Q, generator=g, dtype=torch.float64, device='cuda').to(dtype)] if layer == 'psi' else [])
+    Z, ls, A, B = r(M, Q), 0.3 * r(Q), r(D, M) / M, r(D, M, M) / M
+    B, wm, wv = 0.5 * (B + B.transpose(1, 2)), r(N, D), r(N, D)
+    got = []
+    for shape in ((Q,), (1, Q)):
+        l = ls.reshape(shape).clone().requires_grad_(True)
+        m, v = getattr(autograd, layer + '_moments')(*rows, Z, l, torch.zeros(1, dtype=dtype, device='cuda'), A, B)
+        (wm * m + wv * v).sum().backward()
+        assert l.grad.shape == l.shape and l.grad.dtype == dtype
+        got.append(l.grad.reshape(-1))
+    assert torch.equal(*got)
