@@ -67,8 +67,8 @@ _SIGS = {
     'gpk_triu_pack': [_c_int, _c_int, _vp, _vp, _vp, _c_int, _vp],
     'gpk_hyp_grads': [_c_int, _vp, _vp, _vp, _vp, _vp, _c_int, _vp, _vp, _vp],
     'gpk_moment_grads': [_c_int, _c_int, ctypes.c_long, _vp, _vp, _vp, _vp, ctypes.c_long, _vp, _vp, _vp, _vp],
-    'gpk_psi_layer_bwd': [_c_int] * 5 + [_vp] * 16 + [_vp, ctypes.c_long, _vp],
-    'gpk_det_layer_bwd': [_c_int] * 5 + [_vp, _c_int] + [_vp] * 13 + [_vp, ctypes.c_long, _vp],
+    'gpk_psi_layer_bwd': [_c_int] * 5 + [_vp] * 17 + [_vp, ctypes.c_long, _vp],
+    'gpk_det_layer_bwd': [_c_int] * 5 + [_vp, _c_int] + [_vp] * 14 + [_vp, ctypes.c_long, _vp],
     'gpk_aep_phi': [_c_int, _c_int, _c_dbl, _c_dbl, _vp, _vp, _vp, _vp, _vp, _vp, _c_dbl, _vp, _vp],
     'gpk_work_elems': [_c_int, _c_int, _c_int, _c_int, _c_int, _vp],
     'gpk_cavity_forms': [_c_int, _vp, _vp],

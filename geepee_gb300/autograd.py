@@ -39,24 +39,15 @@ def _up(g, like):
     return torch.zeros_like(like) if g is None else g.contiguous().to(like.dtype)
 
 
-class _Sums:
-    """One backward call's float64 sums, [dsf2 | dl | dZ | dA | dB], with the two chained
-    hyperparameter gradients behind them, and for float32 layers the casts of dZ, dA, dB."""
-
-    def __init__(self, Q, M, D, dtype, device):
-        self.sizes = [1 + Q, M * Q, D * M, D * M * M]
-        n = sum(self.sizes)
-        self.shapes = ((M, Q), (D, M), (D, M, M))
-        buf = torch.empty(n + Q + 1, dtype=torch.float64, device=device)
-        self.acc, self.g_l, self.g_s = buf.split([n, Q, 1])
-        self.cast = None if dtype == torch.float64 else torch.empty(n - 1 - Q, dtype=dtype, device=device)
-
-    def grads(self, hyp):
-        """(dZ, g_lls2, g_lsf2, dA, dB) in the inputs' types."""
-        (lt, lshape), (st, sshape) = hyp
-        rest = self.acc.split(self.sizes)[1:] if self.cast is None else self.cast.split(self.sizes[1:])
-        dZ, dA, dB = [t.view(s) for t, s in zip(rest, self.shapes)]
-        return dZ, self.g_l.reshape(lshape).to(lt), self.g_s.reshape(sshape).to(st), dA, dB
+def _shared_grads(Z, A, hyp):
+    """Gradients of what all rows share, uninitialised, each a tensor of its own: (dZ, dA, dB) in the
+    layer's type, (g_lls2, g_lsf2) in float64 and the hyperparameters' shapes; and the number of
+    float64 sums that the backward keeps beside them (float32 layers sum in float64 first)."""
+    (M, Q), D = Z.shape, A.shape[0]
+    dZ, dA = torch.empty_like(Z), torch.empty_like(A)
+    dB = torch.empty((D, M, M), dtype=A.dtype, device=A.device)
+    g_l, g_s = [torch.empty(shape, dtype=torch.float64, device=Z.device) for _, shape in hyp]
+    return dZ, dA, dB, g_l, g_s, 1 + Q + (0 if Z.dtype == torch.float64 else M * Q + D * M + D * M * M)
 
 
 def _hyp_kind(lls2, lsf2):
@@ -81,12 +72,11 @@ class PsiMoments(torch.autograd.Function):
         N, Q = mu.shape
         M, D = Z.shape[0], A.shape[0]
         dm, dv = _up(dm, m), _up(dv, m)
-        sums = _Sums(Q, M, D, mu.dtype, mu.device)
+        dZ, dA, dB, g_l, g_s, nsums = _shared_grads(Z, A, ctx.hyp)
         dmu, dS = torch.empty_like(mu), torch.empty_like(S)
-        work = torch.empty(gpk.work_elems(gpk.OP_PSI_BWD, N, M, Q, D), dtype=torch.float64, device=mu.device)
-        gpk.psi_layer_bwd(mu, S, Z, l2, s2, A, B, m, dm, dv, sums.acc, dmu, dS, sums.g_l, sums.g_s, sums.cast, work)
-        dZ, g_l, g_s, dA, dB = sums.grads(ctx.hyp)
-        return dmu, dS, dZ, g_l, g_s, dA, dB
+        work = torch.empty(nsums + gpk.work_elems(gpk.OP_PSI_BWD, N, M, Q, D), dtype=torch.float64, device=mu.device)
+        gpk.psi_layer_bwd(mu, S, Z, l2, s2, A, B, m, dm, dv, dZ, dA, dB, dmu, dS, g_l, g_s, work)
+        return dmu, dS, dZ, g_l.to(ctx.hyp[0][0]), g_s.to(ctx.hyp[1][0]), dA, dB
 
 
 class DetMoments(torch.autograd.Function):
@@ -111,13 +101,12 @@ class DetMoments(torch.autograd.Function):
         M, D = Z.shape[0], A.shape[0]
         dm = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dm is None else _up(dm, x)
         dv = torch.zeros((N, D), dtype=x.dtype, device=x.device) if dv is None else _up(dv, x)
-        sums = _Sums(Q, M, D, x.dtype, x.device)
+        dZ, dA, dB, g_l, g_s, nsums = _shared_grads(Z, A, ctx.hyp)
         dx = torch.empty_like(x)
         n1, n2 = gpk.work_elems(gpk.OP_DET_BWD, N, M, Q, D), gpk.work_elems(gpk.OP_GRAM, N, M, Q, D)
-        work = torch.empty(max(n1, n2), dtype=torch.float64, device=x.device)   # one after the other
-        gpk.det_layer_bwd(x, Z, l2, s2, A, kfu, Bk, dm, dv, sums.acc, dx, sums.g_l, sums.g_s, sums.cast, work)
-        dZ, g_l, g_s, dA, dB = sums.grads(ctx.hyp)
-        return dx, dZ, g_l, g_s, dA, dB
+        work = torch.empty(nsums + max(n1, n2), dtype=torch.float64, device=x.device)   # one after the other
+        gpk.det_layer_bwd(x, Z, l2, s2, A, kfu, Bk, dm, dv, dZ, dA, dB, dx, g_l, g_s, work)
+        return dx, dZ, g_l.to(ctx.hyp[0][0]), g_s.to(ctx.hyp[1][0]), dA, dB
 
 
 def psi_moments(mu, S, Z, lls2, lsf2, A, B):

@@ -74,22 +74,26 @@ __global__ void hyp_grads_kernel(int Q, const double* ls, const double* sf, cons
 
 // The tail of a layer's backward in one launch (one cluster of MG_CTAS CTAs):
 //   g_l[q] = acc[1 + q] exp(lls2[q] / 2) / 2,  g_s = exp(lsf2) (acc[0] + sum(dv)),
-//   cast[i] = acc[1 + Q + i] in FP32 (optional).
+//   the sums behind acc[Q], in FP32, to up to three destinations one after the other (optional).
 // The sum over dv is the work (a few doubles a thread): spread over a cluster, whose partial sums
 // meet in the first CTA's view of the others' shared memory, it takes ~4 us for 10000 values
 // where the ten tensor operations it replaces took ~10 us of device and ~60 us of host time.
 constexpr int MG_CTAS = 8, MG_THREADS = 512;
 template <typename S>
 __global__ void __cluster_dims__(MG_CTAS, 1, 1) __launch_bounds__(MG_THREADS)
-    moment_grads_kernel(int Q, long ncast, const double* lls2, const double* lsf2, const double* acc, const S* dv,
-                        long ndv, double* g_l, double* g_s, float* cast) {
+    moment_grads_kernel(int Q, const double* lls2, const double* lsf2, const double* acc, const S* dv, long ndv,
+                        double* g_l, double* g_s, int ncast, gpk::Counts n, gpk::Outputs cast) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ double red[MG_THREADS / 32], total;
   const int rank = (int)cluster.block_rank(), tid = threadIdx.x;
   const long t0 = (long)rank * MG_THREADS + tid, nt = (long)MG_CTAS * MG_THREADS;
-  if (cast)
-    for (long i = t0; i < ncast; i += nt) cast[i] = (float)acc[1 + Q + i];
+  const double* src = acc + 1 + Q;
+  for (int c = 0; c < ncast; ++c) {
+    float* const dst = (float*)cast.p[c];
+    for (long i = t0; i < n.n[c]; i += nt) dst[i] = (float)src[i];
+    src += n.n[c];
+  }
   double s = 0.0;
   for (long i = t0; i < ndv; i += nt) s += (double)dv[i];
   for (int m = 16; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
@@ -532,21 +536,28 @@ extern "C" int gpk_hyp_grads(int Q, const double* ls, const double* sf, const do
   return gpk::check_launch("hyp_grads");
 }
 
+int gpk::moment_grads(int prec, int Q, const double* lls2, const double* lsf2, const double* acc, const void* dv,
+                      long ndv, double* g_l, double* g_s, int ncast, Counts n, Outputs cast, void* stream) {
+  GPK_REQUIRE(prec == GPK_DF64 || prec == GPK_FP32, "moment_grads: unknown precision %d", prec);
+  GPK_REQUIRE(Q >= 1 && ndv >= 0, "moment_grads: bad sizes");
+  GPK_REQUIRE(lls2 && lsf2 && acc && g_l && g_s && (dv || ndv == 0), "moment_grads: null pointer");
+  cudaStream_t st = gpk::as_stream(stream);
+  if (prec == GPK_DF64)
+    moment_grads_kernel<double><<<MG_CTAS, MG_THREADS, 0, st>>>(Q, lls2, lsf2, acc, (const double*)dv, ndv, g_l, g_s, 0,
+                                                               n, cast);
+  else
+    moment_grads_kernel<float><<<MG_CTAS, MG_THREADS, 0, st>>>(Q, lls2, lsf2, acc, (const float*)dv, ndv, g_l, g_s, ncast,
+                                                              n, cast);
+  return gpk::check_launch("moment_grads");
+}
+
 extern "C" int gpk_moment_grads(int prec, int Q, long ncast, const double* lls2, const double* lsf2, const double* acc,
                                 const void* dv, long ndv, double* g_l, double* g_s, void* cast, void* stream) {
   GPK_NVTX("gpk_moment_grads");
-  GPK_REQUIRE(prec == GPK_DF64 || prec == GPK_FP32, "moment_grads: unknown precision %d", prec);
-  GPK_REQUIRE(Q >= 1 && ncast >= 0 && ndv >= 0, "moment_grads: bad sizes");
-  GPK_REQUIRE(lls2 && lsf2 && acc && g_l && g_s && (dv || ndv == 0), "moment_grads: null pointer");
+  GPK_REQUIRE(ncast >= 0, "moment_grads: bad sizes");
   GPK_REQUIRE(!cast || prec == GPK_FP32, "moment_grads: a cast output is FP32");
-  cudaStream_t st = gpk::as_stream(stream);
-  if (prec == GPK_DF64)
-    moment_grads_kernel<double><<<MG_CTAS, MG_THREADS, 0, st>>>(Q, ncast, lls2, lsf2, acc, (const double*)dv, ndv, g_l,
-                                                               g_s, nullptr);
-  else
-    moment_grads_kernel<float><<<MG_CTAS, MG_THREADS, 0, st>>>(Q, ncast, lls2, lsf2, acc, (const float*)dv, ndv, g_l, g_s,
-                                                              (float*)cast);
-  return gpk::check_launch("moment_grads");
+  return gpk::moment_grads(prec, Q, lls2, lsf2, acc, dv, ndv, g_l, g_s, cast ? 1 : 0, {ncast, 0, 0},
+                           {cast, nullptr, nullptr}, stream);
 }
 
 extern "C" int gpk_aep_phi(int D, int M, double N, double alpha, const double* logdetK, const double* ldSuinv,

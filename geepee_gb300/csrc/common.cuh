@@ -90,6 +90,16 @@ struct RedPlan {
 // adds the nparts partial blocks of `part` (stride plan.stride()) into the plan's destinations
 int reduce_partials(const double* part, int nparts, const RedPlan& plan, cudaStream_t st);
 
+// gpk_moment_grads with up to three destinations of the sums behind dl (ncast of them, GPK_FP32 only)
+struct Counts {
+  long n[3];
+};
+struct Outputs {
+  void* p[3];
+};
+int moment_grads(int prec, int Q, const double* lls2, const double* lsf2, const double* acc, const void* dv, long ndv,
+                 double* g_l, double* g_s, int ncast, Counts n, Outputs cast, void* stream);
+
 // An NVTX range named after the C-ABI entry point, open for the call's host-side duration
 // (argument checks and launches); nvtx3 is header-only and costs a pointer test when no tool
 // is attached.

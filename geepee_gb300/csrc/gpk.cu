@@ -1,4 +1,6 @@
 // Library-wide host helpers: version, per-thread error text, device properties.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace gpk {
@@ -114,48 +116,88 @@ int reduce_partials(const double* part, int nparts, const RedPlan& plan, cudaStr
 }
 }  // namespace gpk
 
-// acc = [dsf2 | dl Q | dZ M Q | dA Dout M | dB Dout M M], zeroed
-static int zero_acc(double* acc, int M, int Q, int Dout, long* ncast, cudaStream_t st) {
-  *ncast = (long)M * Q + (long)Dout * M + (long)Dout * M * M;
-  const cudaError_t e = cudaMemsetAsync(acc, 0, (1 + Q + *ncast) * sizeof(double), st);
-  if (e != cudaSuccess) return gpk::fail(GPK_ECUDA, "layer_bwd: %s", cudaGetErrorString(e));
-  return GPK_OK;
+// ---- a layer's whole backward in one call ----
+namespace {
+// the float64 sums of a backward: dsf2 and dl first in the workspace, then (FP32) dZ, dA and dB, which
+// in float64 are the caller's tensors themselves
+struct LayerSums {
+  double *dsf2, *dl, *dZ, *dA, *dB;
+  long nZ, nA, nB, used;   // elements; doubles of the workspace taken
+};
+LayerSums layer_sums(int prec, int M, int Q, int Dout, void* dZ, void* dA, void* dB, double* work) {
+  LayerSums s{};
+  s.nZ = (long)M * Q;
+  s.nA = (long)Dout * M;
+  s.nB = (long)Dout * M * M;
+  s.dsf2 = work;
+  s.dl = work + 1;
+  s.used = 1 + Q;
+  if (prec == GPK_FP32) {
+    s.dZ = work + s.used;
+    s.dA = s.dZ + s.nZ;
+    s.dB = s.dA + s.nA;
+    s.used += s.nZ + s.nA + s.nB;
+  } else {
+    s.dZ = (double*)dZ;
+    s.dA = (double*)dA;
+    s.dB = (double*)dB;
+  }
+  return s;
 }
+__global__ void __launch_bounds__(256) zero_sums_kernel(LayerSums s, int Q) {
+  const long t0 = (long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long)gridDim.x * blockDim.x;
+  if (t0 < 1 + Q) s.dsf2[t0] = 0.0;
+  for (long i = t0; i < s.nZ; i += nt) s.dZ[i] = 0.0;
+  for (long i = t0; i < s.nA; i += nt) s.dA[i] = 0.0;
+  for (long i = t0; i < s.nB; i += nt) s.dB[i] = 0.0;
+}
+int zero_sums(const LayerSums& s, int Q, cudaStream_t st) {
+  zero_sums_kernel<<<(int)std::min((s.nB + 255) / 256, 2L * gpk::sm_count()), 256, 0, st>>>(s, Q);
+  return gpk::check_launch("layer_bwd");
+}
+}  // namespace
 
 extern "C" int gpk_psi_layer_bwd(int prec, int N, int M, int Q, int Dout, const void* mu, const void* var,
                                  const void* Z, const double* lls2, const double* lsf2, const void* A, const void* B,
-                                 const void* m, const void* dm, const void* dv, double* acc, void* dmu, void* dvar,
-                                 double* g_l, double* g_s, void* cast, double* work, long work_elems, void* stream) {
+                                 const void* m, const void* dm, const void* dv, void* dZ, void* dA, void* dB,
+                                 void* dmu, void* dvar, double* g_l, double* g_s, double* work, long work_elems,
+                                 void* stream) {
   GPK_NVTX("gpk_psi_layer_bwd");
+  GPK_REQUIRE(prec == GPK_DF64 || prec == GPK_FP32, "psi_layer_bwd: unknown precision %d", prec);
   GPK_REQUIRE(N >= 0 && M >= 1 && Q >= 1 && Dout >= 1, "psi_layer_bwd: bad sizes N=%d M=%d Q=%d Dout=%d", N, M, Q, Dout);
-  GPK_REQUIRE(acc && work, "psi_layer_bwd: null accumulators or workspace");
-  long nc;
-  int rc = zero_acc(acc, M, Q, Dout, &nc, gpk::as_stream(stream));
-  double *dl = acc + 1, *dZ = dl + Q, *dA = dZ + (long)M * Q, *dB = dA + (long)Dout * M;
+  GPK_REQUIRE(dZ && dA && dB && work, "psi_layer_bwd: null output or workspace");
+  const LayerSums s = layer_sums(prec, M, Q, Dout, dZ, dA, dB, work);
+  GPK_REQUIRE(work_elems > s.used, "psi_layer_bwd: workspace of %ld doubles, more than %ld needed", work_elems, s.used);
+  int rc = zero_sums(s, Q, gpk::as_stream(stream));
   if (rc == GPK_OK)
-    rc = gpk_psi_bwd_ws(prec, N, M, Q, Dout, mu, var, Z, lls2, lsf2, A, B, m, dm, dv, nullptr, 0, acc, dl, dZ, dA, dB,
-                        dmu, dvar, work, work_elems, stream);
+    rc = gpk_psi_bwd_ws(prec, N, M, Q, Dout, mu, var, Z, lls2, lsf2, A, B, m, dm, dv, nullptr, 0, s.dsf2, s.dl, s.dZ,
+                        s.dA, s.dB, dmu, dvar, work + s.used, work_elems - s.used, stream);
   if (rc == GPK_OK)
-    rc = gpk_moment_grads(prec, Q, nc, lls2, lsf2, acc, dv, (long)N * Dout, g_l, g_s, cast, stream);
+    rc = gpk::moment_grads(prec, Q, lls2, lsf2, s.dsf2, dv, (long)N * Dout, g_l, g_s, prec == GPK_FP32 ? 3 : 0,
+                           {s.nZ, s.nA, s.nB}, {dZ, dA, dB}, stream);
   return rc;
 }
 
 extern "C" int gpk_det_layer_bwd(int prec, int N, int M, int D, int Dout, const void* x, int ldx, const void* Z,
                                  const double* lls2, const double* lsf2, const void* A, const void* kfu,
-                                 const void* Bk, const void* dm, const void* dv, double* acc, void* dx, double* g_l,
-                                 double* g_s, void* cast, double* work, long work_elems, void* stream) {
+                                 const void* Bk, const void* dm, const void* dv, void* dZ, void* dA, void* dB,
+                                 void* dx, double* g_l, double* g_s, double* work, long work_elems, void* stream) {
   GPK_NVTX("gpk_det_layer_bwd");
+  GPK_REQUIRE(prec == GPK_DF64 || prec == GPK_FP32, "det_layer_bwd: unknown precision %d", prec);
   GPK_REQUIRE(N >= 0 && M >= 1 && D >= 1 && Dout >= 1, "det_layer_bwd: bad sizes N=%d M=%d D=%d Dout=%d", N, M, D, Dout);
-  GPK_REQUIRE(acc && work, "det_layer_bwd: null accumulators or workspace");
-  long nc;
-  int rc = zero_acc(acc, M, D, Dout, &nc, gpk::as_stream(stream));
-  double *dl = acc + 1, *dZ = dl + D, *dA = dZ + (long)M * D, *dB = dA + (long)Dout * M;
+  GPK_REQUIRE(dZ && dA && dB && work, "det_layer_bwd: null output or workspace");
+  const LayerSums s = layer_sums(prec, M, D, Dout, dZ, dA, dB, work);
+  GPK_REQUIRE(work_elems > s.used, "det_layer_bwd: workspace of %ld doubles, more than %ld needed", work_elems, s.used);
+  double* const rest = work + s.used;
+  const long nrest = work_elems - s.used;
+  int rc = zero_sums(s, D, gpk::as_stream(stream));
   if (rc == GPK_OK)
-    rc = gpk_det_bwd_ws(prec, N, M, D, Dout, x, ldx, Z, lls2, lsf2, A, kfu, Bk, dm, dv, nullptr, acc, dl, dZ, dA, dx,
-                        work, work_elems, stream);
-  if (rc == GPK_OK) rc = gpk_gram_ws(prec, N, M, Dout, kfu, kfu, dv, dB, work, work_elems, stream);
+    rc = gpk_det_bwd_ws(prec, N, M, D, Dout, x, ldx, Z, lls2, lsf2, A, kfu, Bk, dm, dv, nullptr, s.dsf2, s.dl, s.dZ,
+                        s.dA, dx, rest, nrest, stream);
+  if (rc == GPK_OK) rc = gpk_gram_ws(prec, N, M, Dout, kfu, kfu, dv, s.dB, rest, nrest, stream);
   if (rc == GPK_OK)
-    rc = gpk_moment_grads(prec, D, nc, lls2, lsf2, acc, dv, (long)N * Dout, g_l, g_s, cast, stream);
+    rc = gpk::moment_grads(prec, D, lls2, lsf2, s.dsf2, dv, (long)N * Dout, g_l, g_s, prec == GPK_FP32 ? 3 : 0,
+                           {s.nZ, s.nA, s.nB}, {dZ, dA, dB}, stream);
   return rc;
 }
 

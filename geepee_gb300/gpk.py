@@ -404,20 +404,19 @@ def hyp_grads(ls, sf, dl, dsf2, dv, g_ls, g_sf):
          ptr(g_sf), stream())
 
 
-def psi_layer_bwd(mu, var, Z, lls2, lsf2, A, B, m, dm, dv, acc, dmu, dvar, g_l, g_s, cast, work):
-    """gpk_psi_layer_bwd: psi_bwd with fixed-order sums into acc (zeroed here) and moment_grads."""
+def psi_layer_bwd(mu, var, Z, lls2, lsf2, A, B, m, dm, dv, dZ, dA, dB, dmu, dvar, g_l, g_s, work):
+    """gpk_psi_layer_bwd: psi_bwd with fixed-order sums (zeroed here) and moment_grads."""
     N, Q = mu.shape
     call('gpk_psi_layer_bwd', prec_of(mu.dtype), N, Z.shape[0], Q, A.shape[0], ptr(mu), ptr(var), ptr(Z), ptr(lls2),
-         ptr(lsf2), ptr(A), ptr(B), ptr(m), ptr(dm), ptr(dv), ptr(acc), ptr(dmu), ptr(dvar), ptr(g_l), ptr(g_s),
-         ptr(cast), *_ws(work), stream())
+         ptr(lsf2), ptr(A), ptr(B), ptr(m), ptr(dm), ptr(dv), ptr(dZ), ptr(dA), ptr(dB), ptr(dmu), ptr(dvar), ptr(g_l),
+         ptr(g_s), *_ws(work), stream())
 
 
-def det_layer_bwd(x, Z, lls2, lsf2, A, kfu, Bk, dm, dv, acc, dx, g_l, g_s, cast, work):
-    """gpk_det_layer_bwd: det_bwd and gram with fixed-order sums into acc (zeroed here) and
-    moment_grads."""
+def det_layer_bwd(x, Z, lls2, lsf2, A, kfu, Bk, dm, dv, dZ, dA, dB, dx, g_l, g_s, work):
+    """gpk_det_layer_bwd: det_bwd and gram with fixed-order sums (zeroed here) and moment_grads."""
     N, D = x.shape
     call('gpk_det_layer_bwd', prec_of(x.dtype), N, Z.shape[0], D, A.shape[0], ptr(x), D, ptr(Z), ptr(lls2), ptr(lsf2),
-         ptr(A), ptr(kfu), ptr(Bk), ptr(dm), ptr(dv), ptr(acc), ptr(dx), ptr(g_l), ptr(g_s), ptr(cast), *_ws(work),
+         ptr(A), ptr(kfu), ptr(Bk), ptr(dm), ptr(dv), ptr(dZ), ptr(dA), ptr(dB), ptr(dx), ptr(g_l), ptr(g_s), *_ws(work),
          stream())
 
 

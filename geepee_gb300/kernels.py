@@ -156,8 +156,9 @@ def _psi_grads(c, dpsi1, dpsi2, ls, sf2, mu, S, z):
             B = B.unsqueeze(0).contiguous()
     # (per-point weights take no dv)
     ones = torch.ones((N, 1), dtype=torch.float64, device=c.dev) if stride == 0 else None
-    acc = torch.zeros(M * Q + Q + 1, dtype=torch.float64, device=c.dev)   # the sums, in one fill
-    out = dict(dsf2=acc[M * Q + Q:], dl=acc[M * Q:M * Q + Q], dZ=acc[:M * Q].view(M, Q),
+    out = dict(dsf2=torch.zeros(1, dtype=torch.float64, device=c.dev),
+               dl=torch.zeros(Q, dtype=torch.float64, device=c.dev),
+               dZ=torch.zeros((M, Q), dtype=torch.float64, device=c.dev),
                dmu=torch.empty((N, Q), dtype=torch.float64, device=c.dev),
                dS=torch.empty((N, Q), dtype=torch.float64, device=c.dev))
     gpk.psi_bwd(mu_t, S_t, z_t, l2, s2, None, B, None, None, ones, out['dsf2'], out['dl'], out['dZ'],

@@ -435,18 +435,19 @@ int gpk_trace_kzz_ws(int prec, int M, int Q, const void* Mm, const void* Z, cons
                      const double* lsf2, double s_sf, double s_ls, double* g_sf, double* g_ls, double* g_z,
                      double* work, long work_elems, void* stream);
 
-/* A layer's whole backward in one call: acc [1 + Q + M Q + Dout M + Dout M M] (dsf2, dl, dZ, dA, dB)
- * is zeroed, the fixed-order backward adds into it (gpk_psi_bwd_ws; gpk_det_bwd_ws with dx
- * optional, then gpk_gram_ws for dB, which use `work` in turn), and gpk_moment_grads follows (g_l,
- * g_s, cast as there).  work_elems: at least what gpk_work_elems gives for the operations. */
+/* A layer's whole backward in one call: the sums are zeroed, the fixed-order backward adds into them
+ * (gpk_psi_bwd_ws; gpk_det_bwd_ws with dx optional, then gpk_gram_ws for dB, which use `work` in
+ * turn), and the chain rule of gpk_moment_grads follows (g_l, g_s).  dZ [M,Q], dA [Dout,M], dB
+ * [Dout,M,M] and the rows' gradients are overwritten, in the storage type.  work_elems: 1 + Q, for
+ * GPK_FP32 also M Q + Dout M + Dout M M, plus what gpk_work_elems gives for the operations. */
 int gpk_psi_layer_bwd(int prec, int N, int M, int Q, int Dout, const void* mu, const void* var, const void* Z,
                       const double* lls2, const double* lsf2, const void* A, const void* B, const void* m,
-                      const void* dm, const void* dv, double* acc, void* dmu, void* dvar, double* g_l, double* g_s,
-                      void* cast, double* work, long work_elems, void* stream);
+                      const void* dm, const void* dv, void* dZ, void* dA, void* dB, void* dmu, void* dvar,
+                      double* g_l, double* g_s, double* work, long work_elems, void* stream);
 int gpk_det_layer_bwd(int prec, int N, int M, int D, int Dout, const void* x, int ldx, const void* Z,
                       const double* lls2, const double* lsf2, const void* A, const void* kfu, const void* Bk,
-                      const void* dm, const void* dv, double* acc, void* dx, double* g_l, double* g_s, void* cast,
-                      double* work, long work_elems, void* stream);
+                      const void* dm, const void* dv, void* dZ, void* dA, void* dB, void* dx, double* g_l,
+                      double* g_s, double* work, long work_elems, void* stream);
 
 /* Batched inverse and log-determinant of many tiny SPD matrices A[b] (n x n, n <= 8), one
  * thread per matrix; info[b] as in gpk_chol_inv.  Replaces the per-time-step

@@ -134,3 +134,15 @@ def test_lengthscales_as_a_row(layer, dtype):
         assert l.grad.shape == l.shape and l.grad.dtype == dtype
         got.append(l.grad.reshape(-1))
     assert torch.equal(*got)
+
+
+def test_psi_derivatives_are_tensors_of_their_own():
+    """The lengthscale and pseudo-input derivatives keep no other result's memory (the variance's is the
+    element of a one-element tensor)."""
+    from geepee_gb300 import kernels
+    r = lambda *s: torch.rand(*s, dtype=torch.float64, device='cuda')
+    N, M, Q = 9, 6, 3
+    ell, sf2, mu, S, Z = r(Q) + 0.5, r(1) + 0.5, r(N, Q), r(N, Q), r(M, Q)
+    p1, p2 = kernels.compute_psi_weave(2 * torch.log(ell), torch.log(sf2), mu, S, Z)
+    out = kernels.compute_psi_derivatives(r(N, M), p1, r(N, M, M), p2, ell, sf2, mu, S, Z)
+    assert all(t.untyped_storage().nbytes() == t.nbytes for t in out)

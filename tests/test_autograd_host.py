@@ -35,3 +35,19 @@ def test_lengthscale_gradient_has_its_shape(no_kernels, layer, shape, dtype):
     (m + v).sum().backward()
     for a in ins:
         assert a.grad.shape == a.shape and a.grad.dtype == a.dtype
+
+
+@pytest.mark.parametrize('dtype', [torch.float64, torch.float32])
+@pytest.mark.parametrize('layer', ['psi', 'det'])
+def test_gradients_are_tensors_of_their_own(no_kernels, layer, dtype):
+    """No gradient is a view: each can be detached in place, is aligned as an allocation is, and keeps
+    no other gradient's memory."""
+    ins = _leaves(layer, (3,), dtype)
+    m, v = getattr(autograd, layer + '_moments')(*ins)
+    (m + v).sum().backward()
+    held = set()
+    for a in ins:
+        a.grad.detach_()
+        assert a.grad.untyped_storage().nbytes() == a.grad.nbytes
+        held.add(a.grad.untyped_storage().data_ptr())
+    assert len(held) == len(ins)
