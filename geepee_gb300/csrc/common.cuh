@@ -64,6 +64,15 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Lets kernel k take all the dynamic shared memory of a CTA, `reserve` bytes of static words aside.  Every
+// launch asks for the same: the limit is one word per kernel and device that all threads of the process
+// share, and a launch that set it to its own size could lower it between another thread's call
+// and that thread's larger launch, which the runtime would then refuse.
+template <typename K>
+inline void allow_smem(K k, int reserve = 0) {
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - reserve);
+}
+
 // Fixed-order accumulation.  A kernel of the deterministic path writes its per-CTA partial sums
 // to a workspace, part[c * stride + j] for CTA c, instead of adding them into the outputs with
 // atomics; reduce_partials then adds sum_c part[c * stride + j] (in a fixed order of c) into
