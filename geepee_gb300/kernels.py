@@ -156,11 +156,9 @@ def _psi_grads(c, dpsi1, dpsi2, ls, sf2, mu, S, z):
             B = B.unsqueeze(0).contiguous()
     # (per-point weights take no dv)
     ones = torch.ones((N, 1), dtype=torch.float64, device=c.dev) if stride == 0 else None
-    out = dict(dsf2=torch.zeros(1, dtype=torch.float64, device=c.dev),
-               dl=torch.zeros(Q, dtype=torch.float64, device=c.dev),
-               dZ=torch.zeros((M, Q), dtype=torch.float64, device=c.dev),
-               dmu=torch.empty((N, Q), dtype=torch.float64, device=c.dev),
-               dS=torch.empty((N, Q), dtype=torch.float64, device=c.dev))
+    out = {k: torch.empty(s, dtype=torch.float64, device=c.dev)
+           for k, s in (('dsf2', 1), ('dl', Q), ('dZ', (M, Q)), ('dmu', (N, Q)), ('dS', (N, Q)))}
+    torch._foreach_zero_([out['dsf2'], out['dl'], out['dZ']])   # the sums, in one launch
     gpk.psi_bwd(mu_t, S_t, z_t, l2, s2, None, B, None, None, ones, out['dsf2'], out['dl'], out['dZ'],
                 None, None, out['dmu'], out['dS'], dpsi1=d1, b_stride=stride, Dout=1)
     return (c.scalar(out['dsf2'][0]), c.out(out['dl']), c.out(out['dZ']), c.out(out['dmu']),
