@@ -64,13 +64,14 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Lets kernel k take all the dynamic shared memory of a CTA, `reserve` bytes of static words aside.  Every
-// launch asks for the same: the limit is one word per kernel and device that all threads of the process
+// Lets kernel k take sm bytes of dynamic shared memory; above the 48 KB that need no permission, as much
+// as a CTA can have, `reserve` bytes of static words aside.  Every launch that needs permission
+// asks for the same: the limit is one word per kernel and device that all threads of the process
 // share, and a launch that set it to its own size could lower it between another thread's call
 // and that thread's larger launch, which the runtime would then refuse.
 template <typename K>
-inline void allow_smem(K k, int reserve = 0) {
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - reserve);
+inline void allow_smem(K k, size_t sm, int reserve = 0) {
+  if (sm + reserve > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - reserve);
 }
 
 // Fixed-order accumulation.  A kernel of the deterministic path writes its per-CTA partial sums

@@ -852,7 +852,7 @@ void gemm_go(int batch, int m, int n, int k, int tA, int tB, double alpha, const
   dim3 grid(gpk::ceil_div(n, TBM), gpk::ceil_div(m, TBM), batch);
   const size_t sm = 2 * KC * TBM * sizeof(T);
   auto kfn = gemm_kernel<T, TBM, KS, P2>;
-  gpk::allow_smem(kfn);
+  gpk::allow_smem(kfn, sm);
   kfn<<<grid, GemmShape<TBM>::NG * KS, sm, st>>>(m, n, k, tA, tB, alpha, (const S*)A, lda, sA, (const S*)B, ldb, sB,
                                                  beta, (const S*)E, lde, sE, (S*)C, ldc, sC);
 }
@@ -890,7 +890,7 @@ int gemm_group_go(const GemmGroupArgs& g, LincombGroupArgs& l, cudaStream_t st) 
   const int grid = g.first[g.count] + l.first[l.count];
   if (grid == 0) return GPK_OK;
   auto kfn = gemm_group_kernel<T, TBM, KS>;
-  gpk::allow_smem(kfn);
+  gpk::allow_smem(kfn, sm);
   kfn<<<grid, nth, sm, st>>>(g, l);
   return gpk::check_launch("gemm_group");
 }
@@ -1008,7 +1008,7 @@ int spd_factor_launch(int batch, int M, const void* A, T* Lw, double* logdet, in
   typedef typename Num<T>::store_t S;
   const size_t sm = 256 * sizeof(float2) + ((size_t)((M + 1) >> 1) * (M + 32) * 2 + M + NW) * sizeof(T);
   auto k = spd_factor_kernel<T, RS, CS, NW>;
-  gpk::allow_smem(k, 2048);
+  gpk::allow_smem(k, sm, 2048);
   k<<<batch, NW * 32, sm, st>>>(M, (const S*)A, (long)M * M, Lw, logdet, info);
   return gpk::check_launch("spd_factor");
 }
@@ -1017,7 +1017,7 @@ template <typename T, int RS>
 int trinv_launch(int batch, int M, const T* Lw, T* Xt, const int* info, cudaStream_t st) {
   const size_t sm = (size_t)M * M * sizeof(T);
   auto k = trinv_kernel<T, RS>;
-  gpk::allow_smem(k);
+  gpk::allow_smem(k, sm);
   k<<<dim3(gpk::ceil_div(M, TW), batch), TW * 32, sm, st>>>(M, Lw, Xt, info);
   return gpk::check_launch("trinv");
 }
@@ -1053,7 +1053,7 @@ int chol_launch(int batch, int M, const void* A, void* Ainv, void* L, double* lo
   long s = (long)M * M;
   size_t sm = 256 * 8 + ((GMEM ? 0 : (size_t)M * (M + 1)) + 3 * M + 32) * sizeof(T);
   auto k = chol_inv_kernel<T, GMEM>;
-  gpk::allow_smem(k, 64);
+  gpk::allow_smem(k, sm, 64);
   k<<<batch, 1024, sm, st>>>(M, (const S*)A, s, (S*)Ainv, s, (S*)L, s, logdet, info, (S*)work, (S*)Xout);
   return gpk::check_launch("chol_inv");
 }
@@ -1146,7 +1146,7 @@ int trace_launch(int M, int Q, const void* Mm, const void* Z, const double* lls2
   typedef typename Num<T>::store_t S;
   const size_t sm = 256 * sizeof(float2) + (size_t)M * Q * sizeof(T);
   auto k = trace_kzz_kernel<T, QC>;
-  gpk::allow_smem(k, 4096);
+  gpk::allow_smem(k, sm, 4096);
   k<<<M, 32 * std::min(TK_MAXW, gpk::ceil_div(M, 32)), sm, st>>>(M, Q, (const S*)Mm, (const S*)Z, lls2, lsf2, s_sf, s_ls, g_sf, g_ls,
                                              g_z, work);
   int rc = gpk::check_launch("trace_kzz");

@@ -1391,7 +1391,7 @@ int dm_launch(int N, int M, int Dout, const double* lsf2, const double* A, const
   int nrt = per <= 16 ? 1 : (per <= 32 ? 2 : 4);
   while (nrt > 1 && dm_carve(nullptr, nullptr, M, NB, 16 * nrt) > cap) nrt >>= 1;
   const size_t sm = dm_carve(nullptr, nullptr, M, NB, 16 * nrt);
-  gpk::allow_smem(det_mma_kernel, 64);
+  gpk::allow_smem(det_mma_kernel, sm, 64);
   det_mma_kernel<<<dim3(std::min(gx, gpk::ceil_div(N, 16 * nrt)), Dout), DM_T, sm, st>>>(
       N, M, Dout, lsf2, A, B, b_pairs, kin, Bk, m_out, v_out, NB, nrt);
   return gpk::check_launch("det_mma");
@@ -1412,7 +1412,7 @@ int kern_fx_launch(int N, int M, int D, const double* x, int ldx, const double* 
   const long nmb = gpk::ceil_div(M, FC), ntile = gpk::ceil_div(N, FR);
   const long rg = std::min(ntile, std::max(1L, (long)gpk::sm_count() * FCTA / nmb));
   const size_t sm = kFxTab * sizeof(float2) + sizeof(ArdHyp) + ((size_t)2 * FR * D + (size_t)FC * (D | 1)) * 16;
-  gpk::allow_smem(kern_fx_kernel);
+  gpk::allow_smem(kern_fx_kernel, sm);
   kern_fx_kernel<<<(unsigned)(nmb * rg), 256, sm, st>>>(N, M, D, x, ldx, z, ldz, lls2, lsf2, K, ldk);
   return gpk::check_launch("kern");
 }
@@ -1425,7 +1425,7 @@ int kern_launch(int N, int M, int D, const void* x, int ldx, const void* z, int 
   GPK_REQUIRE(grid.y <= 65535, "kern: N=%d too large (at most %d rows)", N, 65535 * KR);
   const size_t sm = 256 * sizeof(float2) + sizeof(Hyp<T>) + (size_t)(KR + KC) * D * sizeof(T);
   auto k = kern_matrix_kernel<T>;
-  gpk::allow_smem(k);
+  gpk::allow_smem(k, sm);
   k<<<grid, 256, sm, st>>>(N, M, D, (const S*)x, ldx, (const S*)z, ldz, lls2, lsf2, jitter, (S*)K, ldk);
   return gpk::check_launch("kern");
 }
@@ -1475,14 +1475,14 @@ extern "C" int gpk_det_fwd(int prec, int N, int M, int D, int Dout, const void* 
   if (prec == GPK_DF64) {
     size_t sm = det_fwd_smem(M, D, zstage, sizeof(df64));
     auto k = det_fwd_kernel<df64>;
-    gpk::allow_smem(k);
+    gpk::allow_smem(k, sm);
     k<<<grid, 256, sm, st>>>(N, M, D, Dout, (const double*)x, ldx, (const double*)Z, lls2, lsf2,
                              (const double*)A, (const double*)B, (double*)kfu, (double*)Bk, (double*)m_out,
                              (double*)v_out, zstage);
   } else if (prec == GPK_FP32) {
     size_t sm = det_fwd_smem(M, D, zstage, sizeof(float));
     auto k = det_fwd_kernel<float>;
-    gpk::allow_smem(k);
+    gpk::allow_smem(k, sm);
     k<<<grid, 256, sm, st>>>(N, M, D, Dout, (const float*)x, ldx, (const float*)Z, lls2, lsf2, (const float*)A,
                              (const float*)B, (float*)kfu, (float*)Bk, (float*)m_out, (float*)v_out, zstage);
   } else {
@@ -1498,7 +1498,7 @@ void contract_launch(int N, int M, int Dout, const void* kfu, const double* lsf2
   typedef typename Num<T>::store_t S;
   const size_t sm = det_contract_smem(M, Dout, sizeof(T));
   auto k = det_contract_kernel<T, DB>;
-  gpk::allow_smem(k);
+  gpk::allow_smem(k, sm);
   k<<<gpk::ceil_div(N, CR), CT, sm, st>>>(N, M, Dout, (const S*)kfu, lsf2, (const S*)A, (const S*)B, (S*)Bk,
                                           (S*)m_out, (S*)v_out);
 }
@@ -1575,7 +1575,7 @@ void det_bwd_launch(int grid, dim3 threads, cudaStream_t st, int N, int M, int D
   typedef typename Num<T>::store_t S;
   const size_t sm = det_bwd_smem(threads.x, threads.y, DC, M, D, dkfu ? 0 : Dout, sizeof(T));
   auto k = det_bwd_kernel<T, DC, DB, EX>;
-  gpk::allow_smem(k);
+  gpk::allow_smem(k, sm);
   k<<<grid, threads, sm, st>>>(N, M, D, Dout, (const S*)x, ldx, (const S*)Z, lls2, lsf2, (const S*)A, (const S*)kfu,
                                (const S*)Bk, (const S*)dm, (const S*)dv, (const S*)dkfu, dsf2, dl, dZ, dA, (S*)dx,
                                work, stride);
@@ -1635,7 +1635,7 @@ void gram_pairs_launch(dim3 grid, size_t sm, cudaStream_t st, int N, int M, int 
                        double* work, long pstride, int GR) {
   typedef typename Num<T>::store_t S;
   auto k = gram_pairs_kernel<T, DB>;
-  gpk::allow_smem(k);
+  gpk::allow_smem(k, sm);
   k<<<grid, GP_T, sm, st>>>(N, M, Dout, (const S*)u, (const S*)w, work, pstride, GR);
 }
 template <typename T>
@@ -1734,7 +1734,7 @@ extern "C" int gpk_gram_ws(int prec, int N, int M, int Dout, const void* u, cons
     const long pstride = (long)Dout * P;
     if (mma) {
       const size_t smm = gm_carve(nullptr, nullptr, M, g.ks);
-      gpk::allow_smem(gram_mma_kernel);
+      gpk::allow_smem(gram_mma_kernel, smm);
       gram_mma_kernel<<<dim3(chunks, Dout, g.groups), GM_T, smm, st>>>(N, M, Dout, (const double*)u, (const double*)w,
                                                                        work, pstride, g.rows, g.ks, g.tw);
     } else if (prec == GPK_DF64) gram_pairs_dispatch<df64>(grid, sm, st, N, M, Dout, u, w, work, pstride, GR);

@@ -2057,7 +2057,7 @@ int run_fwd_gen(const PsiArgs<typename Num<T>::store_t>& a_in, cudaStream_t st) 
   a.g_smem = bytes(P, a.bs_smem ? nbs : 0) <= SMEM_CAP;
   const size_t sm = bytes(a.g_smem ? P : 0, a.bs_smem ? nbs : 0);
   auto k = psi_fwd_gen_kernel<T, NPB, PPT, QC, DB>;
-  gpk::allow_smem(k, SMEM_STATIC);
+  gpk::allow_smem(k, sm, SMEM_STATIC);
   int resident = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k, NT, sm);
   resident = resident < 1 ? 1 : (resident > 2 ? 2 : resident);
@@ -2076,7 +2076,7 @@ int run_chain(const PsiArgs<double>& a, cudaStream_t st) {
   if (sm > SMEM_CAP || a.M > 255) return -1;
   if (a.N < 1) return GPK_OK;
   auto k = P <= CH_KP * CH_SWEEP * 32 ? psi_chain_kernel<QC, true> : psi_chain_kernel<QC, false>;
-  gpk::allow_smem(k, SMEM_STATIC);
+  gpk::allow_smem(k, sm, SMEM_STATIC);
   k<<<1, CH_NTH, sm, st>>>(a);
   return gpk::check_launch("psi_rollout");
 }
@@ -2125,7 +2125,7 @@ int run_fwd(const PsiArgs<typename Num<T>::store_t>& a, size_t cap, cudaStream_t
   if (mcarve<T>(nullptr, nullptr, a.M, QC, P, a.Dout, NPBF, NS, DB, pab) > cap) return -1;
   const size_t sm = mcarve<T>(nullptr, nullptr, a.M, QC, P, a.Dout, NPB, NS, DB, pab);
   auto k = psi_fwd_kernel<T, NPB, QC, DB, NS, NF>;
-  gpk::allow_smem(k, SMEM_STATIC);
+  gpk::allow_smem(k, sm, SMEM_STATIC);
   int grid = gpk::sm_count() * (NS < 16 ? 2 : 1);
   if (grid > a.N) grid = a.N;
   if (grid < 1) return GPK_OK;
@@ -2157,7 +2157,7 @@ int run_out(const PsiArgs<typename Num<T>::store_t>& a_in, size_t cap, cudaStrea
     const size_t sm = ocarve<T>(nullptr, nullptr, a.M, QC, P, a.g_smem ? P : 0, pab, nl);
     if (sm > cap) continue;
     auto k = psi_out_kernel<T, QC, NS, NF>;
-    gpk::allow_smem(k, SMEM_STATIC);
+    gpk::allow_smem(k, sm, SMEM_STATIC);
     int grid = gpk::sm_count() * per_sm;
     if (grid > a.N) grid = a.N;
     if (grid < 1) return GPK_OK;
@@ -2228,7 +2228,7 @@ gpk::RedPlan bwd_plan(const PsiArgs<S>& a) {
 template <typename T, int DB, int QC, int NS, int NB, int NF>
 int run_bwd(const PsiArgs<typename Num<T>::store_t>& a, const BLayout& lo, size_t sm, cudaStream_t st) {
   auto k = psi_bwd_kernel<T, DB, QC, NS, NB, NF>;
-  gpk::allow_smem(k, SMEM_STATIC);
+  gpk::allow_smem(k, sm, SMEM_STATIC);
   int grid = gpk::sm_count() * (NS < 12 ? 2 : 1);
   if (grid > a.N) grid = a.N;
   if (grid < 1) return GPK_OK;
