@@ -632,7 +632,8 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
 #pragma unroll
       for (int i = 0; i < 4; ++i) {   // |entry| < 2^ex
         const int eh = (int)(((unsigned)__double2loint(r[i]) >> 23) & 0xffu) - 126;
-        const int ed = (int)(((__double_as_longlong(r[i]) + (1LL << 28)) >> 52) & 0x7ff) - 1022;   // (rounded as hi is)
+        // (rounded as hi is; a NaN of all ones carries out of the field, which stays above every exponent)
+        const int ed = (int)((((unsigned long long)__double_as_longlong(r[i]) & 0x7fffffffffffffffULL) + (1ULL << 28)) >> 52) - 1022;
         ex = max(ex, pair ? eh : ed);
       }
       atomicMax(&s.bexp[c], ex > 128 ? DM_BAD : ex);

@@ -119,3 +119,23 @@ def test_gram_workspace_of_a_larger_call():
             gpk.gram(ut, ut, dev(w), C, work=work)
             ref = np.einsum('nd,na,nb->dab', w, u, u)
             assert np.abs(C.cpu().numpy() - ref).max() <= 1e-10 * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize('bits', [-1, 0x7fffffffffffffff, 0x7ff8000000000000, 0x7ff0000000000001])
+def test_contraction_of_any_nan(bits):
+    """A NaN of any payload (all ones among them) in B or A makes its column of Bk or its output's m NaN,
+    and v through B; the rest stays finite."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(4)
+    n, m = 20, 30
+    k, A, B = np.exp(-rng.rand(n, m)), rng.randn(2, m), rng.randn(2, m, m)
+    nan = np.array([bits], dtype=np.int64).view(np.float64)
+    B[0, 3, 7], A[1, 5] = nan[0], nan[0]
+    e = lambda *s: torch.zeros(s, dtype=torch.float64, device='cuda')
+    Bk, mo, vo = e(n, 2, m), e(n, 2), e(n, 2)
+    gpk.det_contract(dev(k), dev([0.1]), dev(A), dev(B), Bk, mo, vo)
+    want = np.zeros((2, m), bool)
+    want[0, 7] = True
+    assert (np.isnan(Bk.cpu().numpy()) == want).all()
+    assert (np.isnan(mo.cpu().numpy()) == [False, True]).all()
+    assert (np.isnan(vo.cpu().numpy()) == [True, False]).all()
