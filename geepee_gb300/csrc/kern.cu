@@ -468,22 +468,33 @@ size_t det_contract_smem(int M, int Dout, size_t tsz) {
 
 // ---- the deterministic layer's contraction in double-float precision on the tensor cores ----
 // For rows n and one output d:  Bk_nb = sum_a B[a,b] k_na,  m_n = k_n . A,  v_n = sf2 + k_n . Bk_n, from
-// the kernel rows k.  A is column M of B.  Each row of k and each column of B is scaled by a power of two
-// to less than 1/2 and rounded to 53 bits below the point; the integer is cut into six balanced digits of
-// nine bits (each an exact f16), and a product of two such numbers is the digit products of levels
+// the kernel rows k.  Bk by digits: B is balanced by powers of two along both indices, B'_ab = B_ab 2^-(r_a + c_b)
+// with c_b the largest exponent of column b and r_a <= 0 that of row a beside the c_b, so that every row and
+// every column of B' has its largest entry next to 1; the r_a go over to the rows, k'_a = k_a 2^r_a.  Each row of
+// k' is scaled by its largest entry; the numbers, below 1/2 then, are taken to 53 bits below the point (k rounded;
+// B through its double-float form, ~2^-49 of an entry, truncated), the integer is cut into six balanced digits
+// of nine bits (each an exact f16), and a product of two such numbers is the digit products of levels
 // i + j <= 6: 26 f16 multiply-adds into f32.  Digit products are at most 2^16, so an accumulator that takes
 // at most two of them over 128 terms holds an integer of at most 2^24: the sums of levels 0 to 4 are exact
 // (nine accumulators; a longer contraction is folded into 64-bit integers every 128 terms).  Levels 5
-// and 6 have one accumulator each, whose last place is below 2^-56 of the largest product.  What is left is
-// the rounding to 53 bits, in place of a double-float multiply-add (14 instructions, every term rounded).
+// and 6 have one accumulator each, whose last place is below 2^-56 of the largest product.
+// Errors: Bk_nb is off by a few 2^-52 of max_a k'_a 2^c_b times sqrt(M), where a double-float sum (14 instructions
+// a term, every term rounded) is off by some 2^-48 of sum_a |k_a B_ab|.  Some column b of every row has a sum
+// as large as max_a k'_a 2^c_b, so a row of Bk keeps the double-float accuracy relative to its largest
+// sums; an entry whose terms are all far smaller keeps it relative to those, not to itself.  m and v keep the
+// double-float accuracy relative to their sums of |terms|: A is column M of B' (its own scale, beside the r_a), and
+// the sums of |k'_a B'_ab| are estimated from the first digits by one more product.  Where m's is below 1/16 of its
+// scales, or sum_b |k_b| 2^c_b sum_a |k'_a B'_ab| below 1/16 of max_a k'_a sum_b |k_b| 2^c_b (few rows: none in the
+// deep GP's and the regressions' layers), the row's m, or its v and Bk, are formed again in double-float.
 // A CTA of 16 warps takes R = 16 nrt rows at a time, B's digits resident in shared memory in the order
 // of the matrix instruction's fragments (restaged by column blocks per row chunk when they do not fit);
 // a warp takes 16 x 8 results at a time.  v is summed in an order that depends on M alone, so a row's
 // results are the same in any batch.
-// One-off staging of B (~9 us at M = 100), then per 32 rows ~5500 cycles of digits, ~16000 of products (the
-// matrix pipe itself ~10000) and ~6000 of epilogue.  With the rows' kernel launch before it, N = 20000,
-// M = 100, two outputs take 168 us (752 before); N = 777, M = 200 74 us (159); the contraction
-// alone at N = 1000, M = 100 21 us (27).
+// One-off staging of B (~12 us at M = 100, 3 of them the balance), then per 32 rows ~5500 cycles of digits, ~17000
+// of products (the matrix pipe itself ~10000) and ~7000 of epilogue.  With the rows' kernel launch before it,
+// N = 20000, M = 100, two outputs take 181 us (in double-float 752; scaled by the rows' and columns'
+// largest entries alone, without the balance and the estimate, 168); N = 777, M = 200 75 us (159; 70); the
+// contraction alone at N = 1000, M = 100 22 us (27; 19).
 constexpr int DM_T = 512, DM_W = DM_T / 32, DM_S = 6;
 // an integer (|x| < 2^61) times 2^-F as a double-float
 __device__ __forceinline__ df64 df_of_int(long long x, int F) {
@@ -498,7 +509,7 @@ __device__ __forceinline__ long long fx_bits_by(float x, int F) {
   const long long v = (long long)(((unsigned long long)(((b & 0x7fffffu) | 0x800000u) << 7) << 32) >> s);
   return (int)b < 0 ? -v : v;
 }
-// v 2^(-1 - ex), less than 1/2 in magnitude, in units of 2^-53, rounded
+// v 2^(-1 - ex) (|v| < 2^ex), less than 1/2 in magnitude, in units of 2^-53, rounded
 __device__ __forceinline__ long long digits_of(double v, int ex) {
   const long long b = __double_as_longlong(v);
   const int be = (int)((b >> 52) & 0x7ff), sh = 1023 + ex - be;   // at least 1
@@ -541,14 +552,19 @@ __device__ __forceinline__ long long dm_fold(const float (&acc)[DM_ACC][4], int 
   const long long Y = mad_wide(S(4) + S(5), 1 << 18, mad_wide(S(6) + S(7) + S(8), 1 << 9, (long long)(S(9) + s6)));
   return (X << 20) + (Y >> 7);
 }
-// one k step: all digit products of a row fragment and a column fragment (strides in fragments)
-__device__ __forceinline__ void dm_step(float (&acc)[DM_ACC][4], const uint4* fa, int sa, const uint2* fb, int sb) {
+// one k step: all digit products of a row fragment and a column fragment (strides in fragments), and (MAG) the
+// product of the rows' first digits with the magnitudes of the columns': the sum of magnitudes for rows without
+// negative entries (kernel values), never more than it
+template <bool MAG>
+__device__ __forceinline__ void dm_step(float (&acc)[DM_ACC][4], float (&mag)[4], const uint4* fa, int sa, const uint2* fb,
+                                        int sb) {
   uint4 va[DM_S];
 #pragma unroll
   for (int i = 0; i < DM_S; ++i) va[i] = fa[(size_t)i * sa];
 #pragma unroll
   for (int j = 0; j < DM_S; ++j) {
     const uint2 vb = fb[(size_t)j * sb];
+    if (MAG && j == 0) mma_f16(mag, va[0], make_uint2(vb.x & 0x7fff7fffu, vb.y & 0x7fff7fffu));
 #pragma unroll
     for (int i = 0; i < DM_S; ++i)
       if (i + j <= 6) mma_f16(acc[dm_acc(i, j)], va[i], vb);
@@ -557,7 +573,11 @@ __device__ __forceinline__ void dm_step(float (&acc)[DM_ACC][4], const uint4* fa
 struct DmSmem {
   unsigned *B, *A;      // digit pairs: [digit][column tile][k step][lane][2], [digit][row tile][k step][lane][4]
   df64 *k, *vp, *v;     // [R][M|1] the rows, [R][NT] parts of v, [R] v
-  int *rexp, *bexp;
+  float2* tp;           // [R][NT] sum_b |k_b| 2^c_b times the first digits' sum of |k'_a B'_ab|, by lanes
+  float *t, *e;         // [R] the sum of those; sum_b |k_b| 2^c_b, or -1 where no entry is in the float range
+  float* cw;            // [M] 2^(c_b - the largest); 0: a column with a non-finite entry
+  int *rexp, *mgen;     // [R] exponent of the scaled row; whether its m takes the double-float form
+  int *c, *r;           // [M + 1] exponents c_b (M: A's), [M] r_a
 };
 __host__ __device__ inline size_t dm_carve(DmSmem* out, char* base, int M, int NB, int R) {
   DmSmem s;
@@ -573,13 +593,56 @@ __host__ __device__ inline size_t dm_carve(DmSmem* out, char* base, int M, int N
   s.k = (df64*)take((size_t)R * (M | 1) * 8);
   s.vp = (df64*)take((size_t)R * (NB / 8) * 8);
   s.v = (df64*)take((size_t)R * 8);
+  s.tp = (float2*)take((size_t)R * (NB / 8) * 8);
+  s.t = (float*)take((size_t)R * 4);
+  s.e = (float*)take((size_t)R * 4);
+  s.cw = (float*)take((size_t)M * 4);
   s.rexp = (int*)take((size_t)R * 4);
-  s.bexp = (int*)take((size_t)NB * 4);
+  s.mgen = (int*)take((size_t)R * 4);
+  s.c = (int*)take((size_t)(M + 1) * 4);
+  s.r = (int*)take((size_t)M * 4);
   if (out) *out = s;
   return o;
 }
 constexpr int DM_BAD = 1 << 20;   // exponent of a row or column with a non-finite entry
+constexpr int DM_LOW = -400;      // the smallest exponent of a scaled row (2^-126 of a row and 2^-254 of a balance)
+constexpr float DM_TRUST = 1024.f;   // a sixteenth of the scales, in the first digits' units (2^-7 of each scale)
 constexpr int DM_MAX = 255;       // largest M: four pairs a lane, sums below 2^61
+
+// Bk of one row (optional) and the sum k . Bk in double-float, by a warp
+static __device__ __noinline__ df64 dm_row_general(const double* B, int b_pairs, const df64* k, const int* c, int M,
+                                                   double* Bk) {
+  const int lane = threadIdx.x & 31;
+  df64 v = make_df(0.f);
+  for (int b0 = lane; b0 < M; b0 += 128) {
+    df64 x[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = make_df(0.f);
+    for (int a = 0; a < M; ++a) {
+      const df64 ka = k[a];
+      if (ka.hi == 0.f) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (b0 + 32 * j < M) {
+          const double e = B[(size_t)a * M + b0 + 32 * j];
+          const df64 w = b_pairs ? make_df(__int_as_float(__double2loint(e)), __int_as_float(__double2hiint(e)))
+                                 : df_from_double(e);
+          x[j] = fma_(w, ka, x[j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int b = b0 + 32 * j;
+      if (b < M) {
+        if (c[b] >= DM_BAD) x[j] = make_df(__int_as_float(0x7fffffff));
+        if (Bk) Bk[b] = df_to_double_int(x[j]);
+        v = fma_(k[b], x[j], v);
+      }
+    }
+  }
+  return warp_sum(v);
+}
 
 __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout, const double* lsf2, const double* A,
                                                           const double* B, int b_pairs, const double* kin, double* Bk,
@@ -595,9 +658,92 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
   const float qnan = __int_as_float(0x7fffffff);
   __shared__ df64 s_sf2;
   if (tid == 0) s_sf2 = df_from_double(exp(lsf2[0]));
-  // ---- columns [c0, c0 + NB) of (B, A) as digits; a lane's four entries of a column are the matrix
-  // instruction's fragment, loaded twice (for the column's exponent, then for the digits), the next
-  // item's in flight while one is worked on
+  for (int i = tid; i < M; i += DM_T) s.c[i] = -126;
+  __syncthreads();
+  // ---- the exponents of B's columns, then of its rows beside them.  A warp takes a row's columns by 128, four
+  // such items' loads in flight; the entries' exponents wait in bytes (in the place of B's digits) for the second pass
+  // |entry| < 2^ex_of: of a pair by its high word, of a float64 rounded as that word is (a NaN of all ones carries
+  // out of the field, which stays above every exponent)
+  auto ex_of = [&](double v, bool pair) {
+    const int h = (int)(((unsigned)__double2loint(v) >> 23) & 0xffu);
+    const int e = (int)((((unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL) + (1ULL << 28)) >> 52);
+    return pair ? h - 126 : e - 1022;
+  };
+  const int EP = (M + 3) & ~3, nh = M > 128 ? 2 : 1;   // bytes of a row; items of a row
+  unsigned char* const eb = reinterpret_cast<unsigned char*>(s.B);
+  int ea[8];   // A's exponents
+#pragma unroll
+  for (int j = 0; j < 8; ++j) ea[j] = lane + 32 * j < M ? ex_of(A[lane + 32 * j], false) : 2 * DM_LOW;
+  {
+    const int cb = (warp & (nh - 1)) * 128 + lane;   // (a warp's items are all of one side)
+    int cm[4] = {-126, -126, -126, -126};
+    for (int it = warp; it < nh * M; it += 4 * DM_W) {
+      double v[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int a = (it + u * DM_W) / nh;
+          v[u][j] = a < M && cb + 32 * j < M ? B[(size_t)a * M + cb + 32 * j] : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int a = (it + u * DM_W) / nh;
+          const int e = min(max(ex_of(v[u][j], b_pairs), -126), 129);   // -126: zero or below the float range
+          cm[j] = max(cm[j], e);
+          if (a < M && cb + 32 * j < EP) eb[a * EP + cb + 32 * j] = (unsigned char)(e + 126);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (cb + 32 * j < M) atomicMax(&s.c[cb + 32 * j], cm[j] > 128 ? DM_BAD : cm[j]);
+  }
+  __syncthreads();
+  {
+    int cc[2][4], cmax = 0;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = 4 * (lane + 32 * j) + u;
+        cc[j][u] = c < M ? s.c[c] + 126 : DM_BAD;   // (a column with a NaN takes no part)
+        if (cc[j][u] < DM_BAD) cmax = max(cmax, cc[j][u]);
+      }
+    for (int a = warp; a < M; a += DM_W) {
+      int e = DM_LOW;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (4 * (lane + 32 * j) < M) {
+          const unsigned w = *reinterpret_cast<const unsigned*>(eb + a * EP + 4 * (lane + 32 * j));
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int b = (w >> (8 * u)) & 0xffu;
+            if (b) e = max(e, b - cc[j][u]);
+          }
+        }
+      e = __reduce_max_sync(~0u, e);
+      if (lane == 0) s.r[a] = min(e, 0);
+    }
+    cmax = __reduce_max_sync(~0u, cmax) - 126;
+    for (int i = tid; i < M; i += DM_T) {
+      const int e = s.c[i] - cmax;
+      s.cw[i] = e > 0 || e < -126 ? 0.f : pow2f(e);
+    }
+  }
+  __syncthreads();
+  {
+    int e = 2 * DM_LOW;   // A's column, beside the rows' exponents (every warp alike)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (lane + 32 * j < M) e = max(e, ea[j] > 128 ? DM_BAD : ea[j] - s.r[lane + 32 * j]);
+    e = __reduce_max_sync(~0u, e);
+    if (lane == 0) s.c[M] = e;
+    __syncwarp();
+  }
+  // ---- columns [c0, c0 + NB) of B' as digits; a lane's four entries of a column are the matrix
+  // instruction's fragment, the next item's in flight while one is worked on
   auto stage_B = [&](int c0) {
     double r[4], rn[4];
     auto fetch = [&](int nt, int ks) {
@@ -619,41 +765,21 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
     int nt0 = 0, ks0 = warp - DM_W;
     next(nt0, ks0);
     fetch(nt0, ks0);
-    for (int i = tid; i < NB; i += DM_T) s.bexp[i] = -126;
-    __syncthreads();
     for (int nt = nt0, ks = ks0; nt < NT;) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) r[i] = rn[i];
-      const int c = nt * 8 + (lane >> 2);
-      next(nt, ks);
-      if (nt < NT) fetch(nt, ks);
-      const bool pair = b_pairs && c0 + c < M;
-      int ex = -126;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {   // |entry| < 2^ex
-        const int eh = (int)(((unsigned)__double2loint(r[i]) >> 23) & 0xffu) - 126;
-        // (rounded as hi is; a NaN of all ones carries out of the field, which stays above every exponent)
-        const int ed = (int)((((unsigned long long)__double_as_longlong(r[i]) & 0x7fffffffffffffffULL) + (1ULL << 28)) >> 52) - 1022;
-        ex = max(ex, pair ? eh : ed);
-      }
-      atomicMax(&s.bexp[c], ex > 128 ? DM_BAD : ex);
-    }
-    fetch(nt0, ks0);
-    __syncthreads();
-    for (int nt = nt0, ks = ks0; nt < NT;) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) r[i] = rn[i];
-      const int c = nt * 8 + (lane >> 2), F = 52 - s.bexp[c];
+      const int c = c0 + nt * 8 + (lane >> 2), a0 = ks * 16 + 2 * (lane & 3), F = 52 - (c <= M ? s.c[c] : 0);
       uint2* q = reinterpret_cast<uint2*>(s.B) + (nt * KS + ks) * 32 + lane;
       next(nt, ks);
       if (nt < NT) fetch(nt, ks);
-      const bool pair = b_pairs && c0 + c < M;
+      const bool pair = b_pairs && c < M;
       long long t[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {   // (an exponent of DM_BAD gives zeros)
+        const int a = a0 + (i & 1) + 8 * (i >> 1), Fa = F - (a < M ? s.r[a] : 0);
         df64 v = df_from_double(r[i]);   // (pairs and float64 give the same results)
         if (pair) v = make_df(__int_as_float(__double2loint(r[i])), __int_as_float(__double2hiint(r[i])));
-        t[i] = fx_bits_by(v.hi, F) + fx_bits_by(v.lo, F);
+        t[i] = fx_bits_by(v.hi, Fa) + fx_bits_by(v.lo, Fa);
       }
       unsigned w0[DM_S], w1[DM_S];
       digit_pairs(t[0], t[1], w0);
@@ -666,25 +792,26 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
   const int ntile = (N + R - 1) / R;
   for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
     const int n0 = tile * R, nr = min(R, N - n0);
-    // ---- a warp a row: its largest exponent (|k| < 2^ex), the integers k 2^(-1 - ex) in units of 2^-53
+    // ---- a warp a row: its largest exponent (|k'| < 2^ex), the integers k' 2^(-1 - ex) in units of 2^-53
     // and their digits (rows past nr keep stale digits: their results are not used)
     for (int r = warp; r < nr; r += DM_W) {
       const double* kr = kin + (size_t)(n0 + r) * M;
       double kv[4][2];
-      int ex = -126;
+      int ex = DM_LOW;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int a = 2 * lane + 64 * i;
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           kv[i][u] = a + u < M ? kr[a + u] : 0.0;
-          ex = max(ex, (int)((__double_as_longlong(kv[i][u]) >> 52) & 0x7ff) - 1022);
+          ex = max(ex, (int)((__double_as_longlong(kv[i][u]) >> 52) & 0x7ff) - 1022 + (a + u < M ? s.r[a + u] : 0));
         }
       }
       ex = __reduce_max_sync(~0u, ex);
       if (ex > 128) ex = DM_BAD;
-      if (lane == 0) s.rexp[r] = ex;
       unsigned* q0 = s.A + ((size_t)((r >> 4) * KS) * 32 + (r & 7) * 4) * 4 + ((r >> 3) & 1);
+      float e = 0.f;
+      bool full = false;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int p = lane + 32 * i;
@@ -692,8 +819,15 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
           long long t[2];
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
-            t[u] = digits_of(kv[i][u], ex);
-            if (2 * p + u < M) s.k[r * MP + 2 * p + u] = df_from_double(kv[i][u]);
+            const int a = 2 * p + u;
+            t[u] = 0;
+            if (a < M) {
+              const df64 k = df_from_double(kv[i][u]);
+              t[u] = digits_of(kv[i][u], ex - s.r[a]);
+              s.k[r * MP + a] = k;
+              full |= k.hi != 0.f;
+              e = __fmaf_rn(fabsf(k.hi), s.cw[a], e);
+            }
           }
           unsigned w[DM_S];
           digit_pairs(t[0], t[1], w);
@@ -701,6 +835,12 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
 #pragma unroll
           for (int j = 0; j < DM_S; ++j) q[(size_t)j * nrt * KS * 128] = w[j];
         }
+      }
+      e = warp_sum(e);
+      full = __any_sync(~0u, full);
+      if (lane == 0) {
+        s.rexp[r] = ex;
+        s.e[r] = full ? e : -1.f;
       }
     }
     for (int c0 = 0; c0 <= M; c0 += NB) {
@@ -711,6 +851,7 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
         const uint4* fa = reinterpret_cast<const uint4*>(s.A) + (size_t)rt * KS * 32 + lane;
         const uint2* fb = reinterpret_cast<const uint2*>(s.B) + (size_t)nt * KS * 32 + lane;
         long long Z[4] = {0, 0, 0, 0};
+        float mag[4] = {0.f, 0.f, 0.f, 0.f};   // (at most 255 2^14: exact)
         for (int k0 = 0; k0 < KS; k0 += 8) {
           float acc[DM_ACC][4];
 #pragma unroll
@@ -719,22 +860,28 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
             for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
           const int k1 = min(k0 + 8, KS);
 #pragma unroll 2
-          for (int ks = k0; ks < k1; ++ks) dm_step(acc, fa + ks * 32, nrt * KS * 32, fb + ks * 32, NT * KS * 32);
+          for (int ks = k0; ks < k1; ++ks)
+            dm_step<true>(acc, mag, fa + ks * 32, nrt * KS * 32, fb + ks * 32, NT * KS * 32);
 #pragma unroll
           for (int j = 0; j < 4; ++j) Z[j] += dm_fold(acc, j);
         }
         df64 v[2] = {make_df(0.f), make_df(0.f)};
+        float t[2] = {0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int r = rt * 16 + (lane >> 2) + 8 * (j >> 1), cl = nt * 8 + 2 * (lane & 3) + (j & 1), c = c0 + cl;
           if (r < nr && c <= M) {
-            const int re = s.rexp[r], be = s.bexp[cl];
-            const df64 X = re >= DM_BAD || be >= DM_BAD ? make_df(qnan) : scale2(df_of_int(Z[j], 58), re + be + 6);
+            const int re = s.rexp[r], be = s.c[c];
+            const df64 X = re >= DM_BAD || be >= DM_BAD ? make_df(qnan)
+                                                       : scale2(df_of_int(Z[j], 58), max(-252, min(re + be + 6, 252)));
             if (c < M) {
+              const df64 k = s.k[r * MP + c];
               if (Bk) Bk[((size_t)(n0 + r) * Dout + d) * M + c] = df_to_double_int(X);
-              v[j >> 1] = fma_(s.k[r * MP + c], X, v[j >> 1]);
-            } else if (m_out) {
-              m_out[(size_t)(n0 + r) * Dout + d] = df_to_double_int(X);
+              v[j >> 1] = fma_(k, X, v[j >> 1]);
+              t[j >> 1] = __fmaf_rn(fabsf(k.hi) * s.cw[c], mag[j], t[j >> 1]);
+            } else {
+              s.mgen[r] = mag[j] < DM_TRUST && re < DM_BAD;
+              if (m_out) m_out[(size_t)(n0 + r) * Dout + d] = df_to_double_int(X);
             }
           }
         }
@@ -742,19 +889,45 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
         for (int i = 0; i < 2; ++i) {
 #pragma unroll
           for (int o = 1; o < 4; o <<= 1) v[i] = add(v[i], shfl_xor(v[i], o));
-          if ((lane & 3) == 0) s.vp[(rt * 16 + (lane >> 2) + 8 * i) * NT + nt] = v[i];
+          t[i] += __shfl_xor_sync(~0u, t[i], 1);
+          const int o = (rt * 16 + (lane >> 2) + 8 * i) * NT + nt;
+          if ((lane & 1) == 0) reinterpret_cast<float*>(s.tp + o)[(lane >> 1) & 1] = t[i];
+          if ((lane & 3) == 0) s.vp[o] = v[i];
         }
       }
       __syncthreads();
       // ---- v: a warp a row, the column tiles' parts by one butterfly (NT <= 32)
       for (int r = warp; r < nr; r += DM_W) {
         df64 v = lane < NT ? s.vp[r * NT + lane] : make_df(0.f);
+        const float2 t2 = lane < NT ? s.tp[r * NT + lane] : make_float2(0.f, 0.f);
+        float t = t2.x + t2.y;
 #pragma unroll
-        for (int o = 16; o; o >>= 1) v = add(v, shfl_xor(v, o));
-        if (lane == 0) {
-          if (c0 > 0) v = add(s.v[r], v);
-          s.v[r] = v;
-          if (c0 + NB > M && v_out) v_out[(size_t)(n0 + r) * Dout + d] = df_to_double(add(s_sf2, v));
+        for (int o = 16; o; o >>= 1) {
+          v = add(v, shfl_xor(v, o));
+          t += __shfl_xor_sync(~0u, t, o);
+        }
+        if (c0 > 0) {
+          v = add(s.v[r], v);
+          t += s.t[r];
+        }
+        if (c0 + NB <= M) {
+          __syncwarp();
+          if (lane == 0) {
+            s.v[r] = v;
+            s.t[r] = t;
+          }
+        } else {
+          const float e = s.e[r];
+          const size_t o = (size_t)(n0 + r) * Dout + d;
+          if (s.rexp[r] < DM_BAD && e >= 0.f && !(e > 0.f && t >= DM_TRUST * e))
+            v = dm_row_general(B, b_pairs, s.k + r * MP, s.c, M, Bk ? Bk + o * M : nullptr);
+          if (s.mgen[r] && e >= 0.f && m_out && s.c[M] < DM_BAD) {
+            df64 m = make_df(0.f);
+            for (int a = lane; a < M; a += 32) m = fma_(s.k[r * MP + a], df_from_double(A[a]), m);
+            m = warp_sum(m);
+            if (lane == 0) m_out[o] = df_to_double_int(m);
+          }
+          if (lane == 0 && v_out) v_out[o] = df_to_double(add(s_sf2, v));
         }
       }
     }
@@ -1302,7 +1475,7 @@ __global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dou
 #pragma unroll
     for (int i = 0; i < GM_TW; ++i) {
       if (ti[i] < 0) continue;   // (uniform over the warp)
-      float acc[DM_ACC][4];
+      float acc[DM_ACC][4], none[4];
 #pragma unroll
       for (int k = 0; k < DM_ACC; ++k)
 #pragma unroll
@@ -1310,7 +1483,7 @@ __global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dou
       const uint4* fa = reinterpret_cast<const uint4*>(s.A) + (size_t)ti[i] * KSM * 32 + lane;
       const uint2* fb = reinterpret_cast<const uint2*>(s.B) + (size_t)tj[i] * KSM * 32 + lane;
 #pragma unroll 1
-      for (int ks = 0; ks < KS; ++ks) dm_step(acc, fa + ks * 32, RT * KSM * 32, fb + ks * 32, CT * KSM * 32);
+      for (int ks = 0; ks < KS; ++ks) dm_step<false>(acc, none, fa + ks * 32, RT * KSM * 32, fb + ks * 32, CT * KSM * 32);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int a = ti[i] * 16 + (lane >> 2) + 8 * (j >> 1), b = tj[i] * 8 + 2 * (lane & 3) + (j & 1);

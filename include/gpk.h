@@ -105,6 +105,9 @@ int gpk_psi_bwd_ex(int prec, int N, int M, int Q, int Dout, const void* mu, cons
  *   kfu = K(x, Z) [N,M];  m[n,d] = kfu_n . A_d;  Bk[n,d,b] = sum_a B[d,a,b] kfu[n,a];
  *   v[n,d] = sf2 + kfu_n . Bk[n,d]
  * x [N,D] (row stride ldx), Z [M,D], A [Dout,M], B [Dout,M,M].  kfu/Bk/m/v optional.
+ * GPK_DF64, with kfu given and M <= 255: m and v to some M 2^-47 of their sums of |terms|; Bk[n,d,b] to
+ * some M 2^-48 of max_a(kfu[n,a] r_a) c_b beside the M 2^-47 of its own sum, with c_b the largest |B| of column b and
+ * r_a that of row a over the c_b: as accurate as the row's largest sums allow, not every small entry.
  * Replaces SGP_Layer._forward_prop_deterministic_thru_cav, geepee/aep_models.py:142-158
  * (and _thru_post, base_models.py:265-284). */
 int gpk_det_fwd(int prec, int N, int M, int D, int Dout, const void* x, int ldx, const void* Z,

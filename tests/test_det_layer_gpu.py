@@ -139,3 +139,67 @@ def test_contraction_of_any_nan(bits):
     assert (np.isnan(Bk.cpu().numpy()) == want).all()
     assert (np.isnan(mo.cpu().numpy()) == [False, True]).all()
     assert (np.isnan(vo.cpu().numpy()) == [True, False]).all()
+
+
+def _graded(kind, n, m, rng):
+    """Kernel rows over six lengthscales and a B whose size grows against them."""
+    z, x = np.sort(rng.uniform(0, 6, m)), rng.uniform(0, 1.5, n)
+    k = np.exp(-0.5 * (x[:, None] - z) ** 2)
+    C = rng.uniform(0.5, 1, (m, m)) * rng.choice([-1.0, 1.0], (m, m))
+    g = 10.0 ** (2 * z)                       # 1 to 1e12, along the decay of k
+    if kind == 'rows':
+        return k, g[:, None] * C
+    C = 0.5 * (C + C.T)
+    if kind == 'columns':
+        return k, C * g
+    if kind == 'symmetric':
+        return k, g[:, None] * C * g
+    if kind == 'diagonal':                    # far pseudo-inputs coupled to themselves alone
+        return k, np.diag(np.where(z > 3, 1e20, 1.0))
+    if kind == 'local':                       # most kernel values below the float range
+        return np.exp(-0.5 * (x[:, None] - z) ** 2 * 60), np.diag(rng.uniform(1, 4, m)) + 0.1 * C
+    return k, np.where(C == np.diag(np.diag(C)), 0.0, C * 1e-3) + np.diag(g)   # 'mixed'
+
+
+@pytest.mark.parametrize('m', [7, 60, 130, 201])
+@pytest.mark.parametrize('kind', ['rows', 'columns', 'symmetric', 'diagonal', 'local', 'mixed'])
+def test_contraction_of_graded_weights(kind, m):
+    """Weights graded against the kernel rows keep the double-float form's accuracy: m and v to
+    their sums of |terms| (a sum of M double-float terms: M 2^-47 of it; v's digit products, trusted
+    where the weighted sums of |k B| reach a sixteenth of the scales, another 16 M 2^-50.6), Bk to
+    M 2^-50 of the scales' product beside its own M 2^-47, and where B is dense that is its sum of
+    |terms| too."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(m)
+    L = np.longdouble
+    n = 40
+    k, B = _graded(kind, n, m, rng)
+    A = 10.0 ** (np.argsort(np.argsort(k[0])) * (-12.0 / m)) * rng.randn(1, m)
+    e = lambda *s: torch.zeros(s, dtype=torch.float64, device='cuda')
+    Bk, mo, vo = e(n, 1, m), e(n, 1), e(n, 1)
+    if m <= 128:
+        gpk.det_contract(dev(k), dev([0.0]), dev(A), dev(B[None]), Bk, mo, vo)
+        kg = k
+    else:   # through the fused entry point, whose rows are its own
+        kd = e(n, m)
+        x = rng.uniform(0, 1.5, (n, 1))
+        z = np.sort(rng.uniform(0, 6, m))[:, None]
+        l2 = np.zeros(1) if kind != 'local' else np.full(1, -np.log(60.0))
+        gpk.det_fwd(dev(x), dev(z), dev(l2), dev([0.0]), dev(A), dev(B[None]), kd, Bk, mo, vo)
+        kg = kd.cpu().numpy()
+    kg, Bl = kg.astype(L), B.astype(L)
+    S = np.abs(kg) @ np.abs(Bl)
+    bk, tiny = kg @ Bl, 1e-36
+    sm = (np.abs(kg) @ np.abs(A.astype(L)).T)[:, 0]
+    assert (np.abs(mo.cpu().numpy()[:, 0] - (kg @ A.astype(L).T)[:, 0]) <= (m + 16) * 2.0 ** -47 * sm + tiny).all()
+    T = (S * np.abs(kg)).sum(1)
+    dv = np.abs(vo.cpu().numpy()[:, 0] - (1 + (bk * kg).sum(1)))
+    assert (dv <= (3 * m + 16) * 2.0 ** -47 * (T + 1) + 16 * m * 2.0 ** -50.6 * T).all(), float((dv / (T + 1)).max())
+    c = np.abs(Bl).max(0)
+    r = (np.abs(Bl) / np.where(c > 0, c, 1)).max(1)
+    scale = (kg * r).max(1)[:, None] * c
+    db = np.abs(Bk.cpu().numpy()[:, 0] - bk)
+    # (the scales are powers of two up to four times c r, twice each)
+    assert (db <= m * 2.0 ** -48 * scale + (m + 16) * 2.0 ** -47 * S + tiny).all()
+    if kind in ('rows', 'columns', 'symmetric'):
+        assert (db <= 8 * m * 2.0 ** -48 * S).all(), float((db / S).max())
