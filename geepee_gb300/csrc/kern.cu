@@ -1355,20 +1355,23 @@ __global__ void __launch_bounds__(GP_T) gram_pairs_kernel(int N, int M, int Dout
 }
 
 // ---- the symmetric weighted Gram reduction on the tensor cores (float64) ----
-// C[d]_ab = sum_n (w u_a)(u_b) over a chunk of rows for one output d, by the digit products of
-// det_mma_kernel: the contraction runs over n, so each column of w u and of u is scaled by its largest entry
+// C[d]_ab = sum_n (w u_a 2^-h)(u_b 2^h) over a chunk of rows for one output d, by the digit products of
+// det_mma_kernel: the contraction runs over n, so each column of either factor is scaled by its largest entry
 // of the rows staged (at most 128, so that the digit sums stay exact), and the staged sums, exact
-// integers, are added up in float64.  A CTA of 12 warps owns up to 60 of the 16 x 8 tiles on and below the
+// integers, are added up in float64.  h is half of w's exponent: both factors are then sqrt|w| u in size,
+// and C_ab is off by some 2^-52 sqrt(n) of max_n sqrt|w| |u_a| max_n sqrt|w| |u_b|, at most of
+// sqrt(sum |w| u_a^2 sum |w| u_b^2), however w and u grow along n.  (The double-float pairs' error is some
+// 2^-48 of sum |w u_a u_b|: smaller only where two columns hardly meet.)  A CTA of 12 warps owns up to 60 of the 16 x 8 tiles on and below the
 // diagonal, five a warp, their float64 sums in registers; the next rows arrive by asynchronous copies while
 // these are multiplied.  The chunk's sums leave as a partial block of packed pairs for the
 // fixed-order reduction.
-// N = 20000, M = 100, two outputs: 84 us, a third of it in the matrix pipe, the rest in digits and folds
-// (356 us in double-float pairs); with the reduction 91 us (361); N = 1000, one output 21 us (26).
+// N = 20000, M = 100, two outputs: 86 us, a third of it in the matrix pipe, the rest in digits and folds
+// (356 us in double-float pairs); with the reduction 89 us (361; 87 with h = 0); N = 1000, one output 20 us (26).
 constexpr int GM_T = 384, GM_W = GM_T / 32, GM_TW = 5;
 struct GmSmem {
   unsigned *A, *B;   // digits of w u and of u, as in DmSmem (the columns in the place of the rows)
   double *raw, *w;   // [16 KS][M], [16 KS]
-  int *aexp, *bexp;
+  int *h, *aexp, *bexp;   // [16 KS] half of w's exponent; [M] of the columns of the two factors
 };
 __host__ __device__ inline size_t gm_carve(GmSmem* out, char* base, int M, int KS) {
   GmSmem s;
@@ -1383,6 +1386,7 @@ __host__ __device__ inline size_t gm_carve(GmSmem* out, char* base, int M, int K
   s.B = (unsigned*)take((size_t)DM_S * CT * KS * 256);
   s.raw = (double*)take((size_t)16 * KS * M * 8);
   s.w = (double*)take((size_t)16 * KS * 8);
+  s.h = (int*)take((size_t)16 * KS * 4);
   s.aexp = (int*)take((size_t)M * 4);
   s.bexp = (int*)take((size_t)M * 4);
   if (out) *out = s;
@@ -1427,14 +1431,15 @@ __global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dou
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     // ---- the columns' largest exponents (of w u at most: the factors' sum)
-    for (int i = tid; i < M; i += GM_T) s.aexp[i] = s.bexp[i] = -126;
+    for (int i = tid; i < M; i += GM_T) s.aexp[i] = s.bexp[i] = DM_LOW;
+    for (int r = tid; r < nr; r += GM_T) s.h[r] = expo(s.w[r]) >> 1;
     __syncthreads();
     for (int c = tid & 127; c < M; c += 128) {
-      int ea = -126, eb = -126;
+      int ea = DM_LOW, eb = DM_LOW;
       for (int r = tid >> 7; r < nr; r += GM_T / 128) {
-        const int e = expo(s.raw[r * M + c]), f = expo(s.w[r]);
-        eb = max(eb, e);
-        ea = max(ea, max(e, f) == 1025 ? DM_BAD : e + f);
+        const int e = expo(s.raw[r * M + c]), f = expo(s.w[r]), h = s.h[r];
+        eb = max(eb, e == 1025 ? DM_BAD : e + h);
+        ea = max(ea, max(e, f) == 1025 ? DM_BAD : e + f - h);
       }
       atomicMax(&s.bexp[c], eb > 300 ? DM_BAD : eb);
       atomicMax(&s.aexp[c], ea > 300 ? DM_BAD : ea);
@@ -1450,8 +1455,9 @@ __global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dou
         const int r = r0 + (i & 1) + 8 * (i >> 1);
         const bool on = c < M && r < nr;
         const double v = on ? s.raw[r * M + c] : 0.0, wv = on ? s.w[r] : 0.0;
-        ta[i] = digits_of(v * wv, ea);
-        tb[i] = digits_of(v, eb);
+        const int h = on ? s.h[r] : 0;
+        ta[i] = digits_of(v * wv, ea + h);
+        tb[i] = digits_of(v, eb - h);
       }
       unsigned w0[DM_S], w1[DM_S];
       digit_pairs(ta[0], ta[1], w0);

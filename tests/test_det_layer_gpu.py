@@ -203,3 +203,23 @@ def test_contraction_of_graded_weights(kind, m):
     assert (db <= m * 2.0 ** -48 * scale + (m + 16) * 2.0 ** -47 * S + tiny).all()
     if kind in ('rows', 'columns', 'symmetric'):
         assert (db <= 8 * m * 2.0 ** -48 * S).all(), float((db / S).max())
+
+
+@pytest.mark.parametrize('n,m,dout', [(40, 12, 1), (129, 33, 2), (3000, 100, 1)])
+@pytest.mark.parametrize('p', [-2, -1, 1, 4])
+def test_gram_of_graded_rows(n, m, dout, p):
+    """Rows that grow over twelve decades with weights that grow as a power of them: every sum is good to
+    its sum of |terms| (n 2^-47 of it, as a sum of n double-float terms; the columns are dense)."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(n + m)
+    L = np.longdouble
+    g = 10.0 ** rng.uniform(-6, 6, (n, 1))
+    u = g * rng.uniform(0.5, 1, (n, m)) * rng.choice([-1.0, 1.0], (n, m))
+    w = g ** p * rng.uniform(0.5, 1, (n, dout)) * rng.choice([-1.0, 1.0], (n, dout))
+    z = lambda *s: torch.zeros(s, dtype=torch.float64, device='cuda')
+    C, ut = z(dout, m, m), dev(u)
+    gpk.gram(ut, ut, dev(w), C, work=z(gpk.work_elems(gpk.OP_GRAM, n, m, 1, dout)))
+    ref = np.einsum('nd,na,nb->dab', w.astype(L), u.astype(L), u.astype(L))
+    S = np.einsum('nd,na,nb->dab', np.abs(w).astype(L), np.abs(u).astype(L), np.abs(u).astype(L))
+    err = np.abs(C.cpu().numpy() - ref)
+    assert (err <= n * 2.0 ** -47 * S).all(), float((err / S).max())
