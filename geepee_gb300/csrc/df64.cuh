@@ -359,14 +359,6 @@ __device__ __forceinline__ long long fx57_words_of(df64 v) {
   const int high = (int)(t >> 31), low = (int)((unsigned)t & 0x7fffffffu) - (1 << 30);
   return ((long long)high << 32) | (unsigned)low;
 }
-// a float64 in units of 2^-57, truncated (|v| < 64; the caller checks)
-__device__ __forceinline__ long long fx57_of_double(double v) {
-  const long long b = __double_as_longlong(v);
-  const int s = 1018 - (int)((b >> 52) & 0x7ff);   // v = m 2^(e - 1075): m 2^-s units
-  const long long m = (b & 0xfffffffffffffLL) | 0x10000000000000LL;
-  const long long t = s >= 0 ? m >> min(s, 63) : m << -max(s, -9);
-  return b < 0 ? -t : t;
-}
 // hi + lo as a float64 by integer operations (df_to_double's three FP64-pipe instructions take 48
 // cycles a warp): hi's bits widened, lo added in units of hi's last float64 place (half of it
 // below a power of two).  Values whose words leave the normal range take the FP64 path.

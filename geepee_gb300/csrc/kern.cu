@@ -77,21 +77,35 @@ __global__ void __launch_bounds__(256) kern_matrix_kernel(int N, int M, int D, c
 // as two words, high 2^-26 + low 2^-57: a difference is two integer subtractions, exact, and its
 // square two 32 x 32 -> 64-bit multiply-adds (the low word's square, at most 2^-52, is left out), where
 // the double-float difference, square and scaling take 32 instructions; the exponential then comes from
-// the exponent's bits (exp2_fx).  The sums are taken modulo 2^64 and a float sum of the squares beside them
-// says which are meant: at 256 or more the entry is zero (below 2^-128 with sf^2 < 2^126), below
-// it no sum leaves the range.  A coordinate outside +-16 (or not finite) has NaN for its float, which
-// sends the entries it meets to the double-float form (ard_general).
+// the exponent's bits (exp2_fx).  High words and sums are taken modulo 2^32 and 2^64, so that only differences
+// need the range: a float sum of the squares, of coordinates about the first pseudo-input's, says which are
+// meant.  At 256 or more the entry is zero (below 2^-126 with sf^2 < 2^126), below it no difference and no
+// sum leaves the range.  The floats are good to 2^-6 up to 2^16 lengthscales from that pseudo-input;
+// farther pseudo-inputs, and inputs that are not finite, have NaN for theirs, which sends the entries they
+// meet to the double-float form (ard_general); farther inputs meet no nearer pseudo-input.  Coordinates by
+// their distance from the origin instead took that form beyond 18.8 lengthscales of it, an entry at a time: 109 us
+// at N = 20000, M = 100, D = 8, inputs about 37 lengthscales off, where this takes 28.
 struct __align__(16) ArdHyp {
-  double s[DMAXK];      // sqrt(log2(e)/2) / ell_d
+  unsigned long long ms[DMAXK];   // sqrt(log2(e)/2) / ell_d: its significand,
+  int sh[DMAXK];        // 2093 less its exponent field (ard_coord)
+  float s[DMAXK];       // and its float (NaN out of range: every entry takes the general form)
+  float2 o[DMAXK];      // the first pseudo-input
   df64 inv_l2[DMAXK];   // 1/ell_d^2 (general form)
   df64 lsf;
   long long c0;         // log2 sf^2 in units of 2^-52, plus exp2_fx's half step
   int flag;             // sf^2 outside the fixed-point range: every entry takes the general form
 };
-__device__ __forceinline__ void load_ard(ArdHyp& h, const double* lls2, const double* lsf2, int D, ExpTab tab) {
+__device__ __forceinline__ void load_ard(ArdHyp& h, const double* lls2, const double* lsf2, int D, const double* z,
+                                         ExpTab tab) {
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     const double l = lls2[d];
-    h.s[d] = exp(-0.5 * l) * 0.84932180028801904272;   // times sqrt(log2(e)/2); (in float64: its error counts twice the exponent)
+    const double s = exp(-0.5 * l) * 0.84932180028801904272;   // (in float64: its error counts twice the exponent)
+    const long long b = __double_as_longlong(s);
+    h.ms[d] = ((unsigned long long)b & 0xfffffffffffffULL) | 0x10000000000000ULL;
+    h.sh[d] = 2093 - (int)(b >> 52);
+    h.s[d] = s > 1e-30 && s < 1e30 ? (float)s : __int_as_float(0x7fffffff);
+    const df64 o = fabs(z[d]) < 1e30 ? df_from_double(z[d]) : make_df(0.f);
+    h.o[d] = make_float2(o.hi, o.lo);
     h.inv_l2[d] = exp_tab(df_from_double(-l), tab);
   }
   if (threadIdx.x == 32) {
@@ -101,14 +115,30 @@ __device__ __forceinline__ void load_ard(ArdHyp& h, const double* lls2, const do
     h.c0 = (h.flag ? 0LL : __double2ll_rn(c * 4503599627370496.0)) + kFxHalf;
   }
 }
-// a coordinate in fixed point: (low, high, float, -)
-__device__ __forceinline__ int4 ard_coord(double x, double s) {
-  const double v = x * s;
-  const int e = (int)((__double_as_longlong(v) >> 52) & 0x7ff);
-  if (e >= 1027) return make_int4(0, 0, 0x7fffffff, 0);   // |v| >= 16, infinite or NaN
-  const long long t = fx57_of_double(v) + (1LL << 30);
-  const int h = (int)(t >> 31);
-  return make_int4((int)((unsigned)t & 0x7fffffffu) - (1 << 30), h, __float_as_int(__fmul_rn((float)h, 1.490116119e-08f)), 0);
+// coordinate x of dimension d times the scale in fixed point: (low, high modulo 2^32, float beside the first
+// pseudo-input's, -).  The product of the two 53-bit significands is exact, its bits below 2^-57 cut off; on
+// the integer pipes, because a product and its rounding error by the FP64 pipe made the kernel 8% slower.  The
+// pseudo-inputs' floats end at 2^16 (ZED).
+template <bool ZED>
+__device__ __forceinline__ int4 ard_coord(double x, const ArdHyp& h, int d) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ex = (int)(b >> 52) & 0x7ff, sh = h.sh[d] - ex;
+  const unsigned long long m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL;
+  const unsigned long long lo = m * h.ms[d], hi = __umul64hi(m, h.ms[d]);   // |x| s = (hi : lo) 2^-(57 + sh)
+  unsigned long long u = 0;
+  if (sh >= 64) u = hi >> min(sh - 64, 63);   // (hi < 2^42)
+  else if (sh > 0) u = (lo >> sh) | (hi << (64 - sh));
+  else if (sh > -64) u = lo << -sh;
+  const long long t = ((long long)b < 0 ? -(long long)u : (long long)u) + (1LL << 30);
+  int f = 0x7fffffff;   // not finite
+  if (ex < 1150) {
+    const df64 v = df_from_double(x);
+    f = __float_as_int(__fmul_rn(__fadd_rn(__fsub_rn(v.hi, h.o[d].x), __fsub_rn(v.lo, h.o[d].y)), h.s[d]));
+  } else if (ex < 2047) {
+    f = 0x7f800000 | (int)(b >> 32 & 0x80000000u);   // beyond the float range
+  }
+  if (ZED && (f & 0x7fffffff) > 0x47800000) f = 0x7fffffff;
+  return make_int4((int)((unsigned)t & 0x7fffffffu) - (1 << 30), (int)(t >> 31), f, 0);
 }
 __device__ __forceinline__ int4 lds_i4(saddr a) {
   int4 v;
@@ -150,7 +180,9 @@ __device__ __forceinline__ void ard_exponents(saddr x, saddr xstep, saddr z, int
 __device__ __noinline__ df64 ard_general(const double* x, const double* z, int D, const ArdHyp& h, const float2* tab) {
   df64 rr = make_df(0.f);
   for (int d = 0; d < D; ++d) {
-    const df64 df = sub(df_from_double(x[d]), df_from_double(z[d]));
+    const double diff = x[d] - z[d];   // (far from the origin a coordinate's own 48 bits are too few)
+    if (fabs(diff) < 1.7e308 && fabs(diff) * (double)h.s[d] > 1048576.0) return make_df(0.f);
+    const df64 df = df_from_double(diff);
     rr = fma_(mul(df, df), h.inv_l2[d], rr);
   }
   return exp_tab(sub(h.lsf, scale2(rr, -1)), ExpTab{tab});
@@ -159,8 +191,8 @@ __device__ __noinline__ df64 ard_general(const double* x, const double* z, int D
 // K (float64): a CTA takes FC columns and row tiles of FR; a thread one column and FR / (256 / FC) rows,
 // four at a time, so that a column's coordinate is loaded once for four rows.  As many CTAs as
 // are resident at once share the tiles: the tables and the columns are staged once a CTA.
-// Bound by the integer and FP32 pipes: 20000 x 100, D = 8 in 27 us (49 before), 20000 x 200, D = 16 in
-// 66 us (256 before).
+// Bound by the integer and FP32 pipes: 20000 x 100, D = 8 in 28 us (49 before), 20000 x 200, D = 16 in
+// 68 us (256 before).
 constexpr int FR = 16, FC = 128, FCTA = 3;
 __global__ void __launch_bounds__(256, FCTA) kern_fx_kernel(int N, int M, int D, const double* x, int ldx,
                                                             const double* z, int ldz, const double* lls2,
@@ -176,18 +208,18 @@ __global__ void __launch_bounds__(256, FCTA) kern_fx_kernel(int N, int M, int D,
   const int ntile = (N + FR - 1) / FR, step = (int)(gridDim.x / nmb);
   load_exp2_table(tab);
   __syncthreads();
-  load_ard(*h, lls2, lsf2, D, ExpTab{tab});
+  load_ard(*h, lls2, lsf2, D, z, ExpTab{tab});
   __syncthreads();
   auto rows = [&](int tile, int b) {
     const int n0 = tile * FR, nr = min(FR, N - n0);
     for (int e = tid; e < nr * D; e += 256) {
       const int r = e / D, d = e - r * D;
-      xs[b * FR * D + e] = ard_coord(x[(size_t)(n0 + r) * ldx + d], h->s[d]);
+      xs[b * FR * D + e] = ard_coord<false>(x[(size_t)(n0 + r) * ldx + d], *h, d);
     }
   };
   for (int e = tid; e < nc * D; e += 256) {
     const int c = e / D, d = e - c * D;
-    zs[c * DZ + d] = ard_coord(z[(size_t)(m0 + c) * ldz + d], h->s[d]);
+    zs[c * DZ + d] = ard_coord<true>(z[(size_t)(m0 + c) * ldz + d], *h, d);
   }
   rows((int)(blockIdx.x / nmb), 0);
   __syncthreads();

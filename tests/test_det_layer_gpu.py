@@ -223,3 +223,40 @@ def test_gram_of_graded_rows(n, m, dout, p):
     S = np.einsum('nd,na,nb->dab', np.abs(w).astype(L), np.abs(u).astype(L), np.abs(u).astype(L))
     err = np.abs(C.cpu().numpy() - ref)
     assert (err <= n * 2.0 ** -47 * S).all(), float((err / S).max())
+
+
+@pytest.mark.parametrize('n,m,d', [(1, 1, 1), (50, 17, 2), (33, 129, 5), (300, 100, 8)])
+@pytest.mark.parametrize('shift', [64.0, 2000.0, 1.7e9])
+def test_kernel_rows_do_not_depend_on_the_origin(n, m, d, shift):
+    """Kernel rows of inputs and pseudo-inputs translated together (by exact amounts: multiples of 2^-20) are the
+    same to the fixed point's last places: each coordinate is off by at most 2^-55 either time, which is
+    4 2^-55 sum |x - z| <= 4 2^-55 16 sqrt(d) in an exponent below 256, beside its own 2^-51 d; the exponential's
+    error is below 2^-49."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(n + d)
+    q = lambda a: np.round(a * 2.0 ** 20) / 2.0 ** 20
+    x, z = q(4 * rng.randn(n, d)), q(4 * rng.randn(m, d))
+    l2, s2 = dev(rng.uniform(-0.5, 0.5, d) + np.log(d)), dev([0.2])
+    K = gpk.kern(dev(x), dev(z), l2, s2).cpu().numpy()
+    off = shift * (1 - 2 * (np.arange(d) % 2))
+    Ks = gpk.kern(dev(x + off), dev(z + off), l2, s2).cpu().numpy()
+    tol = 2 * (2.0 ** -49 + 16 * d ** 0.5 * 2.0 ** -53 + d * 2.0 ** -51)
+    assert (np.abs(Ks - K) <= tol * K + 1e-300).all(), float((np.abs(Ks - K) / np.maximum(K, 1e-300)).max())
+
+
+@pytest.mark.parametrize('span', [40.0, 1000.0, 60000.0, 1e6])
+def test_kernel_rows_over_a_wide_range(span):
+    """A one-dimensional range of many lengthscales, with inputs far outside it: each entry to
+    2^-45 (|a| + 1) of itself (a its exponent), zero where it is below the float range."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(3)
+    L = np.longdouble
+    z = np.sort(rng.uniform(0, span, 150))[:, None]
+    x = np.concatenate([z[:, 0] + 3 * rng.randn(150), rng.uniform(0, span, 200), [-1e9, 1e12, 1e200, 7 * span]])[:, None]
+    K = gpk.kern(dev(x), dev(z), dev([0.0]), dev([0.4])).cpu().numpy()
+    a = 0.4 - 0.5 * (x.astype(L) - z.astype(L).T) ** 2
+    k = np.exp(a)
+    assert (np.abs(K - k) <= 2.0 ** -45 * (np.abs(a) + 1) * k + 1e-37).all()
+    assert (K[-4:] == 0).all()
+    Kn = gpk.kern(dev([[np.nan], [0.5]]), dev(z), dev([0.0]), dev([0.4])).cpu().numpy()
+    assert np.isnan(Kn[0]).all() and np.isfinite(Kn[1]).all()
