@@ -1670,23 +1670,26 @@ __global__ void __launch_bounds__((NS + NF) * 32, NS < 8 ? 4 : NS < 12 ? 2 : 1)
 //    exchange), so a step has two barriers: records ready, partial sums ready.  CH_REC warps form
 //    the records (128 rows at a time; those without rows sit out), CH_PSI1 warps psi1 and its sums
 //    beside them, CH_SWEEP warps the pairs;
-//  * the sums over threads are exact integer sums (in units of 2^-60 of sum |A| or sum |B|, which
-//    bound them): three 32-bit warp reductions a sum for what took five shuffle-and-add levels;
+//  * the sums over threads are integer sums, in units of 2^-57 of a warp's largest lane, so that a state far
+//    from every pseudo-input keeps its bits (psi1 beside the warp's nearest pseudo-input's): three 32-bit
+//    warp reductions a sum, and one for the scale, for what took five shuffle-and-add levels.  In units of
+//    2^-60 of sum |A| and sum |B| instead, a mean 2^-40 of sum |A| had 20 bits left (2.47 us a step at M = 50,
+//    Q = 2, 2.56 now; the warps' sums brought to one scale by each thread instead of a lane each 2.8);
 //  * with up to four pairs a thread, their G and B stay in registers.
-// Measured per step: M = 50, Q = 2: 5.2 -> 2.4 us; M = 100: 9.2 -> 4.5; M = 30, Q = 3: 6.0 -> 4.9;
-// M = 10, Q = 1: 3.8 -> 2.2 (the dependent chain alone).  At M = 50 the issue rate of one SM bounds the
+// Measured per step: M = 50, Q = 2: 5.2 -> 2.6 us; M = 100: 9.2 -> 4.6; M = 30, Q = 3: 6.0 -> 5.2;
+// M = 10, Q = 1: 3.8 -> 2.4 (the dependent chain alone).  At M = 50 the issue rate of one SM bounds the
 // pair phase (~5000 instructions a step): twelve sweep warps of four pairs a
 // thread take fewer of them than twenty of two (each warp pays ~100 for its reduction).
 constexpr int CH_REC = 4, CH_PSI1 = 4, CH_SWEEP = 12, CH_KP = 4;
 constexpr int CH_NTH = (CH_REC + CH_PSI1 + CH_SWEEP) * 32;
-// v 2^F as an integer (|v 2^F| < 2^61)
+// v 2^F as an integer (|v 2^F| < 2^57)
 __device__ __forceinline__ long long fx_dyn(float x, int F) {
   const unsigned b = __float_as_uint(x);
   const int s = max(0, min(189 - F - (int)((b >> 23) & 0xffu), 63));
   const long long v = (long long)(((unsigned long long)(((b & 0x7fffffu) | 0x800000u) << 7) << 32) >> s);
   return (int)b < 0 ? -v : v;
 }
-// the warp's sum of |x| < 2^61 (so that 32 lanes stay below 2^63 - the caller's scale leaves room)
+// the warp's sum of |x| < 2^57 (32 lanes stay below 2^62)
 __device__ __forceinline__ long long warp_sum_fx(long long x) {
   const unsigned l0 = (unsigned)x & 0x3ffffffu, l1 = (unsigned)(x >> 26) & 0x3ffffffu;
   const int l2 = (int)(x >> 52);
@@ -1694,20 +1697,42 @@ __device__ __forceinline__ long long warp_sum_fx(long long x) {
   const int s2 = __reduce_add_sync(0xffffffffu, l2);
   return (long long)s0 + ((long long)s1 << 26) + ((long long)s2 << 52);
 }
-// an integer times 2^-F as a double-float
-__device__ __forceinline__ df64 df_of_fx(long long x, int F) {
+// an integer as a double-float in units of 2^16
+__device__ __forceinline__ df64 df_of_fx(long long x) {
   const float h = (float)(int)(x >> 38), m = (float)(int)((x >> 16) & 0x3fffff), l = (float)(int)(x & 0xffff);
   // 26, 22 and 16 bits; h may round (its error is recovered exactly)
   const int he = (int)(x >> 38) - __float2int_rn(h);
-  const df64 a = two_sum(__fmul_rn(h, 4194304.f), __fmaf_rn((float)he, 4194304.f, m));   // units of 2^16
-  const df64 r = add(a, __fmul_rn(l, 1.52587890625e-05f));
-  return scale2(scale2(r, 8), 8 - F);
+  const df64 a = two_sum(__fmul_rn(h, 4194304.f), __fmaf_rn((float)he, 4194304.f, m));
+  return add(a, __fmul_rn(l, 1.52587890625e-05f));
+}
+// the warp's sum of one value a lane, times 2^-off: an integer in units of 2^(e - 183 - off), e the largest
+// lane's exponent field, with e - off + 128 in its last nine bits (2^-48 of that lane); 511: not finite
+__device__ __forceinline__ long long warp_sum_scaled(df64 v, int off) {
+  const int e = __reduce_max_sync(0xffffffffu, (int)((__float_as_uint(v.hi) >> 23) & 0xffu));
+  const long long s = warp_sum_fx(fx_dyn(v.hi, 183 - e) + fx_dyn(v.lo, 183 - e));
+  return ((s + 256) & ~511LL) | (e == 255 ? 511 : e - off + 128);
+}
+// the lanes' such sums x (0: none), G bits that their number needs: the total, a double-float times 2^e (e >= -240:
+// less is zero in any case)
+template <int G>
+__device__ __forceinline__ df64 sum_of_scaled(long long x, int& e) {
+  const int code = (int)x & 511, top = __reduce_max_sync(0xffffffffu, code);
+  const long long s = warp_sum_fx(x >> min(top - code + G, 63));
+  e = max(top + G - 295, -240);
+  df64 r = df_of_fx(s);
+  r.hi = top == 511 ? __int_as_float(0x7fffffff) : r.hi;
+  return r;
+}
+// a 2^e, -252 <= e <= 254, without a branch
+__device__ __forceinline__ df64 scale2_by(df64 a, int e) {
+  const float p = pow2f(e >> 1), q = pow2f(e - (e >> 1));
+  return make_df(a.hi * p * q, a.lo * p * q);
 }
 struct ChSmem {
   float2* tab;
   df64 *z, *As, *ell2, *sl, *inv4l, *misc;   // misc: sf2, then a step's normalisers of psi1 and psi2
   long long* rec;    // [M][rec_len]
-  long long* part;   // [QC][CH_PSI1] sums of m, then [QC][CH_SWEEP] of v
+  long long* part;   // [QC][CH_PSI1] sums of m, then [QC][CH_SWEEP] of v (warp_sum_scaled)
   long long* G;      // [P]
   df64* Bs;          // [QC * P]
   unsigned short* pab;   // [P]
@@ -1779,8 +1804,7 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
   const int M = a.M, Q = a.Q, P = M * (M + 1) / 2, T = a.N;
   ChSmem s;
   chcarve(&s, smem_raw, M, QC, P);
-  __shared__ int s_flag[2], s_bad, s_amax[QC], s_bmax[QC];
-  __shared__ unsigned long long s_asum[QC], s_bsum[QC];
+  __shared__ int s_flag[2];
   const ExpTab etab{s.tab};
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool sweep_warp = warp >= CH_REC + CH_PSI1, rec_warp = warp < CH_REC;
@@ -1791,11 +1815,6 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
     s.z[i] = q < Q ? df_from_double(a.Z[ia * Q + q]) : make_df(0.f);
   }
   if (tid < 2) s_flag[tid] = 0;
-  if (tid == 2) s_bad = 0;
-  if (tid < QC) {
-    s_amax[tid] = s_bmax[tid] = 0;
-    s_asum[tid] = s_bsum[tid] = 0;
-  }
   for (int i = tid; i < QC * (CH_PSI1 + CH_SWEEP); i += NTH) s.part[i] = 0;
   __syncthreads();
   if (tid < QC) {
@@ -1808,9 +1827,7 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
 #pragma unroll 1
   for (int i = tid; i < QC * M; i += NTH) {
     const int d = i / M;
-    const df64 v = d < Q ? df_from_double(a.A[i]) : make_df(0.f);
-    s.As[i] = v;
-    atomicMax(&s_amax[d], __float_as_int(fabsf(v.hi)));
+    s.As[i] = d < Q ? df_from_double(a.A[i]) : make_df(0.f);
   }
   __syncthreads();
 #pragma unroll 1
@@ -1827,36 +1844,9 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
         if (ia != ib) w = add(w, df_from_double(B[ib * M + ia]));
       }
       s.Bs[d * P + p] = w;
-      atomicMax(&s_bmax[d], __float_as_int(fabsf(w.hi)));
     }
   }
   __syncthreads();
-  // scales: |sum psi1 A| <= sum |A| and |sum psi2 B| <= sum |B| (psi1, psi2 without their
-  // normalisers are at most 1), summed as integers relative to the largest so that the result does
-  // not depend on the order; non-finite weights poison the result instead
-  int ea[QC], eb[QC];
-  bool bad_w = false;
-#pragma unroll
-  for (int d = 0; d < QC; ++d) {
-    ea[d] = max((s_amax[d] >> 23) - 126, -60);
-    eb[d] = max((s_bmax[d] >> 23) - 126, -60);
-    bad_w |= ea[d] > 128 || eb[d] > 128;
-    // |x| 2^(32 - e), rounded up (x < 2^e)
-    auto up = [](df64 x, int e) { return (unsigned long long)fx_dyn(fabsf(x.hi), 32 - e) + 2ull; };
-    unsigned long long sa = 0, sb = 0;
-    for (int i = tid; i < M; i += NTH) sa += up(s.As[d * M + i], ea[d]);
-    for (int p = tid; p < P; p += NTH) sb += up(s.Bs[d * P + p], eb[d]);
-    if (sa) atomicAdd(&s_asum[d], sa);
-    if (sb) atomicAdd(&s_bsum[d], sb);
-  }
-  __syncthreads();
-  int Fm[QC], Fv[QC];
-#pragma unroll
-  for (int d = 0; d < QC; ++d) {
-    Fm[d] = 60 - (ea[d] - 32 + 64 - __clzll(s_asum[d]));
-    Fv[d] = 60 - (eb[d] - 32 + 64 - __clzll(s_bsum[d]));
-  }
-  if (bad_w && tid == 0) s_bad = 1;
   const df64 sf2 = s.misc[0], kq = make_df(8.493217826e-01f, 1.769906000e-08f);   // sqrt(log2(e) / 2)
   // the pairs of a sweep thread, their G and B
   const int st = tid - (CH_REC + CH_PSI1) * 32;
@@ -1891,30 +1881,25 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
         } else {
           // ---- the previous step's moments from the partial sums (each warp for itself)
           const df64 K1 = s.misc[1], F2 = s.misc[2];
-          const bool bad = s_bad != 0;
-          const saddr pm = sm_addr(s.part), pv = pm + QC * CH_PSI1 * 8;
+          df64 mu[QC];   // m times 2^64 where it is below ~2^-96 (its low word would leave the float range)
+          int up[QC];
 #pragma unroll
           for (int d = 0; d < QC; ++d) {
-            long long sm = 0, sv = 0, x0, x1;
-#pragma unroll
-            for (int k = 0; k < CH_PSI1; k += 2) {
-              lds_two(pm + (d * CH_PSI1 + k) * 8, x0, x1);
-              sm += x0 + x1;
-            }
-#pragma unroll
-            for (int k = 0; k < CH_SWEEP; k += 2) {
-              lds_two(pv + (d * CH_SWEEP + k) * 8, x0, x1);
-              sv += x0 + x1;
-            }
-            m[d] = mul(K1, df_of_fx(sm, Fm[d]));
-            v[d] = sub(fma_(F2, df_of_fx(sv, Fv[d]), sf2), mul(m[d], m[d]));
-            if (bad) m[d] = v[d] = make_df(__int_as_float(0x7fffffff));
+            int em, ev;
+            const df64 rm = sum_of_scaled<2>(lane < CH_PSI1 ? s.part[d * CH_PSI1 + lane] : 0, em);
+            const df64 rv = sum_of_scaled<4>(lane < CH_SWEEP ? s.part[QC * CH_PSI1 + d * CH_SWEEP + lane] : 0, ev);
+            up[d] = em < -142 ? 64 : 0;
+            mu[d] = mul(K1, scale2_by(rm, em + up[d]));
+            const float down = pow2f(-up[d]);
+            m[d] = make_df(mu[d].hi * down, mu[d].lo * down);
+            v[d] = sub(fma_(F2, scale2_by(rv, ev), sf2), mul(m[d], m[d]));
           }
           if (tid == 0) {   // (before the barrier: the general form reads them)
 #pragma unroll
             for (int d = 0; d < QC; ++d)
               if (d < Q) {
-                a.m_out[(size_t)(t - 1) * Q + d] = df_to_double_int(m[d]);
+                const double md = df_to_double_int(mu[d]);
+                a.m_out[(size_t)(t - 1) * Q + d] = up[d] ? md * 5.42101086242752217e-20 : md;   // 2^-64
                 a.v_out[(size_t)(t - 1) * Q + d] = df_to_double_int(v[d]);
               }
           }
@@ -1962,7 +1947,10 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
       } else {
         // ---- psi1 and its sums
         df64 mm[QC], r1[QC], K1 = sf2;
+        int off = 0;   // the terms are 2^off psi1 / K1, 2^-off that of the warp's nearest row
         if (live_warp) {
+          const bool one_each = M <= CH_PSI1 * 32;   // (the tables of more rows do not fit beside two inputs)
+          const unsigned row_lanes = 0xffffffffu >> max(32 - (M - (r0 & ~31)), 0);
 #pragma unroll
           for (int q = 0; q < QC; ++q) {
             mm[q] = make_df(0.f);
@@ -1978,8 +1966,10 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
               e = fma_(x, x, e);
             }
             // psi1 / K1 = 2^-e
-            const df64 p1 = e.hi < 126.f ? exp2_fx(fx52_of(neg(e)) + kFxHalf, sm_addr(s.tab))
-                                         : (e.hi >= 126.f ? make_df(0.f) : make_df(__int_as_float(0x7fffffff)));
+            if (one_each) off = (int)__reduce_min_sync(row_lanes, (unsigned)fminf(fmaxf(e.hi, 0.f), 120.f));
+            const float left = e.hi - (float)off;
+            const df64 p1 = left < 126.f ? exp2_fx(fx52_of(neg(e)) + kFxHalf + ((long long)off << 52), sm_addr(s.tab))
+                                         : (left >= 126.f ? make_df(0.f) : make_df(__int_as_float(0x7fffffff)));
 #pragma unroll
             for (int d = 0; d < QC; ++d) acc_fma(mm[d], p1, s.As[d * M + ia]);
           }
@@ -1988,8 +1978,7 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
         if (live_warp) {
 #pragma unroll
           for (int d = 0; d < QC; ++d) {
-            if (!(fabsf(mm[d].hi) < 3e38f)) s_bad = 1;
-            const long long x = warp_sum_fx(fx_dyn(mm[d].hi, Fm[d]) + fx_dyn(mm[d].lo, Fm[d]));
+            const long long x = warp_sum_scaled(acc_done(mm[d]), off);
             if (lane == 0) s.part[d * CH_PSI1 + warp - CH_REC] = x;
           }
           if (warp == CH_REC && lane == 0) s.misc[1] = K1;
@@ -2034,10 +2023,8 @@ __global__ void __launch_bounds__(CH_NTH, 1) psi_chain_kernel(PsiArgs<double> a)
       }
 #pragma unroll
       for (int d = 0; d < QC; ++d) {
-        const df64 x = acc_done(vv[d]);
-        if (!(fabsf(x.hi) < 3e38f)) s_bad = 1;
-        const long long f = warp_sum_fx(fx_dyn(x.hi, Fv[d]) + fx_dyn(x.lo, Fv[d]));
-        if (lane == 0) s.part[QC * CH_PSI1 + d * CH_SWEEP + warp - CH_REC - CH_PSI1] = f;
+        const long long x = warp_sum_scaled(acc_done(vv[d]), 0);
+        if (lane == 0) s.part[QC * CH_PSI1 + d * CH_SWEEP + warp - CH_REC - CH_PSI1] = x;
       }
       __syncthreads();
     }

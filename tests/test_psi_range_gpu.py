@@ -233,3 +233,34 @@ def test_psi_moments_where_the_tables_do_not_fit(N):
     assert_close(v.cpu().numpy(), np.exp(0.3) + np.einsum('dab,nab->nd', B, p2) - m_ref ** 2, TOL, 'v')
     m7, v7 = run(777)
     assert torch.equal(m, m7[:N]) and torch.equal(v, v7[:N])
+
+
+@pytest.mark.parametrize('M,Q', [(10, 1), (50, 2), (30, 3), (100, 4), (120, 1)])
+def test_psi_rollout_far_from_the_pseudo_inputs(M, Q):
+    """One step from states ever farther from every pseudo-input: the mean stays good to its own sum of
+    |terms|.  Its exponents e (base 2) are double-float sums, off by e 2^-46 each, the sum of M
+    double-float terms by M 2^-46: (e + M) 2^-44 of sum |psi1 A|, as long as psi1 has not left the
+    float range (e < 126)."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(M + Q)
+    L = np.longdouble
+    Z = rng.uniform(-1, 1, (M, Q))
+    lls2, lsf2 = rng.uniform(-0.4, 0.1, Q), np.array([0.2])
+    A = rng.randn(Q, M)
+    B = rng.randn(Q, M, M) / M
+    B = 0.1 * (B + B.transpose(0, 2, 1))
+    l2, seen = np.exp(lls2.astype(L)), 0
+    for far in np.linspace(3, 13, 21):
+        mu, S = np.zeros(Q), rng.uniform(0.01, 0.05, Q)
+        mu[0] = far * np.exp(0.5 * lls2[0])
+        s1 = l2 + S.astype(L)
+        e = 0.5 * ((mu.astype(L) - Z) ** 2 / s1).sum(1)
+        p1 = np.exp(L(lsf2[0]) + 0.5 * np.log(l2 / s1).sum() - e)
+        e2 = float(e.max()) / np.log(2.0)
+        if e2 > 120:
+            break
+        seen += 1
+        gm, _ = gpk.psi_rollout(dev(mu), dev(S), dev(Z), dev(lls2), dev(lsf2), dev(A), dev(B), 1)
+        err = np.abs(gm[0].cpu().numpy() - A.astype(L) @ p1) / (np.abs(A).astype(L) @ p1)
+        assert (err <= (e2 + M) * 2.0 ** -44).all(), (far, e2, err)
+    assert seen >= 10
