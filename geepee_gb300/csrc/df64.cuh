@@ -436,6 +436,27 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
 // max that returns NaN when either is NaN
 __device__ __forceinline__ float fmax_nan(float a, float b) { return (a != a || b != b) ? __int_as_float(0x7fffffff) : fmaxf(a, b); }
 
+// a running sum kept as (hi, lo) without renormalising: for sums of a few dozen terms (the low
+// word's own rounding stays below the normalised sum's)
+__device__ __forceinline__ void acc_add(df64& a, df64 x) {
+  const df64 s = two_sum(a.hi, x.hi);
+  a.hi = s.hi;
+  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, x.lo));
+}
+__device__ __forceinline__ void acc_fma(df64& a, df64 x, df64 y) {
+  const float p = __fmul_rn(x.hi, y.hi);
+  float e = __fmaf_rn(x.hi, y.hi, -p);
+  e = __fmaf_rn(x.hi, y.lo, e);
+  e = __fmaf_rn(x.lo, y.hi, e);
+  const df64 s = two_sum(a.hi, p);
+  a.hi = s.hi;
+  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, e));
+}
+__device__ __forceinline__ df64 acc_done(df64 a) { return quick_two_sum(a.hi, a.lo); }
+__device__ __forceinline__ void acc_add(float& a, float x) { a += x; }
+__device__ __forceinline__ void acc_fma(float& a, float x, float y) { a = __fmaf_rn(x, y, a); }
+__device__ __forceinline__ float acc_done(float a) { return a; }
+
 // Warp sums of K values at once (K a power of two <= 32): in each of the first log2 K steps
 // of the butterfly a lane keeps half of its values and adds its partner's copies of them,
 // trading the other half, so the K sums take K - 1 + 5 - log2 K exchanges instead of 5 K.

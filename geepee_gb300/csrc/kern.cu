@@ -584,10 +584,11 @@ __device__ __forceinline__ long long dm_fold(const float (&acc)[DM_ACC][4], int 
   const long long Y = mad_wide(S(4) + S(5), 1 << 18, mad_wide(S(6) + S(7) + S(8), 1 << 9, (long long)(S(9) + s6)));
   return (X << 20) + (Y >> 7);
 }
-// one k step: all digit products of a row fragment and a column fragment (strides in fragments), and (MAG) the
-// product of the rows' first digits with the magnitudes of the columns': the sum of magnitudes for rows without
-// negative entries (kernel values), never more than it
-template <bool MAG>
+constexpr unsigned POS2 = 0x7fff7fffu;   // the magnitudes of two f16
+// one k step: all digit products of a row fragment and a column fragment (strides in fragments), and into mag the
+// product of the first digits' magnitudes, of the columns' alone unless BOTH: the sum of magnitudes for rows
+// without negative entries (kernel values), never more than it
+template <bool BOTH>
 __device__ __forceinline__ void dm_step(float (&acc)[DM_ACC][4], float (&mag)[4], const uint4* fa, int sa, const uint2* fb,
                                         int sb) {
   uint4 va[DM_S];
@@ -596,7 +597,10 @@ __device__ __forceinline__ void dm_step(float (&acc)[DM_ACC][4], float (&mag)[4]
 #pragma unroll
   for (int j = 0; j < DM_S; ++j) {
     const uint2 vb = fb[(size_t)j * sb];
-    if (MAG && j == 0) mma_f16(mag, va[0], make_uint2(vb.x & 0x7fff7fffu, vb.y & 0x7fff7fffu));
+    if (j == 0) {
+      const uint4 a = BOTH ? make_uint4(va[0].x & POS2, va[0].y & POS2, va[0].z & POS2, va[0].w & POS2) : va[0];
+      mma_f16(mag, a, make_uint2(vb.x & POS2, vb.y & POS2));
+    }
 #pragma unroll
     for (int i = 0; i < DM_S; ++i)
       if (i + j <= 6) mma_f16(acc[dm_acc(i, j)], va[i], vb);
@@ -893,7 +897,7 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
           const int k1 = min(k0 + 8, KS);
 #pragma unroll 2
           for (int ks = k0; ks < k1; ++ks)
-            dm_step<true>(acc, mag, fa + ks * 32, nrt * KS * 32, fb + ks * 32, NT * KS * 32);
+            dm_step<false>(acc, mag, fa + ks * 32, nrt * KS * 32, fb + ks * 32, NT * KS * 32);
 #pragma unroll
           for (int j = 0; j < 4; ++j) Z[j] += dm_fold(acc, j);
         }
@@ -1391,19 +1395,23 @@ __global__ void __launch_bounds__(GP_T) gram_pairs_kernel(int N, int M, int Dout
 // det_mma_kernel: the contraction runs over n, so each column of either factor is scaled by its largest entry
 // of the rows staged (at most 128, so that the digit sums stay exact), and the staged sums, exact
 // integers, are added up in float64.  h is half of w's exponent: both factors are then sqrt|w| u in size,
-// and C_ab is off by some 2^-52 sqrt(n) of max_n sqrt|w| |u_a| max_n sqrt|w| |u_b|, at most of
-// sqrt(sum |w| u_a^2 sum |w| u_b^2), however w and u grow along n.  (The double-float pairs' error is some
-// 2^-48 of sum |w u_a u_b|: smaller only where two columns hardly meet.)  A CTA of 12 warps owns up to 60 of the 16 x 8 tiles on and below the
+// and the staged sum is off by some 2^-52 of max_n sqrt|w| |u_a| max_n sqrt|w| |u_b| a row, however w and u grow
+// along n.  Where the sum of |terms|, estimated from the first digits, is below 1/32 of that product (two columns
+// that hardly meet), the staged rows are summed in double-float instead: every C_ab is good to some n 2^-47 of its
+// own sum of |terms|, as a double-float sum is.  A CTA of 12 warps owns up to 60 of the 16 x 8 tiles on and below the
 // diagonal, five a warp, their float64 sums in registers; the next rows arrive by asynchronous copies while
 // these are multiplied.  The chunk's sums leave as a partial block of packed pairs for the
 // fixed-order reduction.
-// N = 20000, M = 100, two outputs: 86 us, a third of it in the matrix pipe, the rest in digits and folds
-// (356 us in double-float pairs); with the reduction 89 us (361; 87 with h = 0); N = 1000, one output 20 us (26).
+// N = 20000, M = 100, two outputs, with the reduction 99 us (361 in double-float pairs), a third of it in the matrix
+// pipe, the rest in digits and folds (87 with h = 0 and every result trusted); N = 1000 22 us (30).  Two
+// input dimensions (2% of the results weak) 132 us, one with a lengthscale of 0.04 of the range (most of them) 359.
+constexpr float GM_TRUST = 512.f;   // 1/32 of the scales, in the first digits' units
 constexpr int GM_T = 384, GM_W = GM_T / 32, GM_TW = 5;
 struct GmSmem {
   unsigned *A, *B;   // digits of w u and of u, as in DmSmem (the columns in the place of the rows)
   double *raw, *w;   // [16 KS][M], [16 KS]
   int *h, *aexp, *bexp;   // [16 KS] half of w's exponent; [M] of the columns of the two factors
+  int* list;         // [GM_W][32] a warp's weak results: first time << 31 | row << 16 | column
 };
 __host__ __device__ inline size_t gm_carve(GmSmem* out, char* base, int M, int KS) {
   GmSmem s;
@@ -1421,6 +1429,7 @@ __host__ __device__ inline size_t gm_carve(GmSmem* out, char* base, int M, int K
   s.h = (int*)take((size_t)16 * KS * 4);
   s.aexp = (int*)take((size_t)M * 4);
   s.bexp = (int*)take((size_t)M * 4);
+  s.list = (int*)take((size_t)GM_W * 32 * 4);
   if (out) *out = s;
   return o;
 }
@@ -1451,15 +1460,20 @@ __global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dou
 #pragma unroll
     for (int j = 0; j < 4; ++j) C[i][j] = 0.0;
   }
-  auto fetch = [&](int n0) {
-    const int nr = min(16 * KSM, nend - n0);
+  // the rows by steps of 16, as evenly as at most KSM steps at a time allow (few rows leave more results weak)
+  const int steps = (nend - nbeg + 15) >> 4, nst = (steps + KSM - 1) / KSM;
+  auto begin = [&](int st) { return min(nend, nbeg + 16 * (int)((long)steps * st / nst)); };
+  auto fetch = [&](int st) {
+    const int n0 = begin(st), nr = begin(st + 1) - n0;
     for (int e = tid; e < nr * M; e += GM_T) async_copy(s.raw + e, u + (size_t)n0 * M + e);
     for (int e = tid; e < nr; e += GM_T) async_copy(s.w + e, w + (size_t)(n0 + e) * Dout + d);
   };
   auto expo = [](double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff) - 1022; };   // |v| < 2^expo
-  fetch(nbeg);
-  for (int n0 = nbeg; n0 < nend; n0 += 16 * KSM) {
-    const int nr = min(16 * KSM, nend - n0), KS = (nr + 15) >> 4;
+  double* const pb = part + (size_t)blockIdx.x * pstride + (size_t)d * (M * (M + 1) / 2);
+  unsigned seen = 0;   // results that were weak before: their sums stand in the partial block
+  fetch(0);
+  for (int st = 0; st < nst; ++st) {
+    const int n0 = begin(st), nr = begin(st + 1) - n0, KS = (nr + 15) >> 4;
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     // ---- the columns' largest exponents (of w u at most: the factors' sum)
@@ -1509,11 +1523,12 @@ __global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dou
       }
     }
     __syncthreads();
-    if (n0 + 16 * KSM < nend) fetch(n0 + 16 * KSM);
+    if (st + 1 < nst) fetch(st + 1);
+    unsigned weak = 0;   // the results (bit 4 i + j: result j of tile i) that the digits are too coarse for
 #pragma unroll
     for (int i = 0; i < GM_TW; ++i) {
       if (ti[i] < 0) continue;   // (uniform over the warp)
-      float acc[DM_ACC][4], none[4];
+      float acc[DM_ACC][4], mag[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int k = 0; k < DM_ACC; ++k)
 #pragma unroll
@@ -1521,24 +1536,101 @@ __global__ void __launch_bounds__(GM_T, 1) gram_mma_kernel(int N, int M, int Dou
       const uint4* fa = reinterpret_cast<const uint4*>(s.A) + (size_t)ti[i] * KSM * 32 + lane;
       const uint2* fb = reinterpret_cast<const uint2*>(s.B) + (size_t)tj[i] * KSM * 32 + lane;
 #pragma unroll 1
-      for (int ks = 0; ks < KS; ++ks) dm_step<false>(acc, none, fa + ks * 32, RT * KSM * 32, fb + ks * 32, CT * KSM * 32);
+      for (int ks = 0; ks < KS; ++ks) dm_step<true>(acc, mag, fa + ks * 32, RT * KSM * 32, fb + ks * 32, CT * KSM * 32);
+      const bool strong = __all_sync(~0u, fminf(fminf(mag[0], mag[1]), fminf(mag[2], mag[3])) >= GM_TRUST);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int a = ti[i] * 16 + (lane >> 2) + 8 * (j >> 1), b = tj[i] * 8 + 2 * (lane & 3) + (j & 1);
-        const int e = a < M && b < M ? s.aexp[a] + s.bexp[b] : 0;
+        const int ea = a < M ? s.aexp[a] : 0, eb = b < M ? s.bexp[b] : 0, e = ea + eb;
         // 2^(e - 52), or NaN
         const double f = __hiloint2double(e >= DM_BAD / 2 ? 0x7fffffff : (e + 971) << 20, 0);
-        C[i][j] = fma(__ll2double_rn(dm_fold(acc, j)), f, C[i][j]);
+        if (!strong && mag[j] < GM_TRUST && a < M && b <= a && max(ea, eb) < DM_BAD && min(ea, eb) > DM_LOW)
+          weak |= 1u << (4 * i + j);   // (not: a column of zeros)
+        else
+          C[i][j] = fma(__ll2double_rn(dm_fold(acc, j)), f, C[i][j]);
       }
     }
+    if (__syncthreads_or(weak)) {
+      // ---- the weak results: the staged rows once more, u and w u as double-floats in the place of the digits,
+      // and each warp's results in turn, 32 at a time, a lane each (14 instructions a row)
+      df64* const ud = reinterpret_cast<df64*>(s.B);
+      df64* const wu = reinterpret_cast<df64*>(s.A);
+      for (int r0 = warp; r0 < nr; r0 += 3 * GM_W) {   // a warp a row, three rows' loads in flight
+        for (int c0 = lane; c0 < M; c0 += 128) {
+          double v[3][4], wv[3];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int r = r0 + k * GM_W;
+            wv[k] = r < nr ? w[(size_t)(n0 + r) * Dout + d] : 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[k][j] = r < nr && c0 + 32 * j < M ? u[(size_t)(n0 + r) * M + c0 + 32 * j] : 0.0;
+          }
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const int r = r0 + k * GM_W;
+            const df64 wd = df_from_double(wv[k]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (r < nr && c0 + 32 * j < M) {
+                const df64 x = df_from_double(v[k][j]);
+                ud[r * M + c0 + 32 * j] = x;
+                wu[r * M + c0 + 32 * j] = mul(wd, x);
+              }
+          }
+        }
+      }
+      int first = __popc(weak);   // this lane's first in the warp's order
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(~0u, first, o);
+        first += lane >= o ? x : 0;
+      }
+      const int total = __shfl_sync(~0u, first, 31);
+      first -= __popc(weak);
+      __syncthreads();
+      int* const list = s.list + warp * 32;
+      for (int t0 = 0; t0 < total; t0 += 32) {
+        int k = first - t0;   // the place of this lane's next result among the 32
+        if (k < 32 && k + __popc(weak) > 0) {
+#pragma unroll
+          for (int i = 0; i < GM_TW; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if ((weak >> (4 * i + j)) & 1u) {
+                if (k >= 0 && k < 32)
+                  list[k] = ((seen >> (4 * i + j)) & 1u ? 0 : (int)0x80000000) |
+                            (ti[i] * 16 + (lane >> 2) + 8 * (j >> 1)) << 16 | (tj[i] * 8 + 2 * (lane & 3) + (j & 1));
+                ++k;
+              }
+        }
+        __syncwarp();
+        if (t0 + lane < total) {
+          const int c = list[lane], a = (c >> 16) & 0x7fff, b = c & 0xffff;
+          const df64 *pa = wu + a, *pu = ud + b;
+          df64 x = make_df(0.f);
+#pragma unroll 4
+          for (int r = 0; r < nr; ++r) {
+            const df64 p = pa[r * M], q = pu[r * M];
+            acc_fma(x, p, q);
+          }
+          double* const o = pb + a * (a + 1) / 2 + b;
+          *o = df_to_double(acc_done(x)) + (c < 0 ? 0.0 : *o);
+        }
+        __syncwarp();
+      }
+      seen |= weak;
+    }
   }
-  double* const pb = part + (size_t)blockIdx.x * pstride + (size_t)d * (M * (M + 1) / 2);
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < GM_TW; ++i) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int a = ti[i] * 16 + (lane >> 2) + 8 * (j >> 1), b = tj[i] * 8 + 2 * (lane & 3) + (j & 1);
-      if (ti[i] >= 0 && a < M && b <= a) pb[a * (a + 1) / 2 + b] = C[i][j];
+      if (ti[i] >= 0 && a < M && b <= a) {
+        double* const o = pb + a * (a + 1) / 2 + b;
+        *o = (seen >> (4 * i + j)) & 1u ? *o + C[i][j] : C[i][j];
+      }
     }
   }
 }

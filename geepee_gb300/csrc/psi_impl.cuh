@@ -382,27 +382,6 @@ __device__ __noinline__ T psi2_general(const T* za, const T* zb, const T* pd, co
   return exp_pair(x, ExpTab{tab});
 }
 
-// a running sum kept as (hi, lo) without renormalising: for sums of a few dozen terms (the low
-// word's own rounding stays below the normalised sum's)
-__device__ __forceinline__ void acc_add(df64& a, df64 x) {
-  const df64 s = two_sum(a.hi, x.hi);
-  a.hi = s.hi;
-  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, x.lo));
-}
-__device__ __forceinline__ void acc_fma(df64& a, df64 x, df64 y) {
-  const float p = __fmul_rn(x.hi, y.hi);
-  float e = __fmaf_rn(x.hi, y.hi, -p);
-  e = __fmaf_rn(x.hi, y.lo, e);
-  e = __fmaf_rn(x.lo, y.hi, e);
-  const df64 s = two_sum(a.hi, p);
-  a.hi = s.hi;
-  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, e));
-}
-__device__ __forceinline__ df64 acc_done(df64 a) { return quick_two_sum(a.hi, a.lo); }
-__device__ __forceinline__ void acc_add(float& a, float x) { a += x; }
-__device__ __forceinline__ void acc_fma(float& a, float x, float y) { a = __fmaf_rn(x, y, a); }
-__device__ __forceinline__ float acc_done(float a) { return a; }
-
 // barrier ID over NW warps of the CTA
 template <int ID, int NW>
 __device__ __forceinline__ void warps_sync() {

@@ -149,8 +149,7 @@ int gpk_psi_rollout(int prec, int T, int M, int Q, const void* mu0, const void* 
 /* Weighted Gram reduction over rows:  C[d] += sum_n w[n,d] u_n v_n^T  (u, v [N,M], w [N,Dout],
  * C [Dout,M,M] float64).  The einsum('nd,na,nb->dab') / einsum('na,nd,nb->dab') reductions of
  * geepee/aep_models.py:464,493.  When u and v are the same buffer, C is symmetric: the tiles
- * above the diagonal are formed once and added at both positions; GPK_DF64 with a workspace then
- * forms C_ab to some 2^-52 sqrt(N) of sqrt(sum |w| u_a^2 sum |w| u_b^2), not of its own sum of |terms|. */
+ * above the diagonal are formed once and added at both positions. */
 int gpk_gram(int prec, int N, int M, int Dout, const void* u, const void* v, const void* w, double* C,
              void* stream);
 

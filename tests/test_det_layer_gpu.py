@@ -260,3 +260,35 @@ def test_kernel_rows_over_a_wide_range(span):
     assert (K[-4:] == 0).all()
     Kn = gpk.kern(dev([[np.nan], [0.5]]), dev(z), dev([0.0]), dev([0.4])).cpu().numpy()
     assert np.isnan(Kn[0]).all() and np.isfinite(Kn[1]).all()
+
+
+@pytest.mark.parametrize('n,m,dout', [(17, 9, 1), (130, 40, 2), (2000, 100, 1), (5000, 129, 2)])
+@pytest.mark.parametrize('kind', ['local', 'mixed', 'disjoint'])
+def test_gram_of_columns_that_hardly_meet(n, m, dout, kind):
+    """Kernel rows of a layer whose lengthscale is short against the spread of its pseudo-inputs: the sums of
+    far pseudo-inputs are tens of decades below the near ones' and each is still good to n 2^-47 of its own
+    sum of |terms|."""
+    from geepee_gb300 import gpk
+    rng = np.random.RandomState(n + m)
+    L = np.longdouble
+    z, x = np.sort(rng.uniform(0, 1, m)), rng.uniform(0, 1, n)
+    u = np.exp(-0.5 * (x[:, None] - z) ** 2 / 0.06 ** 2)
+    if kind == 'mixed':                            # broad columns among the narrow ones
+        u[:, ::3] = np.exp(-0.5 * (x[:, None] - z[::3]) ** 2)
+    if kind == 'disjoint':                         # every other column on rows of its own, and a column of zeros
+        u[::2, ::2] = 0.0
+        u[1::2, 1::2] *= 1e-9
+        u[:, m // 2] = 0.0
+    w = rng.randn(n, dout)
+    z0 = lambda *s: torch.zeros(s, dtype=torch.float64, device='cuda')
+    C, ut = z0(dout, m, m), dev(u)
+    gpk.gram(ut, ut, dev(w), C, work=z0(gpk.work_elems(gpk.OP_GRAM, n, m, 1, dout)))
+    ref = np.einsum('nd,na,nb->dab', w.astype(L), u.astype(L), u.astype(L))
+    S = np.einsum('nd,na,nb->dab', np.abs(w).astype(L), u.astype(L), u.astype(L))
+    err = np.abs(C.cpu().numpy() - ref)
+    assert (err <= n * 2.0 ** -47 * S + 1e-37).all(), float((err / (S + 1e-37)).max())
+    u[n // 3, m // 2] = np.nan                     # a NaN in a column of zeros
+    C, ut = z0(dout, m, m), dev(u)
+    gpk.gram(ut, ut, dev(w), C, work=z0(gpk.work_elems(gpk.OP_GRAM, n, m, 1, dout)))
+    g, keep = C.cpu().numpy(), np.arange(m) != m // 2
+    assert np.isnan(g[:, m // 2]).all() and np.isnan(g[:, :, m // 2]).all() and np.isfinite(g[:, keep][:, :, keep]).all()
