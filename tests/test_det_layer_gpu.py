@@ -292,3 +292,22 @@ def test_gram_of_columns_that_hardly_meet(n, m, dout, kind):
     gpk.gram(ut, ut, dev(w), C, work=z0(gpk.work_elems(gpk.OP_GRAM, n, m, 1, dout)))
     g, keep = C.cpu().numpy(), np.arange(m) != m // 2
     assert np.isnan(g[:, m // 2]).all() and np.isnan(g[:, :, m // 2]).all() and np.isfinite(g[:, keep][:, :, keep]).all()
+
+
+@pytest.mark.parametrize('kind', ['rows', 'diagonal', 'mixed'])
+def test_contraction_of_graded_pairs(kind):
+    """The same weights as double-float pairs give the same bits, the rows formed again in double-float
+    among them."""
+    from geepee_gb300 import gpk
+    m, n = 60, 40
+    rng = np.random.RandomState(m)
+    k, B = _graded(kind, n, m, rng)
+    A = rng.randn(1, m)
+    hi = B.astype(np.float32)
+    pairs = np.stack([hi, (B - hi).astype(np.float32)], -1).astype(np.float32).view(np.float64)[..., 0]
+    got = []
+    for Bp, flag in ((B, False), (pairs, True)):
+        out = [torch.zeros(s, dtype=torch.float64, device='cuda') for s in ((n, 1, m), (n, 1), (n, 1))]
+        gpk.det_contract(dev(k), dev([0.0]), dev(A), dev(Bp[None]), *out, b_pairs=flag)
+        got.append(out)
+    assert all(torch.equal(p, q) for p, q in zip(*got))
