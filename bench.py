@@ -151,18 +151,6 @@ def cpu_eval_rate(x, y, params, idx_list, seconds):
 
 
 # ----------------------------------------------------------------------------- roofline helpers
-def df64_ops_psi_bwd(N, M, Q, D):
-    """FP32-pipe operations of the df64 psi backward per launch: the reference formula's
-    float64 operations, each weighted by the FP32-instruction cost of its double-float
-    implementation (add 11, mul 7, fma 18, exp 45, log 60, div 40)."""
-    P = M * (M + 1) // 2
-    add, mul, fma, exp_ = 11, 7, 18, 45
-    pair = (2 * add + Q * fma + add + exp_) + D * (add + fma) + D * fma + mul + add
-    row = 2 * (add + Q * fma)                       # row-sum pass, two entries per pair
-    per_a = exp_ + Q * (4 * add + 6 * mul + 3 * fma) + D * 2 * fma
-    return N * (P * (pair + row) + M * per_a)
-
-
 def psi_flops(N, M, Q, D, backward):
     """Algorithmic FP32-equivalent work of the psi kernels per launch (a fixed convention):
     per point, with P = M(M+1)/2, forward F = 4MQ + 6PQ + 2 D M^2 and E = M + P exps;
@@ -427,7 +415,6 @@ def run_ours(args, world, rank, local):
                                 work=work)
     t_k = time_launches(run_k, flush)
     F, E = psi_flops(MB, M_PSEUDO, HIDDEN, 1, backward=True)
-    ops = df64_ops_psi_bwd(MB, M_PSEUDO, HIDDEN, 1)
     peaks = json.load(open(os.path.join(ROOT, 'MEASURED_PEAKS.json'))) if os.path.exists(
         os.path.join(ROOT, 'MEASURED_PEAKS.json')) else {}
     sm_mhz = peaks.get('sm_max_mhz', 2070.0)
@@ -442,9 +429,6 @@ def run_ours(args, world, rank, local):
                 'peak_source': 'nominal: %d SMs x 128 FP32 lanes x 2 x %.0f MHz (max SM clock, '
                                'MEASURED_PEAKS.json); no measured FP32 peak exists' % (n_sm, sm_mhz),
                 'us_per_launch': round(t_k * 1e6, 2),
-                'df64_issue': {'fp32_ops_per_launch': ops, 'tflops': round(ops / t_k / 1e12, 3),
-                               'frac': round(ops / t_k / 1e12 / fp32_peak, 4),
-                               'note': 'the FP32 operations of the same work in plain double-float arithmetic'},
                 'hbm_algorithmic_gbs': round(psi_bwd_bytes(MB, M_PSEUDO, HIDDEN, 1) / t_k / 1e9, 2),
                 'hbm_peak_gbs': peaks.get('hbm_gbs'),
                 # dram__bytes (read + write) of this launch pair in one ncu capture of the same case
