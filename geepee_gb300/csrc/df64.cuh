@@ -99,6 +99,20 @@ static __device__ __noinline__ df64 df_from_double_rest(double x) {
   }
   return make_df(hi, lo);
 }
+// whether df_from_double_plain does for x: zero, or in the range above
+__device__ __forceinline__ bool df_plain(double x) {
+  const unsigned hw = (unsigned)__double2hiint(x);
+  return ((hw >> 20) & 0x7ff) - 949u <= 201u || ((hw << 1) | (unsigned)__double2loint(x)) == 0u;
+}
+__device__ __forceinline__ df64 df_from_double_plain(double x) {
+  const unsigned hw = (unsigned)__double2hiint(x), lw = (unsigned)__double2loint(x);
+  const int e = (int)((hw >> 20) & 0x7ff);
+  const unsigned long long m = ((unsigned long long)(hw & 0x7fffffffu) << 32) | lw;
+  const unsigned top = (unsigned)((m + 0x0fffffffull + ((m >> 29) & 1u)) >> 29);   // (mod 2^32: the field's excess)
+  const float g = (float)(int)(lw - (top << 29));
+  const unsigned lo = g == 0.f ? 0u : (__float_as_uint(g) + ((unsigned)(e - 1075) << 23)) ^ (hw & 0x80000000u);
+  return make_df(e == 0 ? 0.f : __uint_as_float((top - (896u << 23)) | (hw & 0x80000000u)), __uint_as_float(lo));
+}
 __device__ __forceinline__ df64 df_from_double(double x) {
   const unsigned hw = (unsigned)__double2hiint(x), lw = (unsigned)__double2loint(x);
   const int e = (int)((hw >> 20) & 0x7ff);
@@ -106,11 +120,7 @@ __device__ __forceinline__ df64 df_from_double(double x) {
     if (((hw << 1) | lw) == 0u) return make_df(__int_as_float((int)hw), 0.f);   // +-0
     return df_from_double_rest(x);
   }
-  const unsigned long long m = ((unsigned long long)(hw & 0x7fffffffu) << 32) | lw;
-  const unsigned top = (unsigned)((m + 0x0fffffffull + ((m >> 29) & 1u)) >> 29);   // (mod 2^32: the field's excess)
-  const float g = (float)(int)(lw - (top << 29));
-  const unsigned lo = g == 0.f ? 0u : (__float_as_uint(g) + ((unsigned)(e - 1075) << 23)) ^ (hw & 0x80000000u);
-  return make_df(__uint_as_float((top - (896u << 23)) | (hw & 0x80000000u)), __uint_as_float(lo));
+  return df_from_double_plain(x);
 }
 __device__ __forceinline__ double df_to_double(df64 a) { return (double)a.hi + (double)a.lo; }
 

@@ -645,27 +645,43 @@ constexpr int DM_LOW = -400;      // the smallest exponent of a scaled row (2^-1
 constexpr float DM_TRUST = 1024.f;   // a sixteenth of the scales, in the first digits' units (2^-7 of each scale)
 constexpr int DM_MAX = 255;       // largest M: four pairs a lane, sums below 2^61
 
-// Bk of one row (optional) and the sum k . Bk in double-float, by a warp
+// Bk of one row (optional) and the sum k . Bk in double-float, by a warp: four columns a lane, B's entries of eight
+// rows in flight together and split without a branch where all are ordinary numbers (entry by entry, one row in a
+// thousand made N = 1000, M = 100, two outputs 122 us instead of 22; so, 50)
 static __device__ __noinline__ df64 dm_row_general(const double* B, int b_pairs, const df64* k, const int* c, int M,
                                                    double* Bk) {
+  constexpr int G = 8;
   const int lane = threadIdx.x & 31;
   df64 v = make_df(0.f);
-  for (int b0 = lane; b0 < M; b0 += 128) {
+  for (int b0 = lane; b0 - lane < M; b0 += 128) {
     df64 x[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) x[j] = make_df(0.f);
-    for (int a = 0; a < M; ++a) {
-      const df64 ka = k[a];
-      if (ka.hi == 0.f) continue;
+#pragma unroll 1
+    for (int a0 = 0; a0 < M; a0 += G) {
+      double e[G][4];
+      bool plain = true;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (b0 + 32 * j < M) {
-          const double e = B[(size_t)a * M + b0 + 32 * j];
-          const df64 w = b_pairs ? make_df(__int_as_float(__double2loint(e)), __int_as_float(__double2hiint(e)))
-                                 : df_from_double(e);
-          x[j] = fma_(w, ka, x[j]);
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[g][j] = a0 + g < M && b0 + 32 * j < M ? B[(size_t)(a0 + g) * M + b0 + 32 * j] : 0.0;
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) plain = plain && df_plain(e[g][j]);
+      auto group = [&](auto split) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const df64 ka = k[min(a0 + g, M - 1)];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc_fma(x[j], split(e[g][j]), ka);
         }
-      }
+      };
+      if (b_pairs) group([](double w) { return make_df(__int_as_float(__double2loint(w)), __int_as_float(__double2hiint(w))); });
+      else if (__all_sync(~0u, plain)) group([](double w) { return df_from_double_plain(w); });
+      else group([](double w) { return df_from_double(w); });
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = acc_done(x[j]);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
