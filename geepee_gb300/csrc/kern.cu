@@ -1763,6 +1763,7 @@ extern "C" int gpk_kern(int prec, int N, int M, int D, const void* x, int ldx, c
   // with a jitter the matrix goes into a factorisation, which amplifies its last bits by a condition
   // number of up to 1e7: it keeps the double-float evaluation (its M x M entries cost ~10 us)
   if (prec == GPK_DF64 && jitter != 0.0) return kern_launch<df64>(N, M, D, x, ldx, z, ldz, lls2, lsf2, jitter, K, ldk, st);
+  // (one limit for every form, that of kern_matrix_kernel's grid)
   GPK_REQUIRE(gpk::ceil_div(N, KR) <= 65535, "kern: N=%d too large (at most %d rows)", N, 65535 * KR);
   if (prec == GPK_DF64)
     return kern_fx_launch(N, M, D, (const double*)x, ldx, (const double*)z, ldz, lls2, lsf2, (double*)K, ldk, st);
@@ -1831,6 +1832,8 @@ void contract_dispatch(int N, int M, int Dout, const void* kfu, const double* ls
 }
 }  // namespace
 
+// The sizes this entry point takes, the same in both precisions: B and a few rows in the shared memory of the FP32
+// kernel's layout.  (det_mma_kernel itself takes any Dout and M <= DM_MAX, and serves those through gpk_det_fwd.)
 extern "C" int gpk_det_contract_supported(int prec, int M, int Dout) {
   const size_t tsz = prec == GPK_FP32 ? sizeof(float) : sizeof(df64);
   return M >= 1 && M <= 128 && Dout >= 1 && Dout <= DO_MAX && det_contract_smem(M, Dout, tsz) <= 227 * 1024;

@@ -117,9 +117,10 @@ int gpk_det_fwd(int prec, int N, int M, int D, int Dout, const void* x, int ldx,
 /* The contractions of gpk_det_fwd from given kernel values kfu [N,M] (e.g. from gpk_kern):
  *   m[n,d] = kfu_n . A_d;  Bk[n,d,b] = sum_a B[d,a,b] kfu[n,a];  v[n,d] = sf2 + kfu_n . Bk[n,d]
  * so that kfu, which needs only the inputs and the kernel hyperparameters, can be formed
- * ahead (beside the factorisations that the cavity's A and B wait for).  Needs M <= 128 and
- * Dout M^2 elements in shared memory (gpk_det_contract_supported says whether a size is
- * supported; an unsupported one returns GPK_EUNSUPPORTED).  Bk, m_out, v_out optional.
+ * ahead (beside the factorisations that the cavity's A and B wait for).  Takes M <= 128 with
+ * Dout M^2 compute-type elements within a CTA's shared memory (gpk_det_contract_supported says whether
+ * a size is supported; an unsupported one returns GPK_EUNSUPPORTED).  Bk, m_out, v_out optional;
+ * GPK_DF64 errors as in gpk_det_fwd.
  * b_pairs != 0 (GPK_DF64 only): B holds double-float (hi, lo) float pairs, as gpk_cavity_forms
  * writes them into Bd_pair, and is read without conversion.
  * Replaces the Kfu contractions of geepee/aep_models.py:142-158 (base_models.py:265-284). */
