@@ -709,9 +709,8 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
   B += (size_t)d * M * M;
   const float qnan = __int_as_float(0x7fffffff);
   __shared__ df64 s_sf2;
-  if (tid == 0) s_sf2 = df_from_double(exp(lsf2[0]));
+  const double lsf = lsf2[0];
   for (int i = tid; i < M; i += DM_T) s.c[i] = -126;
-  __syncthreads();
   // ---- the exponents of B's columns, then of its rows beside them.  A warp takes a row's columns by 128, four
   // such items' loads in flight; the entries' exponents wait in bytes (in the place of B's digits) for the second pass
   // |entry| < 2^ex_of: of a pair by its high word, of a float64 rounded as that word is (a NaN of all ones carries
@@ -721,33 +720,34 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
     const int e = (int)((((unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL) + (1ULL << 28)) >> 52);
     return pair ? h - 126 : e - 1022;
   };
-  const int EP = (M + 3) & ~3, nh = M > 128 ? 2 : 1;   // bytes of a row; items of a row
+  const int EP = (M + 3) & ~3, hs = M > 128;   // bytes of a row; a row is 2^hs items
   unsigned char* const eb = reinterpret_cast<unsigned char*>(s.B);
   int ea[8];   // A's exponents
 #pragma unroll
   for (int j = 0; j < 8; ++j) ea[j] = lane + 32 * j < M ? ex_of(A[lane + 32 * j], false) : 2 * DM_LOW;
   {
-    const int cb = (warp & (nh - 1)) * 128 + lane;   // (a warp's items are all of one side)
+    const int cb = (warp & hs) * 128 + lane;   // (a warp's items are all of one side)
     int cm[4] = {-126, -126, -126, -126};
-    for (int it = warp; it < nh * M; it += 4 * DM_W) {
+    for (int it = warp; it < M << hs; it += 4 * DM_W) {
       double v[4][4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int a = (it + u * DM_W) / nh;
+          const int a = (it + u * DM_W) >> hs;
           v[u][j] = a < M && cb + 32 * j < M ? B[(size_t)a * M + cb + 32 * j] : 0.0;
         }
 #pragma unroll
       for (int u = 0; u < 4; ++u)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const int a = (it + u * DM_W) / nh;
+          const int a = (it + u * DM_W) >> hs;
           const int e = min(max(ex_of(v[u][j], b_pairs), -126), 129);   // -126: zero or below the float range
           cm[j] = max(cm[j], e);
           if (a < M && cb + 32 * j < EP) eb[a * EP + cb + 32 * j] = (unsigned char)(e + 126);
         }
     }
+    __syncthreads();
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (cb + 32 * j < M) atomicMax(&s.c[cb + 32 * j], cm[j] > 128 ? DM_BAD : cm[j]);
@@ -841,6 +841,7 @@ __global__ void __launch_bounds__(DM_T, 1) det_mma_kernel(int N, int M, int Dout
     }
   };
   if (nblk == 1) stage_B(0);
+  if (tid == DM_T - 1) s_sf2 = df_from_double(exp(lsf));   // (read after the barriers of the first rows)
   const int ntile = (N + R - 1) / R;
   for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
     const int n0 = tile * R, nr = min(R, N - n0);
