@@ -285,22 +285,31 @@ constexpr long long kFxHalf = 1LL << 40;
 __device__ __forceinline__ void load_exp2_table(float2* s_tab) {
   const float c_hi[8] = {0.000000000e+00f, 3.385080490e-04f, 6.771307089e-04f, 1.015867922e-03f, 1.354719861e-03f, 1.693686470e-03f, 2.032767981e-03f, 2.371964045e-03f};
   const float c_lo[8] = {0.000000000e+00f, 3.656181261e-12f, -1.587024435e-11f, 3.841724161e-11f, 3.069764928e-11f, 5.799375910e-11f, -7.369679866e-11f, 2.371333858e-11f};
-#pragma unroll 1
-  for (int k = threadIdx.x; k < kFxTab; k += blockDim.x) {
-    const int i = k & 7;
-    const float2 t = kExp2Tab[k >> 3];
-    float ch = 0.f, cl = 0.f;
+  // a warp's 32 consecutive entries need four of the 256; eight rounds' worth arrive by one load a lane (a load in
+  // each round made the table ~2 us of a launch)
+  const int lane = threadIdx.x & 31, first = threadIdx.x & ~31, i = lane & 7;
+  float ch = 0.f, cl = 0.f;
 #pragma unroll
-    for (int u = 1; u < 8; ++u) {
-      ch = i == u ? c_hi[u] : ch;
-      cl = i == u ? c_lo[u] : cl;
+  for (int u = 1; u < 8; ++u) {
+    ch = i == u ? c_hi[u] : ch;
+    cl = i == u ? c_lo[u] : cl;
+  }
+#pragma unroll 1
+  for (int b = first; b < kFxTab; b += 8 * blockDim.x) {
+    const int j = ((b + (lane >> 2) * (int)blockDim.x) >> 3) + (lane & 3);
+    const float2 all = j < 256 ? kExp2Tab[j] : make_float2(0.f, 0.f);
+    float2* const out = s_tab + b + lane;
+#pragma unroll 1
+    for (int r = 0; r < 8 && b + r * (int)blockDim.x < kFxTab; ++r) {
+      const float2 t = make_float2(__shfl_sync(0xffffffffu, all.x, 4 * r + (lane >> 3)),
+                                   __shfl_sync(0xffffffffu, all.y, 4 * r + (lane >> 3)));
+      // t (1 + c): the product's exact high part and its cross terms added to t
+      const df64 w = two_prod(t.x, ch);
+      const float e = __fadd_rn(__fmaf_rn(t.x, cl, w.lo), __fmaf_rn(t.y, ch, t.y));
+      df64 q = quick_two_sum(t.x, w.hi);
+      q = quick_two_sum(q.hi, __fadd_rn(q.lo, e));
+      out[r * blockDim.x] = make_float2(q.hi, q.lo);
     }
-    // t (1 + c): the product's exact high part and its cross terms added to t
-    const df64 w = two_prod(t.x, ch);
-    const float e = __fadd_rn(__fmaf_rn(t.x, cl, w.lo), __fmaf_rn(t.y, ch, t.y));
-    df64 r = quick_two_sum(t.x, w.hi);
-    r = quick_two_sum(r.hi, __fadd_rn(r.lo, e));
-    s_tab[k] = make_float2(r.hi, r.lo);
   }
 }
 // the 256-entry exp table of exp_tab inside that table (every 8th entry)
