@@ -1422,6 +1422,7 @@ __global__ void __launch_bounds__(GP_T) gram_pairs_kernel(int N, int M, int Dout
 // N = 20000, M = 100, two outputs, with the reduction 99 us (361 in double-float pairs), a third of it in the matrix
 // pipe, the rest in digits and folds (87 with h = 0 and every result trusted); N = 1000 22 us (30).  Two
 // input dimensions (2% of the results weak) 132 us, one with a lengthscale of 0.04 of the range (most of them) 359.
+constexpr long GM_PAIRS = 1L << 20;
 constexpr float GM_TRUST = 512.f;   // 1/32 of the scales, in the first digits' units
 constexpr int GM_T = 384, GM_W = GM_T / 32, GM_TW = 5;
 struct GmSmem {
@@ -1833,8 +1834,9 @@ void contract_dispatch(int N, int M, int Dout, const void* kfu, const double* ls
 }
 }  // namespace
 
-// The sizes this entry point takes, the same in both precisions: B and a few rows in the shared memory of the FP32
-// kernel's layout.  (det_mma_kernel itself takes any Dout and M <= DM_MAX, and serves those through gpk_det_fwd.)
+// The sizes this entry point takes: M <= 128, and B and a few rows in the compute type within a CTA's shared memory, as
+// det_contract_kernel lays them out.  (det_mma_kernel itself takes any Dout and M <= DM_MAX, and serves those
+// through gpk_det_fwd.)
 extern "C" int gpk_det_contract_supported(int prec, int M, int Dout) {
   const size_t tsz = prec == GPK_FP32 ? sizeof(float) : sizeof(df64);
   return M >= 1 && M <= 128 && Dout >= 1 && Dout <= DO_MAX && det_contract_smem(M, Dout, tsz) <= 227 * 1024;
@@ -2041,8 +2043,11 @@ extern "C" int gpk_gram_ws(int prec, int N, int M, int Dout, const void* u, cons
   GPK_REQUIRE(u && v && w && C, "gram: null pointer");
   const int sym = u == v;   // C symmetric: the upper tiles only
   const int P = M * (M + 1) / 2;
+  // the digits from a million pairs on: below, the tables and digits of a few rows a CTA take longer than the
+  // double-float pairs (M = 100, one output: N = 128 9.9 us in pairs, 12.1 to 15.1 by digits; N = 256 12.8, 12.5 to
+  // 15.1; N = 512 16.5, 14.6 to 17.7; M = 200: N = 64 14.9, 16.3 to 20.0; N = 128 19.0, 16.4 to 20.2)
   GramMma g{};
-  const bool mma = prec == GPK_DF64 && sym && work && gram_mma_plan(N, M, Dout, &g);
+  const bool mma = prec == GPK_DF64 && sym && work && (long)N * P > GM_PAIRS && gram_mma_plan(N, M, Dout, &g);
   const int chunks = mma ? g.chunks : sym ? gram_pair_chunks(N, M) : gram_chunks(N, M, false);
   if (work) {
     const long need = (long)chunks * Dout * (sym ? P : M * M);

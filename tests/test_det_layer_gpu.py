@@ -311,3 +311,20 @@ def test_contraction_of_graded_pairs(kind):
         gpk.det_contract(dev(k), dev([0.0]), dev(A), dev(Bp[None]), *out, b_pairs=flag)
         got.append(out)
     assert all(torch.equal(p, q) for p, q in zip(*got))
+
+
+@pytest.mark.parametrize('m', [16, 33, 100, 255])
+@pytest.mark.parametrize('above', [0, 1])
+def test_gram_where_the_digits_begin(m, above):
+    """The last size of the pair form and the first of the digit form: N M (M + 1) / 2 at and above 2^20."""
+    from geepee_gb300 import gpk
+    n = (1 << 20) // (m * (m + 1) // 2) + above
+    rng = np.random.RandomState(m)
+    L = np.longdouble
+    u, w = np.exp(-rng.rand(n, m) * 8), rng.randn(n, 1)
+    z0 = lambda *s: torch.zeros(s, dtype=torch.float64, device='cuda')
+    C, ut = z0(1, m, m), dev(u)
+    gpk.gram(ut, ut, dev(w), C, work=z0(gpk.work_elems(gpk.OP_GRAM, n, m, 1, 1)))
+    ref = (u.astype(L) * w).T @ u.astype(L)
+    S = (u.astype(L) * np.abs(w)).T @ u.astype(L)
+    assert (np.abs(C.cpu().numpy()[0] - ref) <= n * 2.0 ** -47 * S).all()
