@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) kern_matrix_kernel(int N, int M, int D, c
 // farther pseudo-inputs, and inputs that are not finite, have NaN for theirs, which sends the entries they
 // meet to the double-float form (ard_general); farther inputs meet no nearer pseudo-input.  Coordinates by
 // their distance from the origin instead took that form beyond 18.8 lengthscales of it, an entry at a time: 109 us
-// at N = 20000, M = 100, D = 8, inputs about 37 lengthscales off, where this takes 28.
+// at N = 20000, M = 100, D = 8, inputs about 37 lengthscales off, where this takes 27.
 struct __align__(16) ArdHyp {
   unsigned long long ms[DMAXK];   // sqrt(log2(e)/2) / ell_d: its significand,
   int sh[DMAXK];        // 2093 less its exponent field (ard_coord)
@@ -191,8 +191,8 @@ __device__ __noinline__ df64 ard_general(const double* x, const double* z, int D
 // K (float64): a CTA takes FC columns and row tiles of FR; a thread one column and FR / (256 / FC) rows,
 // four at a time, so that a column's coordinate is loaded once for four rows.  As many CTAs as
 // are resident at once share the tiles: the tables and the columns are staged once a CTA.
-// Bound by the integer and FP32 pipes: 20000 x 100, D = 8 in 28 us (49 before), 20000 x 200, D = 16 in
-// 68 us (256 before).
+// Bound by the integer and FP32 pipes: 20000 x 100, D = 8 in 27 us (49 before), 20000 x 200, D = 16 in
+// 67 us (256 before).
 constexpr int FR = 16, FC = 128, FCTA = 3;
 __global__ void __launch_bounds__(256, FCTA) kern_fx_kernel(int N, int M, int D, const double* x, int ldx,
                                                             const double* z, int ldz, const double* lls2,
