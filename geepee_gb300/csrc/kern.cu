@@ -1932,7 +1932,7 @@ namespace {
 int gram_pair_blocks(int M) { return gpk::ceil_div(M * (M + 1) / 2, GP_T * GP_PPT); }
 int gram_pair_chunks(int N, int M) {
   int c = gpk::ceil_div(gpk::sm_count(), gram_pair_blocks(M));
-  const int cap = gpk::ceil_div(N, 8);
+  const int cap = gpk::ceil_div(N, 3);   // three rows a chunk or more (12 rows: 5.5 to 10.9 us at M = 5 to 200; eight: 5.8 to 11.3)
   if (c > cap) c = cap;
   return c < 1 ? 1 : c;
 }
